@@ -40,20 +40,14 @@ constexpr uint32_t kStreamBlockK = 128;
 //   a2: s9  e2 e1 m0     -> a2 = (w << 6)  & 0x81C081C0
 //   a3: s11 e1@10 e0@14 m13 -> a3 = (((w >> 10) & 0x001B001B) * 0x4108) & 0x81C081C0
 // `bytes` are the four source bytes of a0..a3 (low nibble = even k).
+// Both nibbles of a byte move together: `pair` holds the even-k code in bits 0..3 and the odd-k code in bits 16..19.
 AUGUR_HD uint32_t stream_pack_word(uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3) {
-    const uint32_t bytes[4] = {b0, b1, b2, b3};
-    // destination bit of (sign, e1, e0, m) for each register, inside a 16-bit half
-    const uint32_t where[4][4] = {{15, 8, 7, 6}, {12, 5, 4, 3}, {9, 2, 1, 0}, {11, 10, 14, 13}};
-    uint32_t word = 0;
-    for (uint32_t j = 0; j < 4; ++j) {
-        for (uint32_t half = 0; half < 2; ++half) {
-            const uint32_t code = (bytes[j] >> (4 * half)) & 15u;
-            word |= ((code >> 3) & 1u) << (where[j][0] + 16 * half);
-            word |= ((code >> 2) & 1u) << (where[j][1] + 16 * half);
-            word |= ((code >> 1) & 1u) << (where[j][2] + 16 * half);
-            word |= (code & 1u) << (where[j][3] + 16 * half);
-        }
-    }
+    const uint32_t p0 = (b0 | (b0 << 12)) & 0x000F000Fu, p1 = (b1 | (b1 << 12)) & 0x000F000Fu;
+    const uint32_t p2 = (b2 | (b2 << 12)) & 0x000F000Fu, p3 = (b3 | (b3 << 12)) & 0x000F000Fu;
+    uint32_t word = ((p0 & 0x00080008u) << 12) | ((p0 & 0x00070007u) << 6);
+    word |= ((p1 & 0x00080008u) << 9) | ((p1 & 0x00070007u) << 3);
+    word |= ((p2 & 0x00080008u) << 6) | (p2 & 0x00070007u);
+    word |= ((p3 & 0x000C000Cu) << 8) | ((p3 & 0x00030003u) << 13);
     return word;
 }
 

@@ -37,73 +37,133 @@ uint64_t layout_extent(uint32_t layout, uint32_t rows, uint32_t cols) {
 }
 
 // ---- device repack ----------------------------------------------------------------
-// STREAM / STREAM_PAIR: one thread per destination word (coalesced writes, gathered reads).
-__global__ void repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restrict__ scales_a,
-                                     const uint8_t* __restrict__ codes_b, const uint8_t* __restrict__ scales_b,
-                                     uint8_t* __restrict__ destination, uint32_t rows, uint32_t cols, bool pair) {
+// Both kernels move every byte once and are bound by HBM (reads and writes of the same size). One destination word
+// per thread with byte gathers and a bit-by-bit permutation took 61.5 us for the STREAM layout of a 17408 x 5120
+// weight, and 4-byte copies 35 us for the TCGEN05 layout.
+constexpr uint32_t kRepackWarps = 8;
+
+// STREAM / STREAM_PAIR: one warp per destination block (32 rows x 128 k). A lane's 16 destination bytes hold the codes
+// of rows g and g + 8 for four k-steps, byte columns t4 and t4 + 4 of each: the 32 consecutive source bytes of either
+// row, which the four lanes of a quad read together as 16-byte loads (one sector of DRAM each, fetched once), and of
+// which each lane keeps its own byte of every word. All 16 loads of a lane are in flight together; the eight
+// warps of a CTA take neighbouring blocks of one row group, so the rows are read in runs of 512 bytes.
+__global__ void __launch_bounds__(kRepackWarps * 32)
+repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restrict__ scales_a, const uint8_t* __restrict__ codes_b,
+                     const uint8_t* __restrict__ scales_b, uint8_t* __restrict__ destination, uint32_t blocks, uint32_t cols, bool pair) {
+    const uint32_t block = blockIdx.x * kRepackWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (block >= blocks) return;
     const uint32_t kb_count = cols / kStreamBlockK;
-    const uint64_t groups = pair ? rows / 16 : rows / 32;
-    const uint64_t words = groups * kb_count * (kStreamBlockBytes / 4);
-    const uint64_t index = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (index >= words) return;
-    const uint64_t block = index / (kStreamBlockBytes / 4);
-    const uint32_t word = static_cast<uint32_t>(index % (kStreamBlockBytes / 4));
-    const uint32_t group = static_cast<uint32_t>(block / kb_count);
-    const uint32_t kb = static_cast<uint32_t>(block % kb_count);
-    uint32_t value = 0;
-    if (word < kStreamCodeBytes / 4) {
-        const uint32_t j = word & 3, lane = (word >> 2) & 31, q = (word >> 7) & 1, t = word >> 8;
-        const uint32_t g = lane >> 2, t4 = lane & 3;
-        const uint32_t kstep = kb * 8 + q * 4 + j;
-        const uint8_t* source = (pair && t) ? codes_b : codes_a;
-        const uint32_t row0 = pair ? group * 16 : group * 32 + t * 16;
-        uint32_t bytes[4];
+    const uint32_t group = block / kb_count, kb = block - group * kb_count;
+    const uint32_t g = lane >> 2, t4 = lane & 3;
+    const uint8_t* source[2] = {codes_a, pair ? codes_b : codes_a};
+    uint4 top[2][2][2], bottom[2][2][2];   // [tile][quad][half] of rows g and g + 8
 #pragma unroll
-        for (uint32_t b = 0; b < 4; ++b) {
-            const uint32_t row = row0 + g + (b & 1) * 8;
-            const uint32_t column = kstep * 8 + (b >> 1) * 4 + t4;
-            bytes[b] = source[static_cast<uint64_t>(row) * (cols / 2) + column];
-        }
-        value = stream_pack_word(bytes[0], bytes[1], bytes[2], bytes[3]);
-    } else {
-        // scale word sw of the block: tile t, quad-row g, k-steps 2p and 2p+1, each {row g, row g+8}
-        const uint32_t sw = word - kStreamCodeBytes / 4;  // 0..63
-        const uint32_t p = sw & 3, g = (sw >> 2) & 7, t = sw >> 5;
-        const uint8_t* source = (pair && t) ? scales_b : scales_a;
-        const uint32_t row0 = (pair ? group * 16 : group * 32 + t * 16) + g;
+    for (uint32_t t = 0; t < 2; ++t) {
+        const uint32_t row = (pair ? group * 16 : group * 32 + t * 16) + g;
+        const uint4* from = reinterpret_cast<const uint4*>(source[t] + static_cast<uint64_t>(row) * (cols / 2) + kb * 64);
+        const uint4* below = reinterpret_cast<const uint4*>(source[t] + static_cast<uint64_t>(row + 8) * (cols / 2) + kb * 64);
 #pragma unroll
-        for (uint32_t b = 0; b < 4; ++b) {
-            const uint32_t row = row0 + (b & 1) * 8;
-            const uint32_t sc = kb * 8 + p * 2 + (b >> 1);
-            value |= static_cast<uint32_t>(source[static_cast<uint64_t>(row) * (cols / 16) + sc]) << (8 * b);
+        for (uint32_t q = 0; q < 2; ++q) {
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+                top[t][q][h] = __ldg(from + q * 2 + h);
+                bottom[t][q][h] = __ldg(below + q * 2 + h);
+            }
         }
     }
-    reinterpret_cast<uint32_t*>(destination)[index] = value;
+    // scales: 16 bytes per (tile, g) = k-steps 0..7 of rows g and g + 8, interleaved; lanes 0..15 take one each
+    uint2 scale_top = make_uint2(0, 0), scale_bottom = make_uint2(0, 0);
+    if (lane < 16) {
+        const uint32_t t = lane >> 3, row = (pair ? group * 16 : group * 32 + t * 16) + (lane & 7);
+        const uint8_t* from = ((pair && t) ? scales_b : scales_a) + static_cast<uint64_t>(row) * (cols / 16) + kb * 8;
+        const uint8_t* below = from + static_cast<uint64_t>(8) * (cols / 16);
+        // rows of scales start on 8-byte boundaries (cols is a multiple of 128), the plane itself only on a 4-byte one
+        scale_top = make_uint2(__ldg(reinterpret_cast<const uint32_t*>(from)), __ldg(reinterpret_cast<const uint32_t*>(from) + 1));
+        scale_bottom = make_uint2(__ldg(reinterpret_cast<const uint32_t*>(below)), __ldg(reinterpret_cast<const uint32_t*>(below) + 1));
+    }
+    uint4* out = reinterpret_cast<uint4*>(destination + static_cast<uint64_t>(block) * kStreamBlockBytes);
+    const uint32_t pick = 0x4440u | t4;    // byte t4 of a word, zero-extended
+#pragma unroll
+    for (uint32_t t = 0; t < 2; ++t) {
+#pragma unroll
+        for (uint32_t q = 0; q < 2; ++q) {
+            uint32_t word[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {   // k-step 4 q + j: 8 source bytes, words 2 (j % 2) and 2 (j % 2) + 1 of half j / 2
+                const uint4 a = top[t][q][j >> 1], b = bottom[t][q][j >> 1];
+                word[j] = stream_pack_word(__byte_perm((j & 1) ? a.z : a.x, 0, pick), __byte_perm((j & 1) ? b.z : b.x, 0, pick),
+                                           __byte_perm((j & 1) ? a.w : a.y, 0, pick), __byte_perm((j & 1) ? b.w : b.y, 0, pick));
+            }
+            __stcs(out + (t * 2 + q) * 32 + lane, make_uint4(word[0], word[1], word[2], word[3]));
+        }
+    }
+    if (lane < 16) {
+        __stcs(out + kStreamCodeBytes / 16 + lane,
+               make_uint4(__byte_perm(scale_top.x, scale_bottom.x, 0x5140), __byte_perm(scale_top.x, scale_bottom.x, 0x7362),
+                          __byte_perm(scale_top.y, scale_bottom.y, 0x5140), __byte_perm(scale_top.y, scale_bottom.y, 0x7362)));
+    }
 }
 
-// TCGEN05: codes are copied through; one thread per destination scale word.
-__global__ void repack_tcgen05_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales,
-                                      uint8_t* __restrict__ destination, uint32_t rows, uint32_t cols) {
-    const uint64_t code_words = tcgen05_codes_bytes(rows, cols) / 4;
-    const uint64_t scale_words = tcgen05_scale_bytes(rows, cols) / 4;
-    const uint64_t index = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (index < code_words) {
-        reinterpret_cast<uint32_t*>(destination)[index] = reinterpret_cast<const uint32_t*>(codes)[index];
+// TCGEN05: the codes are copied through, 64 bytes per thread; the scales are re-tiled by one warp per 128-row block and
+// run of kAtoms atoms: a lane loads the run's words of rows lane, lane + 32, + 64 and + 96 and stores the 16 bytes that
+// they make in each atom, a whole atom per store of the warp. kAtoms is what the alignment of the scale rows
+// allows as one load: 4, 2 or 1 words.
+constexpr uint32_t kRepackCopyBytes = kRepackWarps * 32 * 64;   // of one CTA
+
+template <uint32_t kAtoms>
+__device__ __forceinline__ void retile_scales(const uint8_t* __restrict__ scales, uint8_t* __restrict__ out, uint32_t rows, uint32_t cols,
+                                              uint32_t run, uint32_t lane) {
+    const uint32_t atoms_per_row_block = cols / 64, runs = atoms_per_row_block / kAtoms;
+    const uint32_t row_block = run / runs, first = (run - row_block * runs) * kAtoms;
+    if (row_block >= (rows + 127) / 128) return;
+    uint32_t word[4][kAtoms];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        const uint32_t row = row_block * 128 + j * 32 + lane;
+        const uint32_t* from = reinterpret_cast<const uint32_t*>(scales + static_cast<uint64_t>(row) * (cols / 16) + first * 4);
+#pragma unroll
+        for (uint32_t a = 0; a < kAtoms; ++a) word[j][a] = 0;   // rows past the end: padding of the last row block
+        if (row < rows) {
+            if (kAtoms == 4) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(from));
+                word[j][0] = v.x; word[j][1 % kAtoms] = v.y; word[j][2 % kAtoms] = v.z; word[j][3 % kAtoms] = v.w;
+            } else if (kAtoms == 2) {
+                const uint2 v = __ldg(reinterpret_cast<const uint2*>(from));
+                word[j][0] = v.x; word[j][1 % kAtoms] = v.y;
+            } else {
+                word[j][0] = __ldg(from);
+            }
+        }
+    }
+    uint4* atom = reinterpret_cast<uint4*>(out + (static_cast<uint64_t>(row_block) * atoms_per_row_block + first) * kSfAtomBytes) + lane;
+#pragma unroll
+    for (uint32_t a = 0; a < kAtoms; ++a) __stcs(atom + a * (kSfAtomBytes / 16), make_uint4(word[0][a], word[1][a], word[2][a], word[3][a]));
+}
+
+__global__ void __launch_bounds__(kRepackWarps * 32)
+repack_tcgen05_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, uint8_t* __restrict__ destination,
+                      uint32_t rows, uint32_t cols, uint32_t scale_ctas, uint32_t run_atoms) {
+    const uint64_t code_bytes = tcgen05_codes_bytes(rows, cols);
+    if (blockIdx.x < scale_ctas) {   // the scales first: their loads are the scattered ones
+        const uint32_t run = blockIdx.x * kRepackWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+        if (run_atoms == 4) retile_scales<4>(scales, destination + code_bytes, rows, cols, run, lane);
+        else if (run_atoms == 2) retile_scales<2>(scales, destination + code_bytes, rows, cols, run, lane);
+        else retile_scales<1>(scales, destination + code_bytes, rows, cols, run, lane);
         return;
     }
-    const uint64_t sw = index - code_words;
-    if (sw >= scale_words) return;
-    // word sw of the scale region: atom = sw / 128; inside: (r % 32) * 4 + (r / 32) % 4
-    const uint64_t atoms_per_row_block = cols / 64;
-    const uint64_t atom = sw / 128;
-    const uint32_t inner = static_cast<uint32_t>(sw % 128);
-    const uint32_t row = static_cast<uint32_t>(atom / atoms_per_row_block) * 128 + (inner & 3) * 32 + (inner >> 2);
-    const uint32_t sc0 = static_cast<uint32_t>(atom % atoms_per_row_block) * 4;
-    uint32_t value = 0;
-    if (row < rows) {
-        value = *reinterpret_cast<const uint32_t*>(scales + static_cast<uint64_t>(row) * (cols / 16) + sc0);
+    // cols is a multiple of 64, so the plane is a whole number of 16-byte pieces
+    const uint64_t pieces = code_bytes / 16, first = static_cast<uint64_t>(blockIdx.x - scale_ctas) * (kRepackCopyBytes / 16) + threadIdx.x;
+    const uint4* from = reinterpret_cast<const uint4*>(codes);
+    uint4* to = reinterpret_cast<uint4*>(destination);
+    uint4 v[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+        if (first + i * kRepackWarps * 32 < pieces) v[i] = __ldg(from + first + i * kRepackWarps * 32);
     }
-    reinterpret_cast<uint32_t*>(destination)[index] = value;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) {
+        if (first + i * kRepackWarps * 32 < pieces) __stcs(to + first + i * kRepackWarps * 32, v[i]);
+    }
 }
 
 // ---- device dequant ------------------------------------------------------------------
@@ -240,15 +300,20 @@ void launch_repack(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_repack_ar
     const auto* codes = reinterpret_cast<const uint8_t*>(a->codes);
     const auto* scales = reinterpret_cast<const uint8_t*>(a->scales);
     auto* destination = reinterpret_cast<uint8_t*>(a->destination);
-    const uint64_t words = a->destination_len_bytes / 4;
-    const uint32_t blocks = static_cast<uint32_t>((words + 255) / 256);
     if (a->layout == AUGUR_NVFP4_SM100_LAYOUT_TCGEN05) {
-        repack_tcgen05_kernel<<<blocks, 256, 0, s->stream>>>(codes, scales, destination, a->rows, a->cols);
+        // a run of scales is one load: the rows of scales are cols / 16 bytes apart and the plane is 4-byte aligned
+        const uint64_t alignment = a->scales | (a->cols / 16);
+        const uint32_t run_atoms = alignment % 16 == 0 ? 4 : alignment % 8 == 0 ? 2 : 1;
+        const uint64_t runs = static_cast<uint64_t>((a->rows + 127) / 128) * (a->cols / 64 / run_atoms);
+        const uint32_t scale_ctas = static_cast<uint32_t>((runs + kRepackWarps - 1) / kRepackWarps);
+        const uint32_t copy_ctas = static_cast<uint32_t>((tcgen05_codes_bytes(a->rows, a->cols) + kRepackCopyBytes - 1) / kRepackCopyBytes);
+        repack_tcgen05_kernel<<<scale_ctas + copy_ctas, kRepackWarps * 32, 0, s->stream>>>(codes, scales, destination, a->rows, a->cols,
+                                                                                            scale_ctas, run_atoms);
     } else {
-        repack_stream_kernel<<<blocks, 256, 0, s->stream>>>(
-            codes, scales, reinterpret_cast<const uint8_t*>(a->codes_b),
-            reinterpret_cast<const uint8_t*>(a->scales_b), destination, a->rows, a->cols,
-            a->layout == AUGUR_NVFP4_SM100_LAYOUT_STREAM_PAIR);
+        const uint32_t blocks = static_cast<uint32_t>(a->destination_len_bytes / kStreamBlockBytes);
+        repack_stream_kernel<<<(blocks + kRepackWarps - 1) / kRepackWarps, kRepackWarps * 32, 0, s->stream>>>(
+            codes, scales, reinterpret_cast<const uint8_t*>(a->codes_b), reinterpret_cast<const uint8_t*>(a->scales_b), destination,
+            blocks, a->cols, a->layout == AUGUR_NVFP4_SM100_LAYOUT_STREAM_PAIR);
     }
     count_launch();
 }
