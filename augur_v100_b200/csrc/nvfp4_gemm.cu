@@ -3,21 +3,19 @@
 // TMA-fed shared-memory stages and the accumulator in tensor memory.
 //
 // D[token][feature] = g_w * g_a * sum_terms sum_k A_term[token][k] * W[feature][k]
-//   A operand: quantised activations, 128 token rows per tile (UMMA M = 128)
-//   B operand: weights, up to 256 feature rows per tile (UMMA N = 128 or 256)
+//   A operand: quantised activations, 256 token rows per tile on two CTAs
+//   B operand: weights, 256 feature rows per tile (128 in a half tile at the end)
 //   both K-major, packed two E2M1 codes per byte, 128-byte swizzled rows of 256 k
 //   block scales: 512-byte atoms (128 rows x 4 scales) copied smem -> TMEM by tcgen05.cp
 //
-// One persistent CTA per SM, 192 threads: warp 0 issues TMA, warp 1 owns tensor memory
-// and issues the MMAs, warps 2..5 drain the accumulator (tcgen05.ld), scale, round to
-// BF16 and store. Every mbarrier wait is bounded: a wait that runs out records a code in
-// the plan's status word, raises a CTA-wide abort flag, and all roles fall through to the
-// common exit where tensor memory is released.
+// Every mbarrier wait is bounded: a wait that runs out records a code in the plan's status word, raises a CTA-wide
+// abort flag, and all roles fall through to the common exit where tensor memory is released.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 
+#include "nvfp4_gemm.cuh"
 #include "nvfp4_internal.h"
 #include "nvfp4_layout.cuh"
 #include "nvfp4_tc.cuh"
@@ -29,249 +27,21 @@ using namespace tc;
 static_assert(sizeof(augur_cuda_nvfp4_sm100_act_quant_args_v1) == 56, "act_quant ABI");
 static_assert(sizeof(augur_cuda_nvfp4_sm100_gemm_args_v1) == 80, "gemm ABI");
 
-constexpr uint32_t kTileN = 256;          // features per tile (128 for a ragged last tile)
+constexpr uint32_t kTileN = 256;          // features per tile (128 for a half tile at the end)
 constexpr uint32_t kBlockK = 256;         // k per shared-memory stage = one 128-byte swizzled row
-constexpr uint32_t kStages = 4;
 constexpr uint32_t kBytesA = kTileM * 128;            // 16 KB
-constexpr uint32_t kBytesB = kTileN * 128;            // 32 KB
 constexpr uint32_t kBytesSfA = 4 * kSfAtomBytes;      // 2 KB: 4 atoms (k) of one 128-row block
 constexpr uint32_t kBytesSfB = 8 * kSfAtomBytes;      // 4 KB: 2 row blocks x 4 atoms
-constexpr uint32_t kStageBytes = kBytesA + kBytesB + kBytesSfA + kBytesSfB;  // 55296
-constexpr uint32_t kGemmSmemBytes = kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
-constexpr uint32_t kGemmThreads = 192;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemAcc = 0;          // 256 accumulator columns
-constexpr uint32_t kTmemSfA = 256;        // 2 x 16 columns (k-block parity)
-constexpr uint32_t kTmemSfB = 320;        // 2 x 32 columns
 
 constexpr uint32_t kErrProducerWait = 0x101, kErrMmaWaitFull = 0x102, kErrMmaWaitTmem = 0x103,
                    kErrEpilogueWait = 0x104, kErrCopyWait = 0x105, kErrMmaWaitScales = 0x106,
                    kErrSplitWait = 0x107;
 
-struct GemmParams {
-    const uint8_t* weight_sf;      // scale region of the weight tensor
-    const uint8_t* act_sf;         // scale region of term 0; terms are `act_term_stride` bytes apart
-    uint64_t act_term_stride;
-    __nv_bfloat16* out;
-    uint32_t* status_word;
-    uint32_t rows, cols, tokens, terms;
-    uint32_t padded_tokens;        // tokens rounded up to whole 128-row tiles: row stride of the staged activation planes
-    float scale;                   // g_w * g_a
-    float scale_b;                 // SwiGLU: g_w of the up rows * g_a
-    uint32_t swiglu;               // weight rows alternate 16 gate / 16 up; output is bf16(silu(gate) * up), rows / 2 wide
-    // SwiGLU on pair tiles only: the intermediate is also (or only, if `out` is null) quantised for the next GEMM
-    uint8_t* quant_out;            // staged activations: [terms] code planes of whole tiles, then the scale regions
-    uint32_t quant_terms;
-    float quant_global_scale;
-    // Pair tiles whose count is not a multiple of the pairs: the tiles left over are cut along k between all pairs
-    // (null: whole tiles only). Partial accumulators pass through `split_slots`, announced by `split_flags`.
-    float* split_slots;            // [pair][CTA of the pair][epilogue warp][128 columns / 4][lane] x float4
-    uint32_t* split_flags;         // [pair][CTA of the pair][epilogue warp], zero between launches
-    uint32_t split_sharers;        // pairs that share the leftover tiles (0: whole tiles only)
-};
-
-// ---- activation quantiser ------------------------------------------------------------------
-__host__ __device__ constexpr uint32_t padded_tokens(uint32_t tokens) { return (tokens + kTileM - 1) / kTileM * kTileM; }
-// Bytes of the staged activations of one term: code plane of whole tiles, then the scale atoms.
-__host__ __device__ constexpr uint64_t staged_term_bytes(uint32_t tokens, uint32_t cols) {
-    return tcgen05_extent_bytes(padded_tokens(tokens), cols);
-}
-
-
-// 32 accumulator columns of one token row -> packed BF16. Plain: 32 outputs. SwiGLU: the weight rows
-// alternate 16 gate / 16 up, so columns 0..15 are gate sums and 16..31 the matching up sums of 16
-// intermediate columns; the 16 outputs bf16(silu(gate) * up) fill packed[0..8).
-__device__ __forceinline__ void convert_chunk(const uint32_t (&v)[32], float scale, float scale_b, bool swiglu, uint32_t (&packed)[16]) {
-    if (!swiglu) {
-#pragma unroll
-        for (uint32_t i = 0; i < 16; ++i) {
-            const __nv_bfloat162 two = __floats2bfloat162_rn(__uint_as_float(v[2 * i]) * scale, __uint_as_float(v[2 * i + 1]) * scale);
-            packed[i] = *reinterpret_cast<const uint32_t*>(&two);
-        }
-        return;
-    }
-    float h[16];
-#pragma unroll
-    for (uint32_t i = 0; i < 16; ++i) {
-        const float gate = __uint_as_float(v[i]) * scale, up = __uint_as_float(v[16 + i]) * scale_b;
-        // fast exponential and reciprocal (a few 1e-7 relative): this runs between the accumulator read and
-        // its release, in front of the next tile's MMAs. A gate below -87 gives exp = inf and h = -0.
-        h[i] = __fdividef(gate, 1.0f + __expf(-gate)) * up;
-    }
-#pragma unroll
-    for (uint32_t i = 0; i < 8; ++i) {
-        const __nv_bfloat162 two = __floats2bfloat162_rn(h[2 * i], h[2 * i + 1]);
-        packed[i] = *reinterpret_cast<const uint32_t*>(&two);
-    }
-}
-
-__global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant__ CUtensorMap map_weight,
-            const GemmParams p) {
-    extern __shared__ uint8_t smem_raw[];
-    // 128-byte swizzled tiles need 1024-byte alignment.
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
-    // bars[0..S) full, [S..2S) empty, [2S] tmem_full, [2S+1] tmem_empty; then tmem base + abort flag
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 2);
-    volatile uint32_t* abort_flag = tmem_slot + 1;
-
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + kStages);
-    const uint32_t bar_tmem_full = smem_u32(bars + 2 * kStages), bar_tmem_empty = smem_u32(bars + 2 * kStages + 1);
-
-    if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < kStages; ++s) {
-            mbar_init(bar_full + 8 * s, 1);
-            mbar_init(bar_empty + 8 * s, 1);
-        }
-        mbar_init(bar_tmem_full, 1);
-        mbar_init(bar_tmem_empty, 4);   // one arrival per epilogue warp
-        *abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-
-    const uint32_t m_tiles = p.padded_tokens / kTileM;
-    const uint32_t n_tiles = (p.rows + kTileN - 1) / kTileN;
-    const uint32_t total_tiles = m_tiles * n_tiles;
-    const uint32_t k_blocks = (p.cols + kBlockK - 1) / kBlockK;
-    const uint32_t steps = k_blocks * p.terms;              // pipeline steps per tile
-    const uint64_t sf_atoms_per_row_block = p.cols / 64;    // atoms along k
-
-    if (warp == 0 && lane == 0) {
-        // ---------------- TMA producer ----------------
-        uint32_t stage = 0, phase = 0;
-        bool alive = true;
-        for (uint32_t tile = blockIdx.x; alive && tile < total_tiles; tile += gridDim.x) {
-            const uint32_t m_tile = tile % m_tiles, n_tile = tile / m_tiles;
-            const uint32_t n_rows = min(kTileN, p.rows - n_tile * kTileN);
-            for (uint32_t step = 0; step < steps; ++step) {
-                const uint32_t kb = step / p.terms, term = step % p.terms;
-                const uint32_t k_valid = min(kBlockK, p.cols - kb * kBlockK);   // multiple of 64
-                const uint32_t sf_bytes = k_valid / 64 * kSfAtomBytes;
-                if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status_word, kErrProducerWait)) {
-                    alive = false;
-                    break;
-                }
-                uint8_t* base = smem + stage * kStageBytes;
-                const uint32_t full = bar_full + 8 * stage;
-                const uint32_t row_blocks_b = n_rows / 128;
-                mbar_expect_tx(full, kBytesA + n_rows * 128 + sf_bytes * (1 + row_blocks_b));
-                tma_load_2d(smem_u32(base), &map_act, kb * 128, term * p.padded_tokens + m_tile * kTileM, full);
-                tma_load_2d(smem_u32(base + kBytesA), &map_weight, kb * 128, n_tile * kTileN, full);
-                if (n_rows > 128) {
-                    tma_load_2d(smem_u32(base + kBytesA + 128 * 128), &map_weight, kb * 128, n_tile * kTileN + 128, full);
-                }
-                const uint8_t* sfa = p.act_sf + term * p.act_term_stride +
-                                     (static_cast<uint64_t>(m_tile) * sf_atoms_per_row_block + kb * 4) * kSfAtomBytes;
-                bulk_load(smem_u32(base + kBytesA + kBytesB), sfa, sf_bytes, full);
-                for (uint32_t rb = 0; rb < row_blocks_b; ++rb) {
-                    const uint8_t* sfb = p.weight_sf +
-                        ((static_cast<uint64_t>(n_tile) * 2 + rb) * sf_atoms_per_row_block + kb * 4) * kSfAtomBytes;
-                    bulk_load(smem_u32(base + kBytesA + kBytesB + kBytesSfA + rb * kBytesSfA), sfb, sf_bytes, full);
-                }
-                if (++stage == kStages) { stage = 0; phase ^= 1; }
-            }
-        }
-    } else if (warp == 1 && lane == 0) {
-        // ---------------- MMA issuer ----------------
-        uint32_t stage = 0, phase = 0, tmem_phase = 0, sf_buffer = 0;
-        bool alive = true;
-        for (uint32_t tile = blockIdx.x; alive && tile < total_tiles; tile += gridDim.x) {
-            const uint32_t n_tile = tile / m_tiles;
-            const uint32_t n_rows = min(kTileN, p.rows - n_tile * kTileN);
-            const uint32_t idesc = instr_desc(n_rows);
-            // the epilogue must have drained the previous tile's accumulator
-            if (!mbar_wait(bar_tmem_empty, tmem_phase ^ 1, abort_flag, p.status_word, kErrMmaWaitTmem)) break;
-            tc_fence_after();
-            for (uint32_t step = 0; step < steps; ++step) {
-                const uint32_t kb = step / p.terms;
-                const uint32_t k_valid = min(kBlockK, p.cols - kb * kBlockK);
-                if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.status_word, kErrMmaWaitFull)) {
-                    alive = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t base = smem_u32(smem + stage * kStageBytes);
-                const uint32_t sfa_smem = base + kBytesA + kBytesB, sfb_smem = sfa_smem + kBytesSfA;
-                const uint32_t tmem_sfa = tmem_base + kTmemSfA + sf_buffer * 16;
-                const uint32_t tmem_sfb = tmem_base + kTmemSfB + sf_buffer * 32;
-                const uint64_t a_desc = operand_desc(base), b_desc = operand_desc(base + kBytesA);
-                for (uint32_t k = 0; k < k_valid / 64; ++k) {
-                    tc_copy_sf(tmem_sfa + 4 * k, sf_desc(sfa_smem + k * kSfAtomBytes));
-                    tc_copy_sf(tmem_sfb + 8 * k, sf_desc(sfb_smem + k * kSfAtomBytes));
-                    if (n_rows > 128) tc_copy_sf(tmem_sfb + 8 * k + 4, sf_desc(sfb_smem + kBytesSfA + k * kSfAtomBytes));
-                    // each MMA consumes 64 k = 32 bytes of every row: advance the start address by 32 >> 4
-                    tc_mma(tmem_base + kTmemAcc, a_desc + 2 * k, b_desc + 2 * k, idesc, tmem_sfa + 4 * k,
-                           tmem_sfb + 8 * k, (step | k) ? 1u : 0u);
-                }
-                tc_commit(bar_empty + 8 * stage);   // frees the stage when these MMAs have read it
-                sf_buffer ^= 1;
-                if (++stage == kStages) { stage = 0; phase ^= 1; }
-            }
-            if (alive) tc_commit(bar_tmem_full);      // accumulator complete
-            tmem_phase ^= 1;
-        }
-    } else if (warp >= 2) {
-        // ---------------- epilogue: TMEM -> registers -> BF16 -> global ----------------
-        const uint32_t quadrant = warp & 3;          // TMEM lanes this warp may read: 32*quadrant..+31
-        uint32_t tmem_phase = 0;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-            const uint32_t m_tile = tile % m_tiles, n_tile = tile / m_tiles;
-            const uint32_t n_rows = min(kTileN, p.rows - n_tile * kTileN);
-            if (!mbar_wait(bar_tmem_full, tmem_phase, abort_flag, p.status_word, kErrEpilogueWait)) break;
-            tc_fence_after();
-            const uint32_t token = m_tile * kTileM + quadrant * 32 + lane;
-            // SwiGLU halves the output width: 32 accumulator columns give 16 outputs
-            const uint32_t out_width = p.swiglu ? p.rows / 2 : p.rows, out_first = p.swiglu ? n_tile * kTileN / 2 : n_tile * kTileN;
-            __nv_bfloat16* out_row = p.out + static_cast<uint64_t>(token) * out_width + out_first;
-            for (uint32_t c = 0; c < n_rows; c += 32) {
-                uint32_t v[32];
-                tc_load32(tmem_base + kTmemAcc + ((quadrant * 32) << 16) + c, v);
-                tc_wait_ld();
-                if (token >= p.tokens) continue;   // padding rows of the last tile are computed, never stored
-                uint32_t packed[16];
-                convert_chunk(v, p.scale, p.scale_b, p.swiglu != 0, packed);
-                if (p.swiglu) {
-                    uint4* dst = reinterpret_cast<uint4*>(out_row + c / 2);
-                    dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                    dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                } else {
-                    uint4* dst = reinterpret_cast<uint4*>(out_row + c);
-#pragma unroll
-                    for (uint32_t i = 0; i < 4; ++i) {
-                        dst[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
-                    }
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_tmem_empty);
-            tmem_phase ^= 1;
-        }
-    }
-
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
-    }
-}
-
 // ---- two-CTA tiles ------------------------------------------------------------------------------
-// The 128 x 256 tile above pulls 54 KB through L2 -> shared memory per 256-deep k block, and that
-// path, not the tensor pipe, bounds it. Here two CTAs of a cluster (a pair of SMs) share one
+// A 128 x 256 tile on one CTA pulls 54 KB through L2 -> shared memory per 256-deep k block, and that
+// path, not the tensor pipe, would bound it. Here two CTAs of a cluster (a pair of SMs) share one
 // 256 x 256 tile with tcgen05 cta_group::2: each CTA loads its own 128 token rows (A), its own
 // half of the 256 weight rows (B) and the scales of both, 38 KB per k block for the same
 // 128 x 256 x 256 of arithmetic per SM. The even CTA of the pair (the leader) issues the MMAs for
@@ -285,8 +55,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant__
 //   tmem_full one per CTA, same multicast;   tmem_empty leader's only, one arrival per epilogue
 //             warp of either CTA (the peer's through a cluster-scope arrive);
 //   scales_landed[s] leader's only: the stage's block-scale atoms of both CTAs have landed (loaded before
-//             the operand tiles);   scales_ready[s] leader's only: the copy thread has issued the stage's
-//             shared -> tensor memory scale copies.
+//             the operand tiles);   scales_ready[s], weights_ready[slot] leader's only: the copy warps have issued the
+//             shared -> tensor memory copies of the stage's token-row scales, of the k block's weight-row scales.
 constexpr uint32_t kPairStages = 5;
 // Tensor memory of the pair kernel: 256 accumulator columns, then one set of token-row scale columns per stage
 // (16 each) and one set of weight-row scale columns per k-block slot (32 each).
@@ -302,8 +72,8 @@ constexpr uint32_t kPairEpilogueWarps = 8;      // two per tensor-memory lane qu
 constexpr uint32_t kPairOutRowBytes = 64 + 16;
 constexpr uint32_t kPairOutBytes = kPairEpilogueWarps * 32 * kPairOutRowBytes;         // 20480
 constexpr uint32_t kPairSmemBytes = kPairStages * kPairStageBytes + kPairOutBytes + 1024 + 256;
-constexpr uint32_t kPairCopyWarp = 2 + kPairEpilogueWarps;
-constexpr uint32_t kPairThreads = 32 * (kPairCopyWarp + 1);   // TMA warp, MMA warp, epilogue warps, scale-copy warp
+constexpr uint32_t kPairCopyWarp = 2 + kPairEpilogueWarps;    // token-row scales; the warp after it copies the weight-row scales
+constexpr uint32_t kPairThreads = 32 * (kPairCopyWarp + 2);   // TMA warp, MMA warp, epilogue warps, two scale-copy warps
 constexpr uint32_t kSplitWorthSteps = 16;       // pipeline steps a pair issues in the time a hand-over costs
 constexpr uint32_t kSplitWays = 8;              // a leftover tile is cut into this many parts at most
 constexpr uint32_t kSplitWaitLimit = 1u << 20;  // polls of a handed-over part's flag (each a round trip to L2) before giving up
@@ -414,8 +184,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* out_stage = smem + kPairStages * kPairStageBytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + kPairOutBytes);
-    // full[S], empty[S], tmem_full, tmem_empty, scales_ready[S], scales_landed[S]; then the TMEM base and the abort flag
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 * kPairStages + 2);
+    // full[S], empty[S], tmem_full, tmem_empty, scales_ready[S], scales_landed[S], weights_ready[S]; then the TMEM base and the abort flag
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5 * kPairStages + 2);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -424,6 +194,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
     const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + kPairStages);
     const uint32_t bar_tmem_full = smem_u32(bars + 2 * kPairStages), bar_tmem_empty = smem_u32(bars + 2 * kPairStages + 1);
     const uint32_t bar_scales_ready = smem_u32(bars + 2 * kPairStages + 2), bar_scales_landed = smem_u32(bars + 3 * kPairStages + 2);
+    const uint32_t bar_weights_ready = smem_u32(bars + 4 * kPairStages + 2);
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kPairStages; ++s) {
@@ -431,6 +202,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
             mbar_init(bar_empty + 8 * s, 1);
             mbar_init(bar_scales_ready + 8 * s, 1);
             mbar_init(bar_scales_landed + 8 * s, 1);
+            mbar_init(bar_weights_ready + 8 * s, 1);
         }
         mbar_init(bar_tmem_full, 1);
         mbar_init(bar_tmem_empty, 2 * kPairEpilogueWarps);   // one arrival per epilogue warp of either CTA
@@ -448,11 +220,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
     cluster_sync();   // the peer's barriers exist before anything can signal them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // Everything above ran while the launch before this one drained; its results are needed from here on.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     // An odd number of 128-row token tiles leaves the second CTA of the last pair without rows of its own: it
     // loads whatever follows (the next term's rows, or the fill value past the tensor) and stores nothing.
-    const uint32_t m_pairs = (p.padded_tokens + 2 * kTileM - 1) / (2 * kTileM);
-    const uint32_t n_tiles = p.rows / kTileN;
+    const uint32_t m_pairs = p.token_pairs;
+    // With an odd number of 128-row blocks of weights the last tile is half as wide (MMA n = 128): each CTA brings 64 of
+    // its rows, and the epilogue warps of the second column half have nothing to do.
+    const uint32_t n_tiles = (p.rows + kTileN - 1) / kTileN;
+    const uint32_t half_tile = p.rows % kTileN ? n_tiles - 1 : n_tiles;
     const uint32_t total_tiles = m_pairs * n_tiles;
     // A last k block that is only partly inside the tensor is loaded like the others (the TMA fills what lies past
     // the edge); the MMA issuer only consumes the k steps inside.
@@ -461,158 +239,176 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
     const uint32_t act_term_atoms = p.padded_tokens / 128 * atoms_per_row_block;   // scale atoms of one activation term
     const PairWork work = pair_work(pair, pairs, total_tiles, k_blocks, p.split_sharers);
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
-        uint32_t stage = 0, phase = 0;
+        uint32_t stage = 0, phase = 1;
         bool alive = true;
         for (uint32_t index = 0; alive && index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
             const uint32_t m_pair = item.tile % m_pairs, n_tile = item.tile / m_pairs;
-            const uint32_t item_steps = (item.kb1 - item.kb0) * p.terms;
-            for (uint32_t step = 0; step < item_steps; ++step) {
-                const uint32_t kb = item.kb0 + step / p.terms, term = step % p.terms;
-                if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status_word, kErrProducerWait)) {
-                    alive = false;
-                    break;
+            const uint32_t token_row = m_pair * 2 * kTileM + rank * kTileM;
+            const uint32_t weight_row = n_tile * kTileN + rank * (n_tile == half_tile ? 64 : 128);
+            for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb) {
+                for (uint32_t term = 0; term < p.terms; ++term) {
+                    if (!mbar_wait(bar_empty + 8 * stage, phase, abort_flag, p.status_word, kErrProducerWait)) {
+                        alive = false;
+                        break;
+                    }
+                    if (elect_one()) {
+                        const uint32_t base = smem_u32(smem + stage * kPairStageBytes);
+                        // The block scales go first, on a barrier of their own: they are small and land early, so the copy
+                        // warps have them in tensor memory by the time the operand tiles arrive.
+                        const uint32_t landed = bar_scales_landed + 8 * stage, full = bar_full + 8 * stage;
+                        if (rank == 0) mbar_expect_tx(landed, 2 * (kBytesSfA + kBytesSfB));
+                        tma_load_2d_pair(base + kBytesA + kPairBytesB, &map_act_sf, 0,
+                                         term * act_term_atoms + (token_row / 128) * atoms_per_row_block + kb * 4, landed);
+                        tma_load_2d_pair(base + kBytesA + kPairBytesB + kBytesSfA, &map_weight_sf, 0,
+                                         (n_tile * 2) * atoms_per_row_block + kb * 4, landed);
+                        tma_load_2d_pair(base + kBytesA + kPairBytesB + 2 * kBytesSfA, &map_weight_sf, 0,
+                                         (n_tile * 2 + 1) * atoms_per_row_block + kb * 4, landed);
+                        if (rank == 0) mbar_expect_tx(full, 2 * (kBytesA + kPairBytesB));
+                        tma_load_2d_pair(base, &map_act, kb * 128, term * p.padded_tokens + token_row, full);
+                        tma_load_2d_pair(base + kBytesA, &map_weight, kb * 128, weight_row, full);
+                    }
+                    __syncwarp();
+                    if (++stage == kPairStages) { stage = 0; phase ^= 1; }
                 }
-                const uint32_t base = smem_u32(smem + stage * kPairStageBytes);
-                const uint32_t full = bar_full + 8 * stage;
-                // The block scales go first, on a barrier of their own: they are small and land early, so the copy
-                // thread has them in tensor memory by the time the operand tiles arrive.
-                const uint32_t landed = bar_scales_landed + 8 * stage;
-                const uint32_t token_row = m_pair * 2 * kTileM + rank * kTileM;
-                if (rank == 0) mbar_expect_tx(landed, 2 * (kBytesSfA + kBytesSfB));
-                tma_load_2d_pair(base + kBytesA + kPairBytesB, &map_act_sf, 0,
-                                 term * act_term_atoms + (token_row / 128) * atoms_per_row_block + kb * 4, landed);
-                tma_load_2d_pair(base + kBytesA + kPairBytesB + kBytesSfA, &map_weight_sf, 0,
-                                 (n_tile * 2) * atoms_per_row_block + kb * 4, landed);
-                tma_load_2d_pair(base + kBytesA + kPairBytesB + 2 * kBytesSfA, &map_weight_sf, 0,
-                                 (n_tile * 2 + 1) * atoms_per_row_block + kb * 4, landed);
-                if (rank == 0) mbar_expect_tx(full, 2 * (kBytesA + kPairBytesB));
-                tma_load_2d_pair(base, &map_act, kb * 128, term * p.padded_tokens + token_row, full);
-                tma_load_2d_pair(base + kBytesA, &map_weight, kb * 128, n_tile * kTileN + rank * 128, full);
-                if (++stage == kPairStages) { stage = 0; phase ^= 1; }
             }
         }
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+    } else if (warp == 1 && rank == 0) {
         // ---------------- MMA issuer (leader only) ----------------
-        // Issuing a tcgen05 operation keeps a thread busy for tens of cycles, and one thread issuing the
-        // 12 scale copies and the 4 MMAs of every stage could not keep the tensor pipe fed; the copies are
-        // issued by a thread of their own (below) into the stage's scale columns, this thread issues
-        // only the MMAs. Descriptors advance by additions (their low bits hold address >> 4).
+        // Issuing a tcgen05 operation keeps a warp busy for tens of cycles, and one warp issuing the 12 scale copies and
+        // the 4 MMAs of every stage could not keep the tensor pipe fed; the copies are issued by two warps of their own
+        // (below) into the stage's scale columns, this one issues only the MMAs. Descriptors advance by additions (their low
+        // bits hold address >> 4). Looking at a barrier takes as long as issuing an MMA or two, so those of the next
+        // step are looked at before the MMAs of this one are issued, and waited for only if they were not there.
         uint32_t stage = 0, phase = 0, tmem_phase = 0;
-        uint32_t kb_slot = 0;   // k blocks counted across tiles, modulo kPairStages: the weight-row scale buffer
-        bool alive = true;
-        const uint32_t idesc = (1u << 7) | (1u << 10) | ((kTileN >> 3) << 17) | (((2 * kTileM) >> 4) << 24);
+        uint32_t kb_slot = 0, kb_phase = 0;   // k blocks counted across tiles, modulo kPairStages: the weight-row scale buffer
+        bool alive = true, operands_seen = false, scales_seen = false, weights_seen = false;
+        constexpr uint32_t kWideTile = (1u << 7) | (1u << 10) | ((kTileN >> 3) << 17) | (((2 * kTileM) >> 4) << 24);
+        constexpr uint32_t kHalfTile = (1u << 7) | (1u << 10) | ((kTileN / 2 >> 3) << 17) | (((2 * kTileM) >> 4) << 24);
         const uint32_t smem_base = smem_u32(smem);
         const uint64_t a_desc0 = operand_desc(smem_base), b_desc0 = operand_desc(smem_base + kBytesA);
-        constexpr uint64_t kStageStep = kPairStageBytes >> 4;
+        constexpr uint32_t kStageStep = kPairStageBytes >> 4;
         const uint32_t last_k_steps = (p.cols - (k_blocks - 1) * kBlockK) / 64;   // 1..4 k steps of 64 in the last k block
         for (uint32_t index = 0; alive && index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
-            const uint32_t item_steps = (item.kb1 - item.kb0) * p.terms;
             // the epilogues of both CTAs must have drained the previous tile's accumulator
             if (!mbar_wait(bar_tmem_empty, tmem_phase ^ 1, abort_flag, p.status_word, kErrMmaWaitTmem)) break;
             tc_fence_after();
-            uint32_t accumulate = 0, term = 0, kb = item.kb0;
-            for (uint32_t step = 0; step < item_steps; ++step) {
-                // operands in shared memory (TMA) and block scales in tensor memory (copy thread)
-                if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.status_word, kErrMmaWaitFull) ||
-                    !mbar_wait(bar_scales_ready + 8 * stage, phase, abort_flag, p.status_word, kErrMmaWaitScales)) {
+            const uint32_t idesc = item.tile / m_pairs == half_tile ? kHalfTile : kWideTile;
+            uint32_t accumulate = 0;
+            for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb) {
+                const uint32_t k_steps = (kb + 1 < k_blocks) ? 4u : last_k_steps;
+                if (!weights_seen && !mbar_wait(bar_weights_ready + 8 * kb_slot, kb_phase, abort_flag, p.status_word, kErrMmaWaitScales)) {
                     alive = false;
                     break;
                 }
-                tc_fence_after();
-                const uint64_t a_desc = a_desc0 + stage * kStageStep, b_desc = b_desc0 + stage * kStageStep;
-                // the token rows' scales change with every step (term), the weight rows' scales only with the k block
-                const uint32_t tmem_sfa = tmem_base + kTmemPairSfA + stage * 16;
-                const uint32_t tmem_sfb = tmem_base + kTmemPairSfB + kb_slot * 32;
-                // each MMA consumes 64 k = 32 bytes of every row: start address + 2; only k steps inside the tensor
-                const uint32_t k_steps = (kb + 1 < k_blocks) ? 4u : last_k_steps;
-                if (k_steps == 4) {
+                const uint32_t tmem_sfb = tmem_base + kTmemPairSfB + kb_slot * 32;   // the weight rows' scales change with the k block only
+                if (++kb_slot == kPairStages) { kb_slot = 0; kb_phase ^= 1; }
+                for (uint32_t term = 0; term < p.terms; ++term) {
+                    // operands in shared memory (TMA) and block scales in tensor memory (copy warps)
+                    if ((!operands_seen && !mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.status_word, kErrMmaWaitFull)) ||
+                        (!scales_seen && !mbar_wait(bar_scales_ready + 8 * stage, phase, abort_flag, p.status_word, kErrMmaWaitScales))) {
+                        alive = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint64_t a_desc = a_desc0 + stage * kStageStep, b_desc = b_desc0 + stage * kStageStep;
+                    const uint32_t tmem_sfa = tmem_base + kTmemPairSfA + stage * 16, done = bar_empty + 8 * stage;
+                    if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+                    operands_seen = mbar_test(bar_full + 8 * stage, phase);
+                    scales_seen = mbar_test(bar_scales_ready + 8 * stage, phase);
+                    if (term + 1 == p.terms) weights_seen = mbar_test(bar_weights_ready + 8 * kb_slot, kb_phase);
+                    if (elect_one()) {
+                        // each MMA consumes 64 k = 32 bytes of every row: start address + 2; only k steps inside the tensor
+                        if (k_steps == 4) {
 #pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k) {
-                        tc_mma_pair(tmem_base + kTmemAcc, a_desc + 2 * k, b_desc + 2 * k, idesc, tmem_sfa + 4 * k, tmem_sfb + 8 * k,
-                                    accumulate | k);
+                            for (uint32_t k = 0; k < 4; ++k) {
+                                tc_mma_pair(tmem_base + kTmemAcc, a_desc + 2 * k, b_desc + 2 * k, idesc, tmem_sfa + 4 * k, tmem_sfb + 8 * k,
+                                            accumulate | k);
+                            }
+                        } else {
+                            for (uint32_t k = 0; k < k_steps; ++k) {
+                                tc_mma_pair(tmem_base + kTmemAcc, a_desc + 2 * k, b_desc + 2 * k, idesc, tmem_sfa + 4 * k, tmem_sfb + 8 * k,
+                                            accumulate | k);
+                            }
+                        }
+                        tc_commit_pair(done);   // frees the stage, and with it the stage's scale columns, in both CTAs
                     }
-                } else {
-                    for (uint32_t k = 0; k < k_steps; ++k) {
-                        tc_mma_pair(tmem_base + kTmemAcc, a_desc + 2 * k, b_desc + 2 * k, idesc, tmem_sfa + 4 * k, tmem_sfb + 8 * k,
-                                    accumulate | k);
-                    }
+                    __syncwarp();
+                    accumulate = 1;
                 }
-                accumulate = 1;
-                tc_commit_pair(bar_empty + 8 * stage);   // frees the stage, and with it the stage's scale columns, in both CTAs
-                if (++term == p.terms) {
-                    term = 0;
-                    ++kb;
-                    if (++kb_slot == kPairStages) kb_slot = 0;
-                }
-                if (++stage == kPairStages) { stage = 0; phase ^= 1; }
             }
-            if (alive) tc_commit_pair(bar_tmem_full);     // both accumulator halves complete
+            if (alive && elect_one()) tc_commit_pair(bar_tmem_full);     // both accumulator halves complete
+            __syncwarp();
             tmem_phase ^= 1;
         }
-    } else if (warp == kPairCopyWarp && lane == 0 && rank == 0) {
-        // ---------------- scale-copy issuer (leader only): shared memory -> tensor memory, both CTAs ----------------
+    } else if ((warp == kPairCopyWarp || warp == kPairCopyWarp + 1) && rank == 0) {
+        // ---------------- scale-copy issuers (leader only): shared memory -> tensor memory, both CTAs ----------------
+        // One warp copies the token rows' scales of every step, the other the weight rows' scales, which are the same for all
+        // activation terms of a k block, with term 0. (One thread issuing all twelve copies of a one-term step needed longer
+        // than the step's MMAs: 193 us for 4096 tokens on 17408 x 5120.)
+        // A stage's scale atoms have landed. The producer refilled the stage only after the MMAs of the step that used it
+        // last (kPairStages steps ago) were complete, and operations complete in order, so every older MMA is complete
+        // too: the stage's token-row scale columns are free, and so are the weight-row scale columns of this k
+        // block's slot, last read by the k block kPairStages before it (at least kPairStages steps ago for any number
+        // of terms). The copies only have to be issued before the MMAs that read them: a copy and a later MMA execute
+        // in issue order, and the fences on either side of the arrival order the two warps' issues.
+        const bool weights = warp != kPairCopyWarp;
         uint32_t stage = 0, phase = 0, kb_slot = 0;
         const uint32_t smem_base = smem_u32(smem);
         const uint64_t sfa_desc0 = sf_desc(smem_base + kBytesA + kPairBytesB), sfb_desc0 = sf_desc(smem_base + kBytesA + kPairBytesB + kBytesSfA);
-        constexpr uint64_t kStageStep = kPairStageBytes >> 4, kAtomStep = kSfAtomBytes >> 4, kRowBlockStep = kBytesSfA >> 4;
+        constexpr uint32_t kStageStep = kPairStageBytes >> 4, kAtomStep = kSfAtomBytes >> 4, kRowBlockStep = kBytesSfA >> 4;
         const uint32_t last_k_steps = (p.cols - (k_blocks - 1) * kBlockK) / 64;
         bool alive = true;
         for (uint32_t index = 0; alive && index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
-            const uint32_t item_steps = (item.kb1 - item.kb0) * p.terms;
-            uint32_t term = 0, kb = item.kb0;
-            for (uint32_t step = 0; step < item_steps; ++step) {
-                // The stage's scale atoms have landed. The producer refilled the stage only after the MMAs of the
-                // step that used it last (kPairStages steps ago) were complete, and operations complete in
-                // order, so every older MMA is complete too: the stage's token-row scale columns are free, and
-                // so are the weight-row scale columns of this k block's slot, last read by the k block
-                // kPairStages before it (at least kPairStages steps ago for any number of terms).
-                if (!mbar_wait(bar_scales_landed + 8 * stage, phase, abort_flag, p.status_word, kErrCopyWait)) {
-                    alive = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint64_t sfa_desc = sfa_desc0 + stage * kStageStep, sfb_desc = sfb_desc0 + stage * kStageStep;
-                // Token-row scales change with every step; weight-row scales are the same for all activation
-                // terms of a k block and are copied with term 0 only.
-                const uint32_t tmem_sfa = tmem_base + kTmemPairSfA + stage * 16;
-                const uint32_t tmem_sfb = tmem_base + kTmemPairSfB + kb_slot * 32;
+            const bool wide = item.tile / m_pairs != half_tile;   // a half tile has one row block of weight scales
+            for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb) {
                 const uint32_t k_steps = (kb + 1 < k_blocks) ? 4u : last_k_steps;
-                if (k_steps == 4) {
+                for (uint32_t term = 0; term < p.terms; ++term) {
+                    // both warps wait for every step, so that neither can take a phase of the barrier for a later one
+                    if (!mbar_wait(bar_scales_landed + 8 * stage, phase, abort_flag, p.status_word, kErrCopyWait)) {
+                        alive = false;
+                        break;
+                    }
+                    if (!weights || term == 0) {
+                        tc_fence_after();
+                        if (elect_one()) {
+                            if (!weights) {
+                                const uint64_t desc = sfa_desc0 + stage * kStageStep;
+                                const uint32_t columns = tmem_base + kTmemPairSfA + stage * 16;
+                                if (k_steps == 4) {
 #pragma unroll
-                    for (uint32_t k = 0; k < 4; ++k) {
-                        tc_copy_sf_pair(tmem_sfa + 4 * k, sfa_desc + k * kAtomStep);
-                    }
-                    if (term == 0) {
+                                    for (uint32_t k = 0; k < 4; ++k) tc_copy_sf_pair(columns + 4 * k, desc + k * kAtomStep);
+                                } else {
+                                    for (uint32_t k = 0; k < k_steps; ++k) tc_copy_sf_pair(columns + 4 * k, desc + k * kAtomStep);
+                                }
+                            } else {
+                                const uint64_t desc = sfb_desc0 + stage * kStageStep;
+                                const uint32_t columns = tmem_base + kTmemPairSfB + kb_slot * 32;
+                                if (k_steps == 4 && wide) {
 #pragma unroll
-                        for (uint32_t k = 0; k < 4; ++k) {
-                            tc_copy_sf_pair(tmem_sfb + 8 * k, sfb_desc + k * kAtomStep);
-                            tc_copy_sf_pair(tmem_sfb + 8 * k + 4, sfb_desc + kRowBlockStep + k * kAtomStep);
+                                    for (uint32_t k = 0; k < 4; ++k) {
+                                        tc_copy_sf_pair(columns + 8 * k, desc + k * kAtomStep);
+                                        tc_copy_sf_pair(columns + 8 * k + 4, desc + kRowBlockStep + k * kAtomStep);
+                                    }
+                                } else {
+                                    for (uint32_t k = 0; k < k_steps; ++k) {
+                                        tc_copy_sf_pair(columns + 8 * k, desc + k * kAtomStep);
+                                        if (wide) tc_copy_sf_pair(columns + 8 * k + 4, desc + kRowBlockStep + k * kAtomStep);
+                                    }
+                                }
+                            }
+                            tc_fence_before();
+                            mbar_arrive(weights ? bar_weights_ready + 8 * kb_slot : bar_scales_ready + 8 * stage);
                         }
+                        __syncwarp();
                     }
-                } else {
-                    for (uint32_t k = 0; k < k_steps; ++k) {
-                        tc_copy_sf_pair(tmem_sfa + 4 * k, sfa_desc + k * kAtomStep);
-                        if (term == 0) {
-                            tc_copy_sf_pair(tmem_sfb + 8 * k, sfb_desc + k * kAtomStep);
-                            tc_copy_sf_pair(tmem_sfb + 8 * k + 4, sfb_desc + kRowBlockStep + k * kAtomStep);
-                        }
-                    }
+                    if (++stage == kPairStages) { stage = 0; phase ^= 1; }
                 }
-                // The copies only have to be issued before the MMAs that read them: a copy and a later MMA
-                // execute in issue order, and the fences on either side of this arrival order the two threads' issues.
-                tc_fence_before();
-                mbar_arrive(bar_scales_ready + 8 * stage);
-                if (++term == p.terms) {
-                    term = 0;
-                    ++kb;
-                    if (++kb_slot == kPairStages) kb_slot = 0;
-                }
-                if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+                if (++kb_slot == kPairStages) kb_slot = 0;
             }
         }
     } else if (warp >= 2 && warp < 2 + kPairEpilogueWarps) {
@@ -638,6 +434,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive_leader(bar_tmem_empty);
             tmem_phase ^= 1;
+            // Rows past the tokens, and the columns a half tile does not have: nothing to store, hand over or add. (Padding rows
+            // hold whatever the staging buffer held; converting them cost more than real ones, since zeros and non-finite
+            // values leave the quantiser's fast path: 356 us instead of 260 for gate|up of 777 tokens.)
+            const uint32_t first_token = m_pair * 2 * kTileM + rank * kTileM + quadrant * 32;
+            if (first_token >= p.tokens || (half && n_tile == half_tile)) continue;
 
             if (item.kind == 1) {
                 // a part of a leftover tile: the sums go, as they are, to the pair that finishes the tile
@@ -699,7 +500,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
                 }
             }
 
-            const uint32_t first_token = m_pair * 2 * kTileM + rank * kTileM + quadrant * 32;
             if (p.swiglu) {
                 // 32 accumulator columns = gate and up sums of 16 intermediate columns = one quantisation group per row
                 const uint32_t out_width = p.rows / 2;
@@ -711,7 +511,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
                 for (uint32_t c = 0; c < 4; ++c) {
                     uint32_t packed[16];
                     convert_chunk(v[c], p.scale, p.scale_b, true, packed);
-                    if (p.quant_out) {
+                    if (p.quant_out && token < p.tokens) {
                         // The BF16 values this lane holds, quantised for the next GEMM while the next tile's MMAs run.
                         const uint32_t group = n_tile * (kTileN / 32) + half * 4 + c;
                         float2 residual[8];
@@ -725,10 +525,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
                             uint32_t codes[2], scale_code;
                             quantise_term(residual, p.quant_global_scale, term + 1 < p.quant_terms, codes, &scale_code);
                             scale_words[term] |= scale_code << (8 * c);
-                            if (token < p.tokens) {
-                                *reinterpret_cast<uint2*>(p.quant_out + term * code_bytes + static_cast<uint64_t>(token) * (out_width / 2) + group * 8) =
-                                    make_uint2(codes[0], codes[1]);
-                            }
+                            *reinterpret_cast<uint2*>(p.quant_out + term * code_bytes + static_cast<uint64_t>(token) * (out_width / 2) + group * 8) =
+                                make_uint2(codes[0], codes[1]);
                         }
                     }
                     if (p.out) {
@@ -799,8 +597,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
 // One thread per (token, 16-element group). Destination: the code planes of all terms
 // stacked ([terms][tokens][cols/2], one TMA tensor of terms*tokens rows), then the scale
 // regions of all terms.
-__global__ void act_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ destination, uint32_t tokens,
+constexpr uint32_t kQuantThreads = 128;
+__global__ void __launch_bounds__(kQuantThreads) act_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ destination, uint32_t tokens,
                                  uint32_t cols, uint32_t terms, float global_scale) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // x may come from the launch before this one, and the destination may still be read by it
     const uint32_t groups = cols / 16;
     // tokens * cols fits 32 bits, so the group index does too
     const uint32_t index = blockIdx.x * blockDim.x + threadIdx.x;
@@ -855,20 +656,21 @@ EncodeTiled encode_entry() {
     return cached;
 }
 
-// Packed codes as a 2-D byte tensor [rows][cols/2]; boxes of 128 rows x 128 bytes, 128-byte swizzle.
-// A host-side computation: no allocation and no device access.
-bool make_code_map(CUtensorMap* map, uint64_t address, uint64_t rows, uint32_t cols) {
+}  // namespace
+
+bool make_code_map(CUtensorMap* map, uint64_t address, uint64_t rows, uint32_t cols, uint32_t box_rows) {
     const EncodeTiled encode = encode_entry();
     if (!encode) return false;
     const cuuint64_t dims[2] = {cols / 2, rows};
     const cuuint64_t strides[1] = {cols / 2};
-    const cuuint32_t box[2] = {128, 128};
+    const cuuint32_t box[2] = {128, box_rows};
     const cuuint32_t element_strides[2] = {1, 1};
     return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, reinterpret_cast<void*>(address), dims, strides, box,
                   element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+namespace {
 // Block-scale atoms as a 2-D tensor [atoms][256 x u16] (512 bytes each); a box is the 4 atoms of
 // one 128-row block and one 256-deep k block.
 bool make_scale_map(CUtensorMap* map, uint64_t address, uint64_t atoms) {
@@ -975,8 +777,6 @@ uint32_t gemm_pair_resident_clusters() {
 }
 
 cudaError_t gemm_configure_device() {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmemBytes);
-    if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
 }
 
@@ -1016,9 +816,9 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_act_quant
     const uint64_t groups = static_cast<uint64_t>(a->tokens) * (a->cols / 16);
     // Rows past `tokens` in the last 128-row tile (codes and scale bytes) are left as they are: they only
     // feed output rows that the GEMM never stores.
-    act_quant_kernel<<<static_cast<uint32_t>((groups + 255) / 256), 256, 0, s->stream>>>(
-        reinterpret_cast<const uint16_t*>(a->input_bf16), reinterpret_cast<uint8_t*>(a->destination), a->tokens,
-        a->cols, a->terms, a->global_scale);
+    launch_dependent(s->stream, act_quant_kernel, static_cast<uint32_t>((groups + kQuantThreads - 1) / kQuantThreads), kQuantThreads, 0,
+                     reinterpret_cast<const uint16_t*>(a->input_bf16), reinterpret_cast<uint8_t*>(a->destination), a->tokens, a->cols,
+                     a->terms, a->global_scale);
     count_launch();
     return submitted();
 }
@@ -1046,11 +846,8 @@ augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_s
                                  QuantTarget quant = QuantTarget()) {
     // Tensor maps are encoded on the host into kernel parameter space: no allocation, no driver query.
     // The activation map spans the stacked code planes of all terms (terms * padded tokens rows).
-    CUtensorMap map_act, map_weight;
-    if (!make_code_map(&map_weight, a->weight, a->rows, a->cols) ||
-        !make_code_map(&map_act, a->activation, static_cast<uint64_t>(a->activation_terms) * padded_tokens(a->tokens), a->cols)) {
-        return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
-    }
+    CUtensorMap map_weight;
+    if (!make_code_map(&map_weight, a->weight, a->rows, a->cols)) return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
     GemmParams p{};
     p.weight_sf = reinterpret_cast<const uint8_t*>(a->weight) + tcgen05_codes_bytes(a->rows, a->cols);
     const uint32_t padded = padded_tokens(a->tokens);
@@ -1066,17 +863,20 @@ augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_s
     p.quant_out = reinterpret_cast<uint8_t*>(quant.destination);
     p.quant_terms = quant.terms;
     p.quant_global_scale = quant.global_scale;
-    if (a->rows % kTileN == 0 && plan->sm_count >= 2) {
+    const uint32_t all_pairs = plan->pair_clusters;   // pairs that are resident together (at most SMs / 2)
+    if (!all_pairs) return make_result(AUGUR_CUDA_STATUS_UNSUPPORTED_DEVICE);
+    p.token_pairs = (padded + 2 * kTileM - 1) / (2 * kTileM);
+    {
         // 256 x 256 tiles on pairs of CTAs (clusters of two); the grid is a whole number of pairs.
-        CUtensorMap map_act_sf, map_weight_sf;
+        CUtensorMap map_act, map_act_sf, map_weight_sf;
         const uint64_t atoms_per_row_block = a->cols / 64;
-        if (!make_scale_map(&map_weight_sf, reinterpret_cast<uint64_t>(p.weight_sf), (a->rows / 128) * atoms_per_row_block) ||
+        if (!make_code_map(&map_act, a->activation, static_cast<uint64_t>(a->activation_terms) * padded, a->cols) ||
+            !make_scale_map(&map_weight_sf, reinterpret_cast<uint64_t>(p.weight_sf), (a->rows / 128) * atoms_per_row_block) ||
             !make_scale_map(&map_act_sf, reinterpret_cast<uint64_t>(p.act_sf),
                             static_cast<uint64_t>(a->activation_terms) * (padded / 128) * atoms_per_row_block)) {
             return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
         }
-        const uint32_t tiles = ((padded + 2 * kTileM - 1) / (2 * kTileM)) * (a->rows / kTileN);
-        const uint32_t all_pairs = plan->pair_clusters;   // pairs that are resident together (at most SMs / 2)
+        const uint32_t tiles = p.token_pairs * ((a->rows + kTileN - 1) / kTileN);
         uint32_t pairs = tiles < all_pairs ? tiles : all_pairs;
         // Tiles past the last full round of the pairs (all tiles, when there are fewer tiles than pairs) are cut
         // along k between all pairs when the plan's scratch has room for the partial accumulators handed over
@@ -1096,16 +896,10 @@ augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_s
             p.split_flags = reinterpret_cast<uint32_t*>(plan->scratch);
             p.split_slots = reinterpret_cast<float*>(plan->scratch + kCounterBytes);
         }
-        gemm_pair_kernel<<<2 * pairs, kPairThreads, kPairSmemBytes, s->stream>>>(map_act, map_weight, map_act_sf, map_weight_sf, p);
+        launch_dependent(s->stream, gemm_pair_kernel, 2 * pairs, kPairThreads, kPairSmemBytes, map_act, map_weight, map_act_sf, map_weight_sf, p);
         count_launch();
         return submitted();
     }
-    const uint32_t m_tiles = padded / kTileM, n_tiles = (a->rows + kTileN - 1) / kTileN;
-    uint32_t grid = m_tiles * n_tiles;
-    if (grid > plan->sm_count) grid = plan->sm_count;
-    gemm_kernel<<<grid, kGemmThreads, kGemmSmemBytes, s->stream>>>(map_act, map_weight, p);
-    count_launch();
-    return submitted();
 }
 
 static_assert(sizeof(augur_cuda_nvfp4_sm100_gemm_swiglu_args_v1) == 88, "gemm_swiglu ABI");

@@ -100,6 +100,24 @@ void count_allocation();
 void count_free();
 augur_cuda_result_v1 submitted();  // maps cudaGetLastError to SUBMISSION_FAILURE
 
+// Launches with programmatic stream serialisation: the grid may become resident while its predecessor drains, and
+// waits for it in-kernel (griddepcontrol.wait).
+template <class... Parameters, class... Arguments>
+void launch_dependent(cudaStream_t stream, void (*kernel)(Parameters...), uint32_t grid, uint32_t threads, uint32_t smem_bytes,
+                      const Arguments&... arguments) {
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.stream = stream;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = smem_bytes;
+    cudaLaunchKernelEx(&config, kernel, static_cast<Parameters>(arguments)...);
+}
+
 // One-time per-device kernel attribute setup, called from plan creation (bind time).
 cudaError_t gemv_configure_device();
 cudaError_t gemm_configure_device();

@@ -69,6 +69,15 @@ __device__ __forceinline__ bool mbar_wait_suspended(uint32_t bar, uint32_t parit
     return false;
 }
 
+// One lane of a converged warp. The threads that issue tcgen05 and TMA operations run their loops as whole warps and elect
+// a lane around the operations only: addresses and descriptors then live in uniform registers, where those instructions
+// want them. (In a loop that a single thread runs every operand is moved there first: 70 cycles per MMA or copy.)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t elected;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(elected));
+    return elected != 0;
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
