@@ -74,7 +74,6 @@ constexpr uint32_t kPairOutBytes = kPairEpilogueWarps * 32 * kPairOutRowBytes;  
 constexpr uint32_t kPairSmemBytes = kPairStages * kPairStageBytes + kPairOutBytes + 1024 + 256;
 constexpr uint32_t kPairCopyWarp = 2 + kPairEpilogueWarps;    // token-row scales; the warp after it copies the weight-row scales
 constexpr uint32_t kPairThreads = 32 * (kPairCopyWarp + 2);   // TMA warp, MMA warp, epilogue warps, two scale-copy warps
-constexpr uint32_t kSplitWorthSteps = 16;       // pipeline steps a pair issues in the time a hand-over costs
 constexpr uint32_t kSplitWays = 8;              // a leftover tile is cut into this many parts at most
 constexpr uint32_t kSplitWaitLimit = 1u << 20;  // polls of a handed-over part's flag (each a round trip to L2) before giving up
 constexpr uint64_t kSplitSlotBytes = 2ull * kPairEpilogueWarps * 32 * 128 * 4;   // one pair's accumulator: 256 x 256 f32
@@ -425,94 +424,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
             const uint32_t m_pair = item.tile % m_pairs, n_tile = item.tile / m_pairs;
             if (!mbar_wait(bar_tmem_full, tmem_phase, abort_flag, p.status_word, kErrEpilogueWait)) break;
             tc_fence_after();
-            uint32_t v[4][32];
-#pragma unroll
-            for (uint32_t c = 0; c < 4; ++c) tc_load32(tmem_base + kTmemAcc + ((quadrant * 32) << 16) + half * 128 + c * 32, v[c]);
-            tc_wait_ld();
-            // the accumulator is free for the next tile's MMAs from here on
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_leader(bar_tmem_empty);
-            tmem_phase ^= 1;
+            const uint32_t accumulator = tmem_base + kTmemAcc + ((quadrant * 32) << 16) + half * 128;
+            auto release = [&]() {   // the accumulator is free for the next tile's MMAs from here on
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_leader(bar_tmem_empty);
+                tmem_phase ^= 1;
+            };
             // Rows past the tokens, and the columns a half tile does not have: nothing to store, hand over or add. (Padding rows
             // hold whatever the staging buffer held; converting them cost more than real ones, since zeros and non-finite
-            // values leave the quantiser's fast path: 356 us instead of 260 for gate|up of 777 tokens.)
+            // values leave the quantiser's fast path.)
             const uint32_t first_token = m_pair * 2 * kTileM + rank * kTileM + quadrant * 32;
-            if (first_token >= p.tokens || (half && n_tile == half_tile)) continue;
-
-            if (item.kind == 1) {
-                // a part of a leftover tile: the sums go, as they are, to the pair that finishes the tile
-                const uint32_t slot = (pair * 2 + rank) * kPairEpilogueWarps + (warp - 2);
-                float4* dst = reinterpret_cast<float4*>(p.split_slots) + static_cast<uint64_t>(slot) * (32 * 32) + lane;
-#pragma unroll
-                for (uint32_t c = 0; c < 4; ++c) {
-#pragma unroll
-                    for (uint32_t i = 0; i < 8; ++i) {
-                        dst[(c * 8 + i) * 32] = make_float4(__uint_as_float(v[c][4 * i]), __uint_as_float(v[c][4 * i + 1]),
-                                                            __uint_as_float(v[c][4 * i + 2]), __uint_as_float(v[c][4 * i + 3]));
-                    }
-                }
-                __threadfence();
-                __syncwarp();
-                if (lane == 0) atomicExch(p.split_flags + slot, 1u);
+            if (first_token >= p.tokens || (half && n_tile == half_tile)) {
+                release();
                 continue;
             }
-            if (item.kind == 2) {
-                // the part that finishes a leftover tile: add the parts handed over, in pair order
-                bool arrived = true;
-                for (uint32_t giver = item.first_giver; giver < pair; ++giver) {
-                    const uint32_t slot = (giver * 2 + rank) * kPairEpilogueWarps + (warp - 2);
-                    if (lane == 0) {
-                        uint32_t spin = 0;
-                        while (atomicAdd(p.split_flags + slot, 0u) == 0u) {
-                            if (++spin > kSplitWaitLimit || ((spin & 255u) == 255u && *abort_flag)) { arrived = false; break; }
-                        }
-                    }
-                    arrived = __shfl_sync(0xffffffffu, arrived, 0);
-                    if (!arrived) break;
-                    __threadfence();
-                    const float4* src = reinterpret_cast<const float4*>(p.split_slots) + static_cast<uint64_t>(slot) * (32 * 32) + lane;
-#pragma unroll
-                    for (uint32_t c = 0; c < 4; ++c) {
-#pragma unroll
-                        for (uint32_t i = 0; i < 8; ++i) {
-                            const float4 part = __ldcg(src + (c * 8 + i) * 32);
-                            v[c][4 * i] = __float_as_uint(__uint_as_float(v[c][4 * i]) + part.x);
-                            v[c][4 * i + 1] = __float_as_uint(__uint_as_float(v[c][4 * i + 1]) + part.y);
-                            v[c][4 * i + 2] = __float_as_uint(__uint_as_float(v[c][4 * i + 2]) + part.z);
-                            v[c][4 * i + 3] = __float_as_uint(__uint_as_float(v[c][4 * i + 3]) + part.w);
-                        }
-                    }
-                    __syncwarp();
-                    if (lane == 0) p.split_flags[slot] = 0;   // the flags read zero again when the launch is over
-                }
-                if (!arrived) {
-                    if (lane == 0) {
-                        *abort_flag = 1;
-                        atomicCAS(p.status_word, 0u, kErrSplitWait);
-                        // The launch has failed and says so; the flags of the parts it gave up on go back to zero all
-                        // the same, so that a late giver cannot leave one set for the next launch on this plan.
-                        for (uint32_t giver = item.first_giver; giver < pair; ++giver) {
-                            p.split_flags[(giver * 2 + rank) * kPairEpilogueWarps + (warp - 2)] = 0;
-                        }
-                    }
-                    break;
-                }
-            }
 
-            if (p.swiglu) {
-                // 32 accumulator columns = gate and up sums of 16 intermediate columns = one quantisation group per row
-                const uint32_t out_width = p.rows / 2;
-                const uint64_t code_bytes = tcgen05_codes_bytes(p.padded_tokens, out_width);
-                const uint64_t scale_bytes = tcgen05_scale_bytes(p.padded_tokens, out_width);
-                const uint32_t token = first_token + lane;
-                uint32_t scale_words[3] = {0, 0, 0};   // the scale bytes of this row's 4 groups, per term: one word of an atom
-#pragma unroll
-                for (uint32_t c = 0; c < 4; ++c) {
-                    uint32_t packed[16];
-                    convert_chunk(v[c], p.scale, p.scale_b, true, packed);
+            // One 32-column chunk of sums on its way out.
+            const uint32_t out_width = p.swiglu ? p.rows / 2 : p.rows, token = first_token + lane;
+            uint32_t scale_words[3] = {0, 0, 0};   // SwiGLU, quantised: the scale bytes of this row's 4 groups, per term: one word of an atom
+            auto store_chunk = [&](uint32_t c, const uint32_t (&sums)[32]) {
+                uint32_t packed[16];
+                if (p.swiglu) {
+                    // 32 accumulator columns = gate and up sums of 16 intermediate columns = one quantisation group per row
+                    convert_chunk(sums, p.scale, p.scale_b, true, packed);
                     if (p.quant_out && token < p.tokens) {
                         // The BF16 values this lane holds, quantised for the next GEMM while the next tile's MMAs run.
+                        const uint64_t code_bytes = tcgen05_codes_bytes(p.padded_tokens, out_width);
                         const uint32_t group = n_tile * (kTileN / 32) + half * 4 + c;
                         float2 residual[8];
 #pragma unroll
@@ -527,6 +465,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
                             scale_words[term] |= scale_code << (8 * c);
                             *reinterpret_cast<uint2*>(p.quant_out + term * code_bytes + static_cast<uint64_t>(token) * (out_width / 2) + group * 8) =
                                 make_uint2(codes[0], codes[1]);
+                        }
+                        if (c == 3) {
+                            const uint64_t scale_bytes = tcgen05_scale_bytes(p.padded_tokens, out_width);
+#pragma unroll
+                            for (uint32_t term = 0; term < 3; ++term) {
+                                if (term >= p.quant_terms) break;
+                                *reinterpret_cast<uint32_t*>(p.quant_out + p.quant_terms * code_bytes + term * scale_bytes +
+                                                             tcgen05_scale_offset(token, n_tile * (kTileN / 32) + half * 4, out_width)) = scale_words[term];
+                            }
                         }
                     }
                     if (p.out) {
@@ -546,39 +493,131 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
                         }
                         __syncwarp();   // the rows are rewritten for the next chunk
                     }
+                    return;
                 }
-                if (p.quant_out && token < p.tokens) {
+                convert_chunk(sums, p.scale, p.scale_b, false, packed);
+                // transpose through shared memory: 64 bytes of every row, written out as 4 lanes per row
+                uint4* dst = reinterpret_cast<uint4*>(my_rows + lane * kPairOutRowBytes);
 #pragma unroll
-                    for (uint32_t term = 0; term < 3; ++term) {
-                        if (term >= p.quant_terms) break;
-                        *reinterpret_cast<uint32_t*>(p.quant_out + p.quant_terms * code_bytes + term * scale_bytes +
-                                                     tcgen05_scale_offset(token, n_tile * (kTileN / 32) + half * 4, out_width)) = scale_words[term];
+                for (uint32_t i = 0; i < 4; ++i) {
+                    dst[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
+                }
+                __syncwarp();
+                uint8_t* out_base = reinterpret_cast<uint8_t*>(p.out + static_cast<uint64_t>(first_token) * p.rows + n_tile * kTileN +
+                                                               half * 128 + c * 32);
+#pragma unroll
+                for (uint32_t r8 = 0; r8 < 32; r8 += 8) {
+                    const uint32_t r = r8 + (lane >> 2), piece = lane & 3;
+                    if (first_token + r >= p.tokens) continue;   // padding rows of the last tile are computed, never stored
+                    const uint4 value = *reinterpret_cast<const uint4*>(my_rows + r * kPairOutRowBytes + piece * 16);
+                    *reinterpret_cast<uint4*>(out_base + static_cast<uint64_t>(r) * p.rows * 2 + piece * 16) = value;
+                }
+                __syncwarp();   // the rows are rewritten for the next chunk
+            };
+            auto slot_of = [&](uint32_t giver) { return (giver * 2 + rank) * kPairEpilogueWarps + (warp - 2); };
+            auto slot_sums = [&](uint32_t slot) { return reinterpret_cast<float4*>(p.split_slots) + static_cast<uint64_t>(slot) * (32 * 32) + lane; };
+
+            // The part that finishes a leftover tile waits for the parts handed over and adds them in pair order.
+            auto parts_arrived = [&]() {
+                bool arrived = true;
+                for (uint32_t giver = item.first_giver; giver < pair; ++giver) {
+                    const uint32_t slot = slot_of(giver);
+                    if (lane == 0) {
+                        uint32_t spin = 0;
+                        while (atomicAdd(p.split_flags + slot, 0u) == 0u) {
+                            if (++spin > kSplitWaitLimit || ((spin & 255u) == 255u && *abort_flag)) {
+                                arrived = false;
+                                *abort_flag = 1;
+                                atomicCAS(p.status_word, 0u, kErrSplitWait);
+                                break;
+                            }
+                        }
+                        // The flags read zero again when the launch is over, also those of parts that were given up on: that launch has
+                        // failed and says so, and a late giver cannot leave one set for the next launch on this plan.
+                        p.split_flags[slot] = 0;
                     }
                 }
-            } else {
+                __threadfence();
+                return __all_sync(0xffffffffu, arrived) != 0;
+            };
+            if (item.kind == 2 && index + 1 == work.items) {
+                if (!parts_arrived()) break;
+                // Nothing follows that waits for the accumulator: a chunk at a time stays in registers, and the same chunk of several
+                // parts is in flight at once (one part after the other, all 128 columns each, cost 3 us per part).
+#pragma unroll 1
+                for (uint32_t c = 0; c < 4; ++c) {
+                    uint32_t sums[32];
+                    tc_load32(accumulator + c * 32, sums);
+                    tc_wait_ld();
+                    for (uint32_t giver = item.first_giver; giver < pair; giver += 3) {
+                        float4 part[3][8];
+#pragma unroll
+                        for (uint32_t q = 0; q < 3; ++q) {
+                            const float4* src = slot_sums(slot_of(giver + q));
+#pragma unroll
+                            for (uint32_t i = 0; i < 8; ++i) {
+                                part[q][i] = giver + q < pair ? __ldcg(src + (c * 8 + i) * 32) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                            }
+                        }
+#pragma unroll
+                        for (uint32_t q = 0; q < 3; ++q) {
+                            if (giver + q >= pair) break;
+#pragma unroll
+                            for (uint32_t i = 0; i < 8; ++i) {
+                                sums[4 * i] = __float_as_uint(__uint_as_float(sums[4 * i]) + part[q][i].x);
+                                sums[4 * i + 1] = __float_as_uint(__uint_as_float(sums[4 * i + 1]) + part[q][i].y);
+                                sums[4 * i + 2] = __float_as_uint(__uint_as_float(sums[4 * i + 2]) + part[q][i].z);
+                                sums[4 * i + 3] = __float_as_uint(__uint_as_float(sums[4 * i + 3]) + part[q][i].w);
+                            }
+                        }
+                    }
+                    store_chunk(c, sums);
+                }
+                release();
+                continue;
+            }
+
+            uint32_t v[4][32];
+#pragma unroll
+            for (uint32_t c = 0; c < 4; ++c) tc_load32(accumulator + c * 32, v[c]);
+            tc_wait_ld();
+            release();
+            if (item.kind == 1) {
+                // a part of a leftover tile: the sums go, as they are, to the pair that finishes the tile
+                const uint32_t slot = slot_of(pair);
+                float4* dst = slot_sums(slot);
 #pragma unroll
                 for (uint32_t c = 0; c < 4; ++c) {
-                    uint32_t packed[16];
-                    convert_chunk(v[c], p.scale, p.scale_b, false, packed);
-                    // transpose through shared memory: 64 bytes of every row, written out as 4 lanes per row
-                    uint4* dst = reinterpret_cast<uint4*>(my_rows + lane * kPairOutRowBytes);
 #pragma unroll
-                    for (uint32_t i = 0; i < 4; ++i) {
-                        dst[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
+                    for (uint32_t i = 0; i < 8; ++i) {
+                        dst[(c * 8 + i) * 32] = make_float4(__uint_as_float(v[c][4 * i]), __uint_as_float(v[c][4 * i + 1]),
+                                                            __uint_as_float(v[c][4 * i + 2]), __uint_as_float(v[c][4 * i + 3]));
                     }
-                    __syncwarp();
-                    uint8_t* out_base = reinterpret_cast<uint8_t*>(p.out + static_cast<uint64_t>(first_token) * p.rows + n_tile * kTileN +
-                                                                   half * 128 + c * 32);
+                }
+                __threadfence();
+                __syncwarp();
+                if (lane == 0) atomicExch(p.split_flags + slot, 1u);
+                continue;
+            }
+            if (item.kind == 2) {
+                if (!parts_arrived()) break;
+                for (uint32_t giver = item.first_giver; giver < pair; ++giver) {
+                    const float4* src = slot_sums(slot_of(giver));
 #pragma unroll
-                    for (uint32_t r8 = 0; r8 < 32; r8 += 8) {
-                        const uint32_t r = r8 + (lane >> 2), piece = lane & 3;
-                        if (first_token + r >= p.tokens) continue;   // padding rows of the last tile are computed, never stored
-                        const uint4 value = *reinterpret_cast<const uint4*>(my_rows + r * kPairOutRowBytes + piece * 16);
-                        *reinterpret_cast<uint4*>(out_base + static_cast<uint64_t>(r) * p.rows * 2 + piece * 16) = value;
+                    for (uint32_t c = 0; c < 4; ++c) {
+#pragma unroll
+                        for (uint32_t i = 0; i < 8; ++i) {
+                            const float4 part = __ldcg(src + (c * 8 + i) * 32);
+                            v[c][4 * i] = __float_as_uint(__uint_as_float(v[c][4 * i]) + part.x);
+                            v[c][4 * i + 1] = __float_as_uint(__uint_as_float(v[c][4 * i + 1]) + part.y);
+                            v[c][4 * i + 2] = __float_as_uint(__uint_as_float(v[c][4 * i + 2]) + part.z);
+                            v[c][4 * i + 3] = __float_as_uint(__uint_as_float(v[c][4 * i + 3]) + part.w);
+                        }
                     }
-                    __syncwarp();   // the rows are rewritten for the next chunk
                 }
             }
+#pragma unroll
+            for (uint32_t c = 0; c < 4; ++c) store_chunk(c, v[c]);
         }
     }
 
@@ -777,6 +816,8 @@ uint32_t gemm_pair_resident_clusters() {
 }
 
 cudaError_t gemm_configure_device() {
+    const cudaError_t e = gemm_narrow_configure_device();
+    if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
 }
 
@@ -841,6 +882,63 @@ struct QuantTarget {
     float global_scale = 0.0f;
 };
 
+// How a launch of the pair kernel over `token_pairs` x 256 token rows shares its tiles out, and about how long it takes.
+struct PairSplit {
+    uint32_t pairs, sharers;     // sharers: pairs that share the leftover tiles (0: every tile is one pair's)
+    uint32_t ns;
+};
+
+// Measured on a B200: a pipeline step (k block x term) of a pair takes 0.36 us, a launch 8 us beyond its steps. Handing the
+// parts of leftover tiles over takes the time of 16 steps and two more per part when nothing else is left to do, and about
+// 8 when it happens under whole tiles.
+constexpr uint32_t kPairStepNs = 360, kPairLaunchNs = 8000;
+constexpr uint32_t kSplitSteps = 16, kSplitPartSteps = 2, kSplitCoveredSteps = 8;
+
+// Tiles past the last full round of the pairs (all tiles, when there are fewer tiles than pairs) may be cut along k, in `ways`
+// parts each at most and over all pairs at most, when the plan's scratch has room for the partial accumulators handed
+// over: one slot per pair behind the counter regions, whose first words serve as the flags. Of the numbers of parts up to
+// kSplitWays the one with the least steps is taken: cut in eight, the 4 tiles of 1024 rows and 256 tokens took 25 us, whole 15.
+PairSplit pair_split(uint32_t token_pairs, uint32_t rows, uint32_t cols, uint32_t terms, uint32_t all_pairs, uint64_t scratch_bytes) {
+    const uint32_t tiles = token_pairs * ((rows + kTileN - 1) / kTileN), k_blocks = (cols + kBlockK - 1) / kBlockK;
+    const uint32_t whole = tiles / all_pairs, left = tiles % all_pairs;
+    PairSplit best{tiles < all_pairs ? tiles : all_pairs, 0, 0};
+    uint64_t least = static_cast<uint64_t>(whole + (left ? 1 : 0)) * k_blocks * terms;
+    for (uint32_t ways = 2; left && ways <= kSplitWays; ++ways) {
+        uint32_t sharers = left * ways < all_pairs ? left * ways : all_pairs;
+        if (sharers > static_cast<uint64_t>(left) * k_blocks) sharers = left * k_blocks;      // every part holds a k block
+        if (sharers <= left || scratch_bytes < kCounterBytes + sharers * kSplitSlotBytes) break;
+        const uint32_t parts = (sharers + left - 1) / left;
+        const uint64_t steps = static_cast<uint64_t>(whole) * k_blocks * terms + static_cast<uint64_t>(left * k_blocks + sharers - 1) / sharers * terms +
+                               (whole ? kSplitCoveredSteps : kSplitSteps + kSplitPartSteps * parts);
+        if (steps < least) {
+            least = steps;
+            best.sharers = sharers;
+        }
+    }
+    if (best.pairs < best.sharers) best.pairs = best.sharers;
+    best.ns = static_cast<uint32_t>(least * kPairStepNs > UINT32_MAX / 2 ? UINT32_MAX / 2 : least * kPairStepNs) + kPairLaunchNs;
+    return best;
+}
+
+// How many of the token rows the pair kernel takes (in 256-row pairs); the narrow kernel takes the rest. The choice is the
+// quickest by the estimates of the two: narrow up to 128 tokens nearly always (6144 x 5120, three terms, 48 tokens: 12 us
+// against 23), pairs from about 256 on (17408 x 5120, 256 tokens: 29 against 37) unless the weight is small (1024 x 5120: 22
+// against 14), and pairs with a narrow tail when the tokens just exceed whole pairs (17408 x 5120, 300 tokens: 49 against
+// 54). The tail starts when the pairs are nearly done, so it has to be clearly quicker to be taken.
+uint32_t token_pairs_for(const augur_cuda_nvfp4_sm100_plan_v1* plan, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
+    const uint32_t all_pairs = plan->pair_clusters, pairs = (tokens + 2 * kTileM - 1) / (2 * kTileM), rest = tokens % (2 * kTileM);
+    if (!all_pairs) return 0;
+    const uint32_t narrow_ns = gemm_narrow_ns(plan->ordinal, rows, cols, tokens, terms);
+    const uint32_t pair_ns = pair_split(pairs, rows, cols, terms, all_pairs, plan->scratch_bytes).ns;
+    uint32_t best = pair_ns < narrow_ns ? pairs : 0;
+    if (pairs > 1 && rest != 0 && rest <= kTileM) {
+        const uint64_t mixed = static_cast<uint64_t>(pair_split(pairs - 1, rows, cols, terms, all_pairs, plan->scratch_bytes).ns) +
+                               gemm_narrow_ns(plan->ordinal, rows, cols, rest, terms) - 3000;
+        if (mixed * 100 < static_cast<uint64_t>(best ? pair_ns : narrow_ns) * 93) best = pairs - 1;
+    }
+    return best;
+}
+
 augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
                                  const augur_cuda_nvfp4_sm100_gemm_args_v1* a, bool swiglu, float up_global_scale,
                                  QuantTarget quant = QuantTarget()) {
@@ -863,10 +961,8 @@ augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_s
     p.quant_out = reinterpret_cast<uint8_t*>(quant.destination);
     p.quant_terms = quant.terms;
     p.quant_global_scale = quant.global_scale;
-    const uint32_t all_pairs = plan->pair_clusters;   // pairs that are resident together (at most SMs / 2)
-    if (!all_pairs) return make_result(AUGUR_CUDA_STATUS_UNSUPPORTED_DEVICE);
-    p.token_pairs = (padded + 2 * kTileM - 1) / (2 * kTileM);
-    {
+    p.token_pairs = token_pairs_for(plan, a->rows, a->cols, a->tokens, a->activation_terms);
+    if (p.token_pairs) {
         // 256 x 256 tiles on pairs of CTAs (clusters of two); the grid is a whole number of pairs.
         CUtensorMap map_act, map_act_sf, map_weight_sf;
         const uint64_t atoms_per_row_block = a->cols / 64;
@@ -876,30 +972,18 @@ augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_s
                             static_cast<uint64_t>(a->activation_terms) * (padded / 128) * atoms_per_row_block)) {
             return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
         }
-        const uint32_t tiles = p.token_pairs * ((a->rows + kTileN - 1) / kTileN);
-        uint32_t pairs = tiles < all_pairs ? tiles : all_pairs;
-        // Tiles past the last full round of the pairs (all tiles, when there are fewer tiles than pairs) are cut
-        // along k between all pairs when the plan's scratch has room for the partial accumulators handed over
-        // (one slot per pair behind the counter regions, whose first words serve as the flags) and those tiles
-        // hold at least one k block per pair.
-        const uint32_t k_blocks = (a->cols + kBlockK - 1) / kBlockK;
-        const uint32_t left = tiles % all_pairs;
-        uint32_t sharers = left * kSplitWays < all_pairs ? left * kSplitWays : all_pairs;   // a tile is cut in kSplitWays parts at most
-        if (sharers > static_cast<uint64_t>(left) * k_blocks) sharers = left * k_blocks;      // and every part holds a k block
-        // Handing parts over costs about as much as 16 pipeline steps (k block x term) of a pair: the cut is made
-        // when the pairs would otherwise idle for longer than that, on average, in the last round.
-        const uint64_t idle_steps = static_cast<uint64_t>(all_pairs - left) * k_blocks * a->activation_terms;
-        if (left != 0 && sharers > left && idle_steps >= static_cast<uint64_t>(kSplitWorthSteps) * all_pairs &&
-            plan->scratch_bytes >= kCounterBytes + sharers * kSplitSlotBytes) {
-            if (pairs < sharers) pairs = sharers;
-            p.split_sharers = sharers;
+        const PairSplit split = pair_split(p.token_pairs, a->rows, a->cols, a->activation_terms, plan->pair_clusters, plan->scratch_bytes);
+        if (split.sharers) {
+            p.split_sharers = split.sharers;
             p.split_flags = reinterpret_cast<uint32_t*>(plan->scratch);
             p.split_slots = reinterpret_cast<float*>(plan->scratch + kCounterBytes);
         }
-        launch_dependent(s->stream, gemm_pair_kernel, 2 * pairs, kPairThreads, kPairSmemBytes, map_act, map_weight, map_act_sf, map_weight_sf, p);
+        launch_dependent(s->stream, gemm_pair_kernel, 2 * split.pairs, kPairThreads, kPairSmemBytes, map_act, map_weight, map_act_sf, map_weight_sf, p);
         count_launch();
-        return submitted();
+        const augur_cuda_result_v1 result = submitted();
+        if (result.status != AUGUR_CUDA_STATUS_OK || p.token_pairs * 2 * kTileM >= a->tokens) return result;
     }
+    return launch_gemm_narrow(s, plan, map_weight, a->activation, p, p.token_pairs * 2 * kTileM, p.token_pairs != 0);
 }
 
 static_assert(sizeof(augur_cuda_nvfp4_sm100_gemm_swiglu_args_v1) == 88, "gemm_swiglu ABI");

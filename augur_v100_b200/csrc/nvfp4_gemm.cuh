@@ -1,4 +1,4 @@
-// Prefill GEMM: launch parameters, accumulator conversion and the tensor map of packed codes.
+// What the prefill GEMM kernels share: launch parameters, accumulator conversion and the tensor map of packed codes.
 #pragma once
 
 #include <cuda.h>
@@ -71,5 +71,13 @@ __device__ __forceinline__ void convert_chunk(const uint32_t (&v)[32], float sca
 // Packed codes as a 2-D byte tensor [rows][cols/2]; boxes of `box_rows` rows x 128 bytes, 128-byte swizzle. A host-side
 // computation: no allocation and no device access.
 bool make_code_map(CUtensorMap* map, uint64_t address, uint64_t rows, uint32_t cols, uint32_t box_rows = 128);
+
+// The GEMM over the token rows from `token0` (a multiple of 128) on, for a range that is narrow next to the weights
+// (csrc/nvfp4_gemm_narrow.cu). `map_weight`: boxes of 128 rows. `p` describes the whole GEMM. With `after_main` the launch
+// before it on the stream is the pair kernel on the token rows before `token0`.
+augur_cuda_result_v1 launch_gemm_narrow(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan, const CUtensorMap& map_weight,
+                                        uint64_t activation, const GemmParams& p, uint32_t token0, bool after_main);
+// About how long it takes.
+uint32_t gemm_narrow_ns(int32_t ordinal, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms);
 
 }  // namespace augur_sm100

@@ -1,0 +1,493 @@
+// Prefill NVFP4 GEMM for token ranges that are narrow next to the weights (sm_100a): short prompts, batched decode of
+// more users than the small-token kernels take, and the tail of a longer prompt.
+//
+// The pair kernel of nvfp4_gemm.cu puts 256 token rows on its tile, so 9 tokens cost what 256 do. Here the weights are the
+// 128-row operand and the tokens sit on the MMA n dimension, whose size follows their number in steps of 16 (at most
+// 128): the work is that of the tokens there are, and what is left is streaming the weights once. Up to that width the
+// launch is bound by HBM (one term) or by the tensor pipe's queue of MMAs and scale copies (three terms).
+//
+//   D[feature][token] = sum over k blocks of 256, terms, k steps of 64:  W[128 x 64] * A_term[tokens x 64]^T
+//
+// Two rings in shared memory, because a weight stage (16 KB of codes, 2 KB of block scales) serves all terms of its k block
+// while an activation slot (tokens x 128 bytes of codes, 2 KB of scales) serves one term.
+//
+// An item is (128-row tile, token tile of at most 128), one per CTA. Two CTAs share an SM (113 KB of shared and half of tensor
+// memory each): while one waits for its rings or stores its results the other feeds the tensor pipe (one CTA per SM with
+// deeper rings took 30.4 us where this takes 22 for 17408 x 5120, 128 tokens, three terms). With fewer tiles than
+// places a cluster of up to 8 CTAs shares an item, each CTA an equal range of its k blocks; when all are done (a cluster
+// barrier, after which nobody reads its rings any more) every CTA sends its partial sums, by column, to the CTA that owns the
+// column, over distributed shared memory into the space the rings took, and finishes its own columns, adding in CTA
+// order: no scratch, no fences to global memory, no atomics, and results that do not depend on scheduling. (The pair
+// kernel's hand-over of leftover tiles through global memory is what most of its time goes to at these sizes.)
+//
+// Roles: warp 0 TMA and scale copies of the weights, 1 MMA, 2 TMA of the activations, 3 their scale copies to tensor memory,
+// 4..11 epilogue. What a step costs beyond its bytes is the time its warps take to issue it: each waits on as few barriers
+// as possible, its MMAs and copies are unrolled and come from one elected lane of a converged warp. (One thread copying all
+// scales in a loop took 980 cycles per step.)
+// Every wait is bounded; a wait that runs out records a code in the plan's status word, raises a CTA-wide abort flag, and
+// all roles fall through to the common exits.
+#include "nvfp4_gemm.cuh"
+
+namespace augur_sm100 {
+namespace {
+using namespace tc;
+
+constexpr uint32_t kNarrowK = 256;                                    // k per stage = one 128-byte swizzled row of codes
+constexpr uint32_t kNarrowCodes = kTileM * 128;                       // 16 KB
+constexpr uint32_t kNarrowScales = 4 * kSfAtomBytes;                  // 2 KB: the 4 atoms of 128 rows
+constexpr uint32_t kNarrowStage = kNarrowCodes + kNarrowScales;       // one weight stage
+constexpr uint32_t kNarrowMaxDepth = 8;                               // slots of either ring
+constexpr uint32_t kNarrowEpilogueWarps = 8;                          // two per tensor-memory lane quadrant
+constexpr uint32_t kNarrowThreads = 32 * (4 + kNarrowEpilogueWarps);   // 12 warps: registers are handed out to warps by fours
+constexpr uint32_t kNarrowState = 1024;                               // barriers, tensor-memory base, abort flag
+constexpr uint32_t kNarrowTurnPitch = 36;                             // floats between columns of the transposition area: 16-byte reads hit all banks
+constexpr uint32_t kNarrowSumPitch = 129;                             // 16-byte rows between groups of four columns of the partial sums, likewise
+constexpr uint32_t kNarrowSmem = 113 * 1024;                          // of two CTAs per SM
+constexpr uint32_t kNarrowTmemColumns = 256;
+constexpr uint32_t kNarrowMaxParts = 8;                               // portable cluster size
+
+constexpr uint32_t kErrNarrowWeights = 0x111, kErrNarrowTokens = 0x112, kErrNarrowFull = 0x113, kErrNarrowScales = 0x114,
+                   kErrNarrowCopy = 0x115, kErrNarrowAccFull = 0x116;
+
+struct NarrowParams {
+    GemmParams g;
+    uint32_t token0, tile_tokens, token_tiles, columns;   // columns: MMA n, tile_tokens rounded up to 16
+    uint32_t parts;                                       // CTAs per item (the cluster size)
+    uint32_t after_main;
+    uint32_t weight_depth, token_depth, slot_bytes;       // ring slots, size of an activation slot
+    uint32_t sf_weight, sf_token;                         // first tensor-memory columns of either ring's scales
+};
+
+// A row of 32 accumulator values of one token (weight rows row0 .. row0 + 31) -> output, quantised output.
+__device__ __forceinline__ void narrow_store(const GemmParams& g, uint32_t token, uint32_t row0, const uint32_t (&v)[32]) {
+    uint32_t packed[16];
+    convert_chunk(v, g.scale, g.scale_b, g.swiglu != 0, packed);
+    if (!g.swiglu) {
+        uint4* dst = reinterpret_cast<uint4*>(g.out + static_cast<uint64_t>(token) * g.rows + row0);
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) dst[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
+        return;
+    }
+    const uint32_t out_width = g.rows / 2;
+    if (g.out) {
+        uint4* dst = reinterpret_cast<uint4*>(g.out + static_cast<uint64_t>(token) * out_width + row0 / 2);
+        dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+    }
+    if (g.quant_out) {
+        // the 16 outputs are one quantisation group of the next GEMM's activations
+        const uint32_t group = row0 / 32;
+        const uint64_t code_bytes = tcgen05_codes_bytes(g.padded_tokens, out_width), scale_bytes = tcgen05_scale_bytes(g.padded_tokens, out_width);
+        float2 residual[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) residual[i] = make_float2(__uint_as_float(packed[i] << 16), __uint_as_float(packed[i] & 0xffff0000u));
+#pragma unroll 1
+        for (uint32_t term = 0; term < g.quant_terms; ++term) {
+            uint32_t codes[2], scale_code;
+            quantise_term(residual, g.quant_global_scale, term + 1 < g.quant_terms, codes, &scale_code);
+            *reinterpret_cast<uint2*>(g.quant_out + term * code_bytes + static_cast<uint64_t>(token) * (out_width / 2) + group * 8) = make_uint2(codes[0], codes[1]);
+            g.quant_out[g.quant_terms * code_bytes + term * scale_bytes + tcgen05_scale_offset(token, group, out_width)] = static_cast<uint8_t>(scale_code);
+        }
+    }
+}
+
+// The scale atoms of up to four k steps (four tensor-memory columns each).
+__device__ __forceinline__ void narrow_copy_scales(uint32_t columns, uint64_t desc, uint32_t k_steps) {
+    if (k_steps == 4) {
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) tc_copy_sf(columns + 4 * k, desc + k * (kSfAtomBytes >> 4));
+    } else {
+        for (uint32_t k = 0; k < k_steps; ++k) tc_copy_sf(columns + 4 * k, desc + k * (kSfAtomBytes >> 4));
+    }
+}
+
+__device__ __forceinline__ void narrow_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kNarrowThreads, 2)
+gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_constant__ CUtensorMap map_act, const NarrowParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const GemmParams& g = p.g;
+    uint8_t* slots = smem + p.weight_depth * kNarrowStage;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kNarrowSmem - 1024 - kNarrowState);
+    const uint32_t bar0 = smem_u32(bars);
+    // per slot of either ring: landed, free, scales in tensor memory (and with them the codes in shared memory)
+    const uint32_t w_full = bar0, w_empty = bar0 + 8 * kNarrowMaxDepth, w_ready = bar0 + 16 * kNarrowMaxDepth;
+    const uint32_t t_full = bar0 + 24 * kNarrowMaxDepth, t_empty = bar0 + 32 * kNarrowMaxDepth, t_ready = bar0 + 40 * kNarrowMaxDepth;
+    const uint32_t acc_full = bar0 + 48 * kNarrowMaxDepth;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6 * kNarrowMaxDepth + 1);
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    // Normally the next kernel of the stream may become resident from here on (it waits for this one's end before it reads).
+    if (!p.after_main) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (threadIdx.x == 0) {
+        for (uint32_t b = 0; b < 6 * kNarrowMaxDepth + 1; ++b) mbar_init(bar0 + 8 * b, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kNarrowTmemColumns) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    const uint32_t part = blockIdx.x % p.parts, item = blockIdx.x / p.parts;
+    const uint32_t row_tile = item / p.token_tiles, token_row = p.token0 + item % p.token_tiles * p.tile_tokens;
+    const uint32_t token_end = min(token_row + p.tile_tokens, g.tokens);
+    const uint32_t k_blocks = (g.cols + kNarrowK - 1) / kNarrowK, atoms = g.cols / 64;      // scale atoms of a 128-row block along k
+    const uint32_t kb0 = part * k_blocks / p.parts, kb1 = (part + 1) * k_blocks / p.parts;
+    const uint32_t last_k_steps = atoms - (k_blocks - 1) * 4;                               // 1..4 k steps of 64 in the last k block
+
+    if (warp == 0) {
+        // ---------------- weights: TMA, and scale copies to tensor memory ----------------
+        // They are constant, so nothing is waited for before the ring is filled. From then on the copies of a stage come first and
+        // the load into the stage before it, whose MMAs are the ones under way, second: the copies stay a k block ahead.
+        const uint64_t desc0 = sf_desc(smem_u32(smem) + kNarrowCodes);
+        const uint8_t* scales = g.weight_sf + static_cast<uint64_t>(row_tile) * atoms * kSfAtomBytes;
+        uint32_t load_kb = kb0, load_stage = 0, load_phase = 1, stage = 0, phase = 0;
+        auto load = [&]() {
+            if (!mbar_wait(w_empty + 8 * load_stage, load_phase, abort_flag, g.status_word, kErrNarrowWeights)) return false;
+            const uint32_t full = w_full + 8 * load_stage, to = smem_u32(smem + load_stage * kNarrowStage);
+            const uint32_t sf_bytes = (load_kb + 1 < k_blocks ? 4u : last_k_steps) * kSfAtomBytes;
+            if (elect_one()) {
+                mbar_expect_tx(full, kNarrowCodes + sf_bytes);
+                tma_load_2d(to, &map_weight, load_kb * 128, row_tile * kTileM, full);
+                bulk_load(to + kNarrowCodes, scales + static_cast<uint64_t>(load_kb) * kNarrowScales, sf_bytes, full);
+            }
+            __syncwarp();
+            ++load_kb;
+            if (++load_stage == p.weight_depth) { load_stage = 0; load_phase ^= 1; }
+            return true;
+        };
+        bool alive = true;
+        while (alive && load_kb < kb1 && load_kb < kb0 + p.weight_depth) alive = load();
+        for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
+            if (!mbar_wait(w_full + 8 * stage, phase, abort_flag, g.status_word, kErrNarrowCopy)) break;
+            tc_fence_after();
+            if (elect_one()) {
+                narrow_copy_scales(tmem_base + p.sf_weight + stage * 16, desc0 + stage * (kNarrowStage >> 4), kb + 1 < k_blocks ? 4u : last_k_steps);
+                tc_fence_before();
+                mbar_arrive(w_ready + 8 * stage);
+            }
+            __syncwarp();
+            if (++stage == p.weight_depth) { stage = 0; phase ^= 1; }
+            if (kb != kb0 && load_kb < kb1) alive = load();
+        }
+    } else if (warp == 2) {
+        // ---------------- TMA of activations ----------------
+        // They come from the launch before this one; after the pair kernel on the other tokens, from the launch before that,
+        // which is complete since that kernel lets its successor start only once its own wait is over.
+        if (!p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");
+        uint32_t slot = 0, phase = 1;
+        bool alive = true;
+        const uint8_t* scales = g.act_sf + static_cast<uint64_t>(token_row / 128) * atoms * kSfAtomBytes;
+        for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
+            const uint32_t sf_bytes = (kb + 1 < k_blocks ? 4u : last_k_steps) * kSfAtomBytes;
+            const uint8_t* from = scales + static_cast<uint64_t>(kb) * kNarrowScales;
+            uint32_t row = token_row;
+            for (uint32_t term = 0; term < g.terms; ++term) {
+                if (!mbar_wait(t_empty + 8 * slot, phase, abort_flag, g.status_word, kErrNarrowTokens)) {
+                    alive = false;
+                    break;
+                }
+                const uint32_t to = smem_u32(slots + slot * p.slot_bytes), full = t_full + 8 * slot;
+                if (elect_one()) {
+                    mbar_expect_tx(full, p.columns * 128 + sf_bytes);
+                    tma_load_2d(to, &map_act, kb * 128, row, full);
+                    bulk_load(to + p.columns * 128, from, sf_bytes, full);
+                }
+                __syncwarp();
+                from += g.act_term_stride;
+                row += g.padded_tokens;
+                if (++slot == p.token_depth) { slot = 0; phase ^= 1; }
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------- MMA issuer ----------------
+        uint32_t stage = 0, w_phase = 0, slot = 0, t_phase = 0, accumulate = 0;
+        bool alive = true;
+        const uint32_t idesc = instr_desc(p.columns);
+        const uint64_t w_desc0 = operand_desc(smem_u32(smem)), t_desc0 = operand_desc(smem_u32(slots));
+        const uint32_t slot_step = p.slot_bytes >> 4;
+        // Looking at a barrier takes as long as issuing an MMA or two, so the barriers of the next step are looked at before the
+        // MMAs of this one are issued, and waited for only if they were not there.
+        bool w_seen = false, t_seen = false;
+        for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
+            if (!w_seen && !mbar_wait(w_ready + 8 * stage, w_phase, abort_flag, g.status_word, kErrNarrowFull)) break;
+            const uint32_t k_steps = kb + 1 < k_blocks ? 4u : last_k_steps;
+            const uint64_t w_desc = w_desc0 + stage * (kNarrowStage >> 4);
+            const uint32_t sf_w = tmem_base + p.sf_weight + stage * 16, w_done = w_empty + 8 * stage;
+            if (++stage == p.weight_depth) { stage = 0; w_phase ^= 1; }
+            for (uint32_t term = 0; term < g.terms; ++term) {
+                if (!t_seen && !mbar_wait(t_ready + 8 * slot, t_phase, abort_flag, g.status_word, kErrNarrowScales)) {
+                    alive = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint64_t t_desc = t_desc0 + slot * slot_step;
+                const uint32_t sf_t = tmem_base + p.sf_token + slot * 16, t_done = t_empty + 8 * slot;
+                if (++slot == p.token_depth) { slot = 0; t_phase ^= 1; }
+                t_seen = mbar_test(t_ready + 8 * slot, t_phase);
+                if (term + 1 == g.terms) w_seen = mbar_test(w_ready + 8 * stage, w_phase);
+                if (elect_one()) {
+                    if (k_steps == 4) {   // an MMA takes 64 k = 32 bytes of every row: start address + 2
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k) tc_mma(tmem_base, w_desc + 2 * k, t_desc + 2 * k, idesc, sf_w + 4 * k, sf_t + 4 * k, accumulate | k);
+                    } else {
+                        for (uint32_t k = 0; k < k_steps; ++k) tc_mma(tmem_base, w_desc + 2 * k, t_desc + 2 * k, idesc, sf_w + 4 * k, sf_t + 4 * k, accumulate | k);
+                    }
+                    tc_commit(t_done);
+                    if (term + 1 == g.terms) tc_commit(w_done);
+                }
+                __syncwarp();
+                accumulate = 1;
+            }
+        }
+        if (alive && elect_one()) tc_commit(acc_full);
+        __syncwarp();
+    } else if (warp == 3) {
+        // ---------------- scale copies of the activations, shared memory -> tensor memory ----------------
+        // A slot lands after the MMAs that used it last are complete, so its scale columns are free. The copies only have to be
+        // issued before the MMAs that read them: both execute in issue order, and the fences on either side of the arrival
+        // order the two warps' issues. The codes landed on the same barrier, so the MMA warp waits for this arrival only.
+        uint32_t slot = 0, phase = 0;
+        bool alive = true;
+        const uint64_t desc0 = sf_desc(smem_u32(slots) + p.columns * 128);
+        const uint32_t slot_step = p.slot_bytes >> 4;
+        for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
+            const uint32_t k_steps = kb + 1 < k_blocks ? 4u : last_k_steps;
+            for (uint32_t term = 0; term < g.terms; ++term) {
+                if (!mbar_wait(t_full + 8 * slot, phase, abort_flag, g.status_word, kErrNarrowCopy)) {
+                    alive = false;
+                    break;
+                }
+                tc_fence_after();
+                if (elect_one()) {
+                    narrow_copy_scales(tmem_base + p.sf_token + slot * 16, desc0 + slot * slot_step, k_steps);
+                    tc_fence_before();
+                    mbar_arrive(t_ready + 8 * slot);
+                }
+                __syncwarp();
+                if (++slot == p.token_depth) { slot = 0; phase ^= 1; }
+            }
+        }
+    }
+
+    // ---------------- epilogue: tensor memory -> sums of 32 weight rows per lane and token -> global ----------------
+    const bool epilogue = warp >= 4;
+    const uint32_t quadrant = warp & 3, first_chunk = (warp - 4) >> 2;   // tensor-memory lanes 32 * quadrant .. + 31; every other 32 columns
+    const uint32_t row0 = row_tile * kTileM + quadrant * 32;
+    bool complete = true;
+    if (epilogue) {
+        if (!p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing is written while an earlier kernel may still read it
+        complete = mbar_wait(acc_full, 0, abort_flag, g.status_word, kErrNarrowAccFull);
+        tc_fence_after();
+    }
+    __syncwarp();
+    if (p.parts == 1) {
+        if (epilogue && complete) {
+            // all loads have landed and all MMAs have read them: the rings' space turns a chunk so that a lane holds the rows of one token
+            float* turn = reinterpret_cast<float*>(smem) + (warp - 4) * 32 * kNarrowTurnPitch;
+            for (uint32_t column = first_chunk * 32; token_row + column < token_end; column += 64) {
+                uint32_t v[32];
+                tc_load32(tmem_base + ((quadrant * 32) << 16) + column, v);
+                tc_wait_ld();
+#pragma unroll
+                for (uint32_t i = 0; i < 32; ++i) turn[i * kNarrowTurnPitch + lane] = __uint_as_float(v[i]);
+                __syncwarp();
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) {
+                    const uint4 four = *reinterpret_cast<const uint4*>(turn + lane * kNarrowTurnPitch + 4 * i);
+                    v[4 * i] = four.x; v[4 * i + 1] = four.y; v[4 * i + 2] = four.z; v[4 * i + 3] = four.w;
+                }
+                __syncwarp();   // the area is rewritten for the next chunk
+                if (token_row + column + lane < token_end) narrow_store(g, token_row + column + lane, row0, v);
+            }
+        }
+    } else {
+        // every CTA of the cluster owns a share of the columns
+        const uint32_t share = ((p.columns + p.parts - 1) / p.parts + 3) / 4 * 4;
+        narrow_cluster_sync();   // all MMAs of the cluster are complete: the rings may be overwritten
+        if (epilogue && complete) {
+            for (uint32_t column = first_chunk * 32; column < p.columns; column += 64) {
+                uint32_t v[32];
+                tc_load32(tmem_base + ((quadrant * 32) << 16) + column, v);
+                tc_wait_ld();
+                uint32_t owner = column / share, local = column - owner * share;
+#pragma unroll
+                for (uint32_t i = 0; i < 32; i += 4) {   // shares are multiples of 4 columns
+                    if (column + i < p.columns) {
+                        uint32_t to;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                                     : "=r"(to)
+                                     : "r"(smem_u32(smem) + ((part * share + local) / 4 * kNarrowSumPitch + quadrant * 32 + lane) * 16), "r"(owner));
+                        asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"(to), "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3]) : "memory");
+                    }
+                    local += 4;
+                    if (local >= share) { local -= share; ++owner; }
+                }
+            }
+        }
+        __syncwarp();
+        narrow_cluster_sync();   // every partial sum has arrived; nobody writes this CTA's memory from here on
+        if (epilogue && complete) {
+            const float* base = reinterpret_cast<const float*>(smem);
+            for (uint32_t first = first_chunk * 32; first < share; first += 64) {
+                const uint32_t column = first + lane, token = token_row + part * share + column;
+                if (column >= share || token >= token_end) continue;
+                float sum[32];
+#pragma unroll
+                for (uint32_t i = 0; i < 32; ++i) sum[i] = 0.0f;
+                for (uint32_t from = 0; from < p.parts; ++from) {
+                    // [group of four columns][row]{column}: four lanes read neighbouring words, the eight groups of a warp other banks
+                    const float* src = base + ((from * share + column) / 4 * kNarrowSumPitch + quadrant * 32) * 4 + column % 4;
+#pragma unroll
+                    for (uint32_t i = 0; i < 32; ++i) sum[i] += src[4 * i];
+                }
+                uint32_t v[32];
+#pragma unroll
+                for (uint32_t i = 0; i < 32; ++i) v[i] = __float_as_uint(sum[i]);
+                narrow_store(g, token, row0, v);
+            }
+        }
+    }
+    // the successor's wait covers this launch only, so this launch ends after the one before it
+    if (p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kNarrowTmemColumns) : "memory");
+    }
+}
+
+// ---- host side ----------------------------------------------------------------------------------
+// Clusters of `parts` CTAs that the device holds at once (clusters do not fill its SMs evenly: 148 of 2, 93 of 3, 71 of 4,
+// 56 of 5, 45 of 6, 37 of 7, 33 of 8 on a B200). Asked once per device; bind time fills the table. The question is put for
+// a kernel of the same size that uses no tensor memory: for one that does the runtime always answers for one CTA per
+// SM, although two fit when each allocates half of it.
+__global__ void __launch_bounds__(kNarrowThreads, 2) narrow_shape_kernel() {}
+
+struct NarrowDevice {
+    std::atomic<uint32_t> clusters[kNarrowMaxParts + 1];
+};
+NarrowDevice g_narrow_devices[64];
+
+uint32_t narrow_clusters(int32_t ordinal, uint32_t parts) {
+    std::atomic<uint32_t>& known = g_narrow_devices[ordinal & 63].clusters[parts];
+    const uint32_t clusters = known.load();
+    if (clusters) return clusters;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = parts;
+    attribute.val.clusterDim.y = 1;
+    attribute.val.clusterDim.z = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(parts);
+    config.blockDim = dim3(kNarrowThreads);
+    config.dynamicSmemBytes = kNarrowSmem;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    int found = 0;
+    if (cudaOccupancyMaxActiveClusters(&found, narrow_shape_kernel, &config) != cudaSuccess || found < 1) {
+        cudaGetLastError();
+        found = 1;
+    }
+    known.store(static_cast<uint32_t>(found));
+    return static_cast<uint32_t>(found);
+}
+
+// How a launch cuts its work, and about how long it takes: the waves of clusters times the pipeline steps of a part, of the
+// numbers of CTAs per item the one with the least. Measured on a B200 with two CTAs on every SM: a step (k block x term) of a
+// CTA takes 0.33 us at 16 tokens and 0.44 at 128, a launch about 6 us beyond its steps, a wave after the first 3; exchanging
+// the parts' sums takes 4 us more at 128 tokens.
+struct NarrowCut {
+    uint32_t token_tiles, tile_tokens, columns, parts, ns;
+};
+NarrowCut narrow_cut(int32_t ordinal, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
+    NarrowCut cut{};
+    cut.token_tiles = (tokens + kTileM - 1) / kTileM;
+    cut.tile_tokens = tokens < kTileM ? tokens : kTileM;
+    cut.columns = (cut.tile_tokens + 15) / 16 * 16;
+    const uint64_t items = static_cast<uint64_t>(rows / kTileM) * cut.token_tiles;
+    const uint32_t k_blocks = (cols + kNarrowK - 1) / kNarrowK, step_ns = 320 + cut.columns * 120 / kTileM;
+    uint64_t least = ~uint64_t(0);
+    for (uint32_t parts = 1; parts <= kNarrowMaxParts && parts <= k_blocks; ++parts) {
+        const uint32_t clusters = narrow_clusters(ordinal, parts);
+        const uint64_t waves = (items + clusters - 1) / clusters;
+        const uint64_t ns = waves * ((k_blocks + parts - 1) / parts * terms * step_ns + 3000) + 3000 + cut.columns * 4000 / kTileM;
+        if (ns < least) {
+            least = ns;
+            cut.parts = parts;
+        }
+    }
+    cut.ns = static_cast<uint32_t>(least < UINT32_MAX / 2 ? least : UINT32_MAX / 2);
+    return cut;
+}
+}  // namespace
+
+uint32_t gemm_narrow_ns(int32_t ordinal, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
+    return narrow_cut(ordinal, rows, cols, tokens, terms).ns;
+}
+
+augur_cuda_result_v1 launch_gemm_narrow(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan, const CUtensorMap& map_weight,
+                                        uint64_t activation, const GemmParams& g, uint32_t token0, bool after_main) {
+    NarrowParams p{};
+    p.g = g;
+    p.token0 = token0;
+    const NarrowCut cut = narrow_cut(plan->ordinal, g.rows, g.cols, g.tokens - token0, g.terms);
+    p.token_tiles = cut.token_tiles;
+    p.tile_tokens = cut.tile_tokens;
+    p.columns = cut.columns;
+    p.parts = cut.parts;
+    p.after_main = after_main ? 1u : 0u;
+    // Two k blocks of activations ahead, but not at the price of fewer than four weight stages; three slots at least.
+    const uint32_t room = kNarrowSmem - 1024 /*alignment*/ - kNarrowState;
+    p.slot_bytes = p.columns * 128 + kNarrowScales;
+    p.token_depth = 2 * g.terms < 4 ? 4 : 2 * g.terms;
+    while (p.token_depth > 3 && room < p.token_depth * p.slot_bytes + 4 * kNarrowStage) --p.token_depth;
+    p.weight_depth = (room - p.token_depth * p.slot_bytes) / kNarrowStage;
+    p.sf_weight = (p.columns + 31) / 32 * 32;
+    p.sf_token = p.sf_weight + 16 * p.weight_depth;
+    static_assert(128 + 16 * (kNarrowSmem / kNarrowStage) <= kNarrowTmemColumns, "scale columns of all slots fit beside the accumulator");
+    CUtensorMap map_act;
+    if (!make_code_map(&map_act, activation, static_cast<uint64_t>(g.terms) * g.padded_tokens, g.cols, p.columns)) {
+        return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
+    }
+    cudaLaunchAttribute attributes[2]{};
+    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[0].val.programmaticStreamSerializationAllowed = 1;
+    attributes[1].id = cudaLaunchAttributeClusterDimension;
+    attributes[1].val.clusterDim.x = p.parts;
+    attributes[1].val.clusterDim.y = 1;
+    attributes[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t config{};
+    config.stream = s->stream;
+    config.attrs = attributes;
+    config.numAttrs = p.parts > 1 ? 2 : 1;
+    config.gridDim = dim3(g.rows / kTileM * p.token_tiles * p.parts);
+    config.blockDim = dim3(kNarrowThreads);
+    config.dynamicSmemBytes = kNarrowSmem;
+    cudaLaunchKernelEx(&config, gemm_narrow_kernel, map_weight, map_act, p);
+    count_launch();
+    return submitted();
+}
+
+cudaError_t gemm_narrow_configure_device() {
+    cudaError_t e = cudaFuncSetAttribute(gemm_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNarrowSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(narrow_shape_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNarrowSmem);
+    int ordinal = 0;
+    if (e == cudaSuccess) e = cudaGetDevice(&ordinal);
+    if (e != cudaSuccess) return e;
+    for (uint32_t parts = 1; parts <= kNarrowMaxParts; ++parts) narrow_clusters(ordinal, parts);
+    return cudaSuccess;
+}
+
+}  // namespace augur_sm100

@@ -122,6 +122,7 @@ void launch_dependent(cudaStream_t stream, void (*kernel)(Parameters...), uint32
 cudaError_t gemv_configure_device();
 cudaError_t gemm_configure_device();
 cudaError_t gemv_tc_configure_device();
+cudaError_t gemm_narrow_configure_device();
 // Two-CTA clusters of the pair GEMM that the device can hold at once (0 if the query fails).
 uint32_t gemm_pair_resident_clusters();
 

@@ -42,11 +42,27 @@ uint64_t layout_extent(uint32_t layout, uint32_t rows, uint32_t cols) {
 // weight, and 4-byte copies 35 us for the TCGEN05 layout.
 constexpr uint32_t kRepackWarps = 8;
 
-// STREAM / STREAM_PAIR: one warp per destination block (32 rows x 128 k). A lane's 16 destination bytes hold the codes
-// of rows g and g + 8 for four k-steps, byte columns t4 and t4 + 4 of each: the 32 consecutive source bytes of either
-// row, which the four lanes of a quad read together as 16-byte loads (one sector of DRAM each, fetched once), and of
-// which each lane keeps its own byte of every word. All 16 loads of a lane are in flight together; the eight
-// warps of a CTA take neighbouring blocks of one row group, so the rows are read in runs of 512 bytes.
+// Four words of each lane of a quad, word j meant for lane j of it -> one word from each lane, in lane order.
+__device__ __forceinline__ void quad_transpose(uint32_t (&v)[4], uint32_t t4) {
+    const bool high = t4 & 2, odd = t4 & 1;
+    const uint32_t keep0 = high ? v[2] : v[0], keep1 = high ? v[3] : v[1];
+    const uint32_t got0 = __shfl_xor_sync(0xffffffffu, high ? v[0] : v[2], 2), got1 = __shfl_xor_sync(0xffffffffu, high ? v[1] : v[3], 2);
+    // keep: this pair of lanes' own words; got: the other pair's; index = the parity of the lane they are meant for
+    const uint32_t mine = odd ? keep1 : keep0, theirs = odd ? got1 : got0;
+    const uint32_t mine2 = __shfl_xor_sync(0xffffffffu, odd ? keep0 : keep1, 1), theirs2 = __shfl_xor_sync(0xffffffffu, odd ? got0 : got1, 1);
+    const uint32_t own_even = odd ? mine2 : mine, own_odd = odd ? mine : mine2;
+    const uint32_t far_even = odd ? theirs2 : theirs, far_odd = odd ? theirs : theirs2;
+    v[0] = high ? far_even : own_even;
+    v[1] = high ? far_odd : own_odd;
+    v[2] = high ? own_even : far_even;
+    v[3] = high ? own_odd : far_odd;
+}
+
+// STREAM / STREAM_PAIR: one warp per destination block (32 rows x 128 k). A lane reads 16 bytes (two k-steps) of each of
+// four rows, so that a quad reads the 64 bytes of a row and the warp every source byte once; its 16 destination bytes
+// hold byte columns t4 and t4 + 4 of every k-step, which the lanes of a quad exchange after sorting their bytes by column.
+// (Having every lane of a quad read the whole row instead, four times the L1 traffic, took 26.5 us for 17408 x 5120.)
+// The eight warps of a CTA take neighbouring blocks of one row group, so the rows are read in runs of 512 bytes.
 __global__ void __launch_bounds__(kRepackWarps * 32)
 repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restrict__ scales_a, const uint8_t* __restrict__ codes_b,
                      const uint8_t* __restrict__ scales_b, uint8_t* __restrict__ destination, uint32_t blocks, uint32_t cols, bool pair) {
@@ -55,21 +71,13 @@ repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restr
     const uint32_t kb_count = cols / kStreamBlockK;
     const uint32_t group = block / kb_count, kb = block - group * kb_count;
     const uint32_t g = lane >> 2, t4 = lane & 3;
-    const uint8_t* source[2] = {codes_a, pair ? codes_b : codes_a};
-    uint4 top[2][2][2], bottom[2][2][2];   // [tile][quad][half] of rows g and g + 8
+    uint4 piece[2][2];   // [tile][row g, row g + 8]: k-steps 2 t4 and 2 t4 + 1
 #pragma unroll
     for (uint32_t t = 0; t < 2; ++t) {
         const uint32_t row = (pair ? group * 16 : group * 32 + t * 16) + g;
-        const uint4* from = reinterpret_cast<const uint4*>(source[t] + static_cast<uint64_t>(row) * (cols / 2) + kb * 64);
-        const uint4* below = reinterpret_cast<const uint4*>(source[t] + static_cast<uint64_t>(row + 8) * (cols / 2) + kb * 64);
-#pragma unroll
-        for (uint32_t q = 0; q < 2; ++q) {
-#pragma unroll
-            for (uint32_t h = 0; h < 2; ++h) {
-                top[t][q][h] = __ldg(from + q * 2 + h);
-                bottom[t][q][h] = __ldg(below + q * 2 + h);
-            }
-        }
+        const uint8_t* from = ((pair && t) ? codes_b : codes_a) + static_cast<uint64_t>(row) * (cols / 2) + kb * 64 + t4 * 16;
+        piece[t][0] = __ldg(reinterpret_cast<const uint4*>(from));
+        piece[t][1] = __ldg(reinterpret_cast<const uint4*>(from + static_cast<uint64_t>(8) * (cols / 2)));
     }
     // scales: 16 bytes per (tile, g) = k-steps 0..7 of rows g and g + 8, interleaved; lanes 0..15 take one each
     uint2 scale_top = make_uint2(0, 0), scale_bottom = make_uint2(0, 0);
@@ -82,25 +90,37 @@ repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restr
         scale_bottom = make_uint2(__ldg(reinterpret_cast<const uint32_t*>(below)), __ldg(reinterpret_cast<const uint32_t*>(below) + 1));
     }
     uint4* out = reinterpret_cast<uint4*>(destination + static_cast<uint64_t>(block) * kStreamBlockBytes);
-    const uint32_t pick = 0x4440u | t4;    // byte t4 of a word, zero-extended
 #pragma unroll
     for (uint32_t t = 0; t < 2; ++t) {
+        // words[half][lane s of the quad]: of its two k-steps 2s and 2s + 1, this lane's byte columns {t4, t4 + 4} each
+        uint32_t words[2][4];
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+            const uint4 v = piece[t][h];
+            const uint32_t xy01 = __byte_perm(v.x, v.y, 0x5140), xy23 = __byte_perm(v.x, v.y, 0x7362);
+            const uint32_t zw01 = __byte_perm(v.z, v.w, 0x5140), zw23 = __byte_perm(v.z, v.w, 0x7362);
+            words[h][0] = __byte_perm(xy01, zw01, 0x5410);
+            words[h][1] = __byte_perm(xy01, zw01, 0x7632);
+            words[h][2] = __byte_perm(xy23, zw23, 0x5410);
+            words[h][3] = __byte_perm(xy23, zw23, 0x7632);
+            quad_transpose(words[h], t4);
+        }
 #pragma unroll
         for (uint32_t q = 0; q < 2; ++q) {
             uint32_t word[4];
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) {   // k-step 4 q + j: 8 source bytes, words 2 (j % 2) and 2 (j % 2) + 1 of half j / 2
-                const uint4 a = top[t][q][j >> 1], b = bottom[t][q][j >> 1];
-                word[j] = stream_pack_word(__byte_perm((j & 1) ? a.z : a.x, 0, pick), __byte_perm((j & 1) ? b.z : b.x, 0, pick),
-                                           __byte_perm((j & 1) ? a.w : a.y, 0, pick), __byte_perm((j & 1) ? b.w : b.y, 0, pick));
+            for (uint32_t j = 0; j < 4; ++j) {   // k-step 4 q + j, from lane (4 q + j) / 2, the lower or upper half of its word
+                const uint32_t above = words[0][2 * q + (j >> 1)], below = words[1][2 * q + (j >> 1)], at = (j & 1) * 2;
+                word[j] = stream_pack_word(__byte_perm(above, 0, 0x4440u | at), __byte_perm(below, 0, 0x4440u | at),
+                                           __byte_perm(above, 0, 0x4441u + at), __byte_perm(below, 0, 0x4441u + at));
             }
-            __stcs(out + (t * 2 + q) * 32 + lane, make_uint4(word[0], word[1], word[2], word[3]));
+            out[(t * 2 + q) * 32 + lane] = make_uint4(word[0], word[1], word[2], word[3]);
         }
     }
     if (lane < 16) {
-        __stcs(out + kStreamCodeBytes / 16 + lane,
-               make_uint4(__byte_perm(scale_top.x, scale_bottom.x, 0x5140), __byte_perm(scale_top.x, scale_bottom.x, 0x7362),
-                          __byte_perm(scale_top.y, scale_bottom.y, 0x5140), __byte_perm(scale_top.y, scale_bottom.y, 0x7362)));
+        out[kStreamCodeBytes / 16 + lane] =
+            make_uint4(__byte_perm(scale_top.x, scale_bottom.x, 0x5140), __byte_perm(scale_top.x, scale_bottom.x, 0x7362),
+                       __byte_perm(scale_top.y, scale_bottom.y, 0x5140), __byte_perm(scale_top.y, scale_bottom.y, 0x7362));
     }
 }
 
@@ -137,7 +157,7 @@ __device__ __forceinline__ void retile_scales(const uint8_t* __restrict__ scales
     }
     uint4* atom = reinterpret_cast<uint4*>(out + (static_cast<uint64_t>(row_block) * atoms_per_row_block + first) * kSfAtomBytes) + lane;
 #pragma unroll
-    for (uint32_t a = 0; a < kAtoms; ++a) __stcs(atom + a * (kSfAtomBytes / 16), make_uint4(word[0][a], word[1][a], word[2][a], word[3][a]));
+    for (uint32_t a = 0; a < kAtoms; ++a) atom[a * (kSfAtomBytes / 16)] = make_uint4(word[0][a], word[1][a], word[2][a], word[3][a]);
 }
 
 __global__ void __launch_bounds__(kRepackWarps * 32)
@@ -162,7 +182,7 @@ repack_tcgen05_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restri
     }
 #pragma unroll
     for (uint32_t i = 0; i < 4; ++i) {
-        if (first + i * kRepackWarps * 32 < pieces) __stcs(to + first + i * kRepackWarps * 32, v[i]);
+        if (first + i * kRepackWarps * 32 < pieces) to[first + i * kRepackWarps * 32] = v[i];
     }
 }
 
