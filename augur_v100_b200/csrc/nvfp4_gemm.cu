@@ -816,8 +816,6 @@ uint32_t gemm_pair_resident_clusters() {
 }
 
 cudaError_t gemm_configure_device() {
-    const cudaError_t e = gemm_narrow_configure_device();
-    if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
 }
 

@@ -380,7 +380,9 @@ struct NarrowDevice {
 };
 NarrowDevice g_narrow_devices[64];
 
-uint32_t narrow_clusters(int32_t ordinal, uint32_t parts) {
+}  // namespace
+
+uint32_t two_cta_clusters(int32_t ordinal, uint32_t parts) {
     std::atomic<uint32_t>& known = g_narrow_devices[ordinal & 63].clusters[parts];
     const uint32_t clusters = known.load();
     if (clusters) return clusters;
@@ -404,6 +406,7 @@ uint32_t narrow_clusters(int32_t ordinal, uint32_t parts) {
     return static_cast<uint32_t>(found);
 }
 
+namespace {
 // How a launch cuts its work, and about how long it takes: the waves of clusters times the pipeline steps of a part, of the
 // numbers of CTAs per item the one with the least. Measured on a B200 with two CTAs on every SM: a step (k block x term) of a
 // CTA takes 0.33 us at 16 tokens and 0.44 at 128, a launch about 6 us beyond its steps, a wave after the first 3; exchanging
@@ -420,7 +423,7 @@ NarrowCut narrow_cut(int32_t ordinal, uint32_t rows, uint32_t cols, uint32_t tok
     const uint32_t k_blocks = (cols + kNarrowK - 1) / kNarrowK, step_ns = 320 + cut.columns * 120 / kTileM;
     uint64_t least = ~uint64_t(0);
     for (uint32_t parts = 1; parts <= kNarrowMaxParts && parts <= k_blocks; ++parts) {
-        const uint32_t clusters = narrow_clusters(ordinal, parts);
+        const uint32_t clusters = two_cta_clusters(ordinal, parts);
         const uint64_t waves = (items + clusters - 1) / clusters;
         const uint64_t ns = waves * ((k_blocks + parts - 1) / parts * terms * step_ns + 3000) + 3000 + cut.columns * 4000 / kTileM;
         if (ns < least) {
@@ -486,7 +489,7 @@ cudaError_t gemm_narrow_configure_device() {
     int ordinal = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&ordinal);
     if (e != cudaSuccess) return e;
-    for (uint32_t parts = 1; parts <= kNarrowMaxParts; ++parts) narrow_clusters(ordinal, parts);
+    for (uint32_t parts = 1; parts <= kNarrowMaxParts; ++parts) two_cta_clusters(ordinal, parts);
     return cudaSuccess;
 }
 

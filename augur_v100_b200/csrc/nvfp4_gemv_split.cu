@@ -1,0 +1,394 @@
+// Small-token (1..8) NVFP4 linear on tensor memory for sm_100a as two dependent launches.
+//
+//   split    every token row's largest magnitude and its radix-8 digits (nvfp4_digits.cuh), a row slice per CTA;
+//   stream   the weights from HBM to the tensor cores (tcgen05.mma kind::mxf4nvf4, 128 weight rows x 64 columns of
+//            term * 8 + token), one (128-row tile, k range) per CTA, the k ranges of a tile in a cluster.
+//
+// What bounds a linear of a decode step is the chain of things that wait for one another, not its bytes: 10 to 50 MB are 2 to 8
+// us of HBM time. As one launch (the form the MLP block keeps, nvfp4_gemv_tc.cu) every CTA split a share of the activations
+// and all CTAs met before anyone could load them, 6 us in front of the first MMA, and the k parts of a tile met again
+// through global memory. As two launches there is no meeting: the stream kernel becomes resident while the kernel
+// before the split still runs (both starts are programmatic), fills its rings with weights, 21 MB over the GPU, and
+// then waits only for the split, a kernel of two microseconds; the parts of a tile meet in distributed shared memory.
+//
+// Roles, rings and issue as in nvfp4_gemm_narrow.cu: warp 0 weights (TMA, scale copies), 1 MMA, 2 TMA of the activations, 3 their
+// scale copies, 4..11 epilogue. Every wait is bounded; a wait that runs out records a code in the plan's status word, raises a
+// CTA-wide abort flag, and all roles fall through to the common exit.
+#include "nvfp4_digits.cuh"
+#include "nvfp4_gemm.cuh"
+#include "nvfp4_internal.h"
+
+namespace augur_sm100 {
+namespace {
+using namespace tc;
+
+constexpr uint32_t kSplitThreads = 256;
+constexpr uint32_t kSliceGroups = 16;                                  // 16-element groups of a row per split CTA: one pair per warp
+
+constexpr uint32_t kStreamWeightStage = kStageCodeBytes + kStageSfBytes;   // 18 KB
+constexpr uint32_t kStreamActStage = kChunkBytes + kStageSfBytes;          // 10 KB
+constexpr uint32_t kStreamWeightDepth = 4, kStreamActDepth = 3;
+constexpr uint32_t kStreamExchange = 8 * 1024;                         // the cluster's sums of the token rows and weight rows this CTA finishes
+constexpr uint32_t kStreamState = 512;
+constexpr uint32_t kStreamRings = kStreamWeightDepth * kStreamWeightStage + kStreamActDepth * kStreamActStage;
+constexpr uint32_t kStreamSmem = kStreamRings + kStreamExchange + kStreamState + 1024 /*alignment*/;
+constexpr uint32_t kStreamThreads = 32 * 12;
+constexpr uint32_t kStreamTmemColumns = 256;
+constexpr uint32_t kStreamSfWeight = 64, kStreamSfAct = kStreamSfWeight + 16 * kStreamWeightDepth;   // behind the accumulator's 64 columns
+static_assert(kStreamSfAct + 16 * kStreamActDepth <= kStreamTmemColumns, "tensor memory columns");
+static_assert(2 * (kStreamSmem + 1024) <= 228 * 1024, "two CTAs per SM, a kilobyte each reserved by the system");
+constexpr uint32_t kNonFinite = 255;                                   // anchor of a row with an infinity or a NaN
+
+constexpr uint32_t kErrStreamWeights = 0x311, kErrStreamTokens = 0x312, kErrStreamFull = 0x313, kErrStreamScales = 0x314,
+                   kErrStreamCopy = 0x315, kErrStreamAccFull = 0x316;
+
+// ---- split ----------------------------------------------------------------------------------------
+// grid (slices, token rows). Every CTA reads its whole row for the largest magnitude (10 KB from L2 at 5120 columns; sharing the
+// maximum between CTAs would cost a meeting) and splits its slice with the exact anchor.
+__global__ void __launch_bounds__(kSplitThreads)
+split_rows_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ split, uint32_t* __restrict__ anchors, uint32_t cols) {
+    __shared__ uint32_t maxima[kSplitThreads / 32], row_anchor[8];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, token = blockIdx.y, groups = cols / 16;
+    const uint16_t* row = x + static_cast<uint64_t>(token) * cols;
+    const uint32_t group = blockIdx.x * kSliceGroups + warp * 2 + (lane >> 4);
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // x may come from the launch before, and the split may still be read by it
+    const uint32_t bits = group < groups ? __ldcg(row + group * 16 + (lane & 15)) : 0;
+    uint32_t packed = 0;
+    const uint4* vectors = reinterpret_cast<const uint4*>(row);
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < cols / 8; i += kSplitThreads) {
+        const uint4 v = __ldcg(vectors + i);
+        packed = __vmaxu2(packed, __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu)));
+    }
+    // the codes only need the group's own maximum: they are formed and stored while the row is still arriving
+    const SplitTarget to{split, static_cast<uint32_t>(split_code_bytes(cols)), 0, groups, 8};
+    const uint2 where = make_uint2(group < groups ? token : ~0u, group);
+    const uint32_t group_largest = split_codes(to, where, bits, 0, lane);
+    const uint32_t most = __reduce_max_sync(0xffffffffu, max(packed & 0xffffu, packed >> 16));
+    if (lane == 0) maxima[warp] = most;
+    __syncthreads();
+    uint32_t largest = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < kSplitThreads / 32; ++i) largest = max(largest, maxima[i]);
+    // term 0 of the row has the global scale 2^(A - 155), term 7 2^(A - 134): all normal f32 numbers
+    const uint32_t a = min(max(largest >> 7, 40u), 250u);
+    if (threadIdx.x == 0 && blockIdx.x == 0) anchors[token] = largest >= 0x7f80u ? kNonFinite : a;   // the row's outputs are NaN then
+    if (lane == 0) row_anchor[token] = a;   // every warp the same value
+    __syncwarp();
+    split_scales(to, row_anchor, where, bits, group_largest, lane);
+}
+
+// ---- stream ---------------------------------------------------------------------------------------
+struct StreamParams {
+    const uint8_t* weight_sf;     // scale region of the weight
+    const uint8_t* split;         // the split activations
+    const uint32_t* anchors;
+    void* out;
+    uint32_t* status_word;
+    uint32_t out_rows, cols, tokens, epilogue, parts;
+    float global_a, global_b;
+};
+
+__device__ __forceinline__ void copy_scales(uint32_t columns, uint64_t desc, uint32_t k_steps) {
+    if (k_steps == 4) {
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) tc_copy_sf(columns + 4 * k, desc + k * (kSfAtomBytes >> 4));
+    } else {
+        for (uint32_t k = 0; k < k_steps; ++k) tc_copy_sf(columns + 4 * k, desc + k * (kSfAtomBytes >> 4));
+    }
+}
+
+// Four neighbouring columns of this warp's 32 accumulator rows.
+__device__ __forceinline__ void load_columns(uint32_t taddr, uint32_t (&v)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr) : "memory");
+}
+
+// Finished sums of 32 weight rows (lane = row) for the token rows token0 .. token0 + 3.
+__device__ __forceinline__ void store_rows(const StreamParams& p, uint32_t row0, uint32_t token0, uint32_t lane, const float (&y)[4]) {
+    if (p.epilogue == AUGUR_NVFP4_SM100_EPILOGUE_SWIGLU_BF16) {
+        // 32 physical rows = 16 gate rows (lanes 0..15) and the matching 16 up rows (lanes 16..31)
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            const float up = __shfl_sync(0xffffffffu, y[j], (lane & 15) + 16) * p.global_b, gate = y[j] * p.global_a;
+            if (lane < 16 && token0 + j < p.tokens) {
+                static_cast<__nv_bfloat16*>(p.out)[static_cast<uint64_t>(token0 + j) * p.out_rows + row0 / 2 + lane] =
+                    __float2bfloat16_rn(__fdividef(gate, 1.0f + __expf(-gate)) * up);   // a few ulp of f32, far below the rounding
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        if (token0 + j >= p.tokens) continue;
+        const float value = y[j] * p.global_a;
+        const uint64_t at = static_cast<uint64_t>(token0 + j) * p.out_rows + row0 + lane;
+        if (p.epilogue == AUGUR_NVFP4_SM100_EPILOGUE_LINEAR_F32) static_cast<float*>(p.out)[at] = value;
+        else static_cast<__nv_bfloat16*>(p.out)[at] = __float2bfloat16_rn(value);
+    }
+}
+
+__global__ void __launch_bounds__(kStreamThreads, 2)
+split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const StreamParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* slots = smem + kStreamWeightDepth * kStreamWeightStage;
+    float4* exchange = reinterpret_cast<float4*>(smem + kStreamRings);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStreamRings + kStreamExchange);
+    const uint32_t bar0 = smem_u32(bars);
+    // per slot of either ring: landed, free, scales in tensor memory (and with them the codes in shared memory)
+    constexpr uint32_t kBars = 3 * (kStreamWeightDepth + kStreamActDepth) + 1;
+    const uint32_t w_full = bar0, w_empty = w_full + 8 * kStreamWeightDepth, w_ready = w_empty + 8 * kStreamWeightDepth;
+    const uint32_t t_full = w_ready + 8 * kStreamWeightDepth, t_empty = t_full + 8 * kStreamActDepth, t_ready = t_empty + 8 * kStreamActDepth;
+    const uint32_t acc_full = t_ready + 8 * kStreamActDepth;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kBars);
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (threadIdx.x == 0) {
+        for (uint32_t b = 0; b < kBars; ++b) mbar_init(bar0 + 8 * b, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kStreamTmemColumns) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    // first half of a meeting of the cluster: this CTA runs (its shared memory may be written from the second half on)
+    if (p.parts > 1) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+
+    const uint32_t part = blockIdx.x % p.parts, tile = blockIdx.x / p.parts;
+    const uint32_t k_blocks = (p.cols + kStageK - 1) / kStageK, atoms = p.cols / 64;
+    const uint32_t kb0 = part * k_blocks / p.parts, kb1 = (part + 1) * k_blocks / p.parts;
+    const uint32_t last_k_steps = atoms - (k_blocks - 1) * 4;   // 1..4 k steps of 64 in the last k block
+
+    if (warp == 0) {
+        // ---------------- weights: TMA, and scale copies to tensor memory ----------------
+        // They are constant, so nothing is waited for before the ring is filled. From then on the copies of a stage come first and
+        // the load into the stage before it, whose MMAs are the ones under way, second: the copies stay a k block ahead.
+        const uint64_t desc0 = sf_desc(smem_u32(smem) + kStageCodeBytes);
+        const uint8_t* scales = p.weight_sf + static_cast<uint64_t>(tile) * atoms * kSfAtomBytes;
+        uint32_t load_kb = kb0, load_stage = 0, load_phase = 1, stage = 0, phase = 0;
+        auto load = [&]() {
+            if (!mbar_wait(w_empty + 8 * load_stage, load_phase, abort_flag, p.status_word, kErrStreamWeights)) return false;
+            const uint32_t full = w_full + 8 * load_stage, to = smem_u32(smem + load_stage * kStreamWeightStage);
+            const uint32_t sf_bytes = (load_kb + 1 < k_blocks ? 4u : last_k_steps) * kSfAtomBytes;
+            if (elect_one()) {
+                mbar_expect_tx(full, kStageCodeBytes + sf_bytes);
+                tma_load_2d(to, &map_weight, load_kb * 128, tile * kTileM, full);
+                bulk_load(to + kStageCodeBytes, scales + static_cast<uint64_t>(load_kb) * kStageSfBytes, sf_bytes, full);
+            }
+            __syncwarp();
+            ++load_kb;
+            if (++load_stage == kStreamWeightDepth) { load_stage = 0; load_phase ^= 1; }
+            return true;
+        };
+        bool alive = true;
+        while (alive && load_kb < kb1 && load_kb < kb0 + kStreamWeightDepth) alive = load();
+        for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
+            if (!mbar_wait(w_full + 8 * stage, phase, abort_flag, p.status_word, kErrStreamCopy)) break;
+            tc_fence_after();
+            if (elect_one()) {
+                copy_scales(tmem_base + kStreamSfWeight + stage * 16, desc0 + stage * (kStreamWeightStage >> 4), kb + 1 < k_blocks ? 4u : last_k_steps);
+                tc_fence_before();
+                mbar_arrive(w_ready + 8 * stage);
+            }
+            __syncwarp();
+            if (++stage == kStreamWeightDepth) { stage = 0; phase ^= 1; }
+            if (kb != kb0 && load_kb < kb1) alive = load();
+        }
+    } else if (warp == 2) {
+        // ---------------- TMA of activations (the image in memory is the one the ring holds) ----------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const uint8_t* image_sf = p.split + split_code_bytes(p.cols);
+        uint32_t slot = 0, phase = 1;
+        for (uint32_t kb = kb0; kb < kb1; ++kb) {
+            if (!mbar_wait(t_empty + 8 * slot, phase, abort_flag, p.status_word, kErrStreamTokens)) break;
+            const uint32_t to = smem_u32(slots + slot * kStreamActStage), full = t_full + 8 * slot;
+            if (elect_one()) {
+                mbar_expect_tx(full, kStreamActStage);
+                bulk_load(to, p.split + static_cast<uint64_t>(kb) * kChunkBytes, kChunkBytes, full);
+                bulk_load(to + kChunkBytes, image_sf + static_cast<uint64_t>(kb) * kStageSfBytes, kStageSfBytes, full);
+            }
+            __syncwarp();
+            if (++slot == kStreamActDepth) { slot = 0; phase ^= 1; }
+        }
+    } else if (warp == 1) {
+        // ---------------- MMA issuer (the next step's barriers are looked at before this step's MMAs are issued) ----------------
+        uint32_t stage = 0, w_phase = 0, slot = 0, t_phase = 0, accumulate = 0;
+        bool alive = true, w_seen = false, t_seen = false;
+        const uint32_t idesc = instr_desc(kCols);
+        const uint64_t w_desc0 = operand_desc(smem_u32(smem)), t_desc0 = operand_desc(smem_u32(slots));
+        for (uint32_t kb = kb0; kb < kb1; ++kb) {
+            if ((!w_seen && !mbar_wait(w_ready + 8 * stage, w_phase, abort_flag, p.status_word, kErrStreamFull)) ||
+                (!t_seen && !mbar_wait(t_ready + 8 * slot, t_phase, abort_flag, p.status_word, kErrStreamScales))) {
+                alive = false;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t k_steps = kb + 1 < k_blocks ? 4u : last_k_steps;
+            const uint64_t w_desc = w_desc0 + stage * (kStreamWeightStage >> 4), t_desc = t_desc0 + slot * (kStreamActStage >> 4);
+            const uint32_t sf_w = tmem_base + kStreamSfWeight + stage * 16, sf_t = tmem_base + kStreamSfAct + slot * 16;
+            const uint32_t w_done = w_empty + 8 * stage, t_done = t_empty + 8 * slot;
+            if (++stage == kStreamWeightDepth) { stage = 0; w_phase ^= 1; }
+            if (++slot == kStreamActDepth) { slot = 0; t_phase ^= 1; }
+            w_seen = mbar_test(w_ready + 8 * stage, w_phase);
+            t_seen = mbar_test(t_ready + 8 * slot, t_phase);
+            if (elect_one()) {
+                if (k_steps == 4) {   // an MMA takes 64 k = 32 bytes of every row: start address + 2
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k) tc_mma(tmem_base, w_desc + 2 * k, t_desc + 2 * k, idesc, sf_w + 4 * k, sf_t + 4 * k, accumulate | k);
+                } else {
+                    for (uint32_t k = 0; k < k_steps; ++k) tc_mma(tmem_base, w_desc + 2 * k, t_desc + 2 * k, idesc, sf_w + 4 * k, sf_t + 4 * k, accumulate | k);
+                }
+                tc_commit(t_done);
+                tc_commit(w_done);
+            }
+            __syncwarp();
+            accumulate = 1;
+        }
+        if (alive && elect_one()) tc_commit(acc_full);
+        __syncwarp();
+    } else if (warp == 3) {
+        // ---------------- scale copies of the activations ----------------
+        uint32_t slot = 0, phase = 0;
+        const uint64_t desc0 = sf_desc(smem_u32(slots) + kChunkBytes);
+        for (uint32_t kb = kb0; kb < kb1; ++kb) {
+            if (!mbar_wait(t_full + 8 * slot, phase, abort_flag, p.status_word, kErrStreamCopy)) break;
+            tc_fence_after();
+            if (elect_one()) {
+                copy_scales(tmem_base + kStreamSfAct + slot * 16, desc0 + slot * (kStreamActStage >> 4), kb + 1 < k_blocks ? 4u : last_k_steps);
+                tc_fence_before();
+                mbar_arrive(t_ready + 8 * slot);
+            }
+            __syncwarp();
+            if (++slot == kStreamActDepth) { slot = 0; phase ^= 1; }
+        }
+    }
+
+    // ---------------- epilogue: two warps per quarter of the rows, four token rows each ----------------
+    const bool epilogue = warp >= 4;
+    const uint32_t task = warp - 4, quadrant = task & 3, token0 = (task >> 2) * 4;   // quadrant == warp % 4: the tensor-memory lanes it may read
+    float y[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float scale[4];
+    if (epilogue) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // the anchors; and nothing is written while an earlier kernel may still read it
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            const uint32_t a = token0 + j < p.tokens ? __ldcg(p.anchors + token0 + j) : 40u;
+            scale[j] = __uint_as_float(a == kNonFinite ? 0x7fc00000u : (a - 28) << 23);
+        }
+        if (mbar_wait(acc_full, 0, abort_flag, p.status_word, kErrStreamAccFull)) {
+            tc_fence_after();
+            uint32_t v[kTerms][4];
+#pragma unroll
+            for (uint32_t term = 0; term < kTerms; ++term) load_columns(tmem_base + 8 * term + token0 + ((quadrant * 32) << 16), v[term]);
+            tc_wait_ld();
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                // term t carries the factor 8^t relative to term 0
+                float sum = 0.0f, factor = 1.0f;
+#pragma unroll
+                for (uint32_t term = 0; term < kTerms; ++term) {
+                    sum = fmaf(__uint_as_float(v[term][j]), factor, sum);
+                    factor *= 8.0f;
+                }
+                y[j] = sum * scale[j];
+            }
+        }
+    }
+    if (p.parts > 1) {
+        // every (quarter of the rows, half of the token rows) is finished by one CTA of the cluster, adding in CTA order
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");   // second half: the other CTAs run
+        if (epilogue) {
+            const uint32_t owner = task % p.parts;
+            uint32_t to;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_u32(exchange + (task / p.parts * p.parts + part) * 32 + lane)), "r"(owner));
+            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(y[0]), "f"(y[1]), "f"(y[2]), "f"(y[3]) : "memory");
+        }
+        asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+        if (epilogue && task % p.parts == part) {
+            y[0] = y[1] = y[2] = y[3] = 0.0f;
+            for (uint32_t from = 0; from < p.parts; ++from) {
+                const float4 sums = exchange[(task / p.parts * p.parts + from) * 32 + lane];
+                y[0] += sums.x; y[1] += sums.y; y[2] += sums.z; y[3] += sums.w;
+            }
+        }
+    }
+    if (epilogue && (p.parts == 1 || task % p.parts == part) && *abort_flag == 0) store_rows(p, tile * kTileM + quadrant * 32, token0, lane, y);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kStreamTmemColumns) : "memory");
+    }
+}
+
+// CTAs per tile: of the numbers up to the largest portable cluster the one with the least waves of clusters times k blocks of a
+// part, with six k blocks' worth of start and end each.
+uint32_t stream_parts(int32_t ordinal, uint32_t tiles, uint32_t k_blocks) {
+    uint32_t best = 1, least = ~0u;
+    for (uint32_t parts = 1; parts <= 8 && parts <= k_blocks; ++parts) {
+        const uint32_t clusters = two_cta_clusters(ordinal, parts);
+        const uint32_t cost = (tiles + clusters - 1) / clusters * ((k_blocks + parts - 1) / parts + 6);
+        if (cost < least) {
+            least = cost;
+            best = parts;
+        }
+    }
+    return best;
+}
+
+}  // namespace
+
+augur_cuda_result_v1 launch_split_linear(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
+                                         const augur_cuda_nvfp4_sm100_gemv_args_v1* a, uint32_t physical_rows, uint8_t* split) {
+    CUtensorMap map_weight;
+    if (!make_code_map(&map_weight, a->weight, physical_rows, a->cols)) return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
+    uint32_t* anchors = reinterpret_cast<uint32_t*>(plan->scratch + plan->scratch_bytes + kPlanTrailerBytes - kPlanAnchorBytes);
+    cudaLaunchAttribute attributes[2]{};
+    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.stream = s->stream;
+    config.attrs = attributes;
+    config.numAttrs = 1;
+    config.gridDim = dim3((a->cols / 16 + kSliceGroups - 1) / kSliceGroups, a->tokens);
+    config.blockDim = dim3(kSplitThreads);
+    cudaLaunchKernelEx(&config, split_rows_kernel, reinterpret_cast<const uint16_t*>(a->input_bf16), split, anchors, a->cols);
+    count_launch();
+    const augur_cuda_result_v1 result = submitted();
+    if (result.status != AUGUR_CUDA_STATUS_OK) return result;
+    StreamParams p{};
+    p.weight_sf = reinterpret_cast<const uint8_t*>(a->weight) + tcgen05_codes_bytes(physical_rows, a->cols);
+    p.split = split;
+    p.anchors = anchors;
+    p.out = reinterpret_cast<void*>(a->output);
+    p.status_word = plan->status_word;
+    p.out_rows = a->rows; p.cols = a->cols; p.tokens = a->tokens; p.epilogue = a->epilogue;
+    p.global_a = a->global_scale; p.global_b = a->global_scale_b;
+    const uint32_t tiles = physical_rows / kTileM;
+    p.parts = stream_parts(plan->ordinal, tiles, (a->cols + kStageK - 1) / kStageK);
+    attributes[1].id = cudaLaunchAttributeClusterDimension;
+    attributes[1].val.clusterDim.x = p.parts;
+    attributes[1].val.clusterDim.y = 1;
+    attributes[1].val.clusterDim.z = 1;
+    config.numAttrs = p.parts > 1 ? 2 : 1;
+    config.gridDim = dim3(tiles * p.parts);
+    config.blockDim = dim3(kStreamThreads);
+    config.dynamicSmemBytes = kStreamSmem;
+    cudaLaunchKernelEx(&config, split_stream_kernel, map_weight, p);
+    count_launch();
+    return submitted();
+}
+
+cudaError_t gemv_split_configure_device() {
+    return cudaFuncSetAttribute(split_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem);
+}
+
+}  // namespace augur_sm100

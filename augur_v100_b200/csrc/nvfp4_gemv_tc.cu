@@ -17,10 +17,12 @@
 //                the terms of a token with their scales and finish the rows.
 //
 // A launch is a list of steps, each a set of (row tile, k range) items dealt round-robin to the CTAs (two per
-// SM, all resident: two short rings consumed in order lose less to a late stage than one long ring). A linear
-// is one step: whole tiles when there are at least about as many as CTAs, else every tile cut along k into equal
+// SM, all resident: two short rings consumed in order lose less to a late stage than one long ring): whole tiles when
+// there are at least about as many as CTAs, else every tile cut along k into equal
 // parts whose partial sums meet in plan scratch (arrival counter per 32 rows; the last arriver adds the parts in
-// a fixed order and finishes the rows; bit-reproducible). The MLP block is two steps when the
+// a fixed order and finishes the rows; bit-reproducible). (A single linear is a program of one step; it runs as the two
+// launches of nvfp4_gemv_split.cu, which have no meeting: 17408 x 5120 at 8 tokens 14.8 us against 17.3 as a program, 5120 x
+// 5120 9.6 against 12.7.) The MLP block is two steps when the
 // gate|up tiles fit the CTAs: gate|up in whole tiles, then down in k parts. The second product needs every CTA's
 // outputs of the first and their largest magnitudes per token row before it can split them: the CTAs arrive at
 // a counter when their outputs are stored, wait for all, split, arrive at a second counter, and the activation
@@ -43,6 +45,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "nvfp4_digits.cuh"
 #include "nvfp4_internal.h"
 #include "nvfp4_layout.cuh"
 #include "nvfp4_tc.cuh"
@@ -51,12 +54,6 @@ namespace augur_sm100 {
 namespace {
 using namespace tc;
 
-constexpr uint32_t kTerms = 8;                         // radix-8 digits of the activation split
-constexpr uint32_t kCols = 8 * kTerms;                 // MMA n: column = term * 8 + token
-constexpr uint32_t kStageK = 256;                      // k per ring stage = one 128-byte swizzled row of codes
-constexpr uint32_t kStageCodeBytes = kTileM * 128;     // 16 KB of weight codes
-constexpr uint32_t kStageSfBytes = 4 * kSfAtomBytes;   // 2 KB: the 4 scale atoms of a stage (weights; activations alike)
-constexpr uint32_t kChunkBytes = kCols * 128;          // 8 KB: activation codes of one 256-k chunk, 64 rows x 128 bytes
 constexpr uint32_t kStageActCodes = kStageCodeBytes + kStageSfBytes;        // offsets inside a stage
 constexpr uint32_t kStageActSf = kStageActCodes + kChunkBytes;
 constexpr uint32_t kStageBytes = kStageActSf + kStageSfBytes;               // 28 KB
@@ -92,15 +89,8 @@ constexpr uint32_t kHeaderWave = 20;       // [launch parity][wave]{outputs stor
 constexpr uint32_t kHeaderParity = 28;     // launches so far, modulo 2
 // The plan's trailer: [launch parity][wave][CTA] one 64-bit word per CTA with the exponent fields of the largest
 // magnitudes of its outputs, one byte per token row (0: not written yet).
-constexpr uint32_t kMaxCtas = static_cast<uint32_t>(kPlanTrailerBytes / 32);
+constexpr uint32_t kMaxCtas = static_cast<uint32_t>((kPlanTrailerBytes - kPlanAnchorBytes) / 32);
 constexpr uint32_t kHeaderRowMax = 32;     // [job][token] bits of the row's largest magnitude
-
-// The split activations in global memory (plan scratch): the image the ring stages want, chunk by chunk.
-//   [chunk = k / 256][64 rows][128 bytes]   codes, rows already in the 128-byte swizzle of a shared-memory operand tile
-//   [k / 64][512 bytes]                     block-scale atoms (row n at byte (n % 32) * 16 + (n / 32) * 4 + (k / 16) % 4)
-__host__ __device__ constexpr uint64_t split_code_bytes(uint32_t cols) { return static_cast<uint64_t>((cols + kStageK - 1) / kStageK) * kChunkBytes; }
-__host__ __device__ constexpr uint64_t split_sf_bytes(uint32_t cols) { return static_cast<uint64_t>((cols + kStageK - 1) / kStageK) * kStageSfBytes; }
-__host__ __device__ constexpr uint64_t split_bytes(uint32_t cols) { return split_code_bytes(cols) + split_sf_bytes(cols); }
 
 struct TcPhase {
     const uint8_t* weight_sf;     // scale region of the weight
@@ -211,34 +201,13 @@ __device__ __forceinline__ bool grid_meet(const TcParams& p, bool leader, uint32
     return *abort_flag == 0;
 }
 
-// ---- activation split (the four worker warps of every CTA; the grid's worker warps share the groups out) ----
-// One lane per element, sixteen neighbouring lanes per 16-element group; warp w of the grid's W worker warps
-// takes the group pairs w, w + W, ... of a job. With A the exponent field of the largest magnitude of the token
-// row (within the job) and G that of the group's, the group's block scale is 2^q, q = G + 8 - A (the row's
-// largest group gets 2^8; E4M3 holds powers of two down to 2^-9, smaller groups keep 2^-9 and lose low bits),
-// term t has the global scale 2^(A - 155) * 8^t (times the level, half the digit), and the element is the integer I = |x| / 2^(q + A - 156): at
-// most 255 * 2^14 for the group's largest element, exact for every element within 2^-14 of it, rounded to
-// nearest below. I is written in radix 8 with digits -4..3: I plus 4 in every octal place has the digits plus 4
-// as its octal digits (eight of them: 3 * (8^8 - 1) / 7 > 255 * 2^14). Digit t is the code of term t: level
-// |digit| / 2, sign of digit times sign of x; all eight are formed at once in the nibbles of one word. The eight
-// lanes of a half group transpose their words so that lane t holds the eight codes of term t, and store one
-// word each.
+// ---- activation split (the worker warps of every CTA; warp w of the grid's W worker warps takes the group pairs w, w + W, ... of a job) ----
 __device__ __forceinline__ uint32_t load_element(const TcPhase& ph, const TcJob& job, uint32_t tokens, uint32_t index, uint32_t lane) {
     if (index >= tokens * job.groups) return 0;
     const uint32_t token = index / job.groups, group = job.group0 + (index - token * job.groups);
     return __ldcg(ph.x + static_cast<uint64_t>(token) * ph.cols + group * 16 + (lane & 15));
 }
 
-// (Both halves are real functions, not inlined: the code that runs at the boundary between the two products is
-// then the code the launch has already run for its input, and is still in the instruction cache.)
-// First half of a group's split, before the row's anchor is known: the group's largest magnitude (returned), the
-// digits relative to it (`drop` low bits fewer), the codes stored. Whole warps; `index` past the job is inactive.
-struct SplitTarget {
-    uint8_t* split;               // the phase's split activations
-    uint32_t sf_offset;           // of its block-scale atoms
-    uint32_t group0, groups;      // the job's groups of every token row
-    uint32_t tokens;
-};
 __device__ __forceinline__ SplitTarget split_target(const TcParams& p, uint32_t job_index) {
     const TcJob& job = p.job[job_index];
     const TcPhase& ph = p.phase[job.phase];
@@ -250,68 +219,6 @@ __device__ __forceinline__ uint2 group_of(const SplitTarget& to, uint32_t index)
     if (index >= to.tokens * to.groups) return make_uint2(~0u, 0u);
     const uint32_t token = index / to.groups;
     return make_uint2(token, to.group0 + (index - token * to.groups));
-}
-
-__device__ __noinline__ uint32_t split_codes(const SplitTarget to, uint2 where, uint32_t bits, uint32_t drop, uint32_t lane) {
-    const bool active = where.x != ~0u;
-    const uint32_t token = active ? where.x : 0, group = where.y;
-    const uint32_t magnitude = bits & 0x7fffu, negative = (bits >> 15) & 1u;
-    uint32_t largest = max(magnitude, __shfl_xor_sync(0xffffffffu, magnitude, 8));
-    largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, 4));
-    largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, 2));
-    largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, 1));
-    const int g = max(static_cast<int>(largest >> 7), 1);           // a subnormal has the exponent of field 1
-    const uint32_t field = magnitude >> 7;
-    const uint32_t significand = field ? 128u + (magnitude & 127u) : magnitude;
-    // |x| = significand * 2^(max(field, 1) - 134); I = |x| * 2^(156 - q - A) = significand * 2^(field - G + 14) with q = G + 8 - A
-    const int shift = max(static_cast<int>(max(field, 1u)) - g + 14 - static_cast<int>(drop), -16);
-    const uint32_t value = shift >= 0 ? significand << shift : (significand + (1u << (-shift - 1))) >> -shift;
-    // octal digits of I + 44444444 (octal), one per nibble: d = digit + 4 in 0..7
-    uint32_t d = (value + 0x924924u) & 0xffffffu;
-    d = (d & 0x00000fffu) | ((d & 0x00fff000u) << 4);
-    d = (d & 0x003f003fu) | ((d & 0x0fc00fc0u) << 2);
-    d = (d & 0x07070707u) | ((d & 0x38383838u) << 1);
-    // level = |d - 4|: d & 3 where d >= 4, else 4 - d = (~d & 3) + 1; the digit is negative where d < 4
-    const uint32_t upper = (d >> 2) & 0x11111111u, upper_mask = upper * 15u;
-    const uint32_t level = ((d & 0x33333333u) & upper_mask) | (((~d & 0x33333333u) + 0x11111111u) & ~upper_mask);
-    const uint32_t nonzero = (level | (level >> 1) | (level >> 2)) & 0x11111111u;
-    const uint32_t minus = ((upper ^ 0x11111111u) ^ (negative * 0x11111111u)) & nonzero;
-    uint32_t digits = level | (minus << 3);    // code of term t in bits 4t .. 4t + 3
-    // 8 lanes x 8 nibbles, transposed: lane t of the eight ends up with nibble t of all eight, in lane order
-    uint32_t other = __shfl_xor_sync(0xffffffffu, digits, 4);
-    digits = (lane & 4) ? (other >> 16) | (digits & 0xffff0000u) : (digits & 0x0000ffffu) | (other << 16);
-    other = __shfl_xor_sync(0xffffffffu, digits, 2);
-    digits = (lane & 2) ? ((other & 0xff00ff00u) >> 8) | (digits & 0xff00ff00u) : (digits & 0x00ff00ffu) | ((other & 0x00ff00ffu) << 8);
-    other = __shfl_xor_sync(0xffffffffu, digits, 1);
-    digits = (lane & 1) ? ((other & 0xf0f0f0f0u) >> 4) | (digits & 0xf0f0f0f0u) : (digits & 0x0f0f0f0fu) | ((other & 0x0f0f0f0fu) << 4);
-    // lanes t and t + 8 hold the two words of the group's eight bytes in row n = t * 8 + token
-    other = __shfl_xor_sync(0xffffffffu, digits, 8);
-    if (active && (lane & 8) == 0) {
-        const uint32_t n = (lane & 7) * 8 + token, chunk = group >> 4, unit = (group & 15) >> 1, half = group & 1;
-        uint8_t* codes = to.split + static_cast<uint64_t>(chunk) * kChunkBytes + (n >> 3) * 1024 + (n & 7) * 128 + ((unit ^ (n & 7)) << 4);
-        *reinterpret_cast<uint2*>(codes + half * 8) = make_uint2(digits, other);
-    }
-    return largest;
-}
-
-// Second half, with the row's anchor: the group's block scale 2^q, q = G + 8 - A. A group more than 2^17 below its
-// row's largest magnitude keeps 2^-9 and has its codes redone with that many low bits fewer (rare). True if the
-// group is larger than the anchor provides for (an anchor that was guessed).
-__device__ __noinline__ bool split_scales(const SplitTarget to, const uint32_t* anchor, uint2 where, uint32_t bits, uint32_t largest,
-                                          uint32_t lane) {
-    const bool active = where.x != ~0u;
-    const uint32_t token = active ? where.x : 0, group = where.y;
-    const int q = max(static_cast<int>(largest >> 7), 1) + 8 - static_cast<int>(anchor[token]);
-    const uint32_t drop = active && q < -9 ? static_cast<uint32_t>(-9 - q) : 0u;
-    if (__any_sync(0xffffffffu, drop != 0)) split_codes(to, where, bits, drop, lane);
-    if (active && (lane & 8) == 0) {
-        const int clamped = min(max(q, -9), 8);
-        const uint32_t scale_code = clamped >= -6 ? static_cast<uint32_t>(clamped + 7) << 3 : 1u << (clamped + 9);
-        const uint32_t n = (lane & 7) * 8 + token;
-        uint8_t* sf = to.split + to.sf_offset + static_cast<uint64_t>(group >> 2) * kSfAtomBytes + (group & 3);
-        sf[(n & 31) * 16 + (n >> 5) * 4] = static_cast<uint8_t>(scale_code);
-    }
-    return active && q > 8;   // the group is larger than the anchor allows for
 }
 
 // The term scales of a job from the row maxima every CTA has contributed to (workers 0..7, one token row each).
@@ -1147,7 +1054,7 @@ bool weight_map(CUtensorMap* map, uint64_t address, uint64_t rows, uint32_t cols
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// One launch for a linear (`b` null) or the MLP block. Member m uses counter region m and the scratch at offsets[m].
+// The MLP block. Member m uses counter region m and the scratch at offsets[m].
 augur_cuda_result_v1 launch_tc(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
                                const augur_cuda_nvfp4_sm100_gemv_args_v1* a, const augur_cuda_nvfp4_sm100_gemv_args_v1* b,
                                const uint64_t (&offsets)[2]) {
@@ -1162,7 +1069,7 @@ augur_cuda_result_v1 launch_tc(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm1
     p.steps = g.steps;
     for (uint32_t j = 0; j < g.jobs; ++j) p.job[j] = g.job[j];
     for (uint32_t i = 0; i < g.steps; ++i) p.step[i] = g.step[i];
-    for (uint32_t m = 0; m < (b ? 2u : 1u); ++m) {
+    for (uint32_t m = 0; m < 2; ++m) {
         const augur_cuda_nvfp4_sm100_gemv_args_v1* args = members[m];
         const uint32_t physical_rows = physical_rows_of(args);
         if (!weight_map(&maps[m], args->weight, physical_rows, args->cols)) return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
@@ -1177,7 +1084,6 @@ augur_cuda_result_v1 launch_tc(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm1
         ph.contributors = g.contributors[m];
         ph.global_a = args->global_scale; ph.global_b = args->global_scale_b;
     }
-    if (!b) maps[1] = maps[0];
     cudaLaunchAttribute attribute{};
     attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attribute.val.programmaticStreamSerializationAllowed = 1;
@@ -1280,8 +1186,7 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_gemv_tc_b
     if (consume_injected_fault()) return make_result(AUGUR_CUDA_STATUS_DIAGNOSTIC_FAULT_INJECTED);
     const cudaError_t e = cudaSetDevice(d);
     if (e != cudaSuccess) return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE, e);
-    const uint64_t offsets[2] = {kCounterBytes, 0};
-    return launch_tc(s, plan, a, nullptr, offsets);
+    return launch_split_linear(s, plan, a, physical, plan->scratch + kCounterBytes);
 }
 
 // ---- the MLP block as one launch ----------------------------------------------------------------------

@@ -38,8 +38,9 @@ namespace augur_sm100 {
 
 constexpr uint32_t kPlanMagic = 0x4e56'4634u;  // "NVF4"
 constexpr uint64_t kPlanHeaderBytes = 256;     // status word + padding in front of the scratch
-constexpr uint64_t kPlanTrailerBytes = 16384;  // behind the scratch, outside what `scratch_bytes` counts: words that only the
-                                               // tensor-memory small-token kernel writes (one per CTA, four sets)
+constexpr uint64_t kPlanAnchorBytes = 256;     // the trailer's end: the token rows' anchors of a split (nvfp4_gemv_split.cu)
+constexpr uint64_t kPlanTrailerBytes = 16384 + kPlanAnchorBytes;  // behind the scratch, outside what `scratch_bytes` counts: words that only
+                                               // the tensor-memory small-token kernels write (one per CTA, four sets; the anchors)
 
 struct Range {
     uint64_t address, bytes, alignment;
@@ -123,6 +124,12 @@ cudaError_t gemv_configure_device();
 cudaError_t gemm_configure_device();
 cudaError_t gemv_tc_configure_device();
 cudaError_t gemm_narrow_configure_device();
+cudaError_t gemv_split_configure_device();
+// Clusters of `parts` CTAs of 384 threads and 113 KB of shared memory (two per SM) that the device holds at once.
+uint32_t two_cta_clusters(int32_t ordinal, uint32_t parts);
+// A small-token linear on tensor memory as two launches (nvfp4_gemv_split.cu); `split`: split_bytes(cols) of plan scratch.
+augur_cuda_result_v1 launch_split_linear(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
+                                         const augur_cuda_nvfp4_sm100_gemv_args_v1* a, uint32_t physical_rows, uint8_t* split);
 // Two-CTA clusters of the pair GEMM that the device can hold at once (0 if the query fails).
 uint32_t gemm_pair_resident_clusters();
 

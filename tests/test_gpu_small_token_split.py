@@ -1,0 +1,38 @@
+"""GPU parity of the small-token linear on tensor memory at the edges of its two launches: one k step, ragged last k block and row
+slice, every cluster size, more tiles than places on the GPU, rows whose groups are far apart in magnitude, non-finite rows, and
+projections of different shapes in turn on one plan. Bound as elsewhere: helpers.rel_error <= 2e-2 against the fp64 oracle."""
+import numpy as np
+import pytest
+
+import oracle
+from augur_v100_b200 import abi, host, synth
+from helpers import TOLERANCE, bits_from_torch_bf16, rel_error, torch_bf16_from_bits
+from test_gpu_small_token_tc import ctx  # noqa: F401  (the fixture)
+
+pytestmark = pytest.mark.gpu
+
+
+def _bind(ctx, rows, cols, tokens, seed):  # noqa: F811
+    codes, scales, glob = synth.make_weight(seed, 92, "w", rows, cols)
+    x = np.random.default_rng(seed).standard_normal((tokens, cols)).astype(np.float32)
+    x[:, : cols // 4] *= 2.0 ** -19       # groups that keep the smallest block scale and lose low digits, beside full ones
+    x_bits = synth.f32_to_bf16_bits(x)
+    weight = host.Nvfp4Sm100Weight.upload_checkpoint_nvfp4(ctx["stream"], abi.LAYOUT_TCGEN05, rows, cols, codes, scales, glob)
+    projection = host.Nvfp4Sm100TcProjection.bind(ctx["plan"], weight, torch_bf16_from_bits(x_bits, ctx["device"]))
+    return projection, oracle.linear_f64(codes, scales, glob, rows, cols, x_bits, threads=oracle.max_threads())
+
+
+# (128, 64): one MMA; 17408 columns: clusters of 8; 37 and 45 tiles: of 7 and 6; 49920 rows: 390 tiles, more than fit at once
+@pytest.mark.parametrize("rows,cols,tokens", [(128, 64, 1), (128, 17408, 3), (4736, 2112, 8), (5760, 1600, 7), (9088, 1344, 5), (49920, 64, 2), (384, 320, 4)])
+def test_split_linear_edges(ctx, rows, cols, tokens):  # noqa: F811
+    projection, y64 = _bind(ctx, rows, cols, tokens, rows + cols)
+    other, other64 = _bind(ctx, 256, 1024, 8, 5)
+    results = []
+    for _ in range(3):      # the other shape's split overwrites this one's in the plan's scratch in between
+        projection.submit_for_plan()
+        other.submit_for_plan()
+        ctx["stream"].synchronize()
+        results.append(bits_from_torch_bf16(projection.out))
+    assert ctx["plan"].device_status() == 0
+    assert rel_error(results[0], y64) <= TOLERANCE and all(np.array_equal(results[0], again) for again in results[1:])
+    assert rel_error(bits_from_torch_bf16(other.out), other64) <= TOLERANCE
