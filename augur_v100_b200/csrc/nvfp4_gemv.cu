@@ -14,16 +14,21 @@
 // input is staged by each CTA for its own k-slab; an intermediate produced by the SwiGLU
 // epilogue of this kernel is written staged (fixed exponent) and bulk-copied in.
 //
-// Work split (balanced over any grid): the block space of a k-slab is cut into equal
-// contiguous spans, one per CTA, and each CTA's span into equal contiguous spans, one
-// per warp. Row groups that straddle a warp boundary are combined in shared memory in
-// warp order; row groups that straddle a CTA or slab boundary are combined through
-// plan scratch with an arrival counter, the last arriver summing the slots in a fixed
-// order. Nothing spins on another CTA, and the result does not depend on scheduling.
+// Work split: the row groups are dealt out to clusters of 1, 2, 4 or 8 CTAs in equal contiguous ranges, and the CTAs of a
+// cluster take an equal part of k each (their slab); a CTA's blocks are cut into equal contiguous spans, one per warp. Row
+// groups that straddle a warp boundary are combined in shared memory in warp order, the slabs of a group through
+// distributed shared memory in slab order by the CTA of the cluster that owns it: no scratch, no counters. What a cluster
+// buys is small parts: 1024 rows are 32 groups, which as whole groups keep 32 of 148 SMs busy for two and a half blocks per
+// warp, each SM staging all of k; cut in four they keep 128 busy for less than one, staging a quarter.
+// Where that is not possible (more than 8 slabs, more groups per cluster than the exchange area holds, tensor-parallel
+// launches) the block space of a slab is cut into equal spans, one per CTA, and row groups that straddle a CTA or slab
+// boundary are combined through plan scratch with an arrival counter, the last arriver summing the slots in a fixed
+// order. Nothing spins on another CTA of the grid, and the result does not depend on scheduling.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "nvfp4_internal.h"
@@ -42,21 +47,34 @@ constexpr uint32_t kWaitLimit = 1u << 18;   // bounded polls of a ring slot befo
 constexpr uint32_t kMaxSlabBlocks = 40;    // 40 * 128 k = 5120 activations columns per slab (80 KB)
 constexpr uint32_t kSlotFloats = 256;      // one partial tile: 32 lanes x 8 f32
 constexpr uint32_t kCombineBlocks = 48;    // weight blocks a CTA streams in the time of one cross-CTA combine
+constexpr uint32_t kMaxClusterSize = 8;
+constexpr uint32_t kExchangeSlots = 16;    // tiles a CTA of a cluster takes in from the slabs of the groups it finishes
+constexpr uint32_t kMaxGroupMembers = 4;
+
+// One weight matrix of a launch: the row groups [first_group, the next member's) of the launch.
+struct GemvMember {
+    const uint8_t* weight;
+    void* out;
+    uint32_t first_group, rows;
+    uint32_t store_rows;       // rows that are written (the output is [tokens][store_rows]); the rest of the weight rows is padding
+    float global_a;
+    uint32_t epilogue;
+};
 
 struct GemvParams {
-    const uint8_t* weight;
+    GemvMember member[kMaxGroupMembers];   // one for a linear, up to four that read the same staged activations for a norm group
+    uint32_t members;
     const uint16_t* x;
-    void* out;
     float* partials;
     uint32_t* counters;
     uint32_t* status_word;
     const uint8_t* staged;     // activations already staged by the producing launch (fixed exponent), or unused
     float fixed_factor;        // non-zero: input is `staged`, and both rescale factors are this constant
     uint16_t* staged_out;      // SwiGLU epilogue: also write the result as staged fragments (or null)
-    uint32_t groups, kb_count, slabs, ctas_per_slab, max_contrib, unit;
-    uint32_t rows, cols, tokens, epilogue;
-    uint32_t store_rows;       // rows that are written (the output is [tokens][store_rows]); the rest of the weight rows is padding
-    float global_a, global_b;
+    uint32_t groups, kb_count, slabs, ctas_per_slab, max_contrib;
+    uint32_t aligned;          // spans are cut at row-group boundaries; with slabs > 1 these are the CTAs of a cluster
+    uint32_t cols, tokens;
+    float global_b;
     // Tensor-parallel exchange (tp_world == 0: none): every rank's exchange buffer as mapped here.
     uint64_t exchange[AUGUR_NVFP4_SM100_MAX_TP_RANKS];
     uint32_t tp_world, tp_rank;
@@ -65,15 +83,16 @@ struct GemvParams {
 };
 
 struct GemvGeometry {
-    uint32_t groups, kb_count, slabs, ctas_per_slab, max_contrib, unit;
+    uint32_t groups, kb_count, slabs, ctas_per_slab, max_contrib;
+    bool aligned, cluster;
     uint64_t partial_bytes;   // partial-sum slots
     uint64_t staged_bytes;    // staged activations + factors
 };
 
-// Host-side geometry; `sm_count` CTAs at most.
-GemvGeometry geometry(uint32_t rows, uint32_t cols, bool pair, uint32_t sm_count) {
+// The split without clusters; `sm_count` CTAs at most.
+GemvGeometry plain_geometry(uint32_t groups, uint32_t cols, uint32_t sm_count) {
     GemvGeometry g{};
-    g.groups = pair ? rows / 16 : rows / 32;
+    g.groups = groups;
     g.kb_count = cols / kStreamBlockK;
     g.slabs = (g.kb_count + kMaxSlabBlocks - 1) / kMaxSlabBlocks;
     const uint32_t min_kbs = g.kb_count / g.slabs;
@@ -91,14 +110,48 @@ GemvGeometry geometry(uint32_t rows, uint32_t cols, bool pair, uint32_t sm_count
         // imbalance = most - groups / sm_count groups, compared in blocks and scaled by sm_count to stay in integers
         aligned = (most * sm_count - g.groups) * min_kbs <= static_cast<uint64_t>(kCombineBlocks) * sm_count;
     }
-    g.unit = aligned ? min_kbs : 1;
-    const uint64_t least_units = static_cast<uint64_t>(g.groups) * min_kbs / g.unit;
+    g.aligned = aligned;
+    const uint64_t least_units = aligned ? g.groups : static_cast<uint64_t>(g.groups) * min_kbs;
     if (per_slab > least_units) per_slab = least_units;  // every CTA owns at least one unit
     g.ctas_per_slab = static_cast<uint32_t>(per_slab);
     g.max_contrib = g.slabs * ((g.ctas_per_slab + g.groups - 1) / g.groups + 1);
     g.partial_bytes = static_cast<uint64_t>(g.groups) * g.max_contrib * kSlotFloats * 4;
     g.staged_bytes = static_cast<uint64_t>(cols) * 16 + 256;
     return g;
+}
+
+// Clusters of `size` CTAs of this kernel that the device holds at once, one CTA per SM (74 of 2, 33 of 4, 15 of 8 on a
+// B200). Asked once per device, at bind time.
+std::atomic<uint32_t> g_gemv_clusters[64][kMaxClusterSize + 1];
+
+// The split that takes the least time. Measured on a B200: a warp takes 1.1 us per block with all warps of the SM busy; bringing a
+// slab block's activations in costs a CTA 0.018 us where they are staged already and 0.02 us and 0.006 us per token row where
+// the CTA stages them; the exchange within a cluster takes 1.2 us and 0.15 us per row group, the one through scratch 2.6 us.
+// (1024 x 5120 at one token row: 6.8 us in whole groups, 6.2, 5.6 and 5.7 with 2, 4 and 8 CTAs per cluster; 17408 x 5120: 15.6
+// in whole groups, 16.8 in pairs of CTAs, which have the same number of blocks.)
+GemvGeometry geometry(uint32_t groups, uint32_t cols, uint32_t tokens, bool input_is_staged, const augur_cuda_nvfp4_sm100_plan_v1* plan) {
+    const uint32_t kb_count = cols / kStreamBlockK, stage_ns = input_is_staged ? 18 : 20 + 6 * tokens;
+    auto stream_ns = [&](uint64_t blocks, uint32_t kbs) { return (blocks > kWarps ? blocks : kWarps) * 1100 / kWarps + kbs * stage_ns; };
+    GemvGeometry best = plain_geometry(groups, cols, plan->sm_count);
+    const uint32_t plain_kbs = (kb_count + best.slabs - 1) / best.slabs;
+    uint64_t least = best.aligned ? stream_ns(static_cast<uint64_t>((groups + best.ctas_per_slab - 1) / best.ctas_per_slab) * plain_kbs, plain_kbs)
+                                  : stream_ns(static_cast<uint64_t>(groups) * plain_kbs / best.ctas_per_slab + 1, plain_kbs) + 2600;
+    for (uint32_t size = 2; size <= kMaxClusterSize && size <= kb_count; size *= 2) {
+        const uint32_t kbs = (kb_count + size - 1) / size, resident = g_gemv_clusters[plan->ordinal & 63][size].load();
+        if (kbs > kMaxSlabBlocks || resident == 0) continue;
+        const uint32_t clusters = groups < resident ? groups : resident, most = (groups + clusters - 1) / clusters;
+        if ((most + size - 1) / size * size > kExchangeSlots) continue;
+        const uint64_t ns = stream_ns(static_cast<uint64_t>(most) * kbs, kbs) + 1200 + most * 150;
+        if (ns < least) {
+            least = ns;
+            best.slabs = size;
+            best.ctas_per_slab = clusters;
+            best.aligned = best.cluster = true;
+            best.max_contrib = 0;
+            best.partial_bytes = 0;
+        }
+    }
+    return best;
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -247,6 +300,18 @@ __device__ __forceinline__ uint32_t shift_bf16(uint32_t bits, int shift) {
     return (bits & 0x807fu) | (static_cast<uint32_t>(moved > 254 ? 254 : moved) << 7);
 }
 
+// The member that holds a row group, by a chain of selects: a run-time index into kernel parameters would put the table
+// on the stack.
+template <uint32_t kMembers>
+__device__ __forceinline__ GemvMember member_of(const GemvParams& p, uint32_t group) {
+    GemvMember m = p.member[0];
+#pragma unroll
+    for (uint32_t i = 1; i < kMembers; ++i) {
+        if (i < p.members && group >= p.member[i].first_group) m = p.member[i];
+    }
+    return m;
+}
+
 // ---- tensor-parallel exchange ------------------------------------------------------------------
 // Row-parallel down projection over `tp_world` GPUs: every rank holds a k-slice and produces a
 // full-width partial sum; the all-reduce is done inside this kernel instead of by a collective
@@ -307,8 +372,8 @@ __device__ __forceinline__ void exchange_push(const GemvParams& p, uint32_t seq,
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j) {
                 asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};"
-                             ::"l"(dst + j * 16), "r"(__float_as_uint(v[2 * j] * p.global_a)), "r"(seq),
-                               "r"(__float_as_uint(v[2 * j + 1] * p.global_a))
+                             ::"l"(dst + j * 16), "r"(__float_as_uint(v[2 * j] * p.member[0].global_a)), "r"(seq),
+                               "r"(__float_as_uint(v[2 * j + 1] * p.member[0].global_a))
                              : "memory");
             }
         }
@@ -369,55 +434,56 @@ __device__ __forceinline__ void exchange_reduce(const GemvParams& p, uint32_t se
             const uint32_t token = 2 * t4 + (i & 1);
             const uint32_t row = group * 32 + (i >> 2) * 16 + g + ((i >> 1) & 1) * 8;
             if (token < p.tokens) {
-                static_cast<__nv_bfloat16*>(p.out)[static_cast<uint64_t>(token) * p.rows + row] = __float2bfloat16_rn(sum[i]);
+                static_cast<__nv_bfloat16*>(p.member[0].out)[static_cast<uint64_t>(token) * p.member[0].rows + row] = __float2bfloat16_rn(sum[i]);
             }
         }
     }
     if (!__all_sync(0xffffffffu, arrived) && lane == 0) atomicCAS(p.status_word, 0u, 0x203u);   // a tile never arrived
 }
 
+// Finished sums of one lane's elements i (0..3: the first 16 rows of the group, or the gate rows) and i + 4 (the other 16
+// rows, or the up rows): scale, activation, rounding, store.
+template <uint32_t kMembers>
+__device__ __forceinline__ void finish_pair(const GemvParams& p, uint32_t group, uint32_t lane, uint32_t i, float first, float second) {
+    const uint32_t g = lane >> 2, token = 2 * (lane & 3) + (i & 1);
+    if (token >= p.tokens) return;
+    const GemvMember m = member_of<kMembers>(p, group);
+    group -= m.first_group;
+    if (m.epilogue == AUGUR_NVFP4_SM100_EPILOGUE_SWIGLU_BF16) {
+        const uint32_t row = group * 16 + g + (i >> 1) * 8;
+        const float gate = first * m.global_a;
+        const float up = second * p.global_b;
+        const __nv_bfloat16 h = __float2bfloat16_rn(gate / (1.0f + expf(-gate)) * up);
+        static_cast<__nv_bfloat16*>(m.out)[static_cast<uint64_t>(token) * m.rows + row] = h;
+        if (p.staged_out) {
+            // The same value as the next projection's B fragment: k = row, so k-step = group, fragment register i>>1
+            // (rows g / g+8 are k%16 = g / g+8), pair g/2, half g%2; shifted by the fixed staging exponent instead of
+            // a per-token one.
+            const uint32_t word = ((group >> 1) * 32 + token * 4 + (g >> 1)) * 4 + (group & 1) * 2 + (i >> 1);
+            p.staged_out[word * 2 + (g & 1)] = static_cast<uint16_t>(shift_bf16(__bfloat16_as_ushort(h), kFixedStageShift));
+        }
+        return;
+    }
+#pragma unroll
+    for (uint32_t t = 0; t < 2; ++t) {
+        const uint32_t row = group * 32 + t * 16 + g + (i >> 1) * 8;
+        if (row >= m.store_rows) continue;
+        const float value = (t ? second : first) * m.global_a;
+        const uint64_t at = static_cast<uint64_t>(token) * m.store_rows + row;
+        if (m.epilogue == AUGUR_NVFP4_SM100_EPILOGUE_LINEAR_F32) static_cast<float*>(m.out)[at] = value;
+        else static_cast<__nv_bfloat16*>(m.out)[at] = __float2bfloat16_rn(value);
+    }
+}
+
+// The same for a whole tile (8 values per lane).
+template <uint32_t kMembers>
 __device__ __forceinline__ void epilogue(const GemvParams& p, uint32_t seq, uint32_t group, const float (&v)[8], uint32_t lane) {
     if (p.tp_world) {
         exchange_push(p, seq, group, v, lane);   // the sum over ranks is written by exchange_reduce
         return;
     }
-    const uint32_t g = lane >> 2, t4 = lane & 3;
-    if (p.epilogue == AUGUR_NVFP4_SM100_EPILOGUE_SWIGLU_BF16) {
-        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
 #pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-            const uint32_t token = 2 * t4 + (i & 1);
-            const uint32_t row = group * 16 + g + (i >> 1) * 8;
-            if (token < p.tokens) {
-                const float gate = v[i] * p.global_a;
-                const float up = v[4 + i] * p.global_b;
-                const __nv_bfloat16 h = __float2bfloat16_rn(gate / (1.0f + expf(-gate)) * up);
-                out[static_cast<uint64_t>(token) * p.rows + row] = h;
-                if (p.staged_out) {
-                    // The same value as the next projection's B fragment: k = row, so k-step = group,
-                    // fragment register i>>1 (rows g / g+8 are k%16 = g / g+8), pair g/2, half g%2;
-                    // shifted by the fixed staging exponent instead of a per-token one.
-                    const uint32_t word = ((group >> 1) * 32 + token * 4 + (g >> 1)) * 4 + (group & 1) * 2 + (i >> 1);
-                    p.staged_out[word * 2 + (g & 1)] =
-                        static_cast<uint16_t>(shift_bf16(__bfloat16_as_ushort(h), kFixedStageShift));
-                }
-            }
-        }
-        return;
-    }
-#pragma unroll
-    for (uint32_t i = 0; i < 8; ++i) {
-        const uint32_t token = 2 * t4 + (i & 1);
-        const uint32_t row = group * 32 + (i >> 2) * 16 + g + ((i >> 1) & 1) * 8;
-        if (token < p.tokens && row < p.store_rows) {
-            const float value = v[i] * p.global_a;
-            if (p.epilogue == AUGUR_NVFP4_SM100_EPILOGUE_LINEAR_F32) {
-                static_cast<float*>(p.out)[static_cast<uint64_t>(token) * p.store_rows + row] = value;
-            } else {
-                static_cast<__nv_bfloat16*>(p.out)[static_cast<uint64_t>(token) * p.store_rows + row] = __float2bfloat16_rn(value);
-            }
-        }
-    }
+    for (uint32_t i = 0; i < 4; ++i) finish_pair<kMembers>(p, group, lane, i, v[i], v[4 + i]);
 }
 
 // ---- activation staging --------------------------------------------------------------------
@@ -501,12 +567,101 @@ __device__ __forceinline__ void stage_activations(const GemvParams& p, uint32_t 
     }
 }
 
-// One CTA's finished share of row group `group` in k-slab `slab` (whole warp calls this).
+// The same for up to four token rows: a warp takes chunks of 1, 2 or 4 rows at once, as many as there are (17408 x 5120 at one row
+// 15.6 us against 16.6 with the code above; at eight rows, its index arithmetic costs 0.4). The columns of rows that do not
+// exist are left as they are: they only feed outputs that are not stored. The order of the four words is rotated by lane so
+// that the 32 lanes of a store hit 32 (one row: 16) different banks.
+__device__ __forceinline__ void stage_few_rows(const GemvParams& p, uint32_t kbs, uint32_t* act_words,
+                                                  float* amax_scratch, float* factor_out, uint32_t lane, uint32_t warp) {
+    const uint32_t shift = p.tokens > 2 ? 3 : p.tokens > 1 ? 4 : 5;   // lanes per token row, as a power of two
+    const uint32_t token = lane >> shift, mine = lane & ((1u << shift) - 1);
+    const uint32_t chunks = kbs * 16;     // of every token row in the slab
+    const bool live = token < p.tokens;
+    // The slab's columns of every token row were bulk-copied, as they are, to the front of the
+    // activation area ([token][kbs*256 bytes]); each lane takes its chunks into registers, and the
+    // area is rewritten in fragment order once every lane has (the barrier below).
+    const uint4* row = reinterpret_cast<const uint4*>(act_words) + token * chunks;
+    uint4 v[kStageChunks];
+#pragma unroll
+    for (uint32_t j = 0; j < kStageChunks; ++j) {
+        const uint32_t chunk = ((warp + kWarps * j) << shift) + mine;
+        if (((warp + kWarps * j) << shift) >= chunks) break;
+        v[j] = make_uint4(0, 0, 0, 0);
+        if (live && chunk < chunks) v[j] = row[chunk];
+    }
+    // largest magnitude, two BF16 lanes at a time
+    __nv_bfloat162 amax2 = __float2bfloat162_rn(0.0f);
+#pragma unroll
+    for (uint32_t j = 0; j < kStageChunks; ++j) {
+        if (((warp + kWarps * j) << shift) >= chunks) break;
+        const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) amax2 = __hmax2_nan(amax2, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[i])));
+    }
+    float amax = fmaxf(__low2float(amax2), __high2float(amax2));
+    if (!(amax == amax)) amax = __int_as_float(0x7f800000);   // a NaN anywhere: the row is staged unshifted
+#pragma unroll
+    for (uint32_t offset = 1; offset < 32; offset <<= 1) {
+        const float other = __shfl_xor_sync(0xffffffffu, amax, offset);
+        if (offset >> shift == 0) amax = fmaxf(amax, other);
+    }
+    if (mine == 0) amax_scratch[warp * 8 + token] = amax;
+    __syncthreads();
+    float m = 0.0f;
+#pragma unroll
+    for (uint32_t w = 0; w < kWarps; ++w) m = fmaxf(m, amax_scratch[w * 8 + token]);
+    int e = 0;   // zero or non-finite rows are staged unshifted
+    const int field = static_cast<int>((__float_as_uint(m) >> 23) & 0xff);
+    if (m > 0.0f && field != 0xff && field != 0) e = 227 - field;
+    if (warp == 0 && mine == 0) {
+        // partial sums are multiplied by 2^(126 - e), split in two factors that are always finite
+        const int q = 126 - e, q0 = q / 2, q1 = q - q0;
+        factor_out[2 * token] = __uint_as_float(static_cast<uint32_t>(127 + q0) << 23);
+        factor_out[2 * token + 1] = __uint_as_float(static_cast<uint32_t>(127 + q1) << 23);
+    }
+    // x * 2^e as two exact BF16 multiplications by 2^(e/2) and 2^(e - e/2) (e is in [-27, 226]);
+    // the values only move toward the staged row's magnitude, so neither step can overflow.
+    const int e0 = e / 2, e1 = e - e0;
+    const __nv_bfloat162 f0 = __float2bfloat162_rn(__uint_as_float(static_cast<uint32_t>(127 + e0) << 23));
+    const __nv_bfloat162 f1 = __float2bfloat162_rn(__uint_as_float(static_cast<uint32_t>(127 + e1) << 23));
+    const uint32_t turn = shift == 3 ? ((lane >> 2) & 1) | ((lane >> 4) << 1) : (lane >> 2) & 3;
+#pragma unroll
+    for (uint32_t j = 0; j < kStageChunks; ++j) {
+        const uint32_t chunk = ((warp + kWarps * j) << shift) + mine, q = chunk >> 2, cc = chunk & 3;
+        if (((warp + kWarps * j) << shift) >= chunks) break;
+        if (!live || chunk >= chunks) continue;
+        // chunk (q, cc) holds k-step 2q + cc/2, fragment register cc%2; its word i is the pair
+        // k%16 = 8(cc%2) + 2i, +1 and belongs to B-fragment lane token*4 + i
+        uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+        if (turn & 1) { const uint32_t t = w[0]; w[0] = w[1]; w[1] = w[2]; w[2] = w[3]; w[3] = t; }
+        if (turn & 2) { uint32_t t = w[0]; w[0] = w[2]; w[2] = t; t = w[1]; w[1] = w[3]; w[3] = t; }
+        uint32_t* dst = act_words + q * 128 + token * 16 + cc;
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            const uint32_t word = (i + turn) & 3;
+            const __nv_bfloat162 moved = __hmul2(__hmul2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]), f0), f1);
+            dst[word * 4] = *reinterpret_cast<const uint32_t*>(&moved);
+        }
+    }
+}
+
+// One CTA's finished share of row group `group` in k-slab `slab` (whole warp calls this). `first_group`: the first of the
+// CTA's (cluster's) row groups, `exchange`: its exchange area.
+template <uint32_t kMembers>
 __device__ __forceinline__ void contribute(const GemvParams& p, uint32_t seq, uint32_t group, uint32_t slab, uint32_t cta_in_slab,
-                                           const float (&v)[8], uint32_t lane) {
-    // Spans cut at row-group boundaries (one k-slab): the group was finished inside this CTA.
-    if (p.unit != 1) {
-        epilogue(p, seq, group, v, lane);
+                                           uint32_t first_group, uint32_t exchange, const float (&v)[8], uint32_t lane) {
+    if (p.aligned) {
+        // Spans cut at row-group boundaries: the group was finished inside this CTA, or the CTA of the cluster that owns it
+        // takes this slab's share in.
+        if (p.slabs == 1) {
+            epilogue<kMembers>(p, seq, group, v, lane);
+            return;
+        }
+        const uint32_t index = group - first_group, owner = index % p.slabs;
+        uint32_t to;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(exchange + (index - owner + slab) * (kSlotFloats * 4) + lane * 16), "r"(owner));
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + 512), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
         return;
     }
     // How many CTAs hold a share of this group, over all k-slabs, and which of them this one is.
@@ -529,7 +684,7 @@ __device__ __forceinline__ void contribute(const GemvParams& p, uint32_t seq, ui
         }
     }
     if (total == 1) {
-        epilogue(p, seq, group, v, lane);
+        epilogue<kMembers>(p, seq, group, v, lane);
         return;
     }
     float* slots = p.partials + static_cast<uint64_t>(group) * p.max_contrib * kSlotFloats;
@@ -564,12 +719,14 @@ __device__ __forceinline__ void contribute(const GemvParams& p, uint32_t seq, ui
             }
         }
     }
-    epilogue(p, seq, group, sum, lane);
+    epilogue<kMembers>(p, seq, group, sum, lane);
     if (lane == 0) p.counters[group] = 0;  // leave the counter clean for the next launch
 }
 
-// The work of CTA `cta` of the `ctas` that share the linear `p`.
-__device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uint32_t ctas, uint8_t* smem) {
+template <uint32_t kMembers>
+__global__ void __launch_bounds__(kWarps * 32, 1) gemv_kernel(const __grid_constant__ GemvParams p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    const uint32_t cta = blockIdx.x;
     // Let the next kernel in the stream become resident on SMs as this grid drains; every
     // kernel of this library defers its global reads of produced data, and all of its global
     // writes, until its own griddepcontrol.wait.
@@ -577,13 +734,15 @@ __device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uin
     uint4* act = reinterpret_cast<uint4*>(smem);                              // [kbs*4][32] x 16 B
     uint8_t* ring = smem + kMaxSlabBlocks * 4 * 512;                          // [warps][kDepth] x 2304 B
     uint8_t* scale_area = ring + kWarps * kDepth * kStreamBlockBytes;         // [warps] x 1 KB
-    uint64_t* bars = reinterpret_cast<uint64_t*>(scale_area + kWarps * kScaleScratchBytes);   // ring slots, then one for act
+    uint8_t* exchange = scale_area + kWarps * kScaleScratchBytes;              // [kExchangeSlots] x 1 KB
+    uint64_t* bars = reinterpret_cast<uint64_t*>(exchange + kExchangeSlots * kSlotFloats * 4);   // ring slots, then one for act
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t slab = cta / p.ctas_per_slab, cta_in_slab = cta % p.ctas_per_slab;
+    const bool cluster = p.aligned && p.slabs > 1;   // the CTAs of a cluster are neighbours: the slab is the rank
+    const uint32_t slab = cluster ? cta % p.slabs : cta / p.ctas_per_slab, cta_in_slab = cluster ? cta / p.slabs : cta % p.ctas_per_slab;
     const uint32_t kb_lo = slab * p.kb_count / p.slabs;
     const uint32_t kbs = (slab + 1) * p.kb_count / p.slabs - kb_lo;
-    const uint32_t units = p.groups * kbs / p.unit;
-    const uint32_t c0 = cta_in_slab * units / p.ctas_per_slab * p.unit, c1 = (cta_in_slab + 1) * units / p.ctas_per_slab * p.unit;
+    const uint32_t unit = p.aligned ? kbs : 1, units = p.aligned ? p.groups : p.groups * kbs;
+    const uint32_t c0 = cta_in_slab * units / p.ctas_per_slab * unit, c1 = (cta_in_slab + 1) * units / p.ctas_per_slab * unit;
     const uint32_t len = c1 - c0;
     const uint32_t w0 = c0 + warp * len / kWarps, w1 = c0 + (warp + 1) * len / kWarps;
 
@@ -598,7 +757,8 @@ __device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uin
         Cursor c;
         c.group = at / kbs;
         c.kbi = at - c.group * kbs;
-        c.ptr = p.weight + (static_cast<uint64_t>(c.group) * p.kb_count + kb_lo + c.kbi) * kStreamBlockBytes;
+        const GemvMember m = member_of<kMembers>(p, c.group);
+        c.ptr = m.weight + (static_cast<uint64_t>(c.group - m.first_group) * p.kb_count + kb_lo + c.kbi) * kStreamBlockBytes;
         return c;
     };
     auto step = [&](Cursor& c) {
@@ -607,6 +767,10 @@ __device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uin
             c.kbi = 0;
             ++c.group;
             c.ptr += group_skip;
+            if (kMembers > 1) {
+                const GemvMember m = member_of<kMembers>(p, c.group);
+                c.ptr = m.weight + (static_cast<uint64_t>(c.group - m.first_group) * p.kb_count + kb_lo) * kStreamBlockBytes;
+            }
         }
     };
     Cursor fetch = cursor_at(w0);
@@ -618,6 +782,7 @@ __device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uin
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    if (cluster) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");   // this CTA runs: its exchange area may be written
     // Weight copies go out first so that HBM is busy while the activations are staged.
     if (lane == 0) {
         for (uint32_t d = 0; d < kDepth; ++d) {
@@ -631,6 +796,14 @@ __device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uin
     // ---- activations of this k-slab ----
     // Everything above touched only this CTA's shared memory and read-only weights, so it may
     // run while the kernel before this one is still in flight; from here on its output is needed.
+    // A plain input that is not in L2 would queue behind the weight copies that all CTAs have just issued, so its lines are
+    // asked for now, a share by every CTA. (They may be written by the launch before this one; L2 then holds what it writes.)
+    if (p.fixed_factor == 0.0f) {
+        const uint32_t lines = p.tokens * p.cols / 64;   // 128 bytes each
+        for (uint32_t line = cta * (kWarps * 32) + threadIdx.x; line < lines; line += gridDim.x * (kWarps * 32)) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.x + static_cast<uint64_t>(line) * 64));
+        }
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // Tensor-parallel launches that count their sequence on the device read the counter here: the launch
     // before this one is complete, and nobody advances the counter before every CTA of this grid is done.
@@ -677,7 +850,8 @@ __device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uin
         if (!arrived && threadIdx.x == 0) atomicCAS(p.status_word, 0u, 0x202u);   // the activations never arrived
     }
     if (plain) {
-        stage_activations(p, kbs, reinterpret_cast<uint32_t*>(smem), stage_scratch, stage_scratch + kWarps * 8, lane, warp);
+        if (p.tokens > 4) stage_activations(p, kbs, reinterpret_cast<uint32_t*>(smem), stage_scratch, stage_scratch + kWarps * 8, lane, warp);
+        else stage_few_rows(p, kbs, reinterpret_cast<uint32_t*>(smem), stage_scratch, stage_scratch + kWarps * 8, lane, warp);
         __syncthreads();
     }
 
@@ -690,7 +864,9 @@ __device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uin
         __syncthreads();   // the scratch becomes the block-scale area of the streaming loop
     }
     Cursor now = cursor_at(w0);
-    const uint32_t first_group = now.group;
+    const uint32_t first_group = now.group, cta_first_group = c0 / kbs;
+    const uint32_t exchange_area = smem_u32(exchange);
+    if (cluster) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");   // the other CTAs of the cluster run
 
     // ---- stream this warp's span of blocks ----
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -706,7 +882,7 @@ __device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uin
 #pragma unroll
         for (uint32_t i = 0; i < 8; ++i) v[i] = acc[i] * ((i & 1) ? inv1a : inv0a) * ((i & 1) ? inv1b : inv0b);
         if (first_kbi == 0 && last_kbi + 1 == kbs) {
-            contribute(p, seq, group, slab, cta_in_slab, v, lane);
+            contribute<kMembers>(p, seq, group, slab, cta_in_slab, cta_first_group, exchange_area, v, lane);
         } else if (group == first_group) {
 #pragma unroll
             for (uint32_t i = 0; i < 8; ++i) head[i] = v[i];
@@ -756,20 +932,49 @@ __device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uin
     float* warp_partial = reinterpret_cast<float*>(ring);
     constexpr uint32_t kWarpPartialFloats = kDepth * kStreamBlockBytes / 4;   // floats per warp ring
     if (have_head) {
-        float4* dst = reinterpret_cast<float4*>(warp_partial + warp * kWarpPartialFloats) + lane * 2;
+        float4* dst = reinterpret_cast<float4*>(warp_partial + warp * kWarpPartialFloats) + lane;
         dst[0] = make_float4(head[0], head[1], head[2], head[3]);
-        dst[1] = make_float4(head[4], head[5], head[6], head[7]);
+        dst[32] = make_float4(head[4], head[5], head[6], head[7]);
     }
     if (have_tail) {
-        float4* dst = reinterpret_cast<float4*>(warp_partial + warp * kWarpPartialFloats + kSlotFloats) + lane * 2;
+        float4* dst = reinterpret_cast<float4*>(warp_partial + warp * kWarpPartialFloats + kSlotFloats) + lane;
         dst[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-        dst[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+        dst[32] = make_float4(acc[4], acc[5], acc[6], acc[7]);
     }
     __syncthreads();
 
     // ---- combine row groups that were split between warps of this CTA ----
-    if (len != 0) {
-        const uint32_t cta_first_group = c0 / kbs;
+    if (p.aligned && !p.tp_world) {
+        // Two elements of a tile per thread, so that all of the CTA adds: a warp per row group, as below, leaves the other
+        // warps idle and its sums of up to sixteen tiles one behind the other.
+        const uint32_t cta_groups = (c1 - c0) / kbs;
+#pragma unroll 1
+        for (uint32_t at = threadIdx.x; at < cta_groups * 128; at += kWarps * 32) {
+            const uint32_t index = at >> 7, element = at & 127, group = cta_first_group + index;
+            const uint32_t lo = index * kbs;                     // in the CTA's blocks
+            uint32_t w = span_of(lo, len, kWarps);
+            const uint32_t w_hi = span_of(lo + kbs - 1, len, kWarps);
+            if (w == w_hi) continue;                             // one warp had it all
+            float first = 0.0f, second = 0.0f;
+            const float* src = warp_partial + w * kWarpPartialFloats + element;
+#pragma unroll 4
+            for (; w <= w_hi; ++w, src += kWarpPartialFloats) {
+                const uint32_t b0 = w * len / kWarps, b1 = (w + 1) * len / kWarps, slot = b0 >= lo ? 0 : kSlotFloats;   // the span's first row group parks in slot 0
+                const float one = src[slot], other = src[slot + 128];
+                first += b1 != b0 ? one : 0.0f;
+                second += b1 != b0 ? other : 0.0f;
+            }
+            if (!cluster) {
+                finish_pair<kMembers>(p, group, element >> 2, element & 3, first, second);
+                continue;
+            }
+            const uint32_t owner = index % p.slabs;
+            uint32_t to;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(exchange_area + ((index - owner + slab) * kSlotFloats + element) * 4), "r"(owner));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to), "f"(first) : "memory");
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + 512), "f"(second) : "memory");
+        }
+    } else if (len != 0) {
         const uint32_t cta_groups = (c1 - 1) / kbs - cta_first_group + 1;
         for (uint32_t index = warp; index < cta_groups; index += kWarps) {
             const uint32_t group = cta_first_group + index;
@@ -782,16 +987,35 @@ __device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uin
                 const uint32_t b0 = c0 + w * len / kWarps, b1 = c0 + (w + 1) * len / kWarps;
                 if (b1 == b0) continue;
                 const uint32_t slot = (b0 >= group * kbs) ? 0 : 1;   // the span's first row group parks in slot 0
-                const float4* src = reinterpret_cast<const float4*>(warp_partial + w * kWarpPartialFloats + slot * kSlotFloats) + lane * 2;
-                const float4 a = src[0], b = src[1];
+                const float4* src = reinterpret_cast<const float4*>(warp_partial + w * kWarpPartialFloats + slot * kSlotFloats) + lane;
+                const float4 a = src[0], b = src[32];
                 sum[0] += a.x; sum[1] += a.y; sum[2] += a.z; sum[3] += a.w;
                 sum[4] += b.x; sum[5] += b.y; sum[6] += b.z; sum[7] += b.w;
             }
-            contribute(p, seq, group, slab, cta_in_slab, sum, lane);
+            contribute<kMembers>(p, seq, group, slab, cta_in_slab, cta_first_group, exchange_area, sum, lane);
+        }
+    }
+    // ---- the slabs of the row groups that this CTA of the cluster owns ----
+    if (cluster) {
+        asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+        const uint32_t groups = (c1 - c0) / kbs, owned = groups > slab ? (groups - slab + p.slabs - 1) / p.slabs : 0;
+        for (uint32_t at = threadIdx.x; at < owned * 128; at += kWarps * 32) {
+            const uint32_t turn = at >> 7, element = at & 127;
+            const float* tile = reinterpret_cast<const float*>(exchange) + turn * p.slabs * kSlotFloats + element;
+            float first = 0.0f, second = 0.0f;
+#pragma unroll
+            for (uint32_t from = 0; from < kMaxClusterSize; ++from) {
+                if (from < p.slabs) {
+                    first += tile[from * kSlotFloats];
+                    second += tile[from * kSlotFloats + 128];
+                }
+            }
+            finish_pair<kMembers>(p, cta_first_group + turn * p.slabs + slab, element >> 2, element & 3, first, second);
         }
     }
     // ---- tensor-parallel: add the ranks' tiles of the row groups assigned to this warp ----
     if (p.tp_world) {
+        const uint32_t ctas = gridDim.x;
         exchange_reduce(p, seq, warp, lane, cta, ctas);
         if (p.tp_sequence == 0) {
             // the last CTA to get here advances the counter for the next launch and clears the arrivals
@@ -807,35 +1031,9 @@ __device__ __forceinline__ void gemv_body(const GemvParams& p, uint32_t cta, uin
     }
 }
 
-__global__ void __launch_bounds__(kWarps * 32, 1) gemv_kernel(const GemvParams p) {
-    extern __shared__ __align__(128) uint8_t smem[];
-    gemv_body(p, blockIdx.x, gridDim.x, smem);
-}
-
-// Up to four linears that read the same staged activations, as one grid (the grouped projections of a norm
-// group): CTA b works for the member whose CTA range holds b. The members share nothing but the input; each has
-// its own counters and partial-sum slots.
-constexpr uint32_t kMaxGroupMembers = 4;
-struct GemvGroupParams {
-    GemvParams member[kMaxGroupMembers];
-    uint32_t first_cta[kMaxGroupMembers + 1];
-};
-__global__ void __launch_bounds__(kWarps * 32, 1) gemv_group_kernel(const __grid_constant__ GemvGroupParams g) {
-    extern __shared__ __align__(128) uint8_t smem[];
-    // a chain of compile-time indices: a run-time index into kernel parameters would copy them to the stack
-    if (blockIdx.x < g.first_cta[1]) {
-        gemv_body(g.member[0], blockIdx.x, g.first_cta[1], smem);
-    } else if (blockIdx.x < g.first_cta[2]) {
-        gemv_body(g.member[1], blockIdx.x - g.first_cta[1], g.first_cta[2] - g.first_cta[1], smem);
-    } else if (blockIdx.x < g.first_cta[3]) {
-        gemv_body(g.member[2], blockIdx.x - g.first_cta[2], g.first_cta[3] - g.first_cta[2], smem);
-    } else {
-        gemv_body(g.member[3], blockIdx.x - g.first_cta[3], g.first_cta[4] - g.first_cta[3], smem);
-    }
-}
-
 constexpr uint32_t kGemvSmemBytes = kMaxSlabBlocks * 4 * 512 + kWarps * kDepth * kStreamBlockBytes +
-                                    kWarps * kScaleScratchBytes + (kWarps * kDepth + 1) * 8;
+                                    kWarps * kScaleScratchBytes + kExchangeSlots * kSlotFloats * 4 + (kWarps * kDepth + 1) * 8;
+static_assert(kGemvSmemBytes <= 227 * 1024, "shared memory of a CTA");
 
 // ---- validation ---------------------------------------------------------------------------
 bool check_gemv_scalars(const augur_cuda_nvfp4_sm100_gemv_args_v1* a, bool* pair) {
@@ -874,7 +1072,8 @@ bool check_gemv(int32_t d, augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_p
     }
     bool pair = false;
     if (!plan_ok(plan, d, s) || !check_gemv_scalars(a, &pair)) return false;
-    const GemvGeometry g = geometry(a->rows, a->cols, pair, plan->sm_count);
+    // the room that the split without clusters needs, whichever is taken
+    const GemvGeometry g = plain_geometry(pair ? a->rows / 16 : a->rows / 32, a->cols, plan->sm_count);
     if (g.ctas_per_slab == 0 || g.groups > kMaxGroups || partial_offset < kCounterBytes ||
         partial_limit < partial_offset || g.staged_bytes + g.partial_bytes > partial_limit - partial_offset) {
         return false;
@@ -894,63 +1093,70 @@ struct ExchangeTable {
     uint32_t world, rank, sequence;
 };
 
-// `staged_out_offset` (non-zero): the SwiGLU result is also written, staged, at that offset of the plan
-// scratch. `input_is_staged`: the activations were staged there by the producing launch (fixed
+GemvMember make_member(const augur_cuda_nvfp4_sm100_gemv_args_v1* a, uint32_t first_group) {
+    return GemvMember{reinterpret_cast<const uint8_t*>(a->weight), reinterpret_cast<void*>(a->output), first_group, a->rows,
+                      a->stored_rows ? a->stored_rows : a->rows, a->global_scale, a->epilogue};
+}
+
+// What all members of a launch share. `counters`: the arrival counters, `staged` / `partials`: where the staged activations
+// are and where the slots go; `input_is_staged`: the activations were staged there by the producing launch (fixed
 // exponent) and are copied in as they are instead of being staged by the kernel.
-// Kernel parameters of one linear. `sm_share`: the SMs this linear may fill (all of them, or its share of a grouped grid);
-// `counters`: its arrival counters; `staged` / `partials`: where its staged activations are and where its slots go.
-GemvParams make_params(const augur_cuda_nvfp4_sm100_plan_v1* plan, const augur_cuda_nvfp4_sm100_gemv_args_v1* a, uint32_t sm_share,
-                       uint32_t* counters, const uint8_t* staged, float* partials, bool input_is_staged, uint32_t* ctas) {
-    const bool pair = a->epilogue == AUGUR_NVFP4_SM100_EPILOGUE_SWIGLU_BF16;
-    const GemvGeometry g = geometry(a->rows, a->cols, pair, sm_share);
+GemvParams make_params(const augur_cuda_nvfp4_sm100_plan_v1* plan, const augur_cuda_nvfp4_sm100_gemv_args_v1* a, const GemvGeometry& g,
+                       uint32_t* counters, const uint8_t* staged, float* partials, bool input_is_staged) {
     GemvParams p{};
-    p.weight = reinterpret_cast<const uint8_t*>(a->weight);
+    p.member[0] = make_member(a, 0);
+    p.members = 1;
     p.x = reinterpret_cast<const uint16_t*>(a->input_bf16);
-    p.out = reinterpret_cast<void*>(a->output);
     p.counters = counters;
     p.staged = staged;
     p.partials = partials;
-    p.unit = g.unit;
     p.fixed_factor = input_is_staged ? 0x1p31f : 0.0f;      // (2^31)^2 = 2^(126 - kFixedStageShift)
     p.status_word = plan->status_word;
     p.groups = g.groups; p.kb_count = g.kb_count; p.slabs = g.slabs; p.ctas_per_slab = g.ctas_per_slab;
     p.max_contrib = g.max_contrib;
-    p.rows = a->rows; p.cols = a->cols; p.tokens = a->tokens; p.epilogue = a->epilogue;
-    p.store_rows = a->stored_rows ? a->stored_rows : a->rows;
-    p.global_a = a->global_scale; p.global_b = a->global_scale_b;
-    *ctas = g.slabs * g.ctas_per_slab;
+    p.aligned = g.aligned ? 1u : 0u;
+    p.cols = a->cols; p.tokens = a->tokens;
+    p.global_b = a->global_scale_b;
     return p;
 }
 
+// Launched with programmatic stream serialisation: the grid may become resident while its predecessor drains, and waits for
+// it in-kernel (griddepcontrol.wait).
+template <uint32_t kMembers>
+void launch_params(augur_cuda_stream_t s, const GemvGeometry& g, const GemvParams& p) {
+    cudaLaunchAttribute attributes[2]{};
+    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[0].val.programmaticStreamSerializationAllowed = 1;
+    attributes[1].id = cudaLaunchAttributeClusterDimension;
+    attributes[1].val.clusterDim.x = g.slabs;
+    attributes[1].val.clusterDim.y = 1;
+    attributes[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t config{};
+    config.stream = s->stream;
+    config.attrs = attributes;
+    config.numAttrs = g.cluster ? 2 : 1;
+    config.gridDim = dim3(g.slabs * g.ctas_per_slab);
+    config.blockDim = dim3(kWarps * 32);
+    config.dynamicSmemBytes = kGemvSmemBytes;
+    cudaLaunchKernelEx(&config, gemv_kernel<kMembers>, p);
+    count_launch();
+}
+
+// `staged_out_offset` (non-zero): the SwiGLU result is also written, staged, at that offset of the plan scratch.
 void launch_gemv(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
                  const augur_cuda_nvfp4_sm100_gemv_args_v1* a, uint32_t member, uint64_t partial_offset,
                  uint64_t staged_out_offset = 0, bool input_is_staged = false, const ExchangeTable* tp = nullptr) {
-    const bool pair = a->epilogue == AUGUR_NVFP4_SM100_EPILOGUE_SWIGLU_BF16;
-    const GemvGeometry g = geometry(a->rows, a->cols, pair, plan->sm_count);
-    uint32_t ctas = 0;
-    GemvParams p = make_params(plan, a, plan->sm_count, reinterpret_cast<uint32_t*>(plan->scratch + member * kCounterRegionBytes),
-                               plan->scratch + partial_offset, reinterpret_cast<float*>(plan->scratch + partial_offset + g.staged_bytes),
-                               input_is_staged, &ctas);
+    const uint32_t groups = a->epilogue == AUGUR_NVFP4_SM100_EPILOGUE_SWIGLU_BF16 ? a->rows / 16 : a->rows / 32;
+    const GemvGeometry g = tp ? plain_geometry(groups, a->cols, plan->sm_count) : geometry(groups, a->cols, a->tokens, input_is_staged, plan);
+    GemvParams p = make_params(plan, a, g, reinterpret_cast<uint32_t*>(plan->scratch + member * kCounterRegionBytes), plan->scratch + partial_offset,
+                               reinterpret_cast<float*>(plan->scratch + partial_offset + g.staged_bytes), input_is_staged);
     p.staged_out = staged_out_offset ? reinterpret_cast<uint16_t*>(plan->scratch + staged_out_offset) : nullptr;
     if (tp) {
         for (uint32_t r = 0; r < tp->world; ++r) p.exchange[r] = tp->exchange[r];
         p.tp_world = tp->world; p.tp_rank = tp->rank; p.tp_sequence = tp->sequence;
         p.tp_counter = reinterpret_cast<uint32_t*>(tp->exchange[tp->rank] + exchange_tiles_bytes(tp->world, a->rows / 32));
     }
-    // Launched with programmatic stream serialisation: the grid may become resident while its
-    // predecessor drains, and waits for it in-kernel (griddepcontrol.wait).
-    cudaLaunchAttribute attribute{};
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t config{};
-    config.stream = s->stream;
-    config.attrs = &attribute;
-    config.numAttrs = 1;
-    config.gridDim = dim3(g.slabs * g.ctas_per_slab);
-    config.blockDim = dim3(kWarps * 32);
-    config.dynamicSmemBytes = kGemvSmemBytes;
-    cudaLaunchKernelEx(&config, gemv_kernel, p);
-    count_launch();
+    launch_params<1>(s, g, p);
 }
 
 }  // namespace
@@ -958,9 +1164,31 @@ void launch_gemv(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* pl
 // Called once per device from plan creation (a bind-time call): raises the kernels'
 // dynamic shared-memory limit.
 cudaError_t gemv_configure_device() {
-    const cudaError_t e = cudaFuncSetAttribute(gemv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemBytes);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(gemv_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(gemv_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemv_kernel<kMaxGroupMembers>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmemBytes);
+    int ordinal = 0;
+    if (e == cudaSuccess) e = cudaGetDevice(&ordinal);
+    for (uint32_t size = 2; e == cudaSuccess && size <= kMaxClusterSize; size *= 2) {
+        if (g_gemv_clusters[ordinal & 63][size].load()) continue;
+        cudaLaunchAttribute attribute{};
+        attribute.id = cudaLaunchAttributeClusterDimension;
+        attribute.val.clusterDim.x = size;
+        attribute.val.clusterDim.y = 1;
+        attribute.val.clusterDim.z = 1;
+        cudaLaunchConfig_t config{};
+        config.gridDim = dim3(size);
+        config.blockDim = dim3(kWarps * 32);
+        config.dynamicSmemBytes = kGemvSmemBytes;
+        config.attrs = &attribute;
+        config.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, gemv_kernel<1>, &config) != cudaSuccess) {
+            cudaGetLastError();   // this size is not used then
+            clusters = 0;
+        }
+        g_gemv_clusters[ordinal & 63][size].store(static_cast<uint32_t>(clusters));
+    }
+    return e;
 }
 
 }  // namespace augur_sm100
@@ -978,7 +1206,7 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_gemv_scra
     for (uint32_t pair = 0; pair < 2; ++pair) {
         if (!pair && rows % 32 != 0) continue;
         for (uint32_t sms = 1; sms <= 512; ++sms) {
-            const GemvGeometry g = geometry(rows, cols, pair != 0, sms);
+            const GemvGeometry g = plain_geometry(pair ? rows / 16 : rows / 32, cols, sms);
             if (g.staged_bytes + g.partial_bytes > worst) worst = g.staged_bytes + g.partial_bytes;
         }
     }
@@ -1079,7 +1307,7 @@ static_assert(sizeof(augur_cuda_nvfp4_sm100_mlp_tp_args_v1) == 272, "mlp_tp ABI"
 bool exchange_table_ok(const augur_cuda_nvfp4_sm100_plan_v1* plan, const augur_cuda_nvfp4_sm100_gemv_args_v1& m,
                        const uint64_t (&exchange)[AUGUR_NVFP4_SM100_MAX_TP_RANKS], uint64_t exchange_len_bytes, uint32_t world) {
     if (exchange_len_bytes < exchange_extent(world, m.rows / 32)) return false;
-    const GemvGeometry g = geometry(m.rows, m.cols, false, plan->sm_count);
+    const GemvGeometry g = plain_geometry(m.rows / 32, m.cols, plan->sm_count);
     if (g.slabs * g.ctas_per_slab > plan->sm_count) return false;
     for (uint32_t r = 0; r < AUGUR_NVFP4_SM100_MAX_TP_RANKS; ++r) {
         if (r >= world) {
@@ -1219,9 +1447,15 @@ namespace {
 static_assert(sizeof(augur_cuda_nvfp4_sm100_norm_group_args_v1) == 472, "norm_group ABI");
 
 constexpr uint32_t kNormThreads = 256;
+constexpr uint32_t kNormShares = 4;         // CTAs per token row
 constexpr uint32_t kNormHeld = 24;       // columns of a row that one thread keeps in registers (rows up to 6144 wide)
 
-// One CTA per token row. The arithmetic order is the reference kernel's, so that the F32 output is
+// kNormShares CTAs per token row: each forms the whole row's sum (the same operations, so the same scale) and writes its share of
+// the columns. What the stage costs is latency, not bytes (one CTA per row took 7 us between two launches, 4 of them
+// waiting for a row that was not in L2 behind the weight copies the next launch had already issued and 2 writing three
+// outputs): so the lines are asked for before the wait, all of a thread's loads are in flight at once, the fold has
+// one barrier and the writing is spread over more SMs.
+// The arithmetic order is the reference kernel's, so that the F32 output is
 // reproducible on a CPU: lane l accumulates value * value over columns l, l + 256, ... (multiply and
 // add, never fused), the 256 partial sums are folded by halving strides, y = (value * scale) * weight.
 // scale = 1 / sqrt(mean + epsilon) with correctly rounded operations (the reference's rsqrtf is a
@@ -1232,14 +1466,21 @@ __global__ void __launch_bounds__(kNormThreads) norm_stage_kernel(const float* _
                                                                    uint16_t* __restrict__ fragments, uint32_t cols, float epsilon,
                                                                    uint32_t residual) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");   // the inputs may come from the launch before this one
     __shared__ float partial[kNormThreads];
-    const uint32_t lane = threadIdx.x;
+    const uint32_t lane = threadIdx.x, share = blockIdx.y;
     const uint64_t base = static_cast<uint64_t>(blockIdx.x) * cols;
-    // A row of up to 256 * kNormHeld columns is held in registers: all of a thread's loads are in flight at once
-    // (each is a round trip to L2), and the second pass reads nothing but the weights, which are fetched with them.
+    for (uint32_t line = share * kNormThreads + lane; line < cols / 32; line += kNormShares * kNormThreads) {   // 128 bytes each
+        asm volatile("prefetch.global.L2 [%0];" ::"l"((residual ? add_a : input) + base + line * 32));
+        if (residual) asm volatile("prefetch.global.L2 [%0];" ::"l"(add_b + base + line * 32));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(weight + line * 32));
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // the inputs may come from the launch before this one
+    // A row of up to 256 * kNormHeld columns is held in registers: the second pass reads nothing again.
     // The arithmetic and its order are the same on both paths.
     const bool held_row = cols <= kNormThreads * kNormHeld;
+    auto load = [&](uint32_t col) {
+        return residual ? __fadd_rn(__ldcg(add_a + base + col), __ldcg(add_b + base + col)) : __ldcg(input + base + col);
+    };
     float held[kNormHeld], gain[kNormHeld];
     float sum = 0.0f;
     if (held_row) {
@@ -1251,40 +1492,39 @@ __global__ void __launch_bounds__(kNormThreads) norm_stage_kernel(const float* _
             if (col < cols) {
                 held[i] = residual ? __ldcg(add_a + base + col) : __ldcg(input + base + col);
                 if (residual) other[i] = __ldcg(add_b + base + col);
-                gain[i] = __ldg(weight + col);
+                if (i % kNormShares == share) gain[i] = __ldg(weight + col);
             }
         }
 #pragma unroll
         for (uint32_t i = 0; i < kNormHeld; ++i) {
-            const uint32_t col = lane + i * kNormThreads;
-            if (col < cols) {
-                if (residual) {
-                    held[i] = __fadd_rn(held[i], other[i]);
-                    input[base + col] = held[i];
-                }
+            if (lane + i * kNormThreads < cols) {
+                if (residual) held[i] = __fadd_rn(held[i], other[i]);
                 sum = __fadd_rn(sum, __fmul_rn(held[i], held[i]));
             }
         }
     } else {
         for (uint32_t col = lane; col < cols; col += kNormThreads) {
-            float value;
-            if (residual) {
-                value = __fadd_rn(__ldcg(add_a + base + col), __ldcg(add_b + base + col));
-                input[base + col] = value;
-            } else {
-                value = __ldcg(input + base + col);
-            }
+            const float value = load(col);
             sum = __fadd_rn(sum, __fmul_rn(value, value));
         }
     }
     partial[lane] = sum;
     __syncthreads();
-    for (uint32_t stride = kNormThreads / 2; stride != 0; stride >>= 1) {
-        if (lane < stride) partial[lane] = __fadd_rn(partial[lane], partial[lane + stride]);
-        __syncthreads();
+    // strides 128, 64 and 32 on eight values of a lane, the rest by shuffles; every warp for itself
+    float fold[8];
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) fold[j] = partial[(lane & 31) + 32 * j];
+#pragma unroll
+    for (uint32_t stride = 4; stride != 0; stride >>= 1) {
+#pragma unroll
+        for (uint32_t j = 0; j < stride; ++j) fold[j] = __fadd_rn(fold[j], fold[j + stride]);
     }
-    const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(partial[0], static_cast<float>(cols)), epsilon)));
+#pragma unroll
+    for (uint32_t stride = 16; stride != 0; stride >>= 1) fold[0] = __fadd_rn(fold[0], __shfl_down_sync(0xffffffffu, fold[0], stride));
+    const float total = __shfl_sync(0xffffffffu, fold[0], 0);
+    const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(cols)), epsilon)));
     auto emit = [&](uint32_t col, float value, float w) {
+        if (residual) input[base + col] = value;
         const float y = __fmul_rn(__fmul_rn(value, scale), w);
         output[base + col] = y;
         const __nv_bfloat16 rounded = __float2bfloat16_rn(y);
@@ -1300,48 +1540,22 @@ __global__ void __launch_bounds__(kNormThreads) norm_stage_kernel(const float* _
 #pragma unroll
         for (uint32_t i = 0; i < kNormHeld; ++i) {
             const uint32_t col = lane + i * kNormThreads;
-            if (col < cols) emit(col, held[i], gain[i]);
+            if (i % kNormShares == share && col < cols) emit(col, held[i], gain[i]);
         }
     } else {
-        // this thread wrote input[base + col] itself when there is a residual
-        for (uint32_t col = lane; col < cols; col += kNormThreads) emit(col, input[base + col], __ldg(weight + col));
+        for (uint32_t col = lane + share * kNormThreads; col < cols; col += kNormShares * kNormThreads) emit(col, load(col), __ldg(weight + col));
     }
 }
 
-// The members of a norm group run as ONE grid: the SMs are dealt out in proportion to the members' weight rows
-// (every member at least one), the staged activations sit once behind the counter regions, the members'
-// partial-sum slots follow side by side, and members 0/1 and 2/3 share a counter region by halves.
-struct GroupLayout {
-    uint32_t share[kMaxGroupMembers];
-    uint64_t staged_offset, partial_offset[kMaxGroupMembers], end;
-};
-GroupLayout group_layout(const augur_cuda_nvfp4_sm100_plan_v1* plan, const augur_cuda_nvfp4_sm100_norm_group_args_v1* a) {
-    GroupLayout layout{};
-    uint64_t total_rows = 0;
-    for (uint32_t i = 0; i < a->count; ++i) total_rows += a->projections[i].rows;
-    uint32_t dealt = 0;
-    for (uint32_t i = 0; i < a->count; ++i) {
-        const uint64_t fair = static_cast<uint64_t>(plan->sm_count) * a->projections[i].rows / (total_rows ? total_rows : 1);
-        layout.share[i] = fair ? static_cast<uint32_t>(fair) : 1;
-        dealt += layout.share[i];
-    }
-    // what rounding down left over goes to the largest member; what the minimum of one took too much comes off it
-    uint32_t largest = 0;
-    for (uint32_t i = 1; i < a->count; ++i) {
-        if (a->projections[i].rows > a->projections[largest].rows) largest = i;
-    }
-    if (dealt < plan->sm_count) layout.share[largest] += plan->sm_count - dealt;
-    if (dealt > plan->sm_count && layout.share[largest] > dealt - plan->sm_count) layout.share[largest] -= dealt - plan->sm_count;
-    layout.staged_offset = kCounterBytes;
-    uint64_t at = kCounterBytes + (static_cast<uint64_t>(a->cols) * 16 + 255) / 256 * 256;
-    for (uint32_t i = 0; i < a->count; ++i) {
-        layout.partial_offset[i] = at;
-        const GemvGeometry g = geometry(a->projections[i].rows, a->projections[i].cols, false, layout.share[i]);
-        at += (g.partial_bytes + 255) / 256 * 256;
-    }
-    layout.end = at;
-    return layout;
+// The members of a norm group run as ONE launch over the union of their row groups: the staged activations sit behind the
+// counter regions (which lie side by side and hold the counters of all groups), the partial-sum slots, where the split needs
+// any, behind them.
+uint32_t group_row_groups(const augur_cuda_nvfp4_sm100_norm_group_args_v1* a) {
+    uint32_t groups = 0;
+    for (uint32_t i = 0; i < a->count; ++i) groups += a->projections[i].rows / 32;
+    return groups;
 }
+uint64_t group_partial_offset(uint32_t cols) { return kCounterBytes + (static_cast<uint64_t>(cols) * 16 + 255) / 256 * 256; }
 
 bool check_norm_group(int32_t d, augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
                       const augur_cuda_nvfp4_sm100_norm_group_args_v1* a, bool full, augur_cuda_result_v1* failure) {
@@ -1391,7 +1605,7 @@ bool check_norm_group(int32_t d, augur_cuda_stream_t s, const augur_cuda_nvfp4_s
         *failure = invalid();
         if (m.epilogue == AUGUR_NVFP4_SM100_EPILOGUE_SWIGLU_BF16 || m.input_bf16 != a->staged_bf16 ||
             m.input_len_bytes != a->staged_len_bytes || m.tokens != a->tokens || m.cols != a->cols ||
-            m.rows / 32 > kMaxGroups / 2) {   // two members share a counter region
+            m.rows / 32 > kMaxGroups / 2) {   // the counters of four members fit the two regions
             return false;
         }
         r[n++] = {m.weight, m.weight_len_bytes, 256};
@@ -1399,9 +1613,8 @@ bool check_norm_group(int32_t d, augur_cuda_stream_t s, const augur_cuda_nvfp4_s
     }
     r[n++] = plan_scratch_range(plan);
     if (!all_disjoint(r, n)) return false;
-    // the grouped grid: staged activations once, then every member's slots side by side
-    const GroupLayout layout = group_layout(plan, a);
-    if (layout.end > plan->scratch_bytes) return false;
+    // staged activations once, then the slots of the split without clusters over all members
+    if (group_partial_offset(a->cols) + plain_geometry(group_row_groups(a), a->cols, plan->sm_count).partial_bytes > plan->scratch_bytes) return false;
     return !full || inspect_device_ranges(d, r, n - 1, failure);
 }
 }  // namespace
@@ -1429,35 +1642,25 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_norm_grou
     config.stream = s->stream;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    config.gridDim = dim3(a->tokens);
+    config.gridDim = dim3(a->tokens, kNormShares);
     config.blockDim = dim3(kNormThreads);
-    const GroupLayout layout = group_layout(plan, a);
+    uint8_t* fragments = plan->scratch + kCounterBytes;
     cudaLaunchKernelEx(&config, norm_stage_kernel, reinterpret_cast<const float*>(a->add_a), reinterpret_cast<const float*>(a->add_b),
                        reinterpret_cast<float*>(a->input_f32), reinterpret_cast<const float*>(a->weight_f32),
                        reinterpret_cast<float*>(a->output_f32), reinterpret_cast<__nv_bfloat16*>(a->staged_bf16),
-                       reinterpret_cast<uint16_t*>(plan->scratch + layout.staged_offset), a->cols, a->epsilon, a->residual);
+                       reinterpret_cast<uint16_t*>(fragments), a->cols, a->epsilon, a->residual);
     count_launch();
     augur_cuda_result_v1 result = submitted();
     if (result.status != AUGUR_CUDA_STATUS_OK) return result;
     // all projections of the group in one grid; they copy the staged fragments in and stage nothing themselves
-    GemvGroupParams group{};
-    uint32_t next = 0;
-    for (uint32_t i = 0; i < kMaxGroupMembers; ++i) {
-        group.first_cta[i] = next;
-        if (i >= a->count) continue;
-        uint32_t ctas = 0;
-        uint32_t* counters = reinterpret_cast<uint32_t*>(plan->scratch + (i / 2) * kCounterRegionBytes + (i % 2) * (kCounterRegionBytes / 2));
-        group.member[i] = make_params(plan, &a->projections[i], layout.share[i], counters, plan->scratch + layout.staged_offset,
-                                      reinterpret_cast<float*>(plan->scratch + layout.partial_offset[i]), true, &ctas);
-        next += ctas;
+    const GemvGeometry g = geometry(group_row_groups(a), a->cols, a->tokens, true, plan);
+    GemvParams p = make_params(plan, &a->projections[0], g, reinterpret_cast<uint32_t*>(plan->scratch), fragments,
+                               reinterpret_cast<float*>(plan->scratch + group_partial_offset(a->cols)), true);
+    for (uint32_t i = 1; i < a->count; ++i) {
+        p.member[i] = make_member(&a->projections[i], p.member[i - 1].first_group + p.member[i - 1].rows / 32);
     }
-    group.first_cta[kMaxGroupMembers] = next;
-    for (uint32_t i = a->count; i < kMaxGroupMembers; ++i) group.first_cta[i] = next;   // members that do not exist own no CTA
-    config.gridDim = dim3(next);
-    config.blockDim = dim3(kWarps * 32);
-    config.dynamicSmemBytes = kGemvSmemBytes;
-    cudaLaunchKernelEx(&config, gemv_group_kernel, group);
-    count_launch();
+    p.members = a->count;
+    launch_params<kMaxGroupMembers>(s, g, p);
     return submitted();
 }
 

@@ -52,6 +52,11 @@ split_rows_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ split, u
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, token = blockIdx.y, groups = cols / 16;
     const uint16_t* row = x + static_cast<uint64_t>(token) * cols;
     const uint32_t group = blockIdx.x * kSliceGroups + warp * 2 + (lane >> 4);
+    // A row that is not in L2 would queue behind the weight copies that the stream kernel has already issued, so every CTA asks
+    // for its slice of the row now. (The launch before may still write it; L2 then holds what it writes.)
+    if (threadIdx.x < kSliceGroups / 4 && blockIdx.x * kSliceGroups + threadIdx.x * 4 < groups) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(row + (blockIdx.x * kSliceGroups + threadIdx.x * 4) * 16));
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");   // x may come from the launch before, and the split may still be read by it
     const uint32_t bits = group < groups ? __ldcg(row + group * 16 + (lane & 15)) : 0;
     uint32_t packed = 0;

@@ -1,0 +1,54 @@
+"""GPU parity of the mma.sync small-token kernel at the edges of its split: row groups dealt out to clusters of every size, ranges
+of unequal length, slabs of unequal k, more warps than blocks, the split through scratch beside them, and every token count (the
+staging differs by it). Bound as elsewhere: helpers.rel_error <= 2e-2 against the fp64 oracle; two submits give the same bits."""
+import numpy as np
+import pytest
+
+import oracle
+from augur_v100_b200 import abi, host, synth
+from helpers import TOLERANCE, bits_from_torch_bf16, rel_error, torch_bf16_from_bits
+from test_gpu_small_token import ctx  # noqa: F401  (the fixture)
+
+pytestmark = pytest.mark.gpu
+
+
+# 1 group; fewer blocks than warps; 33 and 75 groups over clusters with unequal slabs; 160 groups; 9 slabs, through scratch
+@pytest.mark.parametrize("rows,cols,tokens", [(32, 128, 1), (32, 5120, 8), (64, 1152, 2), (1056, 5248, 3), (2400, 2176, 4), (5120, 5120, 5),
+                                              (1024, 41600, 6), (17408, 256, 7)])
+def test_cluster_split(ctx, rows, cols, tokens):  # noqa: F811
+    codes, scales, glob = synth.make_weight(rows + cols, 93, "w", rows, cols)
+    x_bits = synth.make_activation(rows + cols, 93, "x", tokens, cols)
+    weight = host.Nvfp4Sm100Weight.upload_checkpoint_nvfp4(ctx["stream"], abi.LAYOUT_STREAM, rows, cols, codes, scales, glob)
+    plan = host.Plan(ctx["stream"], host.gemv_scratch_bytes(rows, cols))
+    projection = host.Nvfp4Sm100Projection.bind(plan, weight, torch_bf16_from_bits(x_bits, ctx["device"]))
+    results = []
+    for _ in range(2):
+        projection.out.fill_(float("nan"))
+        projection.submit_for_plan()
+        ctx["stream"].synchronize()
+        results.append(bits_from_torch_bf16(projection.out))
+    assert plan.device_status() == 0
+    plan.close()
+    assert np.array_equal(*results)
+    assert rel_error(results[0], oracle.linear_f64(codes, scales, glob, rows, cols, x_bits, threads=oracle.max_threads())) <= TOLERANCE
+
+
+# members of a norm group whose ranges straddle clusters, one of them trimmed
+@pytest.mark.parametrize("cols,rows,stored", [(1024, (1056, 64, 2080), (0, 48, 0)), (2560, (64, 64, 32, 96), (48, 48, 0, 0)), (5120, (4000,), (0,))])
+def test_group_members_straddle_clusters(ctx, cols, rows, stored):  # noqa: F811
+    torch, tokens = ctx["torch"], 6
+    made = [synth.make_weight(cols + i, 94, "w", r, cols) for i, r in enumerate(rows)]
+    weights = [host.Nvfp4Sm100Weight.upload_checkpoint_nvfp4(ctx["stream"], abi.LAYOUT_STREAM, r, cols, *planes) for r, planes in zip(rows, made)]
+    plan = host.Plan(ctx["stream"], 64 << 20)
+    x = torch.from_numpy(np.random.default_rng(cols).standard_normal((tokens, cols)).astype(np.float32)).to(ctx["device"])
+    gain = torch.ones(cols, dtype=torch.float32, device=ctx["device"])
+    torch.cuda.synchronize()
+    program = host.Nvfp4Sm100NormGroupProgram.bind(plan, weights, x, gain, stored_rows=list(stored))
+    program.submit_for_plan()
+    ctx["stream"].synchronize()
+    assert plan.device_status() == 0
+    plan.close()
+    staged = bits_from_torch_bf16(program.staged)
+    for out, r, keep, planes in zip(program.outputs, rows, stored, made):
+        y64 = oracle.linear_f64(*planes, r, cols, staged, threads=oracle.max_threads())
+        assert rel_error(bits_from_torch_bf16(out), np.ascontiguousarray(y64.reshape(tokens, r)[:, : keep or r])) <= TOLERANCE
