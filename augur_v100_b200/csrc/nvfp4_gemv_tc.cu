@@ -1099,9 +1099,6 @@ augur_cuda_result_v1 launch_tc(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm1
     return submitted();
 }
 
-// Contributors per tile of a single linear on a device with `sm_count` SMs.
-uint32_t linear_contributors(const augur_cuda_nvfp4_sm100_gemv_args_v1* a, uint32_t sm_count) { return tc_program(a, nullptr, sm_count).contributors[0]; }
-
 }  // namespace
 
 cudaError_t gemv_tc_configure_device() {
@@ -1171,7 +1168,7 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_gemv_tc_b
     if (!check_tc_header(d, s, plan, a, a ? a->abi_version : 0, header_ok(d, s, a), &failure)) return failure;
     uint32_t physical = 0;
     if (!check_tc_scalars(a, &physical)) return invalid();
-    if (!check_tc(d, s, plan, a, linear_contributors(a, plan->sm_count), kCounterBytes, plan->scratch_bytes, true, &failure)) return failure;
+    if (!check_tc(d, s, plan, a, 1, kCounterBytes, plan->scratch_bytes, true, &failure)) return failure;
     CUtensorMap probe;
     return weight_map(&probe, a->weight, physical_rows_of(a), a->cols) ? ok() : make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
 }
@@ -1182,7 +1179,7 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_gemv_tc_b
     if (!check_tc_header(d, s, plan, a, a ? a->abi_version : 0, header_ok(d, s, a), &failure)) return failure;
     uint32_t physical = 0;
     if (!check_tc_scalars(a, &physical)) return invalid();
-    if (!check_tc(d, s, plan, a, linear_contributors(a, plan->sm_count), kCounterBytes, plan->scratch_bytes, false, &failure)) return failure;
+    if (!check_tc(d, s, plan, a, 1, kCounterBytes, plan->scratch_bytes, false, &failure)) return failure;
     if (consume_injected_fault()) return make_result(AUGUR_CUDA_STATUS_DIAGNOSTIC_FAULT_INJECTED);
     const cudaError_t e = cudaSetDevice(d);
     if (e != cudaSuccess) return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE, e);

@@ -296,7 +296,7 @@ def gemv_tc_scratch_bytes(rows: int, cols: int, epilogue: int = abi.EPILOGUE_LIN
     return int(out.value)
 
 
-class Nvfp4Sm100TcProjection:
+class Nvfp4Sm100TcProjection(Nvfp4Sm100Projection):
     """A retained small-token projection on the tensor-memory path: the weight is in the tcgen05 layout
     (the one the prefill GEMM uses; for the SwiGLU epilogue the interleaved gate|up tensor of
     `upload_gate_up_interleaved`), the kernel is `gemv_tc`. Same contract as `Nvfp4Sm100Projection`."""
@@ -708,8 +708,13 @@ class Nvfp4Sm100Linear:
     Keeps the weight in both hot layouts (the small-token stream layout and the tcgen05 layout) and
     binds the kernel its shape class calls for: tokens <= 8 -> `Nvfp4Sm100Projection`, otherwise
     `Nvfp4Sm100PrefillLinear` (activation quantiser with `terms` residual terms, then the block-scaled
-    GEMM). Bindings are made per (input, output) pair, exactly like the two classes it chooses between.
+    GEMM). Bindings are made per (input, output) pair, exactly like the classes it chooses between.
     """
+
+    # From this many weights on the tensor-memory kernel is the faster of the two small-token kernels: below, its second
+    # launch costs more than the integer work per weight that it saves (B200, 8 token rows: 4096 x 5120 9.5 us against 9.3 on
+    # mma.sync, 5120 x 7808 12.3 / 12.2, 9856 x 6016 12.0 / 15.9, 17408 x 5120 14.8 / 17.1).
+    TENSOR_MEMORY_WEIGHTS = 1 << 25
 
     def __init__(self, stream: Stream, rows: int, cols: int, codes, scales, global_scale: float):
         self.rows, self.cols = rows, cols
@@ -719,5 +724,10 @@ class Nvfp4Sm100Linear:
     def bind(self, plan: Plan, x: torch.Tensor, out: torch.Tensor | None = None, terms: int = 3,
              activation_global_scale: float = 2.0 ** -8):
         if classify_tokens(x.shape[0]) == SHAPE_SMALL_BATCH:
+            if self.rows % 128 == 0 and self.rows * self.cols >= self.TENSOR_MEMORY_WEIGHTS:
+                try:
+                    return Nvfp4Sm100TcProjection.bind(plan, self.wide, x, out)
+                except CudaRuntimeError:
+                    pass        # a plan with less scratch than it needs; any other fault is reported below
             return Nvfp4Sm100Projection.bind(plan, self.small, x, out)
         return Nvfp4Sm100PrefillLinear.bind(plan, self.wide, x, out, terms=terms, activation_global_scale=activation_global_scale)

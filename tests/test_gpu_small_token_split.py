@@ -36,3 +36,19 @@ def test_split_linear_edges(ctx, rows, cols, tokens):  # noqa: F811
     assert ctx["plan"].device_status() == 0
     assert rel_error(results[0], y64) <= TOLERANCE and all(np.array_equal(results[0], again) for again in results[1:])
     assert rel_error(bits_from_torch_bf16(other.out), other64) <= TOLERANCE
+
+
+# From 2^25 weights on `Nvfp4Sm100Linear` binds this kernel.
+def test_linear_dispatch_by_size(ctx):  # noqa: F811
+    rows, cols, tokens = 32768, 1024, 6
+    codes, scales, glob = synth.make_weight(7, 95, "w", rows, cols)
+    x_bits = synth.make_activation(7, 95, "x", tokens, cols)
+    linear = host.Nvfp4Sm100Linear(ctx["stream"], rows, cols, codes, scales, glob)
+    plan = host.Plan(ctx["stream"], 1 << 20)
+    binding = linear.bind(plan, torch_bf16_from_bits(x_bits, ctx["device"]))
+    binding.submit_for_plan()
+    ctx["stream"].synchronize()
+    y64 = oracle.linear_f64(codes, scales, glob, rows, cols, x_bits, threads=oracle.max_threads())
+    assert plan.device_status() == 0 and isinstance(binding, host.Nvfp4Sm100TcProjection)
+    assert rel_error(bits_from_torch_bf16(binding.out), y64) <= TOLERANCE
+    plan.close()
