@@ -3,39 +3,47 @@
 //
 // What it replaces: the register-blocked FP32 kernel of the reference
 // (crates/augur-cuda-sys/native/augur_dflash_llama_bf16_head.cuh:24-72, f32_rw4: BF16 widened exactly to F32,
-// exact F32 products, F32 accumulation). At 8 token rows the head is bandwidth-bound on a B200 only if the
-// inner product is cheap: 3.2e12 weights per second at HBM rate would need 26e12 FP32 FMAs per second, most of
-// what the FP32 pipes have. Here the weights go to the tensor cores as they are (mma.sync m16n8k16, BF16 A
-// operand straight from global memory in fragment order, the 8 token rows on n), and the F32 activations are
-// split on the fly into three BF16 terms x = hi + mid + lo (8 + 8 + 8 significand bits: exact), one MMA per term.
-// Every product is exact, as in the reference; only the order of the F32 additions differs.
+// exact F32 products, F32 accumulation). The head is one stream over the weights (2.5 GB at 248320 x 5120), and whatever the
+// SMs do beside it costs twice: in issue slots and in power, because at this rate the GPU runs into its power limit within
+// a tenth of a second. So no thread touches a weight: TMA brings tiles of up to 128 rows x 64 k into a ring in
+// shared memory and tcgen05.mma kind::f16 reads them there. (With mma.sync on fragments that every lane loaded for itself, and
+// the activations split by every warp for its own rows, the SM clock fell to 1.58 GHz and a pass took 510 to 540 us.)
 //
-// A warp owns 16-row tiles over the whole k range (no reduction between warps); a lane's weight loads are
-// 16-byte vectors, two per row and 64-k step, kept four steps ahead in registers, so that a CTA of 16 warps has
-// 128 KB in flight. The activations sit in shared memory as F32, each token row padded so that a quarter warp's
-// 16-byte reads fall in different banks, with the 16-byte pieces of a 64-k block ordered the way the lanes
-// consume them.
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-
+//   activations  F32, split into three BF16 terms x = hi + mid + lo (8 + 8 + 8 significand bits: exact), which sit side by side on
+//                the MMA n dimension (column = term * 8 + token): four warps per CTA split the 64 k of every ring stage
+//                once for all its rows. Every product is exact, as in the reference; only the order of the additions differs.
+//   sums         The tensor core adds into its accumulator without rounding to nearest, so the sum of a 64-k block is formed in
+//                an accumulator of its own (four MMAs deep, one column per term) and added to the running sums, in registers of
+//                the epilogue warps, with ordinary round-to-nearest additions: the error grows like that of the
+//                reference's F32 chain.
+//   rows         The tile height is what deals the rows out evenly (120 of 128 at 248320 rows on 148 SMs: 14 tiles for every CTA);
+//                tiles go round the CTAs, so that all of them read one neighbourhood of the weights at a time.
+//
+// Every wait is bounded; a wait that runs out raises a CTA-wide abort flag, all roles fall through to the common exit, and
+// the tiles that were not finished are stored as NaN.
+#include "nvfp4_gemm.cuh"
 #include "nvfp4_internal.h"
 
 namespace augur_sm100 {
 namespace {
+using namespace tc;
 
 static_assert(sizeof(augur_cuda_nvfp4_sm100_bf16_head_args_v1) == 64, "bf16 head ABI");
 
-constexpr uint32_t kHeadWarps = 16;
-constexpr uint32_t kHeadThreads = kHeadWarps * 32;
-constexpr uint32_t kHeadAhead = 4;          // 64-k steps of weights a lane keeps in flight
-constexpr uint32_t kHeadRowPad = 16;        // floats between token rows in shared memory beyond cols (64 bytes)
-constexpr uint32_t kHeadMaxSmem = 200 * 1024;
+constexpr uint32_t kHeadThreads = 32 * 12;                   // warp 0 TMA, 1 MMA, 4..7 split, 8..11 epilogue (2 and 3 have no part)
+constexpr uint32_t kHeadTerms = 3;
+constexpr uint32_t kHeadN = 32;                              // MMA n: 24 columns, rounded up to a multiple of 16
+constexpr uint32_t kHeadTile = kTileM * 128;                 // 16 KB: 128 rows x 64 k of BF16
+constexpr uint32_t kHeadStage = kHeadTile + kHeadN * 128;    // and 4 KB of split activations
+constexpr uint32_t kHeadStages = 11;
+constexpr uint32_t kHeadSmem = kHeadStages * kHeadStage + 512 /*barriers*/ + 1024 /*alignment*/;
+constexpr uint32_t kHeadAccs = 8;                            // accumulators of 32 columns
+constexpr uint32_t kHeadAhead = 4;                           // stages of activations that a split thread has in flight
+constexpr uint32_t kHeadMaxRowBytes = 200 * 1024 / 8 - 64;   // of a token row of activations
+static_assert(kHeadSmem <= 227 * 1024, "shared memory of a CTA");
 
-__device__ __forceinline__ void mma_bf16_acc(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
+__device__ uint32_t g_head_status;   // first wait that ran out (the entry has no plan to report through)
+constexpr uint32_t kErrHeadProducer = 0x401, kErrHeadSplit = 0x402, kErrHeadFull = 0x403, kErrHeadAccEmpty = 0x404, kErrHeadAccFull = 0x405;
 
 // Two F32 values -> their three BF16 terms, packed (low half = first value). x = hi + mid + lo exactly: each
 // subtraction is exact, and after two of them at most 8 significand bits are left.
@@ -47,96 +55,181 @@ __device__ __forceinline__ void split3(float x0, float x1, uint32_t& hi, uint32_
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(s1), "f"(s0));
 }
 
-__device__ __forceinline__ uint4 load_weights(const uint4* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
+__device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+                 : "memory");
+}
+__device__ __forceinline__ void load_columns8(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
 }
 
 __global__ void __launch_bounds__(kHeadThreads, 1)
-bf16_head_kernel(const uint16_t* __restrict__ weight, const float* __restrict__ x, float* __restrict__ out, uint32_t rows,
-                 uint32_t cols, uint32_t tokens) {
-    extern __shared__ __align__(16) float staged[];     // [8 token rows][cols + pad], the 16-byte pieces of a 64-k block reordered
+bf16_head_kernel(const __grid_constant__ CUtensorMap map_weight, const float* __restrict__ x, float* __restrict__ out, uint32_t rows,
+                 uint32_t cols, uint32_t tokens, uint32_t tile_rows) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kHeadStages * kHeadStage);
+    const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + kHeadStages);
+    const uint32_t bar_acc_full = smem_u32(bars + 2 * kHeadStages), bar_acc_empty = smem_u32(bars + 2 * kHeadStages + kHeadAccs);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kHeadStages + 2 * kHeadAccs);
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
-    const uint32_t stride = cols + kHeadRowPad;
-    // Lane (g, t4) takes the weights k = 64c + 16 t4 .. + 15 of a 64-k block c; MMA step j of the block contracts
-    // its k = 64c + 16 t4 + 4j .. + 3 with the same k of token g, which therefore sit at piece j * 4 + t4.
-    for (uint32_t i = threadIdx.x; i < 8 * (cols / 4); i += kHeadThreads) {
-        const uint32_t token = i / (cols / 4), piece = i - token * (cols / 4);          // 16-byte piece of the row
-        const uint32_t block = piece >> 4, owner = (piece >> 2) & 3, step = piece & 3;   // k = 64 block + 16 owner + 4 step
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (token < tokens) v = __ldcg(reinterpret_cast<const float4*>(x + static_cast<uint64_t>(token) * cols) + piece);
-        *reinterpret_cast<float4*>(staged + token * stride + block * 64 + (step * 4 + owner) * 4) = v;
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < kHeadStages; ++s) {
+            mbar_init(bar_full + 8 * s, 1 + 4);   // the TMA's bytes and the four split warps
+            mbar_init(bar_empty + 8 * s, 1);
+        }
+        for (uint32_t b = 0; b < kHeadAccs; ++b) {
+            mbar_init(bar_acc_full + 8 * b, 1);
+            mbar_init(bar_acc_empty + 8 * b, 4);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kHeadAccs * kHeadN) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
     __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tiles = (rows + tile_rows - 1) / tile_rows, blocks = cols / 64;
+    const uint32_t mine = (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x, total = mine * blocks;   // 64-k stages of this CTA
 
-    // this warp's 16-row tiles: equal contiguous shares of all tiles over all warps of the grid
-    const uint32_t tiles = rows / 16, warps = gridDim.x * kHeadWarps, me = blockIdx.x * kHeadWarps + warp;
-    const uint32_t tile0 = static_cast<uint32_t>(static_cast<uint64_t>(me) * tiles / warps);
-    const uint32_t tile1 = static_cast<uint32_t>(static_cast<uint64_t>(me + 1) * tiles / warps);
-    const uint32_t blocks = cols / 64;
-    const uint32_t total = (tile1 - tile0) * blocks;       // 64-k steps of this warp
-    const float* mine = staged + g * stride + t4 * 4;      // token g, this lane's piece of step 0
-
-    // weights of step s: rows g and g + 8 of its tile, 16 k each (two 16-byte vectors per row)
-    auto fetch = [&](uint32_t s, uint4 (&w)[4]) {
-        const uint32_t tile = tile0 + s / blocks, block = s - (s / blocks) * blocks;
-        const uint4* row = reinterpret_cast<const uint4*>(weight + (static_cast<uint64_t>(tile) * 16 + g) * cols + block * 64 + t4 * 16);
-        const uint4* other = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(row) + static_cast<uint64_t>(8) * cols);
-        w[0] = load_weights(row);
-        w[1] = load_weights(row + 1);
-        w[2] = load_weights(other);
-        w[3] = load_weights(other + 1);
-    };
-    uint4 ring[kHeadAhead][4];
+    if (warp == 0) {
+        // ---------------- weights ----------------
+        uint32_t stage = 0, phase = 1, block = 0, row = blockIdx.x * tile_rows;
+        for (uint32_t s = 0; s < total; ++s) {
+            if (!mbar_wait(bar_empty + 8 * stage, phase, abort_flag, &g_head_status, kErrHeadProducer)) break;
+            if (elect_one()) {
+                const uint32_t full = bar_full + 8 * stage;
+                mbar_expect_tx(full, tile_rows * 128);
+                tma_load_2d(smem_u32(smem + stage * kHeadStage), &map_weight, block * 128, row, full);
+            }
+            __syncwarp();
+            if (++stage == kHeadStages) { stage = 0; phase ^= 1; }
+            if (++block == blocks) { block = 0; row += gridDim.x * tile_rows; }
+        }
+    } else if (warp == 1) {
+        // ---------------- MMA issuer ----------------
+        // F32 accumulator, both operands BF16 and K-major
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((kHeadN >> 3) << 17) | ((kTileM >> 4) << 24);
+        const uint64_t w_desc0 = operand_desc(smem_u32(smem)), x_desc0 = operand_desc(smem_u32(smem) + kHeadTile);
+        uint32_t stage = 0, phase = 0, buffer = 0, acc_phase = 1;
+        for (uint32_t s = 0; s < total; ++s) {
+            if (!mbar_wait(bar_acc_empty + 8 * buffer, acc_phase, abort_flag, &g_head_status, kErrHeadAccEmpty) ||
+                !mbar_wait(bar_full + 8 * stage, phase, abort_flag, &g_head_status, kErrHeadFull)) {
+                break;
+            }
+            tc_fence_after();
+            if (elect_one()) {
+                const uint64_t w_desc = w_desc0 + stage * (kHeadStage >> 4), x_desc = x_desc0 + stage * (kHeadStage >> 4);
 #pragma unroll
-    for (uint32_t a = 0; a < kHeadAhead; ++a) {
-        if (a < total) fetch(a, ring[a]);
-    }
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    uint32_t block = 0, tile = tile0;
-    for (uint32_t s0 = 0; s0 < total; s0 += kHeadAhead) {
+                for (uint32_t k = 0; k < 4; ++k) mma_bf16(tmem_base + buffer * kHeadN, w_desc + 2 * k, x_desc + 2 * k, idesc, k);   // 16 k = 32 bytes
+                tc_commit(bar_empty + 8 * stage);
+                tc_commit(bar_acc_full + 8 * buffer);
+            }
+            __syncwarp();
+            if (++stage == kHeadStages) { stage = 0; phase ^= 1; }
+            if (++buffer == kHeadAccs) { buffer = 0; acc_phase ^= 1; }
+        }
+    } else if (warp >= 4 && warp < 8) {
+        // ---------------- split: thread = (token, four neighbouring k) of every stage ----------------
+        // Row term * 8 + token of the operand tile, in its 128-byte swizzle. Columns of tokens that do not exist are never stored,
+        // so neither are their rows here.
+        const uint32_t thread = threadIdx.x - 128, token = thread >> 4, piece = thread & 15;
+        const bool live = token < tokens;
+        const float4* row = reinterpret_cast<const float4*>(x + static_cast<uint64_t>(live ? token : 0) * cols) + piece;
+        uint8_t* place = smem + kHeadTile + token * 128 + (((piece >> 1) ^ token) << 4) + (piece & 1) * 8;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        float4 ahead[kHeadAhead];
+        uint32_t fetch = 0;   // block of the next load (the row is read again for every tile)
 #pragma unroll
         for (uint32_t a = 0; a < kHeadAhead; ++a) {
-            const uint32_t s = s0 + a;
-            if (s >= total) break;
-            const uint4 (&w)[4] = ring[a];
-            const uint32_t row_g[8] = {w[0].x, w[0].y, w[0].z, w[0].w, w[1].x, w[1].y, w[1].z, w[1].w};
-            const uint32_t row_h[8] = {w[2].x, w[2].y, w[2].z, w[2].w, w[3].x, w[3].y, w[3].z, w[3].w};
-            const float* base = mine + block * 64;
-            // The tensor core adds into its accumulator without rounding to nearest, so the sum of a 64-k block is
-            // formed in a register set of its own (twelve MMAs deep) and added to the running sum with ordinary
-            // round-to-nearest additions: the error grows like that of the reference's F32 chain.
-            float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            ahead[a] = __ldcg(row + fetch * 16);
+            if (++fetch == blocks) fetch = 0;
+        }
+        uint32_t stage = 0, phase = 1;
+        bool alive = true;
+        for (uint32_t s0 = 0; alive && s0 < total; s0 += kHeadAhead) {
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) {
-                const float4 v = *reinterpret_cast<const float4*>(base + j * 16);
-                uint32_t hi0, mid0, lo0, hi1, mid1, lo1;
-                split3(v.x, v.y, hi0, mid0, lo0);
-                split3(v.z, v.w, hi1, mid1, lo1);
-                // the smallest terms first, so that they are not lost against a large partial sum
-                mma_bf16_acc(part, row_g[2 * j], row_h[2 * j], row_g[2 * j + 1], row_h[2 * j + 1], lo0, lo1);
-                mma_bf16_acc(part, row_g[2 * j], row_h[2 * j], row_g[2 * j + 1], row_h[2 * j + 1], mid0, mid1);
-                mma_bf16_acc(part, row_g[2 * j], row_h[2 * j], row_g[2 * j + 1], row_h[2 * j + 1], hi0, hi1);
-            }
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) acc[i] += part[i];
-            if (s + kHeadAhead < total) fetch(s + kHeadAhead, ring[a]);
-            if (++block == blocks) {
-                // acc: rows g (first two) and g + 8 (last two) of the tile, tokens 2 t4 and 2 t4 + 1
-                const uint32_t row = tile * 16 + g;
-#pragma unroll
-                for (uint32_t i = 0; i < 4; ++i) {
-                    const uint32_t token = 2 * t4 + (i & 1);
-                    if (token < tokens) out[static_cast<uint64_t>(token) * rows + row + (i >> 1) * 8] = acc[i];
-                    acc[i] = 0.0f;
+            for (uint32_t a = 0; a < kHeadAhead; ++a) {
+                if (s0 + a >= total) break;
+                uint32_t hi[2], mid[2], lo[2];
+                split3(ahead[a].x, ahead[a].y, hi[0], mid[0], lo[0]);
+                split3(ahead[a].z, ahead[a].w, hi[1], mid[1], lo[1]);
+                ahead[a] = __ldcg(row + fetch * 16);
+                if (++fetch == blocks) fetch = 0;
+                if (!mbar_wait(bar_empty + 8 * stage, phase, abort_flag, &g_head_status, kErrHeadSplit)) {
+                    alive = false;
+                    break;
                 }
-                block = 0;
-                ++tile;
+                if (live) {
+                    uint8_t* to = place + stage * kHeadStage;
+                    *reinterpret_cast<uint2*>(to) = make_uint2(hi[0], hi[1]);
+                    *reinterpret_cast<uint2*>(to + 1024) = make_uint2(mid[0], mid[1]);
+                    *reinterpret_cast<uint2*>(to + 2048) = make_uint2(lo[0], lo[1]);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads them through the async proxy
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_full + 8 * stage);
+                if (++stage == kHeadStages) { stage = 0; phase ^= 1; }
             }
         }
+    } else if (warp >= 8) {
+        // ---------------- epilogue: lane = weight row, eight token rows x three terms ----------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing is written while an earlier kernel may still read it
+        const uint32_t quadrant = warp & 3;
+        const uint32_t taddr = tmem_base + ((quadrant * 32) << 16);
+        uint32_t buffer = 0, phase = 0;
+        for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            float sum[kHeadTerms][8];
+#pragma unroll
+            for (uint32_t t = 0; t < kHeadTerms; ++t) {
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) sum[t][i] = 0.0f;
+            }
+            for (uint32_t block = 0; block < blocks; ++block) {
+                if (!mbar_wait(bar_acc_full + 8 * buffer, phase, abort_flag, &g_head_status, kErrHeadAccFull)) {
+                    sum[0][0] = __uint_as_float(0x7fc00000u);
+                    break;
+                }
+                tc_fence_after();
+                uint32_t v[kHeadTerms][8];
+#pragma unroll
+                for (uint32_t t = 0; t < kHeadTerms; ++t) load_columns8(taddr + buffer * kHeadN + 8 * t, v[t]);
+                tc_wait_ld();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buffer);
+                if (++buffer == kHeadAccs) { buffer = 0; phase ^= 1; }
+#pragma unroll
+                for (uint32_t t = 0; t < kHeadTerms; ++t) {
+#pragma unroll
+                    for (uint32_t i = 0; i < 8; ++i) sum[t][i] += __uint_as_float(v[t][i]);
+                }
+            }
+            const bool failed = *abort_flag != 0;
+            const uint32_t local = quadrant * 32 + lane, row = tile * tile_rows + local;
+            if (local < tile_rows && row < rows) {
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) {
+                    if (i < tokens) out[static_cast<uint64_t>(i) * rows + row] = failed ? __uint_as_float(0x7fc00000u) : (sum[2][i] + sum[1][i]) + sum[0][i];
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kHeadAccs * kHeadN) : "memory");
     }
 }
 
@@ -157,14 +250,12 @@ bool check_head(int32_t d, augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_b
     if (count < 1 || count > AUGUR_NVFP4_SM100_MAX_SMALL_TOKENS) return false;
     *tokens = static_cast<uint32_t>(count);
     if (a->output_len_bytes != count * a->rows * 4) return false;
-    if (8ull * (a->cols + kHeadRowPad) * 4 > kHeadMaxSmem) return false;   // the activations must fit shared memory
-    // 16-byte vector loads of weights and activations (the reference's rw4 entry asks the same)
+    if (a->cols * 4 > kHeadMaxRowBytes) return false;   // the widths that this entry has always taken
+    // TMA and 16-byte vector loads (the reference's rw4 entry asks the same alignment)
     const Range r[3] = {{a->weight, a->weight_len_bytes, 16}, {a->input, a->input_len_bytes, 16}, {a->output, a->output_len_bytes, 4}};
     if (!all_disjoint(r, 3)) return false;
     return !full || inspect_device_ranges(d, r, 3, failure);
 }
-
-uint32_t head_smem_bytes(uint32_t cols) { return 8 * (cols + kHeadRowPad) * 4; }
 
 }  // namespace
 }  // namespace augur_sm100
@@ -177,7 +268,7 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_bf16_head
     uint32_t tokens = 0;
     if (!check_head(d, s, a, true, &tokens, &failure)) return failure;
     // a bind-time call: the kernel's shared-memory limit for this width
-    const cudaError_t e = cudaFuncSetAttribute(bf16_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadMaxSmem);
+    const cudaError_t e = cudaFuncSetAttribute(bf16_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadSmem);
     return e == cudaSuccess ? ok() : make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE, e);
 }
 
@@ -194,26 +285,18 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_bf16_head
     if (!sm_count[d]) {
         int sms = 0;
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(bf16_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadMaxSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(bf16_head_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadSmem);
         if (e != cudaSuccess) return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE, e);
         sm_count[d] = sms;
     }
-    const int sms = sm_count[d];
-    const uint32_t tiles = a->rows / 16;
-    uint32_t grid = static_cast<uint32_t>(sms);
-    if (grid * kHeadWarps > tiles) grid = (tiles + kHeadWarps - 1) / kHeadWarps;
-    cudaLaunchAttribute attribute{};
-    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t config{};
-    config.stream = s->stream;
-    config.attrs = &attribute;
-    config.numAttrs = 1;
-    config.gridDim = dim3(grid);
-    config.blockDim = dim3(kHeadThreads);
-    config.dynamicSmemBytes = head_smem_bytes(a->cols);
-    cudaLaunchKernelEx(&config, bf16_head_kernel, reinterpret_cast<const uint16_t*>(a->weight), reinterpret_cast<const float*>(a->input),
-                       reinterpret_cast<float*>(a->output), a->rows, a->cols, tokens);
+    // tiles of equal height, as few rounds of the SMs as 128-row tiles allow
+    const uint32_t sms = static_cast<uint32_t>(sm_count[d]), rounds = (a->rows + kTileM * sms - 1) / (kTileM * sms);
+    const uint32_t tile_rows = ((a->rows + rounds * sms - 1) / (rounds * sms) + 7) / 8 * 8;
+    const uint32_t tiles = (a->rows + tile_rows - 1) / tile_rows;
+    CUtensorMap map_weight;   // rows of cols * 2 bytes, as a map of packed codes with four times the columns
+    if (!make_code_map(&map_weight, a->weight, a->rows, a->cols * 4, tile_rows)) return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
+    launch_dependent(s->stream, bf16_head_kernel, tiles < sms ? tiles : sms, kHeadThreads, kHeadSmem, map_weight,
+                     reinterpret_cast<const float*>(a->input), reinterpret_cast<float*>(a->output), a->rows, a->cols, tokens, tile_rows);
     count_launch();
     return submitted();
 }
