@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(kRepackWarps * 32)
 repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restrict__ scales_a, const uint8_t* __restrict__ codes_b,
                      const uint8_t* __restrict__ scales_b, uint8_t* __restrict__ destination, uint32_t blocks, uint32_t cols, bool pair) {
     const uint32_t block = blockIdx.x * kRepackWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory");
     if (block >= blocks) return;
     const uint32_t kb_count = cols / kStreamBlockK;
     const uint32_t group = block / kb_count, kb = block - group * kb_count;
@@ -163,6 +164,7 @@ __device__ __forceinline__ void retile_scales(const uint8_t* __restrict__ scales
 __global__ void __launch_bounds__(kRepackWarps * 32)
 repack_tcgen05_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, uint8_t* __restrict__ destination,
                       uint32_t rows, uint32_t cols, uint32_t scale_ctas, uint32_t run_atoms) {
+    asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory");
     const uint64_t code_bytes = tcgen05_codes_bytes(rows, cols);
     if (blockIdx.x < scale_ctas) {   // the scales first: their loads are the scattered ones
         const uint32_t run = blockIdx.x * kRepackWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -327,13 +329,13 @@ void launch_repack(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_repack_ar
         const uint64_t runs = static_cast<uint64_t>((a->rows + 127) / 128) * (a->cols / 64 / run_atoms);
         const uint32_t scale_ctas = static_cast<uint32_t>((runs + kRepackWarps - 1) / kRepackWarps);
         const uint32_t copy_ctas = static_cast<uint32_t>((tcgen05_codes_bytes(a->rows, a->cols) + kRepackCopyBytes - 1) / kRepackCopyBytes);
-        repack_tcgen05_kernel<<<scale_ctas + copy_ctas, kRepackWarps * 32, 0, s->stream>>>(codes, scales, destination, a->rows, a->cols,
-                                                                                            scale_ctas, run_atoms);
+        launch_dependent(s->stream, repack_tcgen05_kernel, scale_ctas + copy_ctas, kRepackWarps * 32, 0, codes, scales, destination, a->rows, a->cols,
+                         scale_ctas, run_atoms);
     } else {
         const uint32_t blocks = static_cast<uint32_t>(a->destination_len_bytes / kStreamBlockBytes);
-        repack_stream_kernel<<<(blocks + kRepackWarps - 1) / kRepackWarps, kRepackWarps * 32, 0, s->stream>>>(
-            codes, scales, reinterpret_cast<const uint8_t*>(a->codes_b), reinterpret_cast<const uint8_t*>(a->scales_b), destination,
-            blocks, a->cols, a->layout == AUGUR_NVFP4_SM100_LAYOUT_STREAM_PAIR);
+        launch_dependent(s->stream, repack_stream_kernel, (blocks + kRepackWarps - 1) / kRepackWarps, kRepackWarps * 32, 0, codes, scales,
+                         reinterpret_cast<const uint8_t*>(a->codes_b), reinterpret_cast<const uint8_t*>(a->scales_b), destination, blocks, a->cols,
+                         a->layout == AUGUR_NVFP4_SM100_LAYOUT_STREAM_PAIR);
     }
     count_launch();
 }

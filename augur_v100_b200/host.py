@@ -12,6 +12,7 @@ memory and stream plumbing only; every computation goes through the C ABI.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import byref, c_uint32, c_uint64, c_void_p
 
 import numpy as np
@@ -121,6 +122,7 @@ def gemm_scratch_bytes(rows: int, cols: int, tokens: int, terms: int) -> int:
     return int(out.value)
 
 
+@functools.lru_cache(maxsize=256)
 def repack_extent(layout: int, rows: int, cols: int) -> int:
     out = c_uint64()
     _check("repack_extent", abi.lib().augur_cuda_nvfp4_sm100_repack_extent_host_v1(layout, rows, cols, byref(out)))
