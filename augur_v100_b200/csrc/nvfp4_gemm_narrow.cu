@@ -460,6 +460,8 @@ augur_cuda_result_v1 launch_gemm_narrow(augur_cuda_stream_t s, const augur_cuda_
     p.sf_weight = (p.columns + 31) / 32 * 32;
     p.sf_token = p.sf_weight + 16 * p.weight_depth;
     static_assert(128 + 16 * (kNarrowSmem / kNarrowStage) <= kNarrowTmemColumns, "scale columns of all slots fit beside the accumulator");
+    // A slot index past the barrier arrays would reach the accumulator's barrier and the tensor-memory base word.
+    static_assert(kNarrowSmem / kNarrowStage <= kNarrowMaxDepth && 2 * 3 /*terms*/ <= kNarrowMaxDepth, "every slot of both rings has its barriers");
     CUtensorMap map_act;
     if (!make_code_map(&map_act, activation, static_cast<uint64_t>(g.terms) * g.padded_tokens, g.cols, p.columns)) {
         return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
