@@ -220,6 +220,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // Everything above ran while the launch before this one drained; its results are needed from here on.
+    // The dependents start only after the wait: a narrow launch behind this one (`after_main`) skips its own wait until its
+    // end and relies on the quantiser, which this launch has waited for.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 

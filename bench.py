@@ -371,7 +371,7 @@ def config0_probe(ctx):
     ctx.stream.synchronize()
     other["parity"] = {"rel_error_vs_fp64_oracle": rel_error(bits(projections[0].out), y64), "bound": 2e-2}
     other["device_status"] = plan.device_status()
-    other["kernel"] = KERNELS["tensor_memory"][0]
+    other["kernel"] = "split_stream_kernel"
     entry["tensor_memory_kernel"] = other
     del projections
     plan.close()
