@@ -39,6 +39,10 @@ constexpr uint32_t kNarrowStage = kNarrowCodes + kNarrowScales;       // one wei
 constexpr uint32_t kNarrowMaxDepth = 8;                               // slots of either ring
 constexpr uint32_t kNarrowEpilogueWarps = 8;                          // two per tensor-memory lane quadrant
 constexpr uint32_t kNarrowThreads = 32 * (4 + kNarrowEpilogueWarps);   // 12 warps: registers are handed out to warps by fours
+// As if CTAs had 14 warps: 72 registers a thread instead of 80, no spills. Two CTAs of 12 warps with 80 take all but 4 K of an SM's
+// 64 K registers and a quantiser CTA (5 K) fits beside one of them only, so half the CTAs began to load weights after the quantiser
+// instead of under it (6144 x 5120, three terms, quantiser included: 256 tokens 31.8 -> 29.4 us, 128 tokens 24.2 -> 23.0).
+constexpr uint32_t kNarrowBound = 32 * 14;
 constexpr uint32_t kNarrowState = 1024;                               // barriers, tensor-memory base, abort flag
 constexpr uint32_t kNarrowTurnPitch = 36;                             // floats between columns of the transposition area: 16-byte reads hit all banks
 constexpr uint32_t kNarrowSumPitch = 129;                             // 16-byte rows between groups of four columns of the partial sums, likewise
@@ -105,7 +109,7 @@ __device__ __forceinline__ void narrow_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-__global__ void __launch_bounds__(kNarrowThreads, 2)
+__global__ void __launch_bounds__(kNarrowBound, 2)
 gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_constant__ CUtensorMap map_act, const NarrowParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -373,7 +377,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
 // 56 of 5, 45 of 6, 37 of 7, 33 of 8 on a B200). Asked once per device; bind time fills the table. The question is put for
 // a kernel of the same size that uses no tensor memory: for one that does the runtime always answers for one CTA per
 // SM, although two fit when each allocates half of it.
-__global__ void __launch_bounds__(kNarrowThreads, 2) narrow_shape_kernel() {}
+__global__ void __launch_bounds__(kNarrowBound, 2) narrow_shape_kernel() {}
 
 struct NarrowDevice {
     std::atomic<uint32_t> clusters[kNarrowMaxParts + 1];
