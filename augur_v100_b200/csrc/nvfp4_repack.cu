@@ -40,7 +40,18 @@ uint64_t layout_extent(uint32_t layout, uint32_t rows, uint32_t cols) {
 // Both kernels move every byte once and are bound by HBM (reads and writes of the same size). One destination word
 // per thread with byte gathers and a bit-by-bit permutation took 61.5 us for the STREAM layout of a 17408 x 5120
 // weight, and 4-byte copies 35 us for the TCGEN05 layout.
+//
+// Neither lets the launch behind it start early (griddepcontrol.launch_dependents): every kernel of this library fetches its
+// first weights before its own griddepcontrol.wait, and so may the launch behind an act_quant or a split, which do let theirs
+// start early. A launch of this library behind a repack starts when all of the repack's threads are through with written_out().
 constexpr uint32_t kRepackWarps = 8;
+
+// What this thread has written can be read by any later thread of the device and by its bulk copies: a grid's end says so only
+// to a launch that waits for it.
+__device__ __forceinline__ void written_out() {
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+    __threadfence();
+}
 
 // Four words of each lane of a quad, word j meant for lane j of it -> one word from each lane, in lane order.
 __device__ __forceinline__ void quad_transpose(uint32_t (&v)[4], uint32_t t4) {
@@ -67,7 +78,7 @@ __global__ void __launch_bounds__(kRepackWarps * 32)
 repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restrict__ scales_a, const uint8_t* __restrict__ codes_b,
                      const uint8_t* __restrict__ scales_b, uint8_t* __restrict__ destination, uint32_t blocks, uint32_t cols, bool pair) {
     const uint32_t block = blockIdx.x * kRepackWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (block >= blocks) return;
     const uint32_t kb_count = cols / kStreamBlockK;
     const uint32_t group = block / kb_count, kb = block - group * kb_count;
@@ -123,6 +134,7 @@ repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restr
             make_uint4(__byte_perm(scale_top.x, scale_bottom.x, 0x5140), __byte_perm(scale_top.x, scale_bottom.x, 0x7362),
                        __byte_perm(scale_top.y, scale_bottom.y, 0x5140), __byte_perm(scale_top.y, scale_bottom.y, 0x7362));
     }
+    written_out();
 }
 
 // TCGEN05: the codes are copied through, 64 bytes per thread; the scales are re-tiled by one warp per 128-row block and
@@ -164,13 +176,14 @@ __device__ __forceinline__ void retile_scales(const uint8_t* __restrict__ scales
 __global__ void __launch_bounds__(kRepackWarps * 32)
 repack_tcgen05_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, uint8_t* __restrict__ destination,
                       uint32_t rows, uint32_t cols, uint32_t scale_ctas, uint32_t run_atoms) {
-    asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint64_t code_bytes = tcgen05_codes_bytes(rows, cols);
     if (blockIdx.x < scale_ctas) {   // the scales first: their loads are the scattered ones
         const uint32_t run = blockIdx.x * kRepackWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
         if (run_atoms == 4) retile_scales<4>(scales, destination + code_bytes, rows, cols, run, lane);
         else if (run_atoms == 2) retile_scales<2>(scales, destination + code_bytes, rows, cols, run, lane);
         else retile_scales<1>(scales, destination + code_bytes, rows, cols, run, lane);
+        written_out();
         return;
     }
     // cols is a multiple of 64, so the plane is a whole number of 16-byte pieces
@@ -186,6 +199,7 @@ repack_tcgen05_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restri
     for (uint32_t i = 0; i < 4; ++i) {
         if (first + i * kRepackWarps * 32 < pieces) to[first + i * kRepackWarps * 32] = v[i];
     }
+    written_out();
 }
 
 // ---- device dequant ------------------------------------------------------------------

@@ -149,7 +149,10 @@ augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_plan_destroy_v1(
  * CPU counterpart crates/augur-repack/src/fp4_cpu.rs:45-55). Scale bytes >= 127
  * (sign bit or NaN) are the caller's to reject before upload, as the reference
  * loader does (crates/augur-backend/src/cuda_qwen35_qpn.rs:59-72); the host
- * repack below rejects them itself. */
+ * repack below rejects them itself. Stream order holds: whatever is enqueued behind a repack
+ * finds its destination complete. (Every other entry may fetch its weight while the launches ahead of
+ * it in the stream still run, so a weight must not be the output of another entry of this
+ * library, such as act_quant, that is still in flight.) */
 typedef struct augur_cuda_nvfp4_sm100_repack_args_v1 {
     uint32_t abi_version;
     uint32_t struct_size;

@@ -1,0 +1,73 @@
+"""A repack and the launch behind it on one stream, without a synchronise between them: through the C ABI a submit only enqueues,
+and stream order is all that a caller has. Every consumer that fetches weights early is here, with the destination holding other
+valid weights, so that a stale block shows; results equal those of the synchronised order bit for bit."""
+from ctypes import byref
+
+import pytest
+
+from augur_v100_b200 import abi, host, synth
+
+pytestmark = pytest.mark.gpu
+
+ROWS, COLS = 8192, 4096
+
+
+@pytest.fixture(scope="module")
+def env():
+    import torch
+    torch.cuda.set_device(0)
+    side = torch.cuda.Stream()
+    stream = host.Stream(0, side)
+    plan = host.Plan(stream, 64 << 20)
+    generator = torch.Generator(device="cuda")
+    generator.manual_seed(11)
+    planes = []
+    for _ in range(2):
+        scales = (torch.randn((ROWS, COLS // 16), device="cuda", generator=generator).abs() * 0.5).clamp(2.0 ** -9, 448.0)
+        planes.append((torch.randint(0, 256, (ROWS, COLS // 2), dtype=torch.uint8, device="cuda", generator=generator),
+                       scales.to(torch.float8_e4m3fn).view(torch.uint8).clamp(1, 0x7E)))
+    torch.cuda.synchronize()
+    yield {"torch": torch, "side": side, "stream": stream, "plan": plan, "planes": planes}
+    plan.close()
+    stream.close()
+
+
+def _repack_args(weight, planes):
+    args = abi.header(abi.RepackArgs)
+    for name, tensor in (("codes", planes[0]), ("scales", planes[1]), ("destination", weight.packed)):
+        setattr(args, name, tensor.data_ptr())
+        setattr(args, name + "_len_bytes", tensor.numel())
+    args.rows, args.cols, args.layout = ROWS, COLS, weight.layout
+    return args
+
+
+# one launch; two launches; quantiser and narrow GEMM, whose weights are fetched behind a launch that triggers early; pair GEMM
+@pytest.mark.parametrize("kind,tokens", [("stream", 3), ("split", 8), ("gemm", 16), ("gemm", 300)])
+def test_repack_then_linear(env, kind, tokens):
+    torch, side, stream, plan = env["torch"], env["side"], env["stream"], env["plan"]
+    layout = abi.LAYOUT_STREAM if kind == "stream" else abi.LAYOUT_TCGEN05
+    with torch.cuda.stream(side):
+        generator = torch.Generator(device="cuda")
+        generator.manual_seed(tokens)
+        x = torch.randn((tokens, COLS), device="cuda", generator=generator).to(torch.bfloat16)
+        weight = host.Nvfp4Sm100Weight.repack_device_planes(stream, layout, ROWS, COLS, *env["planes"][0], synth.GLOBAL_SCALE)
+        binding = {"stream": host.Nvfp4Sm100Projection, "split": host.Nvfp4Sm100TcProjection, "gemm": host.Nvfp4Sm100PrefillLinear}[kind]
+        program = binding.bind(plan, weight, x)
+        submit = abi.lib().augur_cuda_nvfp4_sm100_repack_prevalidated_submit_v1
+        args = [_repack_args(weight, planes) for planes in env["planes"]]
+        wanted = []
+        for which in range(2):
+            assert submit(stream.ordinal, stream.handle, byref(args[which])).status == abi.STATUS_OK
+            stream.synchronize()
+            program.submit_for_plan()
+            stream.synchronize()
+            wanted.append(program.out.clone())
+        got = []
+        for turn in range(40):
+            assert submit(stream.ordinal, stream.handle, byref(args[turn % 2])).status == abi.STATUS_OK
+            program.submit_for_plan()
+            got.append(program.out.clone())
+        side.synchronize()
+    assert plan.device_status() == 0
+    assert not torch.equal(wanted[0], wanted[1])
+    assert [torch.equal(out, wanted[turn % 2]) for turn, out in enumerate(got)] == [True] * 40
