@@ -639,8 +639,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
 // stacked ([terms][tokens][cols/2], one TMA tensor of terms*tokens rows), then the scale
 // regions of all terms.
 constexpr uint32_t kQuantThreads = 128;
-__global__ void __launch_bounds__(kQuantThreads) act_quant_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ destination, uint32_t tokens,
-                                 uint32_t cols, uint32_t terms, float global_scale) {
+// `x` is read by coherent loads: the launch before this one may still be writing it when this grid starts, so it is not
+// constant for the life of the grid, which is what __ldg (and a compiler's choice of it) would promise.
+__global__ void __launch_bounds__(kQuantThreads) act_quant_kernel(const uint16_t* x, uint8_t* destination, uint32_t tokens, uint32_t cols,
+                                                                  uint32_t terms, float global_scale) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");   // x may come from the launch before this one, and the destination may still be read by it
     const uint32_t groups = cols / 16;
@@ -649,7 +651,7 @@ __global__ void __launch_bounds__(kQuantThreads) act_quant_kernel(const uint16_t
     if (index >= tokens * groups) return;
     const uint32_t token = index / groups, group = index - token * groups;
     const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<uint64_t>(token) * cols + group * 16);
-    const uint4 lo = __ldg(src), hi = __ldg(src + 1);
+    const uint4 lo = __ldcg(src), hi = __ldcg(src + 1);
     const uint32_t words[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
     float2 residual[8];   // pairs of neighbouring elements, as the two-wide F32 instructions take them
 #pragma unroll

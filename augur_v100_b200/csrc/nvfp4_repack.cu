@@ -41,6 +41,10 @@ uint64_t layout_extent(uint32_t layout, uint32_t rows, uint32_t cols) {
 // per thread with byte gathers and a bit-by-bit permutation took 61.5 us for the STREAM layout of a 17408 x 5120
 // weight, and 4-byte copies 35 us for the TCGEN05 layout.
 //
+// The planes are read by coherent loads and no pointer is __restrict__: the launch before may still be writing them when these
+// grids start, so they are not constant for the grids' life, as __ldg (or a compiler that makes it of such pointers) would
+// have them. STREAM goes through the first-level cache, which gathers its 8-byte pieces of scale rows (17408 x 5120: 23.3 us, 24.1
+// past it); TCGEN05, whose pieces are whole sectors, past it (16.9 us, 17.4 through it).
 // Neither lets the launch behind it start early (griddepcontrol.launch_dependents): every kernel of this library fetches its
 // first weights before its own griddepcontrol.wait, and so may the launch behind an act_quant or a split, which do let theirs
 // start early. A launch of this library behind a repack starts when all of the repack's threads are through with written_out().
@@ -75,8 +79,8 @@ __device__ __forceinline__ void quad_transpose(uint32_t (&v)[4], uint32_t t4) {
 // (Having every lane of a quad read the whole row instead, four times the L1 traffic, took 26.5 us for 17408 x 5120.)
 // The eight warps of a CTA take neighbouring blocks of one row group, so the rows are read in runs of 512 bytes.
 __global__ void __launch_bounds__(kRepackWarps * 32)
-repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restrict__ scales_a, const uint8_t* __restrict__ codes_b,
-                     const uint8_t* __restrict__ scales_b, uint8_t* __restrict__ destination, uint32_t blocks, uint32_t cols, bool pair) {
+repack_stream_kernel(const uint8_t* codes_a, const uint8_t* scales_a, const uint8_t* codes_b, const uint8_t* scales_b, uint8_t* destination,
+                     uint32_t blocks, uint32_t cols, bool pair) {
     const uint32_t block = blockIdx.x * kRepackWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (block >= blocks) return;
@@ -88,8 +92,8 @@ repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restr
     for (uint32_t t = 0; t < 2; ++t) {
         const uint32_t row = (pair ? group * 16 : group * 32 + t * 16) + g;
         const uint8_t* from = ((pair && t) ? codes_b : codes_a) + static_cast<uint64_t>(row) * (cols / 2) + kb * 64 + t4 * 16;
-        piece[t][0] = __ldg(reinterpret_cast<const uint4*>(from));
-        piece[t][1] = __ldg(reinterpret_cast<const uint4*>(from + static_cast<uint64_t>(8) * (cols / 2)));
+        piece[t][0] = *reinterpret_cast<const uint4*>(from);
+        piece[t][1] = *reinterpret_cast<const uint4*>(from + static_cast<uint64_t>(8) * (cols / 2));
     }
     // scales: 16 bytes per (tile, g) = k-steps 0..7 of rows g and g + 8, interleaved; lanes 0..15 take one each
     uint2 scale_top = make_uint2(0, 0), scale_bottom = make_uint2(0, 0);
@@ -98,8 +102,8 @@ repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restr
         const uint8_t* from = ((pair && t) ? scales_b : scales_a) + static_cast<uint64_t>(row) * (cols / 16) + kb * 8;
         const uint8_t* below = from + static_cast<uint64_t>(8) * (cols / 16);
         // rows of scales start on 8-byte boundaries (cols is a multiple of 128), the plane itself only on a 4-byte one
-        scale_top = make_uint2(__ldg(reinterpret_cast<const uint32_t*>(from)), __ldg(reinterpret_cast<const uint32_t*>(from) + 1));
-        scale_bottom = make_uint2(__ldg(reinterpret_cast<const uint32_t*>(below)), __ldg(reinterpret_cast<const uint32_t*>(below) + 1));
+        scale_top = make_uint2(reinterpret_cast<const uint32_t*>(from)[0], reinterpret_cast<const uint32_t*>(from)[1]);
+        scale_bottom = make_uint2(reinterpret_cast<const uint32_t*>(below)[0], reinterpret_cast<const uint32_t*>(below)[1]);
     }
     uint4* out = reinterpret_cast<uint4*>(destination + static_cast<uint64_t>(block) * kStreamBlockBytes);
 #pragma unroll
@@ -144,7 +148,7 @@ repack_stream_kernel(const uint8_t* __restrict__ codes_a, const uint8_t* __restr
 constexpr uint32_t kRepackCopyBytes = kRepackWarps * 32 * 64;   // of one CTA
 
 template <uint32_t kAtoms>
-__device__ __forceinline__ void retile_scales(const uint8_t* __restrict__ scales, uint8_t* __restrict__ out, uint32_t rows, uint32_t cols,
+__device__ __forceinline__ void retile_scales(const uint8_t* scales, uint8_t* out, uint32_t rows, uint32_t cols,
                                               uint32_t run, uint32_t lane) {
     const uint32_t atoms_per_row_block = cols / 64, runs = atoms_per_row_block / kAtoms;
     const uint32_t row_block = run / runs, first = (run - row_block * runs) * kAtoms;
@@ -158,13 +162,13 @@ __device__ __forceinline__ void retile_scales(const uint8_t* __restrict__ scales
         for (uint32_t a = 0; a < kAtoms; ++a) word[j][a] = 0;   // rows past the end: padding of the last row block
         if (row < rows) {
             if (kAtoms == 4) {
-                const uint4 v = __ldg(reinterpret_cast<const uint4*>(from));
+                const uint4 v = __ldcg(reinterpret_cast<const uint4*>(from));
                 word[j][0] = v.x; word[j][1 % kAtoms] = v.y; word[j][2 % kAtoms] = v.z; word[j][3 % kAtoms] = v.w;
             } else if (kAtoms == 2) {
-                const uint2 v = __ldg(reinterpret_cast<const uint2*>(from));
+                const uint2 v = __ldcg(reinterpret_cast<const uint2*>(from));
                 word[j][0] = v.x; word[j][1 % kAtoms] = v.y;
             } else {
-                word[j][0] = __ldg(from);
+                word[j][0] = __ldcg(from);
             }
         }
     }
@@ -174,8 +178,8 @@ __device__ __forceinline__ void retile_scales(const uint8_t* __restrict__ scales
 }
 
 __global__ void __launch_bounds__(kRepackWarps * 32)
-repack_tcgen05_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restrict__ scales, uint8_t* __restrict__ destination,
-                      uint32_t rows, uint32_t cols, uint32_t scale_ctas, uint32_t run_atoms) {
+repack_tcgen05_kernel(const uint8_t* codes, const uint8_t* scales, uint8_t* destination, uint32_t rows, uint32_t cols, uint32_t scale_ctas,
+                      uint32_t run_atoms) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint64_t code_bytes = tcgen05_codes_bytes(rows, cols);
     if (blockIdx.x < scale_ctas) {   // the scales first: their loads are the scattered ones
@@ -193,7 +197,7 @@ repack_tcgen05_kernel(const uint8_t* __restrict__ codes, const uint8_t* __restri
     uint4 v[4];
 #pragma unroll
     for (uint32_t i = 0; i < 4; ++i) {
-        if (first + i * kRepackWarps * 32 < pieces) v[i] = __ldg(from + first + i * kRepackWarps * 32);
+        if (first + i * kRepackWarps * 32 < pieces) v[i] = __ldcg(from + first + i * kRepackWarps * 32);
     }
 #pragma unroll
     for (uint32_t i = 0; i < 4; ++i) {

@@ -71,3 +71,38 @@ def test_repack_then_linear(env, kind, tokens):
     assert plan.device_status() == 0
     assert not torch.equal(wanted[0], wanted[1])
     assert [torch.equal(out, wanted[turn % 2]) for turn, out in enumerate(got)] == [True] * 40
+
+
+# The quantiser reads what the launch before it writes, while that launch still runs: narrow GEMM, pair GEMM with a narrow tail,
+# small-token linear.
+@pytest.mark.parametrize("tokens,producer", [(48, "gemm"), (300, "gemm"), (8, "split")])
+def test_linear_then_quantiser(env, tokens, producer):
+    torch, side, stream, plan = env["torch"], env["side"], env["stream"], env["plan"]
+    with torch.cuda.stream(side):
+        generator = torch.Generator(device="cuda")
+        generator.manual_seed(tokens)
+        inputs = [torch.randn((tokens, COLS), device="cuda", generator=generator).to(torch.bfloat16) for _ in range(2)]
+        x = inputs[0].clone()
+        weight = host.Nvfp4Sm100Weight.repack_device_planes(stream, abi.LAYOUT_TCGEN05, ROWS, COLS, *env["planes"][0], synth.GLOBAL_SCALE)
+        second = host.Nvfp4Sm100Weight.repack_device_planes(
+            stream, abi.LAYOUT_TCGEN05, COLS, ROWS, env["planes"][1][0].view(COLS, ROWS // 2), env["planes"][1][1].view(COLS, ROWS // 16), synth.GLOBAL_SCALE)
+        first = {"gemm": host.Nvfp4Sm100PrefillLinear, "split": host.Nvfp4Sm100TcProjection}[producer].bind(plan, weight, x)
+        then = host.Nvfp4Sm100PrefillLinear.bind(plan, second, first.out, terms=3)
+        wanted = []
+        for value in inputs:
+            x.copy_(value)
+            first.submit_for_plan()
+            stream.synchronize()
+            then.submit_for_plan()
+            stream.synchronize()
+            wanted.append(then.out.clone())
+        got = []
+        for turn in range(40):
+            x.copy_(inputs[turn % 2])
+            first.submit_for_plan()
+            then.submit_for_plan()
+            got.append(then.out.clone())
+        side.synchronize()
+    assert plan.device_status() == 0
+    assert not torch.equal(wanted[0], wanted[1])
+    assert [torch.equal(out, wanted[turn % 2]) for turn, out in enumerate(got)] == [True] * 40
