@@ -129,10 +129,14 @@ std::atomic<uint32_t> g_gemv_clusters[64][kMaxClusterSize + 1];
 // the CTA stages them; the exchange within a cluster takes 1.2 us and 0.15 us per row group, the one through scratch 2.6 us.
 // (1024 x 5120 at one token row: 6.8 us in whole groups, 6.2, 5.6 and 5.7 with 2, 4 and 8 CTAs per cluster; 17408 x 5120: 15.6
 // in whole groups, 16.8 in pairs of CTAs, which have the same number of blocks.)
-GemvGeometry geometry(uint32_t groups, uint32_t cols, uint32_t tokens, bool input_is_staged, const augur_cuda_nvfp4_sm100_plan_v1* plan) {
+// `room`: bytes of scratch for the slots of the split without clusters. Fewer CTAs need fewer of them: with at most as many per
+// slab as there are row groups, a group has two shares per slab.
+GemvGeometry geometry(uint32_t groups, uint32_t cols, uint32_t tokens, bool input_is_staged, const augur_cuda_nvfp4_sm100_plan_v1* plan,
+                      uint64_t room) {
     const uint32_t kb_count = cols / kStreamBlockK, stage_ns = input_is_staged ? 18 : 20 + 6 * tokens;
     auto stream_ns = [&](uint64_t blocks, uint32_t kbs) { return (blocks > kWarps ? blocks : kWarps) * 1100 / kWarps + kbs * stage_ns; };
     GemvGeometry best = plain_geometry(groups, cols, plan->sm_count);
+    if (best.partial_bytes > room) best = plain_geometry(groups, cols, groups * best.slabs);
     const uint32_t plain_kbs = (kb_count + best.slabs - 1) / best.slabs;
     uint64_t least = best.aligned ? stream_ns(static_cast<uint64_t>((groups + best.ctas_per_slab - 1) / best.ctas_per_slab) * plain_kbs, plain_kbs)
                                   : stream_ns(static_cast<uint64_t>(groups) * plain_kbs / best.ctas_per_slab + 1, plain_kbs) + 2600;
@@ -1147,7 +1151,7 @@ void launch_gemv(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* pl
                  const augur_cuda_nvfp4_sm100_gemv_args_v1* a, uint32_t member, uint64_t partial_offset,
                  uint64_t staged_out_offset = 0, bool input_is_staged = false, const ExchangeTable* tp = nullptr) {
     const uint32_t groups = a->epilogue == AUGUR_NVFP4_SM100_EPILOGUE_SWIGLU_BF16 ? a->rows / 16 : a->rows / 32;
-    const GemvGeometry g = tp ? plain_geometry(groups, a->cols, plan->sm_count) : geometry(groups, a->cols, a->tokens, input_is_staged, plan);
+    const GemvGeometry g = tp ? plain_geometry(groups, a->cols, plan->sm_count) : geometry(groups, a->cols, a->tokens, input_is_staged, plan, UINT64_MAX);
     GemvParams p = make_params(plan, a, g, reinterpret_cast<uint32_t*>(plan->scratch + member * kCounterRegionBytes), plan->scratch + partial_offset,
                                reinterpret_cast<float*>(plan->scratch + partial_offset + g.staged_bytes), input_is_staged);
     p.staged_out = staged_out_offset ? reinterpret_cast<uint16_t*>(plan->scratch + staged_out_offset) : nullptr;
@@ -1613,8 +1617,9 @@ bool check_norm_group(int32_t d, augur_cuda_stream_t s, const augur_cuda_nvfp4_s
     }
     r[n++] = plan_scratch_range(plan);
     if (!all_disjoint(r, n)) return false;
-    // staged activations once, then the slots of the split without clusters over all members
-    if (group_partial_offset(a->cols) + plain_geometry(group_row_groups(a), a->cols, plan->sm_count).partial_bytes > plan->scratch_bytes) return false;
+    // staged activations once, then the slots of the split without clusters over all members, on as many CTAs as they fit for
+    const uint32_t groups = group_row_groups(a), slabs = plain_geometry(groups, a->cols, plan->sm_count).slabs;
+    if (group_partial_offset(a->cols) + plain_geometry(groups, a->cols, groups * slabs).partial_bytes > plan->scratch_bytes) return false;
     return !full || inspect_device_ranges(d, r, n - 1, failure);
 }
 }  // namespace
@@ -1653,9 +1658,10 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_norm_grou
     augur_cuda_result_v1 result = submitted();
     if (result.status != AUGUR_CUDA_STATUS_OK) return result;
     // all projections of the group in one grid; they copy the staged fragments in and stage nothing themselves
-    const GemvGeometry g = geometry(group_row_groups(a), a->cols, a->tokens, true, plan);
+    const uint64_t partial_offset = group_partial_offset(a->cols);
+    const GemvGeometry g = geometry(group_row_groups(a), a->cols, a->tokens, true, plan, plan->scratch_bytes - partial_offset);
     GemvParams p = make_params(plan, &a->projections[0], g, reinterpret_cast<uint32_t*>(plan->scratch), fragments,
-                               reinterpret_cast<float*>(plan->scratch + group_partial_offset(a->cols)), true);
+                               reinterpret_cast<float*>(plan->scratch + partial_offset), true);
     for (uint32_t i = 1; i < a->count; ++i) {
         p.member[i] = make_member(&a->projections[i], p.member[i - 1].first_group + p.member[i - 1].rows / 32);
     }

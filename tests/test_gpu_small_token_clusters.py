@@ -52,3 +52,26 @@ def test_group_members_straddle_clusters(ctx, cols, rows, stored):  # noqa: F811
     for out, r, keep, planes in zip(program.outputs, rows, stored, made):
         y64 = oracle.linear_f64(*planes, r, cols, staged, threads=oracle.max_threads())
         assert rel_error(bits_from_torch_bf16(out), np.ascontiguousarray(y64.reshape(tokens, r)[:, : keep or r])) <= TOLERANCE
+
+
+# Scratch that holds the members' slots when every member has its share of the SMs, but not the slots of all SMs over the union
+# of the members' row groups: such a plan is enough. In clusters, which need no slots; nine slabs, through scratch.
+@pytest.mark.parametrize("cols,rows,scratch", [(10496, (768, 768), 594176), (41728, (160, 160, 160), 1075200)])
+def test_group_in_little_scratch(ctx, cols, rows, scratch):  # noqa: F811
+    torch, tokens = ctx["torch"], 5
+    made = [synth.make_weight(cols + i, 96, "w", r, cols) for i, r in enumerate(rows)]
+    weights = [host.Nvfp4Sm100Weight.upload_checkpoint_nvfp4(ctx["stream"], abi.LAYOUT_STREAM, r, cols, *planes) for r, planes in zip(rows, made)]
+    x = torch.from_numpy(np.random.default_rng(cols).standard_normal((tokens, cols)).astype(np.float32)).to(ctx["device"])
+    gain = torch.ones(cols, dtype=torch.float32, device=ctx["device"])
+    torch.cuda.synchronize()
+    plan = host.Plan(ctx["stream"], scratch)
+    program = host.Nvfp4Sm100NormGroupProgram.bind(plan, weights, x, gain)
+    for _ in range(2):       # the counters are clean for the second
+        program.submit_for_plan()
+        ctx["stream"].synchronize()
+        assert plan.device_status() == 0
+        staged = bits_from_torch_bf16(program.staged)
+        for out, r, planes in zip(program.outputs, rows, made):
+            y64 = oracle.linear_f64(*planes, r, cols, staged, threads=oracle.max_threads())
+            assert rel_error(bits_from_torch_bf16(out), y64.reshape(tokens, r)) <= TOLERANCE
+    plan.close()
