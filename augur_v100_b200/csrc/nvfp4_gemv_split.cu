@@ -76,8 +76,7 @@ split_rows_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ split, u
     uint32_t largest = 0;
 #pragma unroll
     for (uint32_t i = 0; i < kSplitThreads / 32; ++i) largest = max(largest, maxima[i]);
-    // term 0 of the row has the global scale 2^(A - 155), term 7 2^(A - 134): all normal f32 numbers
-    const uint32_t a = min(max(largest >> 7, 40u), 250u);
+    const uint32_t a = min(max(largest >> 7, 1u), 254u);   // any finite row, subnormal values with the smallest normal ones
     if (threadIdx.x == 0 && blockIdx.x == 0) anchors[token] = largest >= 0x7f80u ? kNonFinite : a;   // the row's outputs are NaN then
     if (lane == 0) row_anchor[token] = a;   // every warp the same value
     __syncwarp();
@@ -280,13 +279,15 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
     const bool epilogue = warp >= 4;
     const uint32_t task = warp - 4, quadrant = task & 3, token0 = (task >> 2) * 4;   // quadrant == warp % 4: the tensor-memory lanes it may read
     float y[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    float scale[4];
+    float scale[2][4];   // term 0 of a row has the global scale 2^(A - 155), which need not be an F32 number: as the product of two that are
     if (epilogue) {
         asm volatile("griddepcontrol.wait;" ::: "memory");   // the anchors; and nothing is written while an earlier kernel may still read it
 #pragma unroll
         for (uint32_t j = 0; j < 4; ++j) {
-            const uint32_t a = token0 + j < p.tokens ? __ldcg(p.anchors + token0 + j) : 40u;
-            scale[j] = __uint_as_float(a == kNonFinite ? 0x7fc00000u : (a - 28) << 23);
+            const uint32_t a = token0 + j < p.tokens ? __ldcg(p.anchors + token0 + j) : 1u;
+            const int exponent = static_cast<int>(a) - 155, half = exponent / 2;
+            scale[0][j] = __uint_as_float(static_cast<uint32_t>(127 + half) << 23);
+            scale[1][j] = __uint_as_float(a == kNonFinite ? 0x7fc00000u : static_cast<uint32_t>(127 + exponent - half) << 23);
         }
         if (mbar_wait(acc_full, 0, abort_flag, p.status_word, kErrStreamAccFull)) {
             tc_fence_after();
@@ -303,7 +304,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
                     sum = fmaf(__uint_as_float(v[term][j]), factor, sum);
                     factor *= 8.0f;
                 }
-                y[j] = sum * scale[j];
+                y[j] = sum * scale[0][j] * scale[1][j];
             }
         }
     }

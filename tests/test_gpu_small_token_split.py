@@ -38,6 +38,28 @@ def test_split_linear_edges(ctx, rows, cols, tokens):  # noqa: F811
     assert rel_error(bits_from_torch_bf16(other.out), other64) <= TOLERANCE
 
 
+# The largest BF16 exponents (one element of a row far above the rest) and the smallest, subnormal rows among them, with block
+# and global scales that keep the sums inside F32 and the outputs normal.
+@pytest.mark.parametrize("exponents,block_scale,glob", [((122, 123, 124, 125, 126, 127), 0x18, 1.0 / 448.0),
+                                                        ((-86, -88, -99, -110, -124, -130), 0x70, 24.0)])
+def test_split_covers_every_exponent(ctx, exponents, block_scale, glob):  # noqa: F811
+    rows, cols = 256, 1088
+    generator = np.random.default_rng(block_scale)
+    codes = generator.integers(0, 256, (rows, cols // 2), dtype=np.uint8)
+    scales = np.full((rows, cols // 16), block_scale, dtype=np.uint8)
+    x = generator.standard_normal((len(exponents), cols)) * 2.0 ** (np.array(exponents)[:, None] - 8)
+    x[:, 700] = 1.5 * 2.0 ** np.array(exponents)
+    x_bits = synth.f32_to_bf16_bits(x.astype(np.float32))
+    weight = host.Nvfp4Sm100Weight.upload_checkpoint_nvfp4(ctx["stream"], abi.LAYOUT_TCGEN05, rows, cols, codes, scales, glob)
+    projection = host.Nvfp4Sm100TcProjection.bind(ctx["plan"], weight, torch_bf16_from_bits(x_bits, ctx["device"]))
+    projection.submit_for_plan()
+    ctx["stream"].synchronize()
+    y64 = oracle.linear_f64(codes, scales, glob, rows, cols, x_bits, threads=oracle.max_threads()).reshape(len(exponents), rows)
+    got = bits_from_torch_bf16(projection.out).reshape(len(exponents), rows)
+    for row, exponent in enumerate(exponents):
+        assert rel_error(got[row], y64[row]) <= TOLERANCE, exponent
+
+
 # From 2^25 weights on `Nvfp4Sm100Linear` binds this kernel.
 def test_linear_dispatch_by_size(ctx):  # noqa: F811
     rows, cols, tokens = 32768, 1024, 6
