@@ -226,7 +226,7 @@ __device__ __forceinline__ void job_scales(const TcParams& p, uint32_t job, uint
     if (worker < 8) {
         const uint32_t largest = *static_cast<volatile uint32_t*>(p.header + kHeaderRowMax + 8 * job + worker) >> 16;
         // term 0 of the row has the global scale 2^(A - 155), term 7 2^(A - 134): all normal f32 numbers
-        const uint32_t a = min(max(largest >> 7, 40u), 250u);
+        const uint32_t a = min(max(largest >> 7, 40u), 254u);
         float scale = __uint_as_float((a - 28) << 23);
         if (largest >= 0x7f80u) scale = __uint_as_float(0x7fc00000u);   // a NaN or infinity in the row: the row's outputs are NaN
         term_scale[8 * job + worker] = scale;
@@ -688,7 +688,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
                 most = max(most, __shfl_xor_sync(0xffffffffu, most, 1));
                 if (lane == 0) {
                     // term 0 of the row has the global scale 2^(A - 155), term 7 2^(A - 134): all normal f32 numbers
-                    const uint32_t a = min(max((most >> 7) + 3, 40u), 250u);
+                    const uint32_t a = min(max((most >> 7) + 3, 40u), 254u);
                     anchor[token] = a;
                     term_scale[token] = __uint_as_float((a - 28) << 23);
                 }
@@ -771,13 +771,13 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             workers_sync();
             if (st.keeps) {
                 // this CTA's maxima as one word of its own: exponent fields, one byte per token row (40 at least, so the
-                // word is never 0; 251 for a non-finite value). Nothing has to be visible with it, so no release.
+                // word is never 0; 255 for a non-finite value). Nothing has to be visible with it, so no release.
                 if (worker < 32) {   // the first worker warp: lanes 0..7 a token row each, then the eight bytes gathered in lane 0
                     uint32_t low = 0, high = 0;
                     if (lane < 8) {
                         uint32_t field = 0;
                         for (uint32_t k = 0; k < 4; ++k) field = max(field, (gathered[(lane >> 2) * 4 + k] >> (8 * (lane & 3))) & 0xffu);
-                        const uint32_t byte = (field >= 255 ? 251u : min(max(field, 40u), 250u)) << (8 * (lane & 3));
+                        const uint32_t byte = max(field, 40u) << (8 * (lane & 3));
                         low = lane < 4 ? byte : 0;
                         high = lane < 4 ? 0 : byte;
                     }
@@ -854,8 +854,8 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
                     uint32_t field = 0;
                     for (uint32_t k = 0; k < 8; ++k) field = max(field, (gathered[k * 2 + (worker >> 2)] >> (8 * (worker & 3))) & 0xffu);
                     // term 0 of the row has the global scale 2^(A - 155), term 7 2^(A - 134): all normal f32 numbers
-                    const uint32_t a = min(field, 250u);
-                    term_scale[8 * st.feeds + worker] = field > 250 ? __uint_as_float(0x7fc00000u) : __uint_as_float((a - 28) << 23);
+                    const uint32_t a = min(field, 254u);
+                    term_scale[8 * st.feeds + worker] = field > 254 ? __uint_as_float(0x7fc00000u) : __uint_as_float((a - 28) << 23);
                     anchor[8 * st.feeds + worker] = a;
                 }
                 workers_sync();

@@ -329,3 +329,34 @@ def test_one_gate_up_tile_far_larger_than_the_others(ctx):
         assert plan.device_status() == 0
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("hidden,inter", [(1024, 512), (128, 17408)])
+def test_block_with_an_intermediate_of_the_largest_exponents(ctx, hidden, inter):
+    # Every row's intermediate reaches 2^124 to 2^127 (the anchor of the second product), with block scales that keep its sums in
+    # F32. Gate|up tiles cut along k (the intermediate is read back) and whole ones (split from registers).
+    tokens = 4
+    host = ctx["host"]
+    small = lambda name, rows, cols: (synth.make_weight(15, 97, name, rows, cols)[0], np.full((rows, cols // 16), 0x08, dtype=np.uint8), 1.0 / 448.0)
+    gate, up, down = small("gate", inter, hidden), small("up", inter, hidden), small("down", hidden, inter)
+    base = np.random.default_rng(inter).standard_normal((tokens, hidden)) * 2.0 ** 40
+    h64, _ = oracle.mlp_f64(gate, up, down, hidden, inter, synth.f32_to_bf16_bits(base.astype(np.float32)), threads=oracle.max_threads())
+    # the intermediate grows with the square of the input: gates this large are passed or cut to zero
+    grow = np.floor((126 - np.log2(np.abs(h64).max(axis=1))) / 2)
+    x_bits = synth.f32_to_bf16_bits((base * 2.0 ** grow[:, None]).astype(np.float32))
+    h64, _ = oracle.mlp_f64(gate, up, down, hidden, inter, x_bits, threads=oracle.max_threads())
+    assert np.all(np.abs(h64).max(axis=1) >= 2.0 ** 124) and np.abs(h64).max() < 2.0 ** 126.5
+    gate_up_w = host.upload_gate_up_interleaved(ctx["stream"], inter, hidden, *gate, *up)
+    down_w = host.Nvfp4Sm100Weight.upload_checkpoint_nvfp4(ctx["stream"], abi.LAYOUT_TCGEN05, hidden, inter, *down)
+    plan = host.Plan(ctx["stream"], host.mlp_tc_scratch_bytes(hidden, inter))
+    program = host.Nvfp4Sm100TcFfnProgram.bind(plan, gate_up_w, down_w, torch_bf16_from_bits(x_bits, ctx["device"]))
+    program.submit_for_plan()
+    ctx["stream"].synchronize()
+    assert plan.device_status() == 0
+    plan.close()
+    h_bits = bits_from_torch_bf16(program.intermediate).reshape(tokens, inter)
+    got = bits_from_torch_bf16(program.out).reshape(tokens, hidden)
+    y64 = oracle.linear_f64(*down, hidden, inter, h_bits, threads=oracle.max_threads()).reshape(tokens, hidden)   # of the stored intermediate
+    for row in range(tokens):
+        assert rel_error(h_bits[row], h64[row]) <= TOLERANCE
+        assert rel_error(got[row], y64[row]) <= TOLERANCE
