@@ -373,10 +373,13 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
 }
 
 // ---- host side ----------------------------------------------------------------------------------
-// Clusters of `parts` CTAs that the device holds at once (clusters do not fill its SMs evenly: 148 of 2, 93 of 3, 71 of 4,
-// 56 of 5, 45 of 6, 37 of 7, 33 of 8 on a B200). Asked once per device; bind time fills the table. The question is put for
-// a kernel of the same size that uses no tensor memory: for one that does the runtime always answers for one CTA per
-// SM, although two fit when each allocates half of it.
+// Clusters of `parts` CTAs that a launch may count on to run at once. The device holds 148 of 2, 93 of 3, 71 of 4, 56 of 5, 45 of
+// 6, 37 of 7 and 33 of 8 on a B200 (they do not fill its SMs evenly); of those larger than 2 a sixteenth is left out, because they
+// come to lie badly while the launch before still has CTAs of its own on the SMs, and a cluster that finds no place then waits for
+// a whole wave (small-token linear at one token row: 56 clusters of 5 for 7168 x 4736 13.3 us, 56 of 4 9.2; 93 of 3 for
+// 11904 x 5120 16.7 us, 93 of 2 11.1). Asked once per device; bind time fills the table. The question is put for a kernel of
+// the same size that uses no tensor memory: for one that does the runtime always answers for one CTA per SM, although
+// two fit when each allocates half of it.
 __global__ void __launch_bounds__(kNarrowBound, 2) narrow_shape_kernel() {}
 
 struct NarrowDevice {
@@ -406,6 +409,7 @@ uint32_t two_cta_clusters(int32_t ordinal, uint32_t parts) {
         cudaGetLastError();
         found = 1;
     }
+    if (parts > 2) found -= found / 16;
     known.store(static_cast<uint32_t>(found));
     return static_cast<uint32_t>(found);
 }

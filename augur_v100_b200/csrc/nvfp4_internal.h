@@ -125,7 +125,7 @@ cudaError_t gemm_configure_device();
 cudaError_t gemv_tc_configure_device();
 cudaError_t gemm_narrow_configure_device();
 cudaError_t gemv_split_configure_device();
-// Clusters of `parts` CTAs of 384 threads and 113 KB of shared memory (two per SM) that the device holds at once.
+// Clusters of `parts` CTAs of 384 threads and 113 KB of shared memory (two per SM) that a launch may count on to run at once.
 uint32_t two_cta_clusters(int32_t ordinal, uint32_t parts);
 // A small-token linear on tensor memory as two launches (nvfp4_gemv_split.cu); `split`: split_bytes(cols) of plan scratch.
 augur_cuda_result_v1 launch_split_linear(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
