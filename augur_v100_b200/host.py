@@ -298,6 +298,12 @@ def gemv_tc_scratch_bytes(rows: int, cols: int, epilogue: int = abi.EPILOGUE_LIN
     return int(out.value)
 
 
+def gemv_tc_linear_scratch_bytes(cols: int) -> int:
+    """What a plan has to hold for one `gemv_tc` linear: the two counter regions and the eight digits of the activations.
+    (`gemv_tc_scratch_bytes` is larger: it also covers a member of the one-launch block.)"""
+    return 2 * 4 * 16384 + -(-cols // 256) * (8192 + 2048)
+
+
 class Nvfp4Sm100TcProjection(Nvfp4Sm100Projection):
     """A retained small-token projection on the tensor-memory path: the weight is in the tcgen05 layout
     (the one the prefill GEMM uses; for the SwiGLU epilogue the interleaved gate|up tensor of
@@ -708,15 +714,26 @@ class Nvfp4Sm100Linear:
     """One weight matrix, any number of token rows: the dispatch a model runtime does per call site.
 
     Keeps the weight in both hot layouts (the small-token stream layout and the tcgen05 layout) and
-    binds the kernel its shape class calls for: tokens <= 8 -> `Nvfp4Sm100Projection`, otherwise
-    `Nvfp4Sm100PrefillLinear` (activation quantiser with `terms` residual terms, then the block-scaled
-    GEMM). Bindings are made per (input, output) pair, exactly like the classes it chooses between.
+    binds the kernel its shape class calls for: tokens <= 8 -> `Nvfp4Sm100Projection`, or for the larger
+    weights `Nvfp4Sm100TcProjection`, otherwise `Nvfp4Sm100PrefillLinear` (activation quantiser with `terms`
+    residual terms, then the block-scaled GEMM). Bindings are made per (input, output) pair, exactly like the
+    classes it chooses between.
+
+    Both small-token kernels take every BF16 row. The tensor-memory kernel holds an element exactly down to
+    2^-14 of the largest of its 16-element group and to 2^-23 of that below (groups under 2^-17 of their
+    row's largest, to 2^-39 of the latter), and a row with an infinity or a NaN gives NaN in all its outputs.
     """
 
-    # From this many weights on the tensor-memory kernel is the faster of the two small-token kernels: below, its second
-    # launch costs more than the integer work per weight that it saves (B200, 8 token rows: 4096 x 5120 9.5 us against 9.3 on
-    # mma.sync, 5120 x 7808 12.3 / 12.2, 9856 x 6016 12.0 / 15.9, 17408 x 5120 14.8 / 17.1).
     TENSOR_MEMORY_WEIGHTS = 1 << 25
+    TENSOR_MEMORY_MAX_ROWS = 1 << 18        # what the entry takes
+
+    def _on_tensor_memory(self, plan: Plan) -> bool:
+        """From 2^25 weights on the tensor-memory kernel is the faster of the two: below, its second launch costs more than the
+        integer work per weight that it saves (B200, 8 token rows: 4096 x 5120 9.5 us against 9.3 on mma.sync, 17408 x 5120 14.8
+        / 17.1). A plan that does not hold its scratch keeps the other; any other fault of the binding is the caller's to see."""
+        if self.rows % 128 != 0 or self.rows > self.TENSOR_MEMORY_MAX_ROWS or self.rows * self.cols < self.TENSOR_MEMORY_WEIGHTS:
+            return False
+        return plan.snapshot().scratch_len_bytes >= gemv_tc_linear_scratch_bytes(self.cols)
 
     def __init__(self, stream: Stream, rows: int, cols: int, codes, scales, global_scale: float):
         self.rows, self.cols = rows, cols
@@ -726,10 +743,7 @@ class Nvfp4Sm100Linear:
     def bind(self, plan: Plan, x: torch.Tensor, out: torch.Tensor | None = None, terms: int = 3,
              activation_global_scale: float = 2.0 ** -8):
         if classify_tokens(x.shape[0]) == SHAPE_SMALL_BATCH:
-            if self.rows % 128 == 0 and self.rows * self.cols >= self.TENSOR_MEMORY_WEIGHTS:
-                try:
-                    return Nvfp4Sm100TcProjection.bind(plan, self.wide, x, out)
-                except CudaRuntimeError:
-                    pass        # a plan with less scratch than it needs; any other fault is reported below
+            if self._on_tensor_memory(plan):
+                return Nvfp4Sm100TcProjection.bind(plan, self.wide, x, out)
             return Nvfp4Sm100Projection.bind(plan, self.small, x, out)
         return Nvfp4Sm100PrefillLinear.bind(plan, self.wide, x, out, terms=terms, activation_global_scale=activation_global_scale)

@@ -74,3 +74,43 @@ def test_linear_dispatch_by_size(ctx):  # noqa: F811
     assert plan.device_status() == 0 and isinstance(binding, host.Nvfp4Sm100TcProjection)
     assert rel_error(bits_from_torch_bf16(binding.out), y64) <= TOLERANCE
     plan.close()
+
+
+# A plan of one byte less than the kernel's scratch keeps the general kernel, as does a weight of more rows than the kernel takes; a
+# fault of the binding itself is raised and does not change the kernel.
+def test_linear_dispatch_by_scratch_rows_and_faults(ctx):  # noqa: F811
+    rows, cols, tokens = 32768, 1024, 5
+    codes, scales, glob = synth.make_weight(8, 95, "w", rows, cols)
+    linear = host.Nvfp4Sm100Linear(ctx["stream"], rows, cols, codes, scales, glob)
+    x_bits = synth.make_activation(8, 95, "x", tokens, cols)
+    x = torch_bf16_from_bits(x_bits, ctx["device"])
+    y64 = oracle.linear_f64(codes, scales, glob, rows, cols, x_bits, threads=oracle.max_threads())
+    need = host.gemv_tc_linear_scratch_bytes(cols)
+    small_need = host.gemv_scratch_bytes(rows, cols)
+    enough = host.Plan(ctx["stream"], need)
+    binding = linear.bind(enough, x)
+    assert isinstance(binding, host.Nvfp4Sm100TcProjection)
+    binding.submit_for_plan()
+    ctx["stream"].synchronize()
+    assert rel_error(bits_from_torch_bf16(binding.out), y64) <= TOLERANCE
+    less = host.Plan(ctx["stream"], need - 256)
+    with pytest.raises(host.CudaRuntimeError):
+        host.Nvfp4Sm100TcProjection.bind(less, linear.wide, x)
+    assert not linear._on_tensor_memory(less)
+    roomy = host.Plan(ctx["stream"], max(need, small_need))
+    linear.wide.global_scale = float("nan")       # concerns this kernel's copy of the weight only
+    with pytest.raises(host.CudaRuntimeError):
+        linear.bind(roomy, x)
+    for plan in (enough, less, roomy):
+        plan.close()
+    rows, cols = (1 << 18) + 128, 128
+    codes, scales, glob = synth.make_weight(9, 95, "w", rows, cols)
+    linear = host.Nvfp4Sm100Linear(ctx["stream"], rows, cols, codes, scales, glob)
+    x_bits = synth.make_activation(9, 95, "x", tokens, cols)
+    plan = host.Plan(ctx["stream"], host.gemv_scratch_bytes(rows, cols))
+    binding = linear.bind(plan, torch_bf16_from_bits(x_bits, ctx["device"]))
+    binding.submit_for_plan()
+    ctx["stream"].synchronize()
+    y64 = oracle.linear_f64(codes, scales, glob, rows, cols, x_bits, threads=oracle.max_threads())
+    assert type(binding) is host.Nvfp4Sm100Projection and rel_error(bits_from_torch_bf16(binding.out), y64) <= TOLERANCE
+    plan.close()
