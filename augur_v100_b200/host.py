@@ -727,13 +727,18 @@ class Nvfp4Sm100Linear:
     TENSOR_MEMORY_WEIGHTS = 1 << 25
     TENSOR_MEMORY_MAX_ROWS = 1 << 18        # what the entry takes
 
-    def _on_tensor_memory(self, plan: Plan) -> bool:
-        """From 2^25 weights on the tensor-memory kernel is the faster of the two: below, its second launch costs more than the
-        integer work per weight that it saves (B200, 8 token rows: 4096 x 5120 9.5 us against 9.3 on mma.sync, 17408 x 5120 14.8
-        / 17.1). A plan that does not hold its scratch keeps the other; any other fault of the binding is the caller's to see."""
+    def _on_tensor_memory(self, plan: Plan, tokens: int) -> bool:
+        """From 2^25 weights on the tensor-memory kernel is the faster of the two, whatever the token rows: below, its second
+        launch costs more at eight of them than the integer work per weight that it saves (4096 x 5120 9.5 us against 9.2 on
+        mma.sync). It cuts a tile of 128 weight rows in eight parts at most, so that weights of few rows leave SMs idle, which
+        costs the more the more token rows there are. B200, us on tensor memory / mma.sync at 1, 4 and 8 token rows: 17408 x 5120
+        13.3 / 15.4, 13.9 / 16.3, 14.6 / 17.1; 4096 x 8192 9.2 / 10.2, 9.9 / 10.6, 10.8 / 10.9; 3072 x 12288 9.9 / 10.9, 10.8 / 11.5,
+        12.1 / 11.8; 2560 x 13184 10.1 / 11.8, 11.2 / 11.3, 12.6 / 11.6; 2048 x 16384 10.3 / 9.9, 11.6 / 10.6, 12.9 / 11.1. (The
+        worst found above the line: 10880 x 3200 at 8 rows, 11.2 / 10.7.) A plan that does not hold the kernel's scratch keeps
+        the other; any other fault of the binding is the caller's to see."""
         if self.rows % 128 != 0 or self.rows > self.TENSOR_MEMORY_MAX_ROWS or self.rows * self.cols < self.TENSOR_MEMORY_WEIGHTS:
             return False
-        return plan.snapshot().scratch_len_bytes >= gemv_tc_linear_scratch_bytes(self.cols)
+        return self.rows >= (2560 if tokens <= 4 else 4096) and plan.snapshot().scratch_len_bytes >= gemv_tc_linear_scratch_bytes(self.cols)
 
     def __init__(self, stream: Stream, rows: int, cols: int, codes, scales, global_scale: float):
         self.rows, self.cols = rows, cols
@@ -743,7 +748,7 @@ class Nvfp4Sm100Linear:
     def bind(self, plan: Plan, x: torch.Tensor, out: torch.Tensor | None = None, terms: int = 3,
              activation_global_scale: float = 2.0 ** -8):
         if classify_tokens(x.shape[0]) == SHAPE_SMALL_BATCH:
-            if self._on_tensor_memory(plan):
+            if self._on_tensor_memory(plan, x.shape[0]):
                 return Nvfp4Sm100TcProjection.bind(plan, self.wide, x, out)
             return Nvfp4Sm100Projection.bind(plan, self.small, x, out)
         return Nvfp4Sm100PrefillLinear.bind(plan, self.wide, x, out, terms=terms, activation_global_scale=activation_global_scale)

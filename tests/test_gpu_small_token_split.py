@@ -96,7 +96,7 @@ def test_linear_dispatch_by_scratch_rows_and_faults(ctx):  # noqa: F811
     less = host.Plan(ctx["stream"], need - 256)
     with pytest.raises(host.CudaRuntimeError):
         host.Nvfp4Sm100TcProjection.bind(less, linear.wide, x)
-    assert not linear._on_tensor_memory(less)
+    assert not linear._on_tensor_memory(less, tokens)
     roomy = host.Plan(ctx["stream"], max(need, small_need))
     linear.wide.global_scale = float("nan")       # concerns this kernel's copy of the weight only
     with pytest.raises(host.CudaRuntimeError):
