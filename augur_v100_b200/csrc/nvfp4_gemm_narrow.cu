@@ -25,7 +25,8 @@
 // as possible, its MMAs and copies are unrolled and come from one elected lane of a converged warp. (One thread copying all
 // scales in a loop took 980 cycles per step.)
 // Every wait is bounded; a wait that runs out records a code in the plan's status word, raises a CTA-wide abort flag, and
-// all roles fall through to the common exits.
+// all roles fall through to the common exits. What a role waits for on a barrier never includes the launch before: a role that
+// depends on it waits for its end first, so that its time does not count against the bound.
 #include "nvfp4_gemm.cuh"
 
 namespace augur_sm100 {
@@ -181,6 +182,8 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
             }
             __syncwarp();
             if (++stage == p.weight_depth) { stage = 0; phase ^= 1; }
+            // the first wait for a stage to be free, which it is when the activations are there
+            if (kb == kb0 + 1 && !p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");
             if (kb != kb0 && load_kb < kb1) alive = load();
         }
     } else if (warp == 2) {
@@ -214,6 +217,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
+        if (!p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");
         uint32_t stage = 0, w_phase = 0, slot = 0, t_phase = 0, accumulate = 0;
         bool alive = true;
         const uint32_t idesc = instr_desc(p.columns);
@@ -260,6 +264,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         // A slot lands after the MMAs that used it last are complete, so its scale columns are free. The copies only have to be
         // issued before the MMAs that read them: both execute in issue order, and the fences on either side of the arrival
         // order the two warps' issues. The codes landed on the same barrier, so the MMA warp waits for this arrival only.
+        if (!p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");
         uint32_t slot = 0, phase = 0;
         bool alive = true;
         const uint64_t desc0 = sf_desc(smem_u32(slots) + p.columns * 128);

@@ -204,6 +204,8 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
             }
             __syncwarp();
             if (++stage == kStreamWeightDepth) { stage = 0; phase ^= 1; }
+            // the first wait for a stage to be free, which it is when the activations are there
+            if (kb == kb0 + 1) asm volatile("griddepcontrol.wait;" ::: "memory");
             if (kb != kb0 && load_kb < kb1) alive = load();
         }
     } else if (warp == 2) {
@@ -224,6 +226,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (the next step's barriers are looked at before this step's MMAs are issued) ----------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         uint32_t stage = 0, w_phase = 0, slot = 0, t_phase = 0, accumulate = 0;
         bool alive = true, w_seen = false, t_seen = false;
         const uint32_t idesc = instr_desc(kCols);
@@ -260,6 +263,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
         __syncwarp();
     } else if (warp == 3) {
         // ---------------- scale copies of the activations ----------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         uint32_t slot = 0, phase = 0;
         const uint64_t desc0 = sf_desc(smem_u32(slots) + kChunkBytes);
         for (uint32_t kb = kb0; kb < kb1; ++kb) {

@@ -1,7 +1,7 @@
 """A repack and the launch behind it on one stream, without a synchronise between them: through the C ABI a submit only enqueues,
 and stream order is all that a caller has. Every consumer that fetches weights early is here, with the destination holding other
 valid weights, so that a stale block shows; results equal those of the synchronised order bit for bit."""
-from ctypes import byref
+from ctypes import byref, c_uint64
 
 import pytest
 
@@ -106,3 +106,47 @@ def test_linear_then_quantiser(env, tokens, producer):
     assert plan.device_status() == 0
     assert not torch.equal(wanted[0], wanted[1])
     assert [torch.equal(out, wanted[turn % 2]) for turn, out in enumerate(got)] == [True] * 40
+
+
+def _lagging_launch(env, plan):
+    """A tensor-parallel launch of a few CTAs whose peer never answers: it lets its successors start at once and gives up after
+    about a second (bounded polls). What it reads and writes is returned, to be kept."""
+    torch, stream = env["torch"], env["stream"]
+    hidden, inter, tokens, world = 128, 256, 8, 2
+    weights = [host.Nvfp4Sm100Weight.upload_checkpoint_nvfp4(stream, abi.LAYOUT_STREAM_PAIR, inter, hidden, *synth.make_weight(3, 98, "gate", inter, hidden),
+                                                             *synth.make_weight(3, 98, "up", inter, hidden)),
+               host.Nvfp4Sm100Weight.upload_checkpoint_nvfp4(stream, abi.LAYOUT_STREAM, hidden, inter, *synth.make_weight(3, 98, "down", hidden, inter))]
+    program = host.Nvfp4Sm100FfnProgram.bind(plan, *weights, torch.ones((tokens, hidden), dtype=torch.bfloat16, device="cuda"))
+    extent = c_uint64()
+    assert abi.lib().augur_cuda_nvfp4_sm100_mlp_tp_exchange_extent_host_v1(hidden, world, byref(extent)).status == abi.STATUS_OK
+    buffers = [torch.zeros(extent.value, dtype=torch.uint8, device="cuda") for _ in range(world)]
+    args = abi.header(abi.MlpTpArgs)
+    args.gate_up, args.down = program.args.gate_up, program.args.down
+    for rank, buffer in enumerate(buffers):
+        args.exchange[rank] = buffer.data_ptr()
+    args.exchange_len_bytes, args.world, args.rank, args.sequence = extent.value, world, 0, 1
+    torch.cuda.synchronize()
+    submit = abi.lib().augur_cuda_nvfp4_sm100_mlp_tp_prevalidated_submit_v1
+    assert submit(stream.ordinal, stream.handle, plan.handle, byref(args)).status == abi.STATUS_OK
+    return program, buffers
+
+
+# The bounded waits of a launch do not run out while it waits for a launch ahead of it that takes long.
+@pytest.mark.parametrize("kind,tokens", [("split", 8), ("gemm", 16)])
+def test_waits_do_not_count_the_launch_before(env, kind, tokens):
+    torch, side, stream, plan = env["torch"], env["side"], env["stream"], env["plan"]
+    with torch.cuda.stream(side):
+        x = torch.randn((tokens, COLS), device="cuda").to(torch.bfloat16)
+        weight = host.Nvfp4Sm100Weight.repack_device_planes(stream, abi.LAYOUT_TCGEN05, ROWS, COLS, *env["planes"][0], synth.GLOBAL_SCALE)
+        program = {"split": host.Nvfp4Sm100TcProjection, "gemm": host.Nvfp4Sm100PrefillLinear}[kind].bind(plan, weight, x)
+        program.submit_for_plan()
+        wanted = program.out.clone()
+        program.out.zero_()
+        lagging = host.Plan(stream, host.mlp_scratch_bytes(128, 256))
+        kept = _lagging_launch(env, lagging)
+        program.submit_for_plan()
+        stream.synchronize()
+    assert lagging.device_status() == 0x203 and plan.device_status() == 0
+    assert torch.equal(program.out, wanted)
+    del kept
+    lagging.close()
