@@ -99,6 +99,9 @@ bf16_head_kernel(const __grid_constant__ CUtensorMap map_weight, const float* __
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // Everything above runs while the launch before this one drains. From here on its results are needed (the weights are any
+    // BF16 matrix, one that it writes among them), and its time does not count against the bound of the waits below.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t tiles = (rows + tile_rows - 1) / tile_rows, blocks = cols / 64;
     const uint32_t mine = (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x, total = mine * blocks;   // 64-k stages of this CTA
 
@@ -147,7 +150,6 @@ bf16_head_kernel(const __grid_constant__ CUtensorMap map_weight, const float* __
         const bool live = token < tokens;
         const float4* row = reinterpret_cast<const float4*>(x + static_cast<uint64_t>(live ? token : 0) * cols) + piece;
         uint8_t* place = smem + kHeadTile + token * 128 + (((piece >> 1) ^ token) << 4) + (piece & 1) * 8;
-        asm volatile("griddepcontrol.wait;" ::: "memory");
         float4 ahead[kHeadAhead];
         uint32_t fetch = 0;   // block of the next load (the row is read again for every tile)
 #pragma unroll
@@ -184,7 +186,6 @@ bf16_head_kernel(const __grid_constant__ CUtensorMap map_weight, const float* __
         }
     } else if (warp >= 8) {
         // ---------------- epilogue: lane = weight row, eight token rows x three terms ----------------
-        asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing is written while an earlier kernel may still read it
         const uint32_t quadrant = warp & 3;
         const uint32_t taddr = tmem_base + ((quadrant * 32) << 16);
         uint32_t buffer = 0, phase = 0;

@@ -150,3 +150,34 @@ def test_waits_do_not_count_the_launch_before(env, kind, tokens):
     assert torch.equal(program.out, wanted)
     del kept
     lagging.close()
+
+
+# The head's weights are any BF16 matrix: here the output of a linear that lets its successor start before it has stored anything,
+# with other values in the buffer; and the head behind a launch that takes long.
+def test_head_behind_the_launch_that_writes_its_weight(env):
+    torch, side, stream, plan = env["torch"], env["side"], env["stream"], env["plan"]
+    tokens = 48
+    with torch.cuda.stream(side):
+        x = torch.randn((tokens, COLS), device="cuda").to(torch.bfloat16)
+        weight = host.Nvfp4Sm100Weight.repack_device_planes(stream, abi.LAYOUT_TCGEN05, ROWS, COLS, *env["planes"][0], synth.GLOBAL_SCALE)
+        producer = host.Nvfp4Sm100PrefillLinear.bind(plan, weight, x)
+        head = host.Bf16Head.bind(stream, producer.out.view(2 * tokens, ROWS // 2), torch.randn((4, ROWS // 2), device="cuda"))
+        producer.submit_for_plan()
+        stream.synchronize()
+        head.submit()
+        wanted = head.out.clone()
+        got = []
+        for _ in range(20):
+            producer.out.zero_()
+            producer.submit_for_plan()
+            head.submit()
+            got.append(head.out.clone())
+        lagging = host.Plan(stream, host.mlp_scratch_bytes(128, 256))
+        kept = _lagging_launch(env, lagging)
+        head.submit()
+        got.append(head.out.clone())
+        stream.synchronize()
+    assert lagging.device_status() == 0x203 and plan.device_status() == 0
+    assert [torch.equal(out, wanted) for out in got] == [True] * 21
+    del kept
+    lagging.close()
