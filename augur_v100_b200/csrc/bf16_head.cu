@@ -42,8 +42,15 @@ constexpr uint32_t kHeadAhead = 4;                           // stages of activa
 constexpr uint32_t kHeadMaxRowBytes = 200 * 1024 / 8 - 64;   // of a token row of activations
 static_assert(kHeadSmem <= 227 * 1024, "shared memory of a CTA");
 
-__device__ uint32_t g_head_status;   // first wait that ran out (the entry has no plan to report through)
-constexpr uint32_t kErrHeadProducer = 0x401, kErrHeadSplit = 0x402, kErrHeadFull = 0x403, kErrHeadAccEmpty = 0x404, kErrHeadAccFull = 0x405;
+// A bounded wait (the entry has no plan to report through: tiles that were given up on are NaN).
+__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
+    for (uint32_t spin = 0; spin < kWaitLimit; ++spin) {
+        if (mbar_test(bar, parity)) return true;
+        if ((spin & 1023u) == 1023u && *abort_flag) return false;
+    }
+    *abort_flag = 1;
+    return false;
+}
 
 // Two F32 values -> their three BF16 terms, packed (low half = first value). x = hi + mid + lo exactly: each
 // subtraction is exact, and after two of them at most 8 significand bits are left.
@@ -109,7 +116,7 @@ bf16_head_kernel(const __grid_constant__ CUtensorMap map_weight, const float* __
         // ---------------- weights ----------------
         uint32_t stage = 0, phase = 1, block = 0, row = blockIdx.x * tile_rows;
         for (uint32_t s = 0; s < total; ++s) {
-            if (!mbar_wait(bar_empty + 8 * stage, phase, abort_flag, &g_head_status, kErrHeadProducer)) break;
+            if (!wait(bar_empty + 8 * stage, phase, abort_flag)) break;
             if (elect_one()) {
                 const uint32_t full = bar_full + 8 * stage;
                 mbar_expect_tx(full, tile_rows * 128);
@@ -126,10 +133,7 @@ bf16_head_kernel(const __grid_constant__ CUtensorMap map_weight, const float* __
         const uint64_t w_desc0 = operand_desc(smem_u32(smem)), x_desc0 = operand_desc(smem_u32(smem) + kHeadTile);
         uint32_t stage = 0, phase = 0, buffer = 0, acc_phase = 1;
         for (uint32_t s = 0; s < total; ++s) {
-            if (!mbar_wait(bar_acc_empty + 8 * buffer, acc_phase, abort_flag, &g_head_status, kErrHeadAccEmpty) ||
-                !mbar_wait(bar_full + 8 * stage, phase, abort_flag, &g_head_status, kErrHeadFull)) {
-                break;
-            }
+            if (!wait(bar_acc_empty + 8 * buffer, acc_phase, abort_flag) || !wait(bar_full + 8 * stage, phase, abort_flag)) break;
             tc_fence_after();
             if (elect_one()) {
                 const uint64_t w_desc = w_desc0 + stage * (kHeadStage >> 4), x_desc = x_desc0 + stage * (kHeadStage >> 4);
@@ -168,7 +172,7 @@ bf16_head_kernel(const __grid_constant__ CUtensorMap map_weight, const float* __
                 split3(ahead[a].z, ahead[a].w, hi[1], mid[1], lo[1]);
                 ahead[a] = __ldcg(row + fetch * 16);
                 if (++fetch == blocks) fetch = 0;
-                if (!mbar_wait(bar_empty + 8 * stage, phase, abort_flag, &g_head_status, kErrHeadSplit)) {
+                if (!wait(bar_empty + 8 * stage, phase, abort_flag)) {
                     alive = false;
                     break;
                 }
@@ -197,7 +201,7 @@ bf16_head_kernel(const __grid_constant__ CUtensorMap map_weight, const float* __
                 for (uint32_t i = 0; i < 8; ++i) sum[t][i] = 0.0f;
             }
             for (uint32_t block = 0; block < blocks; ++block) {
-                if (!mbar_wait(bar_acc_full + 8 * buffer, phase, abort_flag, &g_head_status, kErrHeadAccFull)) {
+                if (!wait(bar_acc_full + 8 * buffer, phase, abort_flag)) {
                     sum[0][0] = __uint_as_float(0x7fc00000u);
                     break;
                 }
