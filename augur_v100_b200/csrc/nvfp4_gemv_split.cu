@@ -339,13 +339,14 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
     }
 }
 
-// CTAs per tile: of the numbers up to the largest portable cluster the one with the least waves of clusters times k blocks of a
-// part, with six k blocks' worth of start and end each.
-uint32_t stream_parts(int32_t ordinal, uint32_t tiles, uint32_t k_blocks) {
+}  // namespace
+
+// Of the numbers up to the largest portable cluster the one with the least waves of clusters times k blocks of a part, with six k
+// blocks' worth of start and end each.
+uint32_t split_linear_parts(uint32_t tiles, uint32_t k_blocks, const uint32_t (&clusters)[kSplitMaxParts + 1]) {
     uint32_t best = 1, least = ~0u;
-    for (uint32_t parts = 1; parts <= 8 && parts <= k_blocks; ++parts) {
-        const uint32_t clusters = two_cta_clusters(ordinal, parts);
-        const uint32_t cost = (tiles + clusters - 1) / clusters * ((k_blocks + parts - 1) / parts + 6);
+    for (uint32_t parts = 1; parts <= kSplitMaxParts && parts <= k_blocks; ++parts) {
+        const uint32_t cost = (tiles + clusters[parts] - 1) / clusters[parts] * ((k_blocks + parts - 1) / parts + 6);
         if (cost < least) {
             least = cost;
             best = parts;
@@ -353,8 +354,6 @@ uint32_t stream_parts(int32_t ordinal, uint32_t tiles, uint32_t k_blocks) {
     }
     return best;
 }
-
-}  // namespace
 
 augur_cuda_result_v1 launch_split_linear(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
                                          const augur_cuda_nvfp4_sm100_gemv_args_v1* a, uint32_t physical_rows, uint8_t* split) {
@@ -383,7 +382,9 @@ augur_cuda_result_v1 launch_split_linear(augur_cuda_stream_t s, const augur_cuda
     p.out_rows = a->rows; p.cols = a->cols; p.tokens = a->tokens; p.epilogue = a->epilogue;
     p.global_a = a->global_scale; p.global_b = a->global_scale_b;
     const uint32_t tiles = physical_rows / kTileM;
-    p.parts = stream_parts(plan->ordinal, tiles, (a->cols + kStageK - 1) / kStageK);
+    uint32_t clusters[kSplitMaxParts + 1] = {};
+    for (uint32_t parts = 1; parts <= kSplitMaxParts; ++parts) clusters[parts] = two_cta_clusters(plan->ordinal, parts);
+    p.parts = split_linear_parts(tiles, (a->cols + kStageK - 1) / kStageK, clusters);
     attributes[1].id = cudaLaunchAttributeClusterDimension;
     attributes[1].val.clusterDim.x = p.parts;
     attributes[1].val.clusterDim.y = 1;

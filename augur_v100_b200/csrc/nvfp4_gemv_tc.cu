@@ -1,6 +1,7 @@
-// Small-token (1..8) NVFP4 linear and MLP block for sm_100a on the tensor-memory path: the weights go from HBM to
-// the tensor cores without a single per-element instruction on the SMs, and a whole MLP block is ONE launch in
-// which the weight stream does not stop at the boundary between its two products.
+// Small-token (1..8) NVFP4 MLP block for sm_100a on the tensor-memory path: the weights go from HBM to the tensor cores
+// without a single per-element instruction on the SMs, and a whole MLP block is ONE launch in which the weight
+// stream does not stop at the boundary between its two products. (Also the entries of the small-token linear,
+// whose kernels are in nvfp4_gemv_split.cu.)
 //
 //   weights      TCGEN05 layout (codes K-major as in the checkpoint, block scales in 512-byte atoms), the
 //                128-row operand of tcgen05.mma kind::mxf4nvf4: TMA brings 128 rows x 256 k (16 KB of codes
@@ -11,8 +12,8 @@
 //                radix 8 (digits -4..4, i.e. the E2M1 levels 0, 0.5, .., 2 with a sign), all scales powers of
 //                two. The terms sit side by side on the MMA n dimension (column = term * 8 + token); their
 //                codes and block scales (10 KB per 256 k, L2-resident) ride along with every weight stage.
-//                Eight digits hold a BF16 value exactly when it is within 2^-15 of its group's largest magnitude
-//                and to 2^-24 of that magnitude otherwise; one MMA per 64 k covers all tokens and all terms;
+//                Eight digits hold a BF16 value exactly when it is within 2^-14 of its group's largest magnitude
+//                and to 2^-22 of that magnitude otherwise; one MMA per 64 k covers all tokens and all terms;
 //   accumulator  128 weight rows x 64 columns of f32 in tensor memory, two buffers; the epilogue warps add
 //                the terms of a token with their scales and finish the rows.
 //
@@ -20,10 +21,9 @@
 // SM, all resident: two short rings consumed in order lose less to a late stage than one long ring): whole tiles when
 // there are at least about as many as CTAs, else every tile cut along k into equal
 // parts whose partial sums meet in plan scratch (arrival counter per 32 rows; the last arriver adds the parts in
-// a fixed order and finishes the rows; bit-reproducible). (A single linear is a program of one step; it runs as the two
-// launches of nvfp4_gemv_split.cu, which have no meeting: 17408 x 5120 at 8 tokens 14.8 us against 17.3 as a program, 5120 x
-// 5120 9.6 against 12.7.) The MLP block is two steps when the
-// gate|up tiles fit the CTAs: gate|up in whole tiles, then down in k parts. The second product needs every CTA's
+// a fixed order and finishes the rows; bit-reproducible). (A single linear as a program of one step took 17.3 us for
+// 17408 x 5120 at 8 tokens and 12.7 for 5120 x 5120; its two launches, which have no meeting, take 14.8 and 9.6.) The block is
+// two steps when the gate|up tiles fit the CTAs: gate|up in whole tiles, then down in k parts. The second product needs every CTA's
 // outputs of the first and their largest magnitudes per token row before it can split them: the CTAs arrive at
 // a counter when their outputs are stored, wait for all, split, arrive at a second counter, and the activation
 // loads of the second product wait for that one; its weights are in the ring by then. With more gate|up tiles
@@ -928,22 +928,13 @@ struct TcProgram {
     uint32_t contributors[kMaxPhases];
 };
 
-// The steps of a linear (`b` null) or of the MLP block on a device with `sm_count` SMs.
+// The steps of the MLP block on a device with `sm_count` SMs.
 TcProgram tc_program(const augur_cuda_nvfp4_sm100_gemv_args_v1* a, const augur_cuda_nvfp4_sm100_gemv_args_v1* b, uint32_t sm_count) {
     TcProgram g{};
     const uint32_t slots = sm_count * kCtasPerSm;   // CTAs resident at once
-    const uint32_t rows_a = a->epilogue == AUGUR_NVFP4_SM100_EPILOGUE_SWIGLU_BF16 ? 2 * a->rows : a->rows;
-    const uint32_t tiles_a = rows_a / kTileM, kb_a = (a->cols + kStageK - 1) / kStageK;
+    const uint32_t tiles_a = 2 * a->rows / kTileM, kb_a = (a->cols + kStageK - 1) / kStageK;
     g.job[0] = TcJob{0, 0, a->cols / 16};
     g.jobs = 1;
-    if (!b) {
-        const uint32_t parts = parts_for(tiles_a, kb_a, slots);
-        g.step[0] = TcStep{0, 0, 0, tiles_a, 0, kb_a, parts, 0, 0, 0};
-        g.steps = 1;
-        g.contributors[0] = parts;
-        g.ctas = tiles_a * parts < slots ? tiles_a * parts : slots;
-        return g;
-    }
     // gate|up in whole tiles, in two waves when there are more tiles than CTAs: a wave's outputs are 64 columns of
     // the intermediate per tile, and the first wave must end on a k block of the second product
     const uint32_t tiles_b = b->rows / kTileM, kb_b = (b->cols + kStageK - 1) / kStageK;
@@ -1114,8 +1105,8 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_gemv_tc_s
     if (!out_bytes || !rows || !cols || cols % 64 != 0 || epilogue > AUGUR_NVFP4_SM100_EPILOGUE_LINEAR_F32) return invalid();
     const uint64_t physical = epilogue == AUGUR_NVFP4_SM100_EPILOGUE_SWIGLU_BF16 ? 2ull * rows : rows;
     if (physical % kTileM != 0 || physical * cols > UINT32_MAX) return invalid();
-    // on any device with up to 512 SMs; the second product of the MLP block has two k ranges, each cut like a linear,
-    // and the first has its tiles in two halves
+    // Of the MLP block's members on any device with up to 512 SMs: the second product has two k ranges, each cut by parts_for, and
+    // the first has its tiles in two halves. (A lone linear has no partial sums in scratch: its split activations are all it needs.)
     uint32_t contributors = 2;
     for (uint32_t sms = 1; sms <= 512; ++sms) {
         const uint32_t parts = 2 * parts_for(static_cast<uint32_t>(physical / kTileM), (cols + kStageK - 1) / kStageK, sms * kCtasPerSm);
@@ -1148,8 +1139,25 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_tc_progra
         }
     }
     if (rows_b && (cols_b != rows_a || rows_b != cols_a)) return invalid();   // the second product consumes the first's outputs
-    const TcProgram g = tc_program(&a, rows_b ? &b : nullptr, sm_count);
     *out = augur_cuda_nvfp4_sm100_tc_program_v1{};
+    if (!rows_b) {
+        // one CTA per (tile, part), as launch_split_linear cuts it on a device that holds two CTAs on every SM
+        const uint32_t tiles = physical_rows_of(&a) / kTileM, k_blocks = (cols_a + kStageK - 1) / kStageK;
+        uint32_t clusters[kSplitMaxParts + 1] = {};
+        for (uint32_t parts = 1; parts <= kSplitMaxParts; ++parts) {
+            clusters[parts] = sm_count * kCtasPerSm / parts;
+            if (parts > 2) clusters[parts] -= clusters[parts] / 16;
+            if (!clusters[parts]) clusters[parts] = 1;
+        }
+        const uint32_t parts = split_linear_parts(tiles, k_blocks, clusters);
+        out->steps = out->jobs = 1;
+        out->ctas = tiles * parts;
+        out->contributors[0] = parts;
+        out->step[0] = {0, 0, 0, tiles, 0, k_blocks, parts, 0, 0, 0};
+        out->job[0] = {0, 0, cols_a / 16};
+        return ok();
+    }
+    const TcProgram g = tc_program(&a, &b, sm_count);
     out->steps = g.steps;
     out->jobs = g.jobs;
     out->ctas = g.ctas;

@@ -127,7 +127,10 @@ cudaError_t gemm_narrow_configure_device();
 cudaError_t gemv_split_configure_device();
 // Clusters of `parts` CTAs of 384 threads and 113 KB of shared memory (two per SM) that a launch may count on to run at once.
 uint32_t two_cta_clusters(int32_t ordinal, uint32_t parts);
-// A small-token linear on tensor memory as two launches (nvfp4_gemv_split.cu); `split`: split_bytes(cols) of plan scratch.
+// CTAs per 128-row tile of a small-token linear on tensor memory (a cluster) where `clusters[parts]` clusters of `parts` run at once.
+constexpr uint32_t kSplitMaxParts = 8;
+uint32_t split_linear_parts(uint32_t tiles, uint32_t k_blocks, const uint32_t (&clusters)[kSplitMaxParts + 1]);
+// The linear as two launches (nvfp4_gemv_split.cu); `split`: split_bytes(cols) of plan scratch.
 augur_cuda_result_v1 launch_split_linear(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
                                          const augur_cuda_nvfp4_sm100_gemv_args_v1* a, uint32_t physical_rows, uint8_t* split);
 // Two-CTA clusters of the pair GEMM that the device can hold at once (0 if the query fails).

@@ -720,7 +720,7 @@ class Nvfp4Sm100Linear:
     classes it chooses between.
 
     Both small-token kernels take every BF16 row. The tensor-memory kernel holds an element exactly down to
-    2^-14 of the largest of its 16-element group and to 2^-23 of that below (groups under 2^-17 of their
+    2^-14 of the largest of its 16-element group and to 2^-22 of that below (groups under 2^-17 of their
     row's largest, to 2^-39 of the latter), and a row with an infinity or a NaN gives NaN in all its outputs.
     """
 

@@ -279,13 +279,13 @@ augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_gemv_bf16_prevalidat
  * (for EPILOGUE_SWIGLU_BF16: one tensor of 2 * rows physical rows, 16 gate rows alternating with the
  * matching 16 up rows, as interleave_gate_up_host_v1 makes it), rows (physical) a multiple of 128, cols a
  * multiple of 64. The weights reach the tensor cores (tcgen05.mma kind::mxf4nvf4) as TMA delivers them;
- * the BF16 activations are split inside the launch into eight NVFP4 terms (radix-8 digits with power-of-two
- * scales), exact for every element within 2^-14 of its 16-element group's largest magnitude and to 2^-23 of that
- * magnitude below; a token row with a non-finite element gives NaN outputs. The CTAs of the launch meet through
- * counters in the plan's header: it needs all of them (at most two per SM) resident, so keep other long-running
- * kernels off the device meanwhile; a wait that runs out sets the plan's status word to 0x301..0x309, and reading
- * the status word then also clears the counters. Replaces the same reference entry points as
- * gemv_bf16_*_v1 (augur_qwen35_nvfp4_qpn_abi.h:134-156), with one weight layout for every token count. */
+ * the BF16 activations are split, by a launch of their own, into eight NVFP4 terms (radix-8 digits with
+ * power-of-two scales), exact for every element within 2^-14 of its 16-element group's largest magnitude and
+ * to 2^-22 of that magnitude below (in a group more than 2^17 below its row's largest magnitude, to 2^-39 of the
+ * latter); a token row with a non-finite element gives NaN outputs. A wait that runs out sets the plan's
+ * status word to 0x311..0x316. Needs the counter regions and the split activations of the plan's scratch, 10 KB per
+ * 256 columns; the extent below is larger and also covers a member of mlp_tc. Replaces the same reference entry
+ * points as gemv_bf16_*_v1 (augur_qwen35_nvfp4_qpn_abi.h:134-156), with one weight layout for every token count. */
 augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_gemv_tc_scratch_extent_host_v1(
     uint32_t rows, uint32_t cols, uint32_t epilogue, uint64_t* out_bytes);
 augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_gemv_tc_bf16_preflight_v1(
@@ -345,7 +345,11 @@ augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_mlp_prevalidated_sub
  * stream of the down projection already running while the intermediate is completed. Same descriptor and
  * the same cross-member checks as mlp_*_v1 (both members validated before the one enqueue); replaces
  * CudaQwen35QpnFfnProgramV1 (crates/augur-backend/src/cuda_qwen35_prefill_cublas/qpn.rs:391-492) for
- * 1..8 token rows. The plan needs gemv_tc_scratch_extent of each member, side by side. */
+ * 1..8 token rows. The plan needs gemv_tc_scratch_extent of each member, side by side. The input and the
+ * intermediate are split as in gemv_tc, inside the launch, whose CTAs meet through counters in the plan's
+ * header: it needs all of them (at most two per SM) resident, so keep other long-running kernels off the
+ * device meanwhile; a wait that runs out sets the plan's status word to 0x301..0x309, and reading the status word
+ * then also clears the counters. */
 augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_mlp_tc_preflight_v1(
     int32_t ordinal, augur_cuda_stream_t stream, augur_cuda_nvfp4_sm100_plan_v1* plan,
     const augur_cuda_nvfp4_sm100_mlp_args_v1* args);
@@ -361,9 +365,11 @@ augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_mlp_tc_prevalidated_
  * meet in contributor slots slot0 + part of `contributors[phase]`. Its activations are job `job`: the 16-element
  * groups [group0, group0 + groups) of every token row of the input of product `phase`, split inside the launch;
  * `feeds` names the job that this step's outputs become (0: none), `keeps` says that every CTA has at most one item
- * of the step and splits its own outputs from registers. `rows_b` = 0 describes a linear (`epilogue_a` as in the
- * gemv arguments, `rows_a` logical rows), otherwise the MLP block `rows_a` = intermediate, `cols_a` = hidden,
- * `rows_b` = hidden, `cols_b` = intermediate. */
+ * of the step and splits its own outputs from registers. The MLP block is `rows_a` = intermediate, `cols_a` = hidden,
+ * `rows_b` = hidden, `cols_b` = intermediate. `rows_b` = 0 describes the weight stream of a linear (`epilogue_a` as in the
+ * gemv arguments, `rows_a` logical rows): one step with a CTA of its own for every item, whose parts are at most 8,
+ * form a cluster and meet in its shared memory. (The launch asks the device how many clusters of every size it
+ * holds; the description takes what `sm_count` SMs with two CTAs each would hold.) */
 typedef struct augur_cuda_nvfp4_sm100_tc_step_v1 {
     uint32_t phase, job, tile0, tiles, kb0, kb1, parts, slot0, feeds, keeps;
 } augur_cuda_nvfp4_sm100_tc_step_v1;

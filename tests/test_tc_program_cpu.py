@@ -1,9 +1,10 @@
-"""The work split of the tensor-memory launch (csrc/nvfp4_gemv_tc.cu), checked on the CPU for many shapes and SM
-counts through the host-side description entry: every (tile, k block) of every product is streamed exactly once,
+"""The work split of the tensor-memory launches (csrc/nvfp4_gemv_tc.cu; of a linear csrc/nvfp4_gemv_split.cu), checked on the
+CPU for many shapes and SM counts through the host-side description entry: every (tile, k block) of every product is streamed exactly once,
 by exactly one CTA; a tile's parts fill its contributor slots without a gap or a clash; the jobs partition the
 input groups of their product; and a step marked `keeps` gives no CTA a second item. The item arithmetic restated
 here is the kernel's (`cursor_load`): item i of a step belongs to CTA i mod ctas, tile = i / parts, part = i % parts,
-k range [kb0 + part * span / parts, kb0 + (part + 1) * span / parts).
+k range [kb0 + part * span / parts, kb0 + (part + 1) * span / parts). A linear has one CTA per item, and the parts of a
+tile are a cluster of at most 8.
 """
 from ctypes import byref
 
@@ -26,9 +27,9 @@ def describe(rows_a, cols_a, epilogue_a, rows_b, cols_b, sms):
 
 
 def check_program(program, sms, products):
-    """`products`: [(tiles, k_blocks, input_groups)] per phase."""
-    ctas = program.ctas
-    assert 1 <= ctas <= 2 * sms
+    """`products`: [(tiles, k_blocks, input_groups)] per phase, one of a linear, two of the MLP block."""
+    ctas, linear = program.ctas, len(products) == 1
+    assert 1 <= ctas and (linear or ctas <= 2 * sms)
     covered = [dict() for _ in products]          # phase -> {(tile, kb): count}
     slots = [dict() for _ in products]            # phase -> {tile: set of slots}
     for index in range(program.steps):
@@ -36,7 +37,7 @@ def check_program(program, sms, products):
         tiles, k_blocks, _ = products[step.phase]
         assert step.tiles >= 1 and step.parts >= 1 and step.tile0 + step.tiles <= tiles
         assert step.kb0 < step.kb1 <= k_blocks and step.parts <= step.kb1 - step.kb0
-        assert step.parts <= 16 and (step.parts == 1 or (step.kb1 - step.kb0) // step.parts >= 2)
+        assert step.parts <= 8 if linear else step.parts <= 16 and (step.parts == 1 or (step.kb1 - step.kb0) // step.parts >= 2)
         assert 1 <= step.job + 1 <= program.jobs and program.job[step.job].phase == step.phase
         items, span = step.tiles * step.parts, step.kb1 - step.kb0
         per_cta = {}
@@ -85,7 +86,7 @@ def test_linear_programs_cover_every_block_once(sms):
             program = describe(rows, cols, epilogue, 0, 0, sms)
             assert program.steps == 1 and program.jobs == 1
             check_program(program, sms, [(physical // 128, (cols + 255) // 256, cols // 16)])
-            assert program.ctas == min(physical // 128 * program.step[0].parts, 2 * sms)
+            assert program.ctas == physical // 128 * program.step[0].parts
 
 
 @pytest.mark.parametrize("sms", SM_COUNTS)
