@@ -50,6 +50,10 @@ constexpr uint32_t kCombineBlocks = 48;    // weight blocks a CTA streams in the
 constexpr uint32_t kMaxClusterSize = 8;
 constexpr uint32_t kExchangeSlots = 16;    // tiles a CTA of a cluster takes in from the slabs of the groups it finishes
 constexpr uint32_t kMaxGroupMembers = 4;
+// From as many row groups per CTA on (without clusters), a warp adds the shares of a group; below, all threads add by elements. At one token row, by
+// elements / by warps: 6 groups (28416 x 1024) 8.7 us / 9.0, 8 groups (37888 x 512) 7.2 / 7.3, 10 (47360 x 512) 8.7 / 8.5, 52
+// (248320 x 256) 15.5 / 14.7.
+constexpr uint32_t kGroupsByWarp = 9;
 
 // One weight matrix of a launch: the row groups [first_group, the next member's) of the launch.
 struct GemvMember {
@@ -479,15 +483,30 @@ __device__ __forceinline__ void finish_pair(const GemvParams& p, uint32_t group,
     }
 }
 
-// The same for a whole tile (8 values per lane).
+// The same for a whole tile (8 values per lane). The stores of a lone linear are written out here: as pairs of elements they cost up
+// to 5 % where most groups end in one warp (131072 x 256 at 8 token rows 11.8 us against 11.2).
 template <uint32_t kMembers>
 __device__ __forceinline__ void epilogue(const GemvParams& p, uint32_t seq, uint32_t group, const float (&v)[8], uint32_t lane) {
     if (p.tp_world) {
         exchange_push(p, seq, group, v, lane);   // the sum over ranks is written by exchange_reduce
         return;
     }
+    const GemvMember m = member_of<kMembers>(p, group);
+    if (kMembers > 1 || m.epilogue == AUGUR_NVFP4_SM100_EPILOGUE_SWIGLU_BF16) {
 #pragma unroll
-    for (uint32_t i = 0; i < 4; ++i) finish_pair<kMembers>(p, group, lane, i, v[i], v[4 + i]);
+        for (uint32_t i = 0; i < 4; ++i) finish_pair<kMembers>(p, group, lane, i, v[i], v[4 + i]);
+        return;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+        const uint32_t token = 2 * (lane & 3) + (i & 1), row = (group - m.first_group) * 32 + (i >> 2) * 16 + (lane >> 2) + ((i >> 1) & 1) * 8;
+        if (token < p.tokens && row < m.store_rows) {
+            const float value = v[i] * m.global_a;
+            const uint64_t at = static_cast<uint64_t>(token) * m.store_rows + row;
+            if (m.epilogue == AUGUR_NVFP4_SM100_EPILOGUE_LINEAR_F32) static_cast<float*>(m.out)[at] = value;
+            else static_cast<__nv_bfloat16*>(m.out)[at] = __float2bfloat16_rn(value);
+        }
+    }
 }
 
 // ---- activation staging --------------------------------------------------------------------
@@ -948,9 +967,9 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_kernel(const __grid_const
     __syncthreads();
 
     // ---- combine row groups that were split between warps of this CTA ----
-    if (p.aligned && !p.tp_world) {
+    if (p.aligned && !p.tp_world && (cluster || len / kbs < kGroupsByWarp)) {
         // Two elements of a tile per thread, so that all of the CTA adds: a warp per row group, as below, leaves the other
-        // warps idle and its sums of up to sixteen tiles one behind the other.
+        // warps idle and its sums of up to sixteen tiles one behind the other. With many row groups every warp has one of its own.
         const uint32_t cta_groups = (c1 - c0) / kbs;
 #pragma unroll 1
         for (uint32_t at = threadIdx.x; at < cta_groups * 128; at += kWarps * 32) {

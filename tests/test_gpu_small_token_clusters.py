@@ -33,6 +33,12 @@ def test_cluster_split(ctx, rows, cols, tokens):  # noqa: F811
     assert rel_error(results[0], oracle.linear_f64(codes, scales, glob, rows, cols, x_bits, threads=oracle.max_threads())) <= TOLERANCE
 
 
+# many row groups per CTA, whose shares the warps add a group each: 10, 9 and 8 per CTA, a short last one, groups that straddle warps
+@pytest.mark.parametrize("rows,cols,tokens", [(47360, 384, 8), (42560, 640, 3), (37888, 256, 1)])
+def test_many_groups_per_cta(ctx, rows, cols, tokens):  # noqa: F811
+    test_cluster_split(ctx, rows, cols, tokens)
+
+
 # members of a norm group whose ranges straddle clusters, one of them trimmed
 @pytest.mark.parametrize("cols,rows,stored", [(1024, (1056, 64, 2080), (0, 48, 0)), (2560, (64, 64, 32, 96), (48, 48, 0, 0)), (5120, (4000,), (0,))])
 def test_group_members_straddle_clusters(ctx, cols, rows, stored):  # noqa: F811
