@@ -60,7 +60,27 @@ def test_split_covers_every_exponent(ctx, exponents, block_scale, glob):  # noqa
         assert rel_error(got[row], y64[row]) <= TOLERANCE, exponent
 
 
-# From 2^25 weights on `Nvfp4Sm100Linear` binds this kernel.
+# An infinity or a NaN makes its row NaN, whichever part of k holds it, and no other row.
+def test_non_finite_rows(ctx):  # noqa: F811
+    rows, cols, tokens = 384, 4160, 6
+    codes, scales, glob = synth.make_weight(21, 92, "w", rows, cols)
+    x = np.random.default_rng(21).standard_normal((tokens, cols)).astype(np.float32)
+    x[1, 0], x[3, cols - 1], x[4, 2000] = np.inf, -np.inf, np.nan
+    x_bits = synth.f32_to_bf16_bits(x)
+    x_bits[4, 2000] = 0x7FC0       # rounding a NaN is not what is tested
+    weight = host.Nvfp4Sm100Weight.upload_checkpoint_nvfp4(ctx["stream"], abi.LAYOUT_TCGEN05, rows, cols, codes, scales, glob)
+    projection = host.Nvfp4Sm100TcProjection.bind(ctx["plan"], weight, torch_bf16_from_bits(x_bits, ctx["device"]))
+    projection.submit_for_plan()
+    ctx["stream"].synchronize()
+    assert ctx["plan"].device_status() == 0
+    got = bits_from_torch_bf16(projection.out).reshape(tokens, rows)
+    assert np.all((got[[1, 3, 4]] & 0x7FFF) > 0x7F80)
+    finite = [0, 2, 5]
+    y64 = oracle.linear_f64(codes, scales, glob, rows, cols, np.ascontiguousarray(x_bits[finite]), threads=oracle.max_threads())
+    assert rel_error(got[finite], y64.reshape(3, rows)) <= TOLERANCE
+
+
+# `Nvfp4Sm100Linear` binds this kernel for large weights.
 def test_linear_dispatch_by_size(ctx):  # noqa: F811
     rows, cols, tokens = 32768, 1024, 6
     codes, scales, glob = synth.make_weight(7, 95, "w", rows, cols)
