@@ -50,7 +50,7 @@ constexpr uint32_t kCombineBlocks = 48;    // weight blocks a CTA streams in the
 constexpr uint32_t kMaxClusterSize = 8;
 constexpr uint32_t kExchangeSlots = 16;    // tiles a CTA of a cluster takes in from the slabs of the groups it finishes
 constexpr uint32_t kMaxGroupMembers = 4;
-// From as many row groups per CTA on (without clusters), a warp adds the shares of a group; below, all threads add by elements. At one token row, by
+// From as many row groups per CTA on, a warp adds the shares of a group; below, all threads add by elements. At one token row, by
 // elements / by warps: 6 groups (28416 x 1024) 8.7 us / 9.0, 8 groups (37888 x 512) 7.2 / 7.3, 10 (47360 x 512) 8.7 / 8.5, 52
 // (248320 x 256) 15.5 / 14.7.
 constexpr uint32_t kGroupsByWarp = 9;
@@ -967,7 +967,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_kernel(const __grid_const
     __syncthreads();
 
     // ---- combine row groups that were split between warps of this CTA ----
-    if (p.aligned && !p.tp_world && (cluster || len / kbs < kGroupsByWarp)) {
+    if (p.aligned && !p.tp_world && len / kbs < kGroupsByWarp) {
         // Two elements of a tile per thread, so that all of the CTA adds: a warp per row group, as below, leaves the other
         // warps idle and its sums of up to sixteen tiles one behind the other. With many row groups every warp has one of its own.
         const uint32_t cta_groups = (c1 - c0) / kbs;

@@ -33,8 +33,9 @@ def test_cluster_split(ctx, rows, cols, tokens):  # noqa: F811
     assert rel_error(results[0], oracle.linear_f64(codes, scales, glob, rows, cols, x_bits, threads=oracle.max_threads())) <= TOLERANCE
 
 
-# many row groups per CTA, whose shares the warps add a group each: 10, 9 and 8 per CTA, a short last one, groups that straddle warps
-@pytest.mark.parametrize("rows,cols,tokens", [(47360, 384, 8), (42560, 640, 3), (37888, 256, 1)])
+# many row groups per CTA, whose shares the warps add a group each: 10, 9 and 8 per CTA, a short last one, groups that straddle warps;
+# 9 per cluster of four CTAs
+@pytest.mark.parametrize("rows,cols,tokens", [(47360, 384, 8), (42560, 640, 3), (37888, 256, 1), (9504, 5120, 8)])
 def test_many_groups_per_cta(ctx, rows, cols, tokens):  # noqa: F811
     test_cluster_split(ctx, rows, cols, tokens)
 
