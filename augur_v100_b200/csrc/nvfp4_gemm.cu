@@ -1061,7 +1061,7 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_gemm_swig
 namespace {
 static_assert(sizeof(augur_cuda_nvfp4_sm100_gemm_swiglu_quant_args_v1) == 112, "gemm_swiglu_quant ABI");
 
-// Pair tiles only: padded tokens a multiple of 256 and an intermediate size that is a multiple of 128.
+// An intermediate size that is a multiple of 128: its rows of gate and up fill whole 256-row tiles.
 bool check_swiglu_quant(int32_t d, augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
                         const augur_cuda_nvfp4_sm100_gemm_swiglu_quant_args_v1* a, bool full,
                         augur_cuda_nvfp4_sm100_gemm_args_v1* g, augur_cuda_result_v1* failure) {

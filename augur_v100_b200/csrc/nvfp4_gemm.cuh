@@ -23,7 +23,7 @@ struct GemmParams {
     float scale;                   // g_w * g_a
     float scale_b;                 // SwiGLU: g_w of the up rows * g_a
     uint32_t swiglu;               // weight rows alternate 16 gate / 16 up; output is bf16(silu(gate) * up), rows / 2 wide
-    // SwiGLU on pair tiles only: the intermediate is also (or only, if `out` is null) quantised for the next GEMM
+    // SwiGLU: the intermediate is also (or only, if `out` is null) quantised for the next GEMM
     uint8_t* quant_out;            // staged activations: [terms] code planes of whole tiles, then the scale regions
     uint32_t quant_terms;
     float quant_global_scale;

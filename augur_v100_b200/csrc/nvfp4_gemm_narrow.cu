@@ -3,8 +3,9 @@
 //
 // The pair kernel of nvfp4_gemm.cu puts 256 token rows on its tile, so 9 tokens cost what 256 do. Here the weights are the
 // 128-row operand and the tokens sit on the MMA n dimension, whose size follows their number in steps of 16 (at most
-// 128): the work is that of the tokens there are, and what is left is streaming the weights once. Up to that width the
-// launch is bound by HBM (one term) or by the tensor pipe's queue of MMAs and scale copies (three terms).
+// 128): the work is that of the tokens there are, and what is left is streaming the weights once. What bounds a launch is a
+// chain of latencies, a pipeline step (k block x term) of 0.33 to 0.44 us behind the other, not HBM or the tensor pipe: 6144 x 5120 at
+// 48 tokens and three terms has them 13 % and 9 % busy.
 //
 //   D[feature][token] = sum over k blocks of 256, terms, k steps of 64:  W[128 x 64] * A_term[tokens x 64]^T
 //

@@ -9,7 +9,8 @@
 // and all CTAs met before anyone could load them, 6 us in front of the first MMA, and the k parts of a tile met again
 // through global memory. As two launches there is no meeting: the stream kernel becomes resident while the kernel
 // before the split still runs (both starts are programmatic), fills its rings with weights, 21 MB over the GPU, and
-// then waits only for the split, a kernel of two microseconds; the parts of a tile meet in distributed shared memory.
+// then waits only for the split, about four microseconds from its input being there to the first activation load, half of
+// them the split itself and half its end and hand-over; the parts of a tile meet in distributed shared memory.
 //
 // Roles, rings and issue as in nvfp4_gemm_narrow.cu: warp 0 weights (TMA, scale copies), 1 MMA, 2 TMA of the activations, 3 their
 // scale copies, 4..11 epilogue. Every wait is bounded; a wait that runs out records a code in the plan's status word, raises a

@@ -307,7 +307,8 @@ def gemv_tc_linear_scratch_bytes(cols: int) -> int:
 class Nvfp4Sm100TcProjection(Nvfp4Sm100Projection):
     """A retained small-token projection on the tensor-memory path: the weight is in the tcgen05 layout
     (the one the prefill GEMM uses; for the SwiGLU epilogue the interleaved gate|up tensor of
-    `upload_gate_up_interleaved`), the kernel is `gemv_tc`. Same contract as `Nvfp4Sm100Projection`."""
+    `upload_gate_up_interleaved`), the kernel is `gemv_tc`. Same contract as `Nvfp4Sm100Projection`, but for token rows
+    with a non-finite element, whose outputs are all NaN."""
 
     def __init__(self, plan: Plan, weight: Nvfp4Sm100Weight, x: torch.Tensor, out: torch.Tensor, epilogue: int):
         assert weight.layout == abi.LAYOUT_TCGEN05
