@@ -35,8 +35,8 @@ constexpr uint32_t kBytesSfB = 8 * kSfAtomBytes;      // 4 KB: 2 row blocks x 4 
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTmemAcc = 0;          // 256 accumulator columns
 
-constexpr uint32_t kErrProducerWait = 0x101, kErrMmaWaitFull = 0x102, kErrMmaWaitTmem = 0x103,
-                   kErrEpilogueWait = 0x104, kErrCopyWait = 0x105, kErrMmaWaitScales = 0x106,
+constexpr uint32_t kErrProducerWait = 0x101, kErrMmaWaitTokens = 0x102, kErrMmaWaitTmem = 0x103,
+                   kErrEpilogueWait = 0x104, kErrCopyWait = 0x105, kErrMmaWaitWeights = 0x106,
                    kErrSplitWait = 0x107;
 
 // ---- two-CTA tiles ------------------------------------------------------------------------------
@@ -48,30 +48,57 @@ constexpr uint32_t kErrProducerWait = 0x101, kErrMmaWaitFull = 0x102, kErrMmaWai
 // both; each CTA's accumulator half sits in its own tensor memory and is drained by its own
 // epilogue warps.
 //
-// Barriers (same offsets in both CTAs):
-//   full[s]   leader's only: one arrival (leader's producer, expecting the bytes of both CTAs);
-//             both producers' TMA loads complete on it (cta_group::2 loads, leader's address);
-//   empty[s]  one per CTA, arrived by the leader's tcgen05.commit multicast to both CTAs;
-//   tmem_full one per CTA, same multicast;   tmem_empty leader's only, one arrival per epilogue
-//             warp of either CTA (the peer's through a cluster-scope arrive);
-//   scales_landed[s] leader's only: the stage's block-scale atoms of both CTAs have landed (loaded before
-//             the operand tiles);   scales_ready[s], weights_ready[slot] leader's only: the copy warps have issued the
-//             shared -> tensor memory copies of the stage's token-row scales, of the k block's weight-row scales.
-constexpr uint32_t kPairStages = 5;
-// Tensor memory of the pair kernel: 256 accumulator columns, then one set of token-row scale columns per stage
-// (16 each) and one set of weight-row scale columns per k-block slot (32 each).
-constexpr uint32_t kTmemPairSfA = 256;
-constexpr uint32_t kTmemPairSfB = kTmemPairSfA + kPairStages * 16;
-static_assert(kTmemPairSfB + kPairStages * 32 <= kTmemCols, "scale columns of all stages fit beside the accumulator");
-constexpr uint32_t kPairBytesB = 128 * 128;                                            // this CTA's 128 weight rows
-constexpr uint32_t kPairStageBytes = kBytesA + kPairBytesB + kBytesSfA + kBytesSfB;   // 38912
+// Two rings per CTA: a weight stage (20 KB) holds a k block's weight rows and their scales for all activation terms, a token
+// slot (18 KB) one term of it. What bounds the kernel is the board's power (SM clock 1.5 to 1.65 GHz under it) and, within it,
+// about 150 cycles per MMA: so bytes that need not move into shared memory are time. With one ring, whose stages brought the
+// weights again for every term, three terms of 17408 x 5120 x 4096 took 434 us (GEMM alone; 457 in a long loop), with two
+// 384 (418), two terms 291 -> 272; 5120 x 17408 x 777, three terms, 114 -> 97.
+//
+// Barriers per slot of a ring (same offsets in both CTAs):
+//   landed  leader's only: the slot's block-scale atoms of both CTAs have landed (loaded before the operand tiles);
+//   full    leader's only: two arrivals, the leader's producer (expecting the operand bytes of both CTAs; both producers' TMA
+//           loads complete on it: cta_group::2 loads, leader's address) and the ring's copy warp, which has issued the
+//           shared -> tensor memory copies of the slot's scales;
+//   empty   token slots only, one per CTA, arrived by the leader's tcgen05.commit multicast to both CTAs.
+// And: tmem_full one per CTA, same multicast;   tmem_empty leader's only, one arrival per epilogue warp of either CTA (the
+// peer's through a cluster-scope arrive).
+constexpr uint32_t kPairBytesB = 128 * 128;                          // this CTA's 128 weight rows
+constexpr uint32_t kPairWeightStage = kPairBytesB + kBytesSfB;       // 20480
+constexpr uint32_t kPairTokenSlot = kBytesA + kBytesSfA;             // 18432
+constexpr uint32_t kPairMaxDepth = 8;                                // slots of either ring
+// Ring depths by activation terms: about as many k blocks ahead on either ring as shared memory holds. A weight stage is
+// free when the last term's step of its k block is complete, which that step's token slot says (no barrier and no commit of its
+// own: a second commit per step, and scales that queue behind codes, took one term from 157 to 178 us). For the slot's
+// phase to be the one meant, the step must not have left the token ring yet.
+struct PairDepths {
+    uint32_t weights, tokens;
+};
+__host__ __device__ constexpr PairDepths pair_depths(uint32_t terms) { return terms == 1 ? PairDepths{5, 5} : PairDepths{3, 8}; }
+__host__ __device__ constexpr bool pair_depths_ok(uint32_t terms) {
+    return pair_depths(terms).tokens > (pair_depths(terms).weights - 1) * terms && pair_depths(terms).tokens >= terms;
+}
+static_assert(pair_depths_ok(1) && pair_depths_ok(2) && pair_depths_ok(3), "a freed weight stage shows in the token ring");
+__host__ __device__ constexpr uint32_t pair_ring_bytes(uint32_t terms) {
+    return pair_depths(terms).weights * kPairWeightStage + pair_depths(terms).tokens * kPairTokenSlot;
+}
+constexpr uint32_t kPairRingBytes = pair_ring_bytes(3);              // the largest: 208896
+static_assert(pair_ring_bytes(1) <= kPairRingBytes && pair_ring_bytes(2) <= kPairRingBytes, "space for the rings");
+// Tensor memory of the pair kernel: 256 accumulator columns, then one set of weight-row scale columns per weight stage
+// (32 each) and one set of token-row scale columns per token slot (16 each).
+constexpr uint32_t kTmemPairScales = 256;
+constexpr uint32_t pair_tmem_columns(uint32_t terms) { return kTmemPairScales + pair_depths(terms).weights * 32 + pair_depths(terms).tokens * 16; }
+static_assert(pair_tmem_columns(1) <= kTmemCols && pair_tmem_columns(2) <= kTmemCols && pair_tmem_columns(3) <= kTmemCols,
+              "scale columns of both rings fit beside the accumulator");
 // Epilogue transposition rows: an epilogue warp holds one accumulator row per lane; to store row pieces that are
 // contiguous in global memory it parks one 32-column chunk (64 bytes of BF16 per row, rows padded by 16 bytes so
 // that the row-per-lane writes spread over all banks) and reads it back with 4 lanes per row.
 constexpr uint32_t kPairEpilogueWarps = 8;      // two per tensor-memory lane quadrant
 constexpr uint32_t kPairOutRowBytes = 64 + 16;
 constexpr uint32_t kPairOutBytes = kPairEpilogueWarps * 32 * kPairOutRowBytes;         // 20480
-constexpr uint32_t kPairSmemBytes = kPairStages * kPairStageBytes + kPairOutBytes + 1024 + 256;
+constexpr uint32_t kPairBarriers = 5 * kPairMaxDepth + 2;
+constexpr uint32_t kPairSmemBytes = kPairRingBytes + kPairOutBytes + 1024 + 512;
+static_assert(kPairBarriers * 8 + 8 <= 512, "barriers, tensor-memory base and abort flag fit behind the rings");
+static_assert(kPairSmemBytes <= 227 * 1024, "shared memory of a CTA");
 constexpr uint32_t kPairCopyWarp = 2 + kPairEpilogueWarps;    // token-row scales; the warp after it copies the weight-row scales
 constexpr uint32_t kPairThreads = 32 * (kPairCopyWarp + 2);   // TMA warp, MMA warp, epilogue warps, two scale-copy warps
 constexpr uint32_t kSplitWays = 8;              // a leftover tile is cut into this many parts at most
@@ -175,33 +202,36 @@ __device__ __forceinline__ PairWork pair_work(uint32_t pair, uint32_t pairs, uin
     return w;
 }
 
+// One instantiation per set of ring depths: as constants they are worth 1.5 %.
+template <bool kResidualTerms>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant__ CUtensorMap map_weight,
                  const __grid_constant__ CUtensorMap map_act_sf, const __grid_constant__ CUtensorMap map_weight_sf,
                  const GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* out_stage = smem + kPairStages * kPairStageBytes;
+    uint8_t* out_stage = smem + kPairRingBytes;
     uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + kPairOutBytes);
-    // full[S], empty[S], tmem_full, tmem_empty, scales_ready[S], scales_landed[S], weights_ready[S]; then the TMEM base and the abort flag
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5 * kPairStages + 2);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kPairBarriers);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();            // 0 = leader
     const uint32_t pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + kPairStages);
-    const uint32_t bar_tmem_full = smem_u32(bars + 2 * kPairStages), bar_tmem_empty = smem_u32(bars + 2 * kPairStages + 1);
-    const uint32_t bar_scales_ready = smem_u32(bars + 2 * kPairStages + 2), bar_scales_landed = smem_u32(bars + 3 * kPairStages + 2);
-    const uint32_t bar_weights_ready = smem_u32(bars + 4 * kPairStages + 2);
+    constexpr PairDepths depth = pair_depths(kResidualTerms ? 3 : 1);
+    const uint32_t smem_base = smem_u32(smem), tokens_base = smem_base + depth.weights * kPairWeightStage;
+    const uint32_t bar0 = smem_u32(bars);
+    const uint32_t w_full = bar0, w_landed = bar0 + 8 * kPairMaxDepth;
+    const uint32_t t_full = bar0 + 16 * kPairMaxDepth, t_landed = bar0 + 24 * kPairMaxDepth, t_empty = bar0 + 32 * kPairMaxDepth;
+    const uint32_t bar_tmem_full = bar0 + 40 * kPairMaxDepth, bar_tmem_empty = bar_tmem_full + 8;
 
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < kPairStages; ++s) {
-            mbar_init(bar_full + 8 * s, 1);
-            mbar_init(bar_empty + 8 * s, 1);
-            mbar_init(bar_scales_ready + 8 * s, 1);
-            mbar_init(bar_scales_landed + 8 * s, 1);
-            mbar_init(bar_weights_ready + 8 * s, 1);
+        for (uint32_t s = 0; s < kPairMaxDepth; ++s) {
+            mbar_init(w_full + 8 * s, 2);
+            mbar_init(w_landed + 8 * s, 1);
+            mbar_init(t_full + 8 * s, 2);
+            mbar_init(t_empty + 8 * s, 1);
+            mbar_init(t_landed + 8 * s, 1);
         }
         mbar_init(bar_tmem_full, 1);
         mbar_init(bar_tmem_empty, 2 * kPairEpilogueWarps);   // one arrival per epilogue warp of either CTA
@@ -219,11 +249,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
     cluster_sync();   // the peer's barriers exist before anything can signal them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    // Everything above ran while the launch before this one drained; its results are needed from here on.
-    // The dependents start only after the wait: a narrow launch behind this one (`after_main`) skips its own wait until its
-    // end and relies on the quantiser, which this launch has waited for.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (threadIdx.x == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t tmem_weights = tmem_base + kTmemPairScales, tmem_tokens = tmem_weights + depth.weights * 32;
 
     // An odd number of 128-row token tiles leaves the second CTA of the last pair without rows of its own: it
     // loads whatever follows (the next term's rows, or the fill value past the tensor) and stores nothing.
@@ -242,55 +268,84 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
 
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
-        uint32_t stage = 0, phase = 1;
+        // The block scales of a slot go first, on a barrier of their own: they are small and land early, so the copy warps have
+        // them in tensor memory by the time the operand tiles arrive. The weights are constant, so the first ring of them is
+        // under way while the launch before this one, whose results the token rows are, still drains.
+        uint32_t w_stage = 0, slot = 0, t_phase = 1;
         bool alive = true;
+        auto weight_scales = [&](uint32_t n_tile, uint32_t kb, uint32_t stage) {
+            const uint32_t to = smem_base + stage * kPairWeightStage + kPairBytesB, landed = w_landed + 8 * stage;
+            if (rank == 0) mbar_expect_tx(landed, 2 * kBytesSfB);
+            tma_load_2d_pair(to, &map_weight_sf, 0, (n_tile * 2) * atoms_per_row_block + kb * 4, landed);
+            tma_load_2d_pair(to + kBytesSfB / 2, &map_weight_sf, 0, (n_tile * 2 + 1) * atoms_per_row_block + kb * 4, landed);
+        };
+        auto weight_codes = [&](uint32_t n_tile, uint32_t kb, uint32_t stage) {
+            const uint32_t full = w_full + 8 * stage;
+            if (rank == 0) mbar_expect_tx(full, 2 * kPairBytesB);
+            tma_load_2d_pair(smem_base + stage * kPairWeightStage, &map_weight, kb * 128, n_tile * kTileN + rank * (n_tile == half_tile ? 64 : 128), full);
+        };
+        uint32_t ahead = 0;
+        if (work.items) {
+            const PairItem first = work.item(0, pair, pairs, k_blocks);
+            for (; ahead < depth.weights && first.kb0 + ahead < first.kb1; ++ahead) {
+                if (elect_one()) {
+                    weight_scales(first.tile / m_pairs, first.kb0 + ahead, ahead);
+                    weight_codes(first.tile / m_pairs, first.kb0 + ahead, ahead);
+                }
+                __syncwarp();
+            }
+        }
+        // The dependents start only after the wait: a narrow launch behind this one (`after_main`) skips its own wait until its
+        // end and relies on the quantiser, which this launch has waited for.
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (lane == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        uint32_t done_slot = p.terms - 1, done_phase = 0, blocks = 0;
         for (uint32_t index = 0; alive && index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
-            const uint32_t m_pair = item.tile % m_pairs, n_tile = item.tile / m_pairs;
-            const uint32_t token_row = m_pair * 2 * kTileM + rank * kTileM;
-            const uint32_t weight_row = n_tile * kTileN + rank * (n_tile == half_tile ? 64 : 128);
-            for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb) {
+            const uint32_t n_tile = item.tile / m_pairs, token_row = item.tile % m_pairs * 2 * kTileM + rank * kTileM;
+            for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb, ++blocks) {
+                if (blocks >= depth.weights) {
+                    if (!mbar_wait(t_empty + 8 * done_slot, done_phase, abort_flag, p.status_word, kErrProducerWait)) {
+                        alive = false;
+                        break;
+                    }
+                    done_slot += p.terms;
+                    if (done_slot >= depth.tokens) { done_slot -= depth.tokens; done_phase ^= 1; }
+                }
+                const bool fetch = blocks >= ahead;
                 for (uint32_t term = 0; term < p.terms; ++term) {
-                    if (!mbar_wait(bar_empty + 8 * stage, phase, abort_flag, p.status_word, kErrProducerWait)) {
+                    if (!mbar_wait(t_empty + 8 * slot, t_phase, abort_flag, p.status_word, kErrProducerWait)) {
                         alive = false;
                         break;
                     }
                     if (elect_one()) {
-                        const uint32_t base = smem_u32(smem + stage * kPairStageBytes);
-                        // The block scales go first, on a barrier of their own: they are small and land early, so the copy
-                        // warps have them in tensor memory by the time the operand tiles arrive.
-                        const uint32_t landed = bar_scales_landed + 8 * stage, full = bar_full + 8 * stage;
-                        if (rank == 0) mbar_expect_tx(landed, 2 * (kBytesSfA + kBytesSfB));
-                        tma_load_2d_pair(base + kBytesA + kPairBytesB, &map_act_sf, 0,
+                        const uint32_t base = tokens_base + slot * kPairTokenSlot, landed = t_landed + 8 * slot, full = t_full + 8 * slot;
+                        if (rank == 0) mbar_expect_tx(landed, 2 * kBytesSfA);
+                        tma_load_2d_pair(base + kBytesA, &map_act_sf, 0,
                                          term * act_term_atoms + (token_row / 128) * atoms_per_row_block + kb * 4, landed);
-                        tma_load_2d_pair(base + kBytesA + kPairBytesB + kBytesSfA, &map_weight_sf, 0,
-                                         (n_tile * 2) * atoms_per_row_block + kb * 4, landed);
-                        tma_load_2d_pair(base + kBytesA + kPairBytesB + 2 * kBytesSfA, &map_weight_sf, 0,
-                                         (n_tile * 2 + 1) * atoms_per_row_block + kb * 4, landed);
-                        if (rank == 0) mbar_expect_tx(full, 2 * (kBytesA + kPairBytesB));
+                        if (fetch && term == 0) weight_scales(n_tile, kb, w_stage);
+                        if (rank == 0) mbar_expect_tx(full, 2 * kBytesA);
                         tma_load_2d_pair(base, &map_act, kb * 128, term * p.padded_tokens + token_row, full);
-                        tma_load_2d_pair(base + kBytesA, &map_weight, kb * 128, weight_row, full);
+                        if (fetch && term == 0) weight_codes(n_tile, kb, w_stage);
                     }
                     __syncwarp();
-                    if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+                    if (++slot == depth.tokens) { slot = 0; t_phase ^= 1; }
                 }
+                if (++w_stage == depth.weights) w_stage = 0;
             }
         }
     } else if (warp == 1 && rank == 0) {
         // ---------------- MMA issuer (leader only) ----------------
         // Issuing a tcgen05 operation keeps a warp busy for tens of cycles, and one warp issuing the 12 scale copies and
-        // the 4 MMAs of every stage could not keep the tensor pipe fed; the copies are issued by two warps of their own
-        // (below) into the stage's scale columns, this one issues only the MMAs. Descriptors advance by additions (their low
+        // the 4 MMAs of every step could not keep the tensor pipe fed; the copies are issued by two warps of their own
+        // (below) into the slots' scale columns, this one issues only the MMAs. Descriptors advance by additions (their low
         // bits hold address >> 4). Looking at a barrier takes as long as issuing an MMA or two, so those of the next
         // step are looked at before the MMAs of this one are issued, and waited for only if they were not there.
-        uint32_t stage = 0, phase = 0, tmem_phase = 0;
-        uint32_t kb_slot = 0, kb_phase = 0;   // k blocks counted across tiles, modulo kPairStages: the weight-row scale buffer
-        bool alive = true, operands_seen = false, scales_seen = false, weights_seen = false;
+        uint32_t w_stage = 0, w_phase = 0, slot = 0, t_phase = 0, tmem_phase = 0;
+        bool alive = true, tokens_seen = false, weights_seen = false;
         constexpr uint32_t kWideTile = (1u << 7) | (1u << 10) | ((kTileN >> 3) << 17) | (((2 * kTileM) >> 4) << 24);
         constexpr uint32_t kHalfTile = (1u << 7) | (1u << 10) | ((kTileN / 2 >> 3) << 17) | (((2 * kTileM) >> 4) << 24);
-        const uint32_t smem_base = smem_u32(smem);
-        const uint64_t a_desc0 = operand_desc(smem_base), b_desc0 = operand_desc(smem_base + kBytesA);
-        constexpr uint32_t kStageStep = kPairStageBytes >> 4;
+        const uint64_t w_desc0 = operand_desc(smem_base), t_desc0 = operand_desc(tokens_base);
         const uint32_t last_k_steps = (p.cols - (k_blocks - 1) * kBlockK) / 64;   // 1..4 k steps of 64 in the last k block
         for (uint32_t index = 0; alive && index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
@@ -301,41 +356,38 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
             uint32_t accumulate = 0;
             for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb) {
                 const uint32_t k_steps = (kb + 1 < k_blocks) ? 4u : last_k_steps;
-                if (!weights_seen && !mbar_wait(bar_weights_ready + 8 * kb_slot, kb_phase, abort_flag, p.status_word, kErrMmaWaitScales)) {
+                if (!weights_seen && !mbar_wait(w_full + 8 * w_stage, w_phase, abort_flag, p.status_word, kErrMmaWaitWeights)) {
                     alive = false;
                     break;
                 }
-                const uint32_t tmem_sfb = tmem_base + kTmemPairSfB + kb_slot * 32;   // the weight rows' scales change with the k block only
-                if (++kb_slot == kPairStages) { kb_slot = 0; kb_phase ^= 1; }
+                const uint64_t w_desc = w_desc0 + w_stage * (kPairWeightStage >> 4);
+                const uint32_t sf_w = tmem_weights + w_stage * 32;
+                if (++w_stage == depth.weights) { w_stage = 0; w_phase ^= 1; }
                 for (uint32_t term = 0; term < p.terms; ++term) {
-                    // operands in shared memory (TMA) and block scales in tensor memory (copy warps)
-                    if ((!operands_seen && !mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.status_word, kErrMmaWaitFull)) ||
-                        (!scales_seen && !mbar_wait(bar_scales_ready + 8 * stage, phase, abort_flag, p.status_word, kErrMmaWaitScales))) {
+                    // codes in shared memory (TMA) and block scales on their way to tensor memory (copy warp)
+                    if (!tokens_seen && !mbar_wait(t_full + 8 * slot, t_phase, abort_flag, p.status_word, kErrMmaWaitTokens)) {
                         alive = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint64_t a_desc = a_desc0 + stage * kStageStep, b_desc = b_desc0 + stage * kStageStep;
-                    const uint32_t tmem_sfa = tmem_base + kTmemPairSfA + stage * 16, done = bar_empty + 8 * stage;
-                    if (++stage == kPairStages) { stage = 0; phase ^= 1; }
-                    operands_seen = mbar_test(bar_full + 8 * stage, phase);
-                    scales_seen = mbar_test(bar_scales_ready + 8 * stage, phase);
-                    if (term + 1 == p.terms) weights_seen = mbar_test(bar_weights_ready + 8 * kb_slot, kb_phase);
+                    const uint64_t t_desc = t_desc0 + slot * (kPairTokenSlot >> 4);
+                    const uint32_t sf_t = tmem_tokens + slot * 16, t_done = t_empty + 8 * slot;
+                    if (++slot == depth.tokens) { slot = 0; t_phase ^= 1; }
+                    tokens_seen = mbar_test(t_full + 8 * slot, t_phase);
+                    if (term + 1 == p.terms) weights_seen = mbar_test(w_full + 8 * w_stage, w_phase);
                     if (elect_one()) {
                         // each MMA consumes 64 k = 32 bytes of every row: start address + 2; only k steps inside the tensor
                         if (k_steps == 4) {
 #pragma unroll
                             for (uint32_t k = 0; k < 4; ++k) {
-                                tc_mma_pair(tmem_base + kTmemAcc, a_desc + 2 * k, b_desc + 2 * k, idesc, tmem_sfa + 4 * k, tmem_sfb + 8 * k,
-                                            accumulate | k);
+                                tc_mma_pair(tmem_base + kTmemAcc, t_desc + 2 * k, w_desc + 2 * k, idesc, sf_t + 4 * k, sf_w + 8 * k, accumulate | k);
                             }
                         } else {
                             for (uint32_t k = 0; k < k_steps; ++k) {
-                                tc_mma_pair(tmem_base + kTmemAcc, a_desc + 2 * k, b_desc + 2 * k, idesc, tmem_sfa + 4 * k, tmem_sfb + 8 * k,
-                                            accumulate | k);
+                                tc_mma_pair(tmem_base + kTmemAcc, t_desc + 2 * k, w_desc + 2 * k, idesc, sf_t + 4 * k, sf_w + 8 * k, accumulate | k);
                             }
                         }
-                        tc_commit_pair(done);   // frees the stage, and with it the stage's scale columns, in both CTAs
+                        tc_commit_pair(t_done);   // frees the slot, and with it the slot's scale columns, in both CTAs
                     }
                     __syncwarp();
                     accumulate = 1;
@@ -348,19 +400,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
     } else if ((warp == kPairCopyWarp || warp == kPairCopyWarp + 1) && rank == 0) {
         // ---------------- scale-copy issuers (leader only): shared memory -> tensor memory, both CTAs ----------------
         // One warp copies the token rows' scales of every step, the other the weight rows' scales, which are the same for all
-        // activation terms of a k block, with term 0. (One thread issuing all twelve copies of a one-term step needed longer
+        // activation terms of a k block. (One thread issuing all twelve copies of a one-term step needed longer
         // than the step's MMAs: 193 us for 4096 tokens on 17408 x 5120.)
-        // A stage's scale atoms have landed. The producer refilled the stage only after the MMAs of the step that used it
-        // last (kPairStages steps ago) were complete, and operations complete in order, so every older MMA is complete
-        // too: the stage's token-row scale columns are free, and so are the weight-row scale columns of this k
-        // block's slot, last read by the k block kPairStages before it (at least kPairStages steps ago for any number
-        // of terms). The copies only have to be issued before the MMAs that read them: a copy and a later MMA execute
-        // in issue order, and the fences on either side of the arrival order the two warps' issues.
+        // A slot's scale atoms have landed. The producer refilled the slot only after the MMAs that used it last were
+        // complete, so the slot's scale columns are free. The copies only have to be issued before the MMAs that read them: a
+        // copy and a later MMA execute in issue order, and the fences on either side of the arrival order the two warps' issues.
         const bool weights = warp != kPairCopyWarp;
-        uint32_t stage = 0, phase = 0, kb_slot = 0;
-        const uint32_t smem_base = smem_u32(smem);
-        const uint64_t sfa_desc0 = sf_desc(smem_base + kBytesA + kPairBytesB), sfb_desc0 = sf_desc(smem_base + kBytesA + kPairBytesB + kBytesSfA);
-        constexpr uint32_t kStageStep = kPairStageBytes >> 4, kAtomStep = kSfAtomBytes >> 4, kRowBlockStep = kBytesSfA >> 4;
+        uint32_t slot = 0, phase = 0;
+        const uint32_t slots = weights ? depth.weights : depth.tokens, per_block = weights ? 1u : p.terms;
+        const uint32_t landed = weights ? w_landed : t_landed, full = weights ? w_full : t_full;
+        const uint64_t desc0 = sf_desc(weights ? smem_base + kPairBytesB : tokens_base + kBytesA);
+        const uint32_t slot_step = (weights ? kPairWeightStage : kPairTokenSlot) >> 4;
+        const uint32_t columns0 = weights ? tmem_weights : tmem_tokens, slot_columns = weights ? 32 : 16;
+        constexpr uint32_t kAtomStep = kSfAtomBytes >> 4, kRowBlockStep = kBytesSfB / 2 >> 4;
         const uint32_t last_k_steps = (p.cols - (k_blocks - 1) * kBlockK) / 64;
         bool alive = true;
         for (uint32_t index = 0; alive && index < work.items; ++index) {
@@ -368,63 +420,57 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
             const bool wide = item.tile / m_pairs != half_tile;   // a half tile has one row block of weight scales
             for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb) {
                 const uint32_t k_steps = (kb + 1 < k_blocks) ? 4u : last_k_steps;
-                for (uint32_t term = 0; term < p.terms; ++term) {
-                    // both warps wait for every step, so that neither can take a phase of the barrier for a later one
-                    if (!mbar_wait(bar_scales_landed + 8 * stage, phase, abort_flag, p.status_word, kErrCopyWait)) {
+                for (uint32_t term = 0; term < per_block; ++term) {
+                    if (!mbar_wait(landed + 8 * slot, phase, abort_flag, p.status_word, kErrCopyWait)) {
                         alive = false;
                         break;
                     }
-                    if (!weights || term == 0) {
-                        tc_fence_after();
-                        if (elect_one()) {
-                            if (!weights) {
-                                const uint64_t desc = sfa_desc0 + stage * kStageStep;
-                                const uint32_t columns = tmem_base + kTmemPairSfA + stage * 16;
-                                if (k_steps == 4) {
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint64_t desc = desc0 + slot * slot_step;
+                        const uint32_t columns = columns0 + slot * slot_columns;
+                        if (!weights) {
+                            if (k_steps == 4) {
 #pragma unroll
-                                    for (uint32_t k = 0; k < 4; ++k) tc_copy_sf_pair(columns + 4 * k, desc + k * kAtomStep);
-                                } else {
-                                    for (uint32_t k = 0; k < k_steps; ++k) tc_copy_sf_pair(columns + 4 * k, desc + k * kAtomStep);
-                                }
+                                for (uint32_t k = 0; k < 4; ++k) tc_copy_sf_pair(columns + 4 * k, desc + k * kAtomStep);
                             } else {
-                                const uint64_t desc = sfb_desc0 + stage * kStageStep;
-                                const uint32_t columns = tmem_base + kTmemPairSfB + kb_slot * 32;
-                                if (k_steps == 4 && wide) {
-#pragma unroll
-                                    for (uint32_t k = 0; k < 4; ++k) {
-                                        tc_copy_sf_pair(columns + 8 * k, desc + k * kAtomStep);
-                                        tc_copy_sf_pair(columns + 8 * k + 4, desc + kRowBlockStep + k * kAtomStep);
-                                    }
-                                } else {
-                                    for (uint32_t k = 0; k < k_steps; ++k) {
-                                        tc_copy_sf_pair(columns + 8 * k, desc + k * kAtomStep);
-                                        if (wide) tc_copy_sf_pair(columns + 8 * k + 4, desc + kRowBlockStep + k * kAtomStep);
-                                    }
-                                }
+                                for (uint32_t k = 0; k < k_steps; ++k) tc_copy_sf_pair(columns + 4 * k, desc + k * kAtomStep);
                             }
-                            tc_fence_before();
-                            mbar_arrive(weights ? bar_weights_ready + 8 * kb_slot : bar_scales_ready + 8 * stage);
+                        } else if (k_steps == 4 && wide) {
+#pragma unroll
+                            for (uint32_t k = 0; k < 4; ++k) {
+                                tc_copy_sf_pair(columns + 8 * k, desc + k * kAtomStep);
+                                tc_copy_sf_pair(columns + 8 * k + 4, desc + kRowBlockStep + k * kAtomStep);
+                            }
+                        } else {
+                            for (uint32_t k = 0; k < k_steps; ++k) {
+                                tc_copy_sf_pair(columns + 8 * k, desc + k * kAtomStep);
+                                if (wide) tc_copy_sf_pair(columns + 8 * k + 4, desc + kRowBlockStep + k * kAtomStep);
+                            }
                         }
-                        __syncwarp();
+                        tc_fence_before();
+                        mbar_arrive(full + 8 * slot);
                     }
-                    if (++stage == kPairStages) { stage = 0; phase ^= 1; }
+                    __syncwarp();
+                    if (++slot == slots) { slot = 0; phase ^= 1; }
                 }
-                if (++kb_slot == kPairStages) kb_slot = 0;
             }
         }
     } else if (warp >= 2 && warp < 2 + kPairEpilogueWarps) {
         // ---------------- epilogue (both CTAs): own TMEM half -> BF16 -> global ----------------
+        // The wait for the tile is a suspended one: eight polling warps cost 2 to 3 % of the time at the board's power cap.
         // Two warps per lane quadrant, 128 accumulator columns each. A warp reads its columns into registers
         // in one go and releases the accumulator at once; conversion, staging and the stores to global memory
         // run while the next tile's MMAs are already under way.
         const uint32_t quadrant = warp & 3, half = (warp - 2) >> 2;
         uint32_t tmem_phase = 0;
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing is written while an earlier kernel may still read it
         // this warp's transposition rows (lane = row): one 32-column chunk at a time
         uint8_t* my_rows = out_stage + (warp - 2) * 32 * kPairOutRowBytes;
         for (uint32_t index = 0; index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
             const uint32_t m_pair = item.tile % m_pairs, n_tile = item.tile / m_pairs;
-            if (!mbar_wait(bar_tmem_full, tmem_phase, abort_flag, p.status_word, kErrEpilogueWait)) break;
+            if (!mbar_wait_suspended(bar_tmem_full, tmem_phase, abort_flag, p.status_word, kErrEpilogueWait)) break;
             tc_fence_after();
             const uint32_t accumulator = tmem_base + kTmemAcc + ((quadrant * 32) << 16) + half * 128;
             auto release = [&]() {   // the accumulator is free for the next tile's MMAs from here on
@@ -811,16 +857,21 @@ uint32_t gemm_pair_resident_clusters() {
     attribute.val.clusterDim.z = 1;
     config.attrs = &attribute;
     config.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, gemm_pair_kernel, &config) != cudaSuccess || clusters < 1) {
-        cudaGetLastError();
-        return 0;
+    int fewest = INT_MAX;
+    for (auto* kernel : {gemm_pair_kernel<false>, gemm_pair_kernel<true>}) {
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess || clusters < 1) {
+            cudaGetLastError();
+            return 0;
+        }
+        if (clusters < fewest) fewest = clusters;
     }
-    return static_cast<uint32_t>(clusters);
+    return static_cast<uint32_t>(fewest);
 }
 
 cudaError_t gemm_configure_device() {
-    return cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
 }
 
 }  // namespace augur_sm100
@@ -980,7 +1031,7 @@ augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_s
             p.split_flags = reinterpret_cast<uint32_t*>(plan->scratch);
             p.split_slots = reinterpret_cast<float*>(plan->scratch + kCounterBytes);
         }
-        launch_dependent(s->stream, gemm_pair_kernel, 2 * split.pairs, kPairThreads, kPairSmemBytes, map_act, map_weight, map_act_sf, map_weight_sf, p);
+        launch_dependent(s->stream, a->activation_terms > 1 ? gemm_pair_kernel<true> : gemm_pair_kernel<false>, 2 * split.pairs, kPairThreads, kPairSmemBytes, map_act, map_weight, map_act_sf, map_weight_sf, p);
         count_launch();
         const augur_cuda_result_v1 result = submitted();
         if (result.status != AUGUR_CUDA_STATUS_OK || p.token_pairs * 2 * kTileM >= a->tokens) return result;
