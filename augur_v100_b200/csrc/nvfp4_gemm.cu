@@ -910,9 +910,10 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_act_quant
     const uint64_t groups = static_cast<uint64_t>(a->tokens) * (a->cols / 16);
     // Rows past `tokens` in the last 128-row tile (codes and scale bytes) are left as they are: they only
     // feed output rows that the GEMM never stores.
-    launch_dependent(s->stream, act_quant_kernel, static_cast<uint32_t>((groups + kQuantThreads - 1) / kQuantThreads), kQuantThreads, 0,
-                     reinterpret_cast<const uint16_t*>(a->input_bf16), reinterpret_cast<uint8_t*>(a->destination), a->tokens, a->cols,
-                     a->terms, a->global_scale);
+    // Spread: 6144 x 5120, three terms, 48 tokens 18.5 -> 17.2 us; 256 tokens 30.7 -> 30.4.
+    launch_dependent_spread(s->stream, act_quant_kernel, static_cast<uint32_t>((groups + kQuantThreads - 1) / kQuantThreads), kQuantThreads,
+                            reinterpret_cast<const uint16_t*>(a->input_bf16), reinterpret_cast<uint8_t*>(a->destination), a->tokens, a->cols,
+                            a->terms, a->global_scale);
     count_launch();
     return submitted();
 }

@@ -12,7 +12,7 @@
 // Two rings in shared memory, because a weight stage (16 KB of codes, 2 KB of block scales) serves all terms of its k block
 // while an activation slot (tokens x 128 bytes of codes, 2 KB of scales) serves one term.
 //
-// An item is (128-row tile, token tile of at most 128), one per CTA. Two CTAs share an SM (113 KB of shared and half of tensor
+// An item is (128-row tile, token tile of at most 128), one per CTA. Two CTAs share an SM (112 KB of shared and half of tensor
 // memory each): while one waits for its rings or stores its results the other feeds the tensor pipe (one CTA per SM with
 // deeper rings took 30.4 us where this takes 22 for 17408 x 5120, 128 tokens, three terms). With fewer tiles than
 // places a cluster of up to 8 CTAs shares an item, each CTA an equal range of its k blocks; when all are done (a cluster
@@ -48,7 +48,9 @@ constexpr uint32_t kNarrowBound = 32 * 14;
 constexpr uint32_t kNarrowState = 1024;                               // barriers, tensor-memory base, abort flag
 constexpr uint32_t kNarrowTurnPitch = 36;                             // floats between columns of the transposition area: 16-byte reads hit all banks
 constexpr uint32_t kNarrowSumPitch = 129;                             // 16-byte rows between groups of four columns of the partial sums, likewise
-constexpr uint32_t kNarrowSmem = 113 * 1024;                          // of two CTAs per SM
+// Of two CTAs per SM. At 113 KB they took all of an SM's shared memory with what the system reserves for each, so that no quantiser
+// CTA found room beside two of them: 17408 x 5120, three terms, 128 tokens 33.8 -> 30.8 us, 48 tokens 26.1 -> 24.4.
+constexpr uint32_t kNarrowSmem = 112 * 1024;
 constexpr uint32_t kNarrowTmemColumns = 256;
 constexpr uint32_t kNarrowMaxParts = 8;                               // portable cluster size
 
@@ -296,7 +298,8 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
     bool complete = true;
     if (epilogue) {
         if (!p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing is written while an earlier kernel may still read it
-        complete = mbar_wait(acc_full, 0, abort_flag, g.status_word, kErrNarrowAccFull);
+        // suspended: sixteen polling warps per SM took 2 to 3 % of the launch from those that issue
+        complete = mbar_wait_suspended(acc_full, 0, abort_flag, g.status_word, kErrNarrowAccFull);
         tc_fence_after();
     }
     __syncwarp();
