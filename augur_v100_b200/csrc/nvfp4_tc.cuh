@@ -106,6 +106,26 @@ __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint3
         ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
         : "memory");
 }
+// One pipeline step of a converged warp: the four MMAs of a 256-deep k block (64 k each: 32 bytes further in every operand row, four
+// scale columns further) and the commits that free what they read, `done` and, where `also` is not zero, `also_done`. The elected
+// lane is a predicate on the instructions, not a branch: the warp does not diverge, and the operands of all six are formed once
+// in uniform registers. Written as a branch around six separate instructions a step takes 400 cycles to issue, whatever its n.
+__device__ __forceinline__ void tc_step(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t accumulate,
+                                        uint32_t done, uint32_t also, uint32_t also_done) {
+    asm volatile(
+        "{\n.reg .pred e, f, p, q;\n.reg .b64 a1, a2, a3, b1, b2, b3;\n.reg .b32 s1, s2, s3, t1, t2, t3;\n"
+        "elect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, %6, 0;\nsetp.eq.u32 q, 0, 0;\nsetp.ne.and.b32 f, %8, 0, e;\n"
+        "add.s64 a1, %1, 2;\nadd.s64 a2, %1, 4;\nadd.s64 a3, %1, 6;\nadd.s64 b1, %2, 2;\nadd.s64 b2, %2, 4;\nadd.s64 b3, %2, 6;\n"
+        "add.s32 s1, %4, 4;\nadd.s32 s2, %4, 8;\nadd.s32 s3, %4, 12;\nadd.s32 t1, %5, 4;\nadd.s32 t2, %5, 8;\nadd.s32 t3, %5, 12;\n"
+        "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n"
+        "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a1, b1, %3, [s1], [t1], q;\n"
+        "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a2, b2, %3, [s2], [t2], q;\n"
+        "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a3, b3, %3, [s3], [t3], q;\n"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n"
+        "@f tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%9];\n}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "r"(done), "r"(also), "r"(also_done)
+        : "memory");
+}
 __device__ __forceinline__ void tc_load32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
