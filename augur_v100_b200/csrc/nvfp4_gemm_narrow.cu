@@ -15,9 +15,8 @@
 // An item is (128-row tile, token tile of at most 128), one per CTA. Two CTAs share an SM (112 KB of shared and half of tensor
 // memory each): while one waits for its rings or stores its results the other feeds the tensor pipe (one CTA per SM with
 // deeper rings took 30.4 us where this takes 22 for 17408 x 5120, 128 tokens, three terms). With fewer tiles than
-// places a cluster of up to 8 CTAs shares an item, each CTA an equal range of its k blocks; when all are done (a cluster
-// barrier, after which nobody reads its rings any more) every CTA sends its partial sums, by column, to the CTA that owns the
-// column, over distributed shared memory into the space the rings took, and finishes its own columns, adding in CTA
+// places a cluster of up to 8 CTAs shares an item, each CTA an equal range of its k blocks; when all are done every CTA
+// reads the partial sums of its share of the columns from all of them over distributed shared memory and adds them in CTA
 // order: no scratch, no fences to global memory, no atomics, and results that do not depend on scheduling. (The pair
 // kernel's hand-over of leftover tiles through global memory is what most of its time goes to at these sizes.)
 //
@@ -48,11 +47,14 @@ constexpr uint32_t kNarrowBound = 32 * 14;
 constexpr uint32_t kNarrowState = 1024;                               // barriers, tensor-memory base, abort flag
 constexpr uint32_t kNarrowTurnPitch = 36;                             // floats between columns of the transposition area: 16-byte reads hit all banks
 constexpr uint32_t kNarrowSumPitch = 129;                             // 16-byte rows between groups of four columns of the partial sums, likewise
+constexpr uint32_t kNarrowRowPitch = kTileM + 4;                      // floats between columns of finished sums on their way to SwiGLU, likewise
 // Of two CTAs per SM. At 113 KB they took all of an SM's shared memory with what the system reserves for each, so that no quantiser
 // CTA found room beside two of them: 17408 x 5120, three terms, 128 tokens 33.8 -> 30.8 us, 48 tokens 26.1 -> 24.4.
 constexpr uint32_t kNarrowSmem = 112 * 1024;
 constexpr uint32_t kNarrowTmemColumns = 256;
 constexpr uint32_t kNarrowMaxParts = 8;                               // portable cluster size
+static_assert(kTileM / 4 * kNarrowSumPitch * 16 + kTileM / 2 * kNarrowRowPitch * 4 <= kNarrowSmem - 1024 - kNarrowState,
+              "partial sums of all columns and finished ones of half of them in the space of the rings");
 
 constexpr uint32_t kErrNarrowWeights = 0x111, kErrNarrowTokens = 0x112, kErrNarrowFull = 0x113, kErrNarrowScales = 0x114,
                    kErrNarrowCopy = 0x115, kErrNarrowAccFull = 0x116;
@@ -107,6 +109,15 @@ __device__ __forceinline__ void narrow_copy_scales(uint32_t columns, uint64_t de
     } else {
         for (uint32_t k = 0; k < k_steps; ++k) tc_copy_sf(columns + 4 * k, desc + k * (kSfAtomBytes >> 4));
     }
+}
+
+// 16 bytes at this offset of another CTA's shared memory.
+__device__ __forceinline__ float4 narrow_read_cluster(uint32_t offset, uint32_t cta) {
+    uint32_t at;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(offset), "r"(cta));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
 }
 
 __device__ __forceinline__ void narrow_cluster_sync() {
@@ -322,52 +333,77 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
             }
         }
     } else {
-        // every CTA of the cluster owns a share of the columns
-        const uint32_t share = ((p.columns + p.parts - 1) / p.parts + 3) / 4 * 4;
-        narrow_cluster_sync();   // all MMAs of the cluster are complete: the rings may be overwritten
+        // Every CTA of the cluster finishes a share of the columns. It parks its sums in the space of its own rings, which are done
+        // with; one meeting later all threads read the share's sums from all CTAs, four columns of a row each, every CTA's at once
+        // (own is a multiple of four and a tile has 128 rows, so a warp's 32 lanes are always 32 rows of the same columns).
+        // Sent to their owners instead, which takes a meeting more, and added by the few lanes that have a column, three terms: 1024 x 5120
+        // at 32 tokens 11.9 us against 11.2, 6144 x 5120 at 48 tokens 15.7 against 15.5, 17408 x 5120 at 128 tokens 28.9 against 28.1.
+        const uint32_t share = ((p.columns + p.parts - 1) / p.parts + 3) / 4 * 4, first = part * share;
+        const uint32_t own = first < p.columns ? min(share, p.columns - first) : 0;
+        float4* sums = reinterpret_cast<float4*>(smem);   // [group of four columns][row]
+        float* turn = reinterpret_cast<float*>(sums + p.columns / 4 * kNarrowSumPitch);
         if (epilogue && complete) {
             for (uint32_t column = first_chunk * 32; column < p.columns; column += 64) {
                 uint32_t v[32];
                 tc_load32(tmem_base + ((quadrant * 32) << 16) + column, v);
                 tc_wait_ld();
-                uint32_t owner = column / share, local = column - owner * share;
 #pragma unroll
-                for (uint32_t i = 0; i < 32; i += 4) {   // shares are multiples of 4 columns
-                    if (column + i < p.columns) {
-                        uint32_t to;
-                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                                     : "=r"(to)
-                                     : "r"(smem_u32(smem) + ((part * share + local) / 4 * kNarrowSumPitch + quadrant * 32 + lane) * 16), "r"(owner));
-                        asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};"
-                                     ::"r"(to), "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3]) : "memory");
-                    }
-                    local += 4;
-                    if (local >= share) { local -= share; ++owner; }
+                for (uint32_t i = 0; i < 32; i += 4) {
+                    if (column + i >= p.columns) break;
+                    sums[(column + i) / 4 * kNarrowSumPitch + quadrant * 32 + lane] =
+                        make_float4(__uint_as_float(v[i]), __uint_as_float(v[i + 1]), __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
                 }
             }
         }
         __syncwarp();
-        narrow_cluster_sync();   // every partial sum has arrived; nobody writes this CTA's memory from here on
-        if (epilogue && complete) {
-            const float* base = reinterpret_cast<const float*>(smem);
-            for (uint32_t first = first_chunk * 32; first < share; first += 64) {
-                const uint32_t column = first + lane, token = token_row + part * share + column;
-                if (column >= share || token >= token_end) continue;
-                float sum[32];
+        narrow_cluster_sync();
+        const bool whole = *abort_flag == 0;
+        for (uint32_t index = threadIdx.x; whole && index < own * (kTileM / 4); index += kNarrowThreads) {
+            const uint32_t row = index % kTileM, column = index / kTileM * 4;
+            const uint32_t here = smem_u32(sums + (first + column) / 4 * kNarrowSumPitch + row);
+            float4 piece[kNarrowMaxParts], sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-                for (uint32_t i = 0; i < 32; ++i) sum[i] = 0.0f;
-                for (uint32_t from = 0; from < p.parts; ++from) {
-                    // [group of four columns][row]{column}: four lanes read neighbouring words, the eight groups of a warp other banks
-                    const float* src = base + ((from * share + column) / 4 * kNarrowSumPitch + quadrant * 32) * 4 + column % 4;
+            for (uint32_t from = 0; from < kNarrowMaxParts; ++from) {
+                if (from < p.parts) piece[from] = narrow_read_cluster(here, from);
+            }
 #pragma unroll
-                    for (uint32_t i = 0; i < 32; ++i) sum[i] += src[4 * i];
-                }
+            for (uint32_t from = 0; from < kNarrowMaxParts; ++from) {
+                if (from >= p.parts) break;
+                sum.x += piece[from].x; sum.y += piece[from].y; sum.z += piece[from].z; sum.w += piece[from].w;
+            }
+            if (g.swiglu) {
+                float* to = turn + column * kNarrowRowPitch + row;
+                to[0] = sum.x; to[kNarrowRowPitch] = sum.y; to[2 * kNarrowRowPitch] = sum.z; to[3 * kNarrowRowPitch] = sum.w;
+                continue;
+            }
+            // two rows go out as one word: the even lane of a pair takes the first two columns, the odd lane the other two
+            const bool odd = row & 1;
+            const float a = __shfl_xor_sync(0xffffffffu, odd ? sum.x : sum.z, 1), b = __shfl_xor_sync(0xffffffffu, odd ? sum.y : sum.w, 1);
+            const __nv_bfloat162 words[2] = {__floats2bfloat162_rn((odd ? a : sum.x) * g.scale, (odd ? sum.z : a) * g.scale),
+                                             __floats2bfloat162_rn((odd ? b : sum.y) * g.scale, (odd ? sum.w : b) * g.scale)};
+            const uint32_t token = token_row + first + column + (odd ? 2 : 0);
+            __nv_bfloat16* to = g.out + static_cast<uint64_t>(token) * g.rows + row_tile * kTileM + (row & ~1u);
+            if (token < token_end) *reinterpret_cast<__nv_bfloat162*>(to) = words[0];
+            if (token + 1 < token_end) *reinterpret_cast<__nv_bfloat162*>(to + g.rows) = words[1];
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // this CTA has read what it needs of the others
+        if (g.swiglu) {
+            __syncthreads();
+            for (uint32_t index = threadIdx.x; whole && index < own * 4; index += kNarrowThreads) {
+                const uint32_t column = index % own, rows32 = index / own;
+                if (token_row + first + column >= token_end) continue;
                 uint32_t v[32];
 #pragma unroll
-                for (uint32_t i = 0; i < 32; ++i) v[i] = __float_as_uint(sum[i]);
-                narrow_store(g, token, row0, v);
+                for (uint32_t i = 0; i < 8; ++i) {
+                    const uint4 four = *reinterpret_cast<const uint4*>(turn + column * kNarrowRowPitch + rows32 * 32 + 4 * i);
+                    v[4 * i] = four.x; v[4 * i + 1] = four.y; v[4 * i + 2] = four.z; v[4 * i + 3] = four.w;
+                }
+                narrow_store(g, token_row + first + column, row_tile * kTileM + rows32 * 32, v);
             }
+            __syncwarp();
         }
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");     // and the others of this one
     }
     // the successor's wait covers this launch only, so this launch ends after the one before it
     if (p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");
