@@ -509,7 +509,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
                         for (uint32_t term = 0; term < 3; ++term) {
                             if (term >= p.quant_terms) break;
                             uint32_t codes[2], scale_code;
-                            quantise_term(residual, p.quant_global_scale, term + 1 < p.quant_terms, codes, &scale_code);
+                            quantise_term(residual, p.quant_scale, term + 1 < p.quant_terms, codes, &scale_code);
                             scale_words[term] |= scale_code << (8 * c);
                             *reinterpret_cast<uint2*>(p.quant_out + term * code_bytes + static_cast<uint64_t>(token) * (out_width / 2) + group * 8) =
                                 make_uint2(codes[0], codes[1]);
@@ -688,7 +688,7 @@ constexpr uint32_t kQuantThreads = 128;
 // `x` is read by coherent loads: the launch before this one may still be writing it when this grid starts, so it is not
 // constant for the life of the grid, which is what __ldg (and a compiler's choice of it) would promise.
 __global__ void __launch_bounds__(kQuantThreads) act_quant_kernel(const uint16_t* x, uint8_t* destination, uint32_t tokens, uint32_t cols,
-                                                                  uint32_t terms, float global_scale) {
+                                                                  uint32_t terms, const QuantScale scale) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");   // x may come from the launch before this one, and the destination may still be read by it
     const uint32_t groups = cols / 16;
@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(kQuantThreads) act_quant_kernel(const uint16_t
     const uint64_t code_bytes = tcgen05_codes_bytes(padded_tokens(tokens), cols), scale_bytes = tcgen05_scale_bytes(tokens, cols);
     for (uint32_t term = 0; term < terms; ++term) {
         uint32_t packed[2], scale_code;
-        quantise_term(residual, global_scale, term + 1 < terms, packed, &scale_code);
+        quantise_term(residual, scale, term + 1 < terms, packed, &scale_code);
         *reinterpret_cast<uint2*>(destination + term * code_bytes + static_cast<uint64_t>(token) * (cols / 2) + group * 8) =
             make_uint2(packed[0], packed[1]);
         // The scales of four consecutive groups of a token are four consecutive bytes of an atom: lanes are
@@ -913,7 +913,7 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_act_quant
     // Spread: 6144 x 5120, three terms, 48 tokens 18.5 -> 17.2 us; 256 tokens 30.7 -> 30.4.
     launch_dependent_spread(s->stream, act_quant_kernel, static_cast<uint32_t>((groups + kQuantThreads - 1) / kQuantThreads), kQuantThreads,
                             reinterpret_cast<const uint16_t*>(a->input_bf16), reinterpret_cast<uint8_t*>(a->destination), a->tokens, a->cols,
-                            a->terms, a->global_scale);
+                            a->terms, quant_scale(a->global_scale));
     count_launch();
     return submitted();
 }
@@ -1014,7 +1014,7 @@ augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_s
     p.swiglu = swiglu ? 1u : 0u;
     p.quant_out = reinterpret_cast<uint8_t*>(quant.destination);
     p.quant_terms = quant.terms;
-    p.quant_global_scale = quant.global_scale;
+    p.quant_scale = quant_scale(quant.global_scale);
     p.token_pairs = token_pairs_for(plan, a->rows, a->cols, a->tokens, a->activation_terms);
     if (p.token_pairs) {
         // 256 x 256 tiles on pairs of CTAs (clusters of two); the grid is a whole number of pairs.

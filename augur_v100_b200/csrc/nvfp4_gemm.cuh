@@ -26,7 +26,7 @@ struct GemmParams {
     // SwiGLU: the intermediate is also (or only, if `out` is null) quantised for the next GEMM
     uint8_t* quant_out;            // staged activations: [terms] code planes of whole tiles, then the scale regions
     uint32_t quant_terms;
-    float quant_global_scale;
+    tc::QuantScale quant_scale;
     // Pair tiles whose count is not a multiple of the pairs: the tiles left over are cut along k between all pairs
     // (null: whole tiles only). Partial accumulators pass through `split_slots`, announced by `split_flags`.
     float* split_slots;            // [pair][CTA of the pair][epilogue warp][128 columns / 4][lane] x float4

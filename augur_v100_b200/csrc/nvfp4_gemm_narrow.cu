@@ -94,7 +94,7 @@ __device__ __forceinline__ void narrow_store(const GemmParams& g, uint32_t token
 #pragma unroll 1
         for (uint32_t term = 0; term < g.quant_terms; ++term) {
             uint32_t codes[2], scale_code;
-            quantise_term(residual, g.quant_global_scale, term + 1 < g.quant_terms, codes, &scale_code);
+            quantise_term(residual, g.quant_scale, term + 1 < g.quant_terms, codes, &scale_code);
             *reinterpret_cast<uint2*>(g.quant_out + term * code_bytes + static_cast<uint64_t>(token) * (out_width / 2) + group * 8) = make_uint2(codes[0], codes[1]);
             g.quant_out[g.quant_terms * code_bytes + term * scale_bytes + tcgen05_scale_offset(token, group, out_width)] = static_cast<uint8_t>(scale_code);
         }

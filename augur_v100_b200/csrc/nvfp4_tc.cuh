@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstring>
 
 namespace augur_sm100 {
 namespace tc {
@@ -210,15 +211,17 @@ __device__ __forceinline__ uint32_t e2m1_nearest(float v, float* level) {
 
 // Eight quotients -> eight codes, element i in nibble i, by the hardware converter: round to nearest even,
 // magnitudes above 6 (infinities too) to 6. It differs from "nearest, ties toward zero, zero always code 0" in
-// three places, put right here. At 0.75, 1.75 and 3.5 "even" is the larger level. A tie is a value of at most
-// three significant bits; every quotient that short (low 21 bits of the pattern zero) goes in one or two ulps
-// nearer to zero, which takes a tie to the level below and changes nothing else: the values passed over
-// are not short, so none of them is a tie, and a zero stays a zero. A negative quotient that rounds to zero
-// comes out as code 8. And a NaN comes out as +6 (the caller keeps groups with a NaN off this path).
-__device__ __forceinline__ float off_the_tie(float q) {
-    return (__float_as_uint(q) & 0x1fffffu) == 0 ? __fmul_rn(q, 0x1.fffffcp-1f) : q;   // q * (1 - 2^-23)
-}
-__device__ __forceinline__ uint32_t e2m1x8_nearest(const float2 (&q)[4]) {
+// three places, put right here. At 0.75, 1.75 and 3.5 "even" is the larger level; at the other ties it is the smaller one. The
+// three have a significand of 1.5 or 1.75, the others of 1 or 1.25, so every quotient goes in one ulp nearer to zero if its
+// significand m is above 1.37 and as it is otherwise: q - q * 1.457 * 2^-25 takes 0.364 m
+// of an ulp off, which rounds to the neighbour once it exceeds half of one. A tie of the three then lies below itself, the value one ulp above it on the tie,
+// which rounds up as it must, and no other boundary has values so close (all F32 values from 2^-6 to 16 were compared). A negative
+// quotient that rounds to zero comes out as code 8. And a NaN comes out as +6 (the caller keeps groups with a NaN off this path).
+__device__ __forceinline__ uint32_t e2m1x8_nearest(const float2 (&quotient)[4]) {
+    const float2 nudge = make_float2(-0x1.75p-25f, -0x1.75p-25f);
+    float2 q[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i) q[i] = __ffma2_rn(quotient[i], nudge, quotient[i]);
     uint32_t codes;
     asm("{\n .reg .b8 b0, b1, b2, b3;\n"
         "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n"
@@ -227,8 +230,7 @@ __device__ __forceinline__ uint32_t e2m1x8_nearest(const float2 (&q)[4]) {
         "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n"
         "mov.b32 %0, {b0, b1, b2, b3};\n}"
         : "=r"(codes)
-        : "f"(off_the_tie(q[0].x)), "f"(off_the_tie(q[0].y)), "f"(off_the_tie(q[1].x)), "f"(off_the_tie(q[1].y)),
-          "f"(off_the_tie(q[2].x)), "f"(off_the_tie(q[2].y)), "f"(off_the_tie(q[3].x)), "f"(off_the_tie(q[3].y)));
+        : "f"(q[0].x), "f"(q[0].y), "f"(q[1].x), "f"(q[1].y), "f"(q[2].x), "f"(q[2].y), "f"(q[3].x), "f"(q[3].y));
     const uint32_t nonzero = (codes | (codes >> 1) | (codes >> 2)) & 0x11111111u;   // bit 0 of every nibble with a magnitude
     return codes & ((nonzero << 3) | 0x77777777u);
 }
@@ -314,21 +316,57 @@ __device__ __forceinline__ float group_divisor(float maximum, float global_scale
     return __fmul_rn(scale, global_scale);
 }
 
+// What a quantiser knows about its global scale before it has seen an element: 6 g, and its rounded reciprocal where the Newton
+// steps below end on the correctly rounded quotient (0 where they need not, see quantise_group_fast).
+struct QuantScale {
+    float global, six, six_reciprocal;
+};
+inline QuantScale quant_scale(float global_scale) {
+    const float six = 6.0f * global_scale;
+    uint32_t bits;
+    memcpy(&bits, &six, 4);
+    const uint32_t field = bits >> 23;
+    return QuantScale{global_scale, six, field >= 64u && field <= 180u && (bits & 0x7fffffu) != 0x7fffffu ? 1.0f / six : 0.0f};
+}
+
+// An E4M3 code as a float (hardware E4M3 -> F16, widened).
+__device__ __forceinline__ float e4m3_value(uint32_t code) {
+    uint32_t pair;
+    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(pair) : "h"(static_cast<uint16_t>(code)));
+    return __half2float(__ushort_as_half(static_cast<uint16_t>(pair & 0xffffu)));
+}
+// group_divisor for a `maximum` from 2^-63 to 2^64 and a scale with a reciprocal, without a branch: the quotient, which is a normal
+// number then, by two Newton steps (compared with IEEE division on 2 * 10^8 random cases), its ceiling as the hardware's nearest
+// value, or the one above where that is smaller.
+__device__ __forceinline__ float group_divisor_fast(float maximum, const QuantScale& s, uint32_t* scale_code_out) {
+    float desired = __fmul_rn(maximum, s.six_reciprocal);
+    float rest = __fmaf_rn(desired, -s.six, maximum);
+    desired = __fmaf_rn(rest, s.six_reciprocal, desired);
+    rest = __fmaf_rn(desired, -s.six, maximum);
+    desired = __fmaf_rn(rest, s.six_reciprocal, desired);
+    uint16_t nearest;
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(nearest) : "f"(0.0f), "f"(desired));
+    uint32_t code = nearest & 0xffu;
+    if (e4m3_value(code) < desired && code < 126u) ++code;
+    *scale_code_out = code;
+    return __fmul_rn(e4m3_value(code), s.global);
+}
+
 // One residual term of one 16-element group: the block scale, the 16 codes (nearest level of x / (scale * g),
 // ties toward zero) and, if another term follows, the residual it quantises.
 // `kMoreTerms` is a compile-time choice: the last term of a group needs neither the levels nor the residual.
 template <bool kMoreTerms>
-__device__ __forceinline__ void quantise_term_as(float2 (&residual)[8], float global_scale, uint32_t (&packed)[2],
+__device__ __forceinline__ void quantise_term_as(float2 (&residual)[8], const QuantScale& s, uint32_t (&packed)[2],
                                                  uint32_t* scale_code_out) {
     // This maximum carries a NaN along, which keeps the group off the fast path; the reference's maximum
     // leaves NaNs out, and only the other path computes it.
     float maximum = 0.0f;
 #pragma unroll
     for (uint32_t i = 0; i < 8; ++i) maximum = max_or_nan(maximum, fabsf(residual[i].x), fabsf(residual[i].y));
-    float divisor = group_divisor(maximum, global_scale, scale_code_out);
+    float divisor = group_divisor_fast(maximum, s, scale_code_out);
     const uint32_t divisor_field = (__float_as_uint(divisor) >> 23) & 0xffu, largest_field = (__float_as_uint(maximum) >> 23) & 0xffu;
     const bool fast = divisor_field >= 64u && divisor_field <= 190u && (__float_as_uint(divisor) & 0x7fffffu) != 0x7fffffu &&
-                      largest_field <= 190u;
+                      largest_field >= 64u && largest_field <= 190u && s.six_reciprocal != 0.0f;
     packed[0] = packed[1] = 0;
     if (fast) {
         quantise_group_fast<kMoreTerms>(residual, divisor, __frcp_rn(divisor), packed);
@@ -336,16 +374,16 @@ __device__ __forceinline__ void quantise_term_as(float2 (&residual)[8], float gl
         maximum = 0.0f;
 #pragma unroll
         for (uint32_t i = 0; i < 8; ++i) maximum = fmaxf(maximum, fmaxf(fabsf(residual[i].x), fabsf(residual[i].y)));
-        divisor = group_divisor(maximum, global_scale, scale_code_out);
+        divisor = group_divisor(maximum, s.global, scale_code_out);
         quantise_group_any<kMoreTerms>(residual, divisor, packed);
     }
 }
-__device__ __forceinline__ void quantise_term(float2 (&residual)[8], float global_scale, bool more_terms, uint32_t (&packed)[2],
+__device__ __forceinline__ void quantise_term(float2 (&residual)[8], const QuantScale& s, bool more_terms, uint32_t (&packed)[2],
                                               uint32_t* scale_code_out) {
     if (more_terms) {
-        quantise_term_as<true>(residual, global_scale, packed, scale_code_out);
+        quantise_term_as<true>(residual, s, packed, scale_code_out);
     } else {
-        quantise_term_as<false>(residual, global_scale, packed, scale_code_out);
+        quantise_term_as<false>(residual, s, packed, scale_code_out);
     }
 }
 
