@@ -556,7 +556,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
                 }
             }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         const uint32_t idesc = instr_desc(kCols);
         uint32_t step = 0, item_count = 0;
@@ -583,22 +583,19 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             const uint64_t weight_desc = operand_desc(stage_smem), act_desc = operand_desc(stage_smem + kStageActCodes);
             const uint32_t tmem_sf_weight = tmem_base + kTmemSfWeight + stage * 16, tmem_sf_act = tmem_base + kTmemSfAct + stage * 16;
             const uint32_t k_steps = min(kStageK, p.phase[p.step[c.step].phase].cols - c.kb * kStageK) / 64;
-            // each MMA consumes 64 k = 32 bytes of every row: advance the start address by 32 >> 4
+            const uint32_t accumulate = c.kb != c.kb0 ? 1u : 0u, last = c.kb + 1 == c.kb1 ? 1u : 0u;
+            // each MMA consumes 64 k = 32 bytes of every row; the commits free the stage and, behind an item's last k block, hand the accumulator over
             if (k_steps == 4) {
-#pragma unroll
-                for (uint32_t k = 0; k < 4; ++k) {
-                    tc_mma(acc, weight_desc + 2 * k, act_desc + 2 * k, idesc, tmem_sf_weight + 4 * k, tmem_sf_act + 4 * k,
-                           (c.kb != c.kb0 || k != 0) ? 1u : 0u);
-                }
-            } else {
+                tc_step(acc, weight_desc, act_desc, idesc, tmem_sf_weight, tmem_sf_act, accumulate, bar_empty + 8 * stage, last, bar_acc_full + 8 * buffer);
+            } else if (elect_one()) {
                 for (uint32_t k = 0; k < k_steps; ++k) {
-                    tc_mma(acc, weight_desc + 2 * k, act_desc + 2 * k, idesc, tmem_sf_weight + 4 * k, tmem_sf_act + 4 * k,
-                           (c.kb != c.kb0 || k != 0) ? 1u : 0u);
+                    tc_mma(acc, weight_desc + 2 * k, act_desc + 2 * k, idesc, tmem_sf_weight + 4 * k, tmem_sf_act + 4 * k, accumulate | k);
                 }
+                tc_commit(bar_empty + 8 * stage);
+                if (last) tc_commit(bar_acc_full + 8 * buffer);
             }
-            tc_commit(bar_empty + 8 * stage);   // frees the stage when these MMAs have read it
-            if (c.kb + 1 == c.kb1) {
-                tc_commit(bar_acc_full + 8 * buffer);
+            __syncwarp();
+            if (last) {
                 acc_phase[buffer] ^= 1;
                 ++item_count;
             }

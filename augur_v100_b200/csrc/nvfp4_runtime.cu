@@ -190,12 +190,12 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_plan_crea
     }
     if (major != 10) return make_result(AUGUR_CUDA_STATUS_UNSUPPORTED_DEVICE);
     // Kernels are loaded in this order. Where a kernel's code comes to lie is worth a few percent to the one-launch MLP block,
-    // whose code is larger than an instruction cache: 39.9 us at 5120 / 17408, 8 tokens, in this order, 40.9 with the split ahead of it;
-    // between linears, two layers 157.2 us in this order, 158.3 with the narrow GEMM ahead of the split. To be measured again
-    // whenever a kernel is added or grows.
-    e = gemv_configure_device();
+    // whose code is larger than an instruction cache, so it comes first, where what the other kernels grow by does not move it: two
+    // layers of linears and blocks 157.1 us in this order, 157.4 to 158.6 with it third, second or ahead of the split; the block
+    // alone 39.8 to 40.0 us in all of them (41.2 before its MMAs became one block of instructions, 39.9 to 40.9 by place).
+    e = gemv_tc_configure_device();
+    if (e == cudaSuccess) e = gemv_configure_device();
     if (e == cudaSuccess) e = gemm_configure_device();
-    if (e == cudaSuccess) e = gemv_tc_configure_device();
     if (e == cudaSuccess) e = gemv_split_configure_device();
     if (e == cudaSuccess) e = gemm_narrow_configure_device();
     if (e != cudaSuccess) return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE, e);
