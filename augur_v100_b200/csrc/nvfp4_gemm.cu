@@ -265,12 +265,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
     const uint32_t atoms_per_row_block = p.cols / 64;
     const uint32_t act_term_atoms = p.padded_tokens / 128 * atoms_per_row_block;   // scale atoms of one activation term
     const PairWork work = pair_work(pair, pairs, total_tiles, k_blocks, p.split_sharers);
+    // The weights are constant, so the first ring of them, `ahead` k blocks of the first item, is under way while the launch before
+    // this one, whose results the token rows are, still drains. What a role waits for on a barrier must not include that launch,
+    // whose time would count against the bound of the wait: a role that depends on it waits for its end first.
+    uint32_t ahead = 0;
+    if (work.items) {
+        const PairItem first = work.item(0, pair, pairs, k_blocks);
+        ahead = min(depth.weights, first.kb1 - first.kb0);
+    }
 
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
         // The block scales of a slot go first, on a barrier of their own: they are small and land early, so the copy warps have
-        // them in tensor memory by the time the operand tiles arrive. The weights are constant, so the first ring of them is
-        // under way while the launch before this one, whose results the token rows are, still drains.
+        // them in tensor memory by the time the operand tiles arrive.
         uint32_t w_stage = 0, slot = 0, t_phase = 1;
         bool alive = true;
         auto weight_scales = [&](uint32_t n_tile, uint32_t kb, uint32_t stage) {
@@ -284,13 +291,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
             if (rank == 0) mbar_expect_tx(full, 2 * kPairBytesB);
             tma_load_2d_pair(smem_base + stage * kPairWeightStage, &map_weight, kb * 128, n_tile * kTileN + rank * (n_tile == half_tile ? 64 : 128), full);
         };
-        uint32_t ahead = 0;
         if (work.items) {
             const PairItem first = work.item(0, pair, pairs, k_blocks);
-            for (; ahead < depth.weights && first.kb0 + ahead < first.kb1; ++ahead) {
+            for (uint32_t stage = 0; stage < ahead; ++stage) {
                 if (elect_one()) {
-                    weight_scales(first.tile / m_pairs, first.kb0 + ahead, ahead);
-                    weight_codes(first.tile / m_pairs, first.kb0 + ahead, ahead);
+                    weight_scales(first.tile / m_pairs, first.kb0 + stage, stage);
+                    weight_codes(first.tile / m_pairs, first.kb0 + stage, stage);
                 }
                 __syncwarp();
             }
@@ -347,6 +353,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         constexpr uint32_t kHalfTile = (1u << 7) | (1u << 10) | ((kTileN / 2 >> 3) << 17) | (((2 * kTileM) >> 4) << 24);
         const uint64_t w_desc0 = operand_desc(smem_base), t_desc0 = operand_desc(tokens_base);
         const uint32_t last_k_steps = (p.cols - (k_blocks - 1) * kBlockK) / 64;   // 1..4 k steps of 64 in the last k block
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // the token rows
         for (uint32_t index = 0; alive && index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
             // the epilogues of both CTAs must have drained the previous tile's accumulator
@@ -414,6 +421,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         const uint32_t columns0 = weights ? tmem_weights : tmem_tokens, slot_columns = weights ? 32 : 16;
         constexpr uint32_t kAtomStep = kSfAtomBytes >> 4, kRowBlockStep = kBytesSfB / 2 >> 4;
         const uint32_t last_k_steps = (p.cols - (k_blocks - 1) * kBlockK) / 64;
+        // the token rows; and weights beyond the first ring, whose stages are free when the token rows have been multiplied with
+        uint32_t before_wait = weights ? ahead : 0;
+        if (!before_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
         bool alive = true;
         for (uint32_t index = 0; alive && index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
@@ -453,6 +463,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
                     }
                     __syncwarp();
                     if (++slot == slots) { slot = 0; phase ^= 1; }
+                    if (before_wait && --before_wait == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
                 }
             }
         }

@@ -131,8 +131,9 @@ def _lagging_launch(env, plan):
     return program, buffers
 
 
-# The bounded waits of a launch do not run out while it waits for a launch ahead of it that takes long.
-@pytest.mark.parametrize("kind,tokens", [("split", 8), ("gemm", 16)])
+# The bounded waits of a launch do not run out while it waits for a launch ahead of it that takes long: small-token linear, narrow
+# GEMM, pair GEMM.
+@pytest.mark.parametrize("kind,tokens", [("split", 8), ("gemm", 16), ("gemm", 300)])
 def test_waits_do_not_count_the_launch_before(env, kind, tokens):
     torch, side, stream, plan = env["torch"], env["side"], env["stream"], env["plan"]
     with torch.cuda.stream(side):
