@@ -501,8 +501,11 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    // What a role waits for on a barrier must not include the launch before this one, whose time would count against the bound of
+    // the wait. Past the first ring of weights everything follows from the activations, so every role waits for its end first.
     if (warp == 0 && lane == 0) {
         // ---------------- TMA producer, weights: runs ahead as far as the ring allows ----------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         while (weights_left) {
             // stage of step `weights_issued`: free once the MMAs of the step kStages before it are complete
             const uint32_t stage = weights_issued % kStages, round = weights_issued / kStages;
@@ -514,6 +517,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
     } else if (warp == 11 && lane == 0) {
         // ---------------- TMA producer, activations: a stage's half follows as soon as the stage is free and the
         // split it comes from is complete in every CTA ----------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         Cursor acts_at;
         bool acts_left = cursor_begin(p, acts_at);
         uint32_t acts_issued = 0, idle = 0, polls = 0, open_jobs = 0;   // jobs 0 .. open_jobs - 1 are known to be complete
@@ -558,6 +562,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         const uint32_t idesc = instr_desc(kCols);
         uint32_t step = 0, item_count = 0;
         uint32_t acc_phase[2] = {0, 0};
@@ -607,6 +612,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
         // Two threads, one for the weights' scales and one for the activations': a thread gets one copy accepted
         // about every hundred cycles. A stage's scale columns in tensor memory are free when its scales land again:
         // the producer refilled the stage only after the MMAs that read those columns were complete.
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         const bool weights = warp == 10;
         uint32_t step = 0;
         Cursor c;

@@ -132,14 +132,20 @@ def _lagging_launch(env, plan):
 
 
 # The bounded waits of a launch do not run out while it waits for a launch ahead of it that takes long: small-token linear, narrow
-# GEMM, pair GEMM.
-@pytest.mark.parametrize("kind,tokens", [("split", 8), ("gemm", 16), ("gemm", 300)])
+# GEMM, pair GEMM, one-launch MLP block.
+@pytest.mark.parametrize("kind,tokens", [("split", 8), ("gemm", 16), ("gemm", 300), ("block", 8)])
 def test_waits_do_not_count_the_launch_before(env, kind, tokens):
     torch, side, stream, plan = env["torch"], env["side"], env["stream"], env["plan"]
     with torch.cuda.stream(side):
         x = torch.randn((tokens, COLS), device="cuda").to(torch.bfloat16)
         weight = host.Nvfp4Sm100Weight.repack_device_planes(stream, abi.LAYOUT_TCGEN05, ROWS, COLS, *env["planes"][0], synth.GLOBAL_SCALE)
-        program = {"split": host.Nvfp4Sm100TcProjection, "gemm": host.Nvfp4Sm100PrefillLinear}[kind].bind(plan, weight, x)
+        if kind == "block":
+            weight.global_scale_b = synth.GLOBAL_SCALE   # the rows as gate and up of an intermediate half as wide
+            codes, scales = (plane[:COLS] for plane in env["planes"][1])
+            down = host.Nvfp4Sm100Weight.repack_device_planes(stream, abi.LAYOUT_TCGEN05, COLS, ROWS // 2, codes, scales, synth.GLOBAL_SCALE)
+            program = host.Nvfp4Sm100TcFfnProgram.bind(plan, weight, down, x)
+        else:
+            program = {"split": host.Nvfp4Sm100TcProjection, "gemm": host.Nvfp4Sm100PrefillLinear}[kind].bind(plan, weight, x)
         program.submit_for_plan()
         wanted = program.out.clone()
         program.out.zero_()
