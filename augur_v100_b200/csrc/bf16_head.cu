@@ -36,20 +36,17 @@ constexpr uint32_t kHeadN = 32;                              // MMA n: 24 column
 constexpr uint32_t kHeadTile = kTileM * 128;                 // 16 KB: 128 rows x 64 k of BF16
 constexpr uint32_t kHeadStage = kHeadTile + kHeadN * 128;    // and 4 KB of split activations
 constexpr uint32_t kHeadStages = 11;
-constexpr uint32_t kHeadSmem = kHeadStages * kHeadStage + 512 /*barriers*/ + 1024 /*alignment*/;
 constexpr uint32_t kHeadAccs = 8;                            // accumulators of 32 columns
+constexpr uint32_t kHeadState = 512;                         // barriers, tensor-memory base, abort flag, a counter per warp
+constexpr uint32_t kHeadSmem = kHeadStages * kHeadStage + kHeadState + 1024 /*alignment*/;
 constexpr uint32_t kHeadAhead = 4;                           // stages of activations that a split thread has in flight
 constexpr uint32_t kHeadMaxRowBytes = 200 * 1024 / 8 - 64;   // of a token row of activations
 static_assert(kHeadSmem <= 227 * 1024, "shared memory of a CTA");
+static_assert((2 * kHeadStages + 2 * kHeadAccs) * 8 + 8 + kHeadThreads / 32 * 4 <= kHeadState, "the small state fits");
 
-// A bounded wait (the entry has no plan to report through: tiles that were given up on are NaN).
+// A bounded wait of a whole warp (the entry has no plan to report through: tiles that were given up on are NaN).
 __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
-    for (uint32_t spin = 0; spin < kWaitLimit; ++spin) {
-        if (mbar_test(bar, parity)) return true;
-        if ((spin & 1023u) == 1023u && *abort_flag) return false;
-    }
-    *abort_flag = 1;
-    return false;
+    return warp_look_wait(bar, parity, abort_flag, nullptr, 0);
 }
 
 // Two F32 values -> their three BF16 terms, packed (low half = first value). x = hi + mid + lo exactly: each
@@ -96,6 +93,7 @@ bf16_head_kernel(const __grid_constant__ CUtensorMap map_weight, const float* __
             mbar_init(bar_acc_empty + 8 * b, 4);
         }
         *abort_flag = 0;
+        for (uint32_t w = 0; w < kHeadThreads / 32; ++w) abort_flag[1 + w] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {

@@ -97,10 +97,10 @@ constexpr uint32_t kPairOutRowBytes = 64 + 16;
 constexpr uint32_t kPairOutBytes = kPairEpilogueWarps * 32 * kPairOutRowBytes;         // 20480
 constexpr uint32_t kPairBarriers = 5 * kPairMaxDepth + 2;
 constexpr uint32_t kPairSmemBytes = kPairRingBytes + kPairOutBytes + 1024 + 512;
-static_assert(kPairBarriers * 8 + 8 <= 512, "barriers, tensor-memory base and abort flag fit behind the rings");
 static_assert(kPairSmemBytes <= 227 * 1024, "shared memory of a CTA");
 constexpr uint32_t kPairCopyWarp = 2 + kPairEpilogueWarps;    // token-row scales; the warp after it copies the weight-row scales
 constexpr uint32_t kPairThreads = 32 * (kPairCopyWarp + 2);   // TMA warp, MMA warp, epilogue warps, two scale-copy warps
+static_assert(kPairBarriers * 8 + 8 + kPairThreads / 32 * 4 <= 512, "barriers, tensor-memory base, abort flag and the warps' counters fit behind the rings");
 constexpr uint32_t kSplitWays = 8;              // a leftover tile is cut into this many parts at most
 constexpr uint32_t kSplitWaitLimit = 1u << 20;  // polls of a handed-over part's flag (each a round trip to L2) before giving up
 constexpr uint64_t kSplitSlotBytes = 2ull * kPairEpilogueWarps * 32 * 128 * 4;   // one pair's accumulator: 256 x 256 f32
@@ -236,6 +236,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         mbar_init(bar_tmem_full, 1);
         mbar_init(bar_tmem_empty, 2 * kPairEpilogueWarps);   // one arrival per epilogue warp of either CTA
         *abort_flag = 0;
+        for (uint32_t w = 0; w < kPairThreads / 32; ++w) abort_flag[1 + w] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -311,7 +312,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
             const uint32_t n_tile = item.tile / m_pairs, token_row = item.tile % m_pairs * 2 * kTileM + rank * kTileM;
             for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb, ++blocks) {
                 if (blocks >= depth.weights) {
-                    if (!mbar_wait(t_empty + 8 * done_slot, done_phase, abort_flag, p.status_word, kErrProducerWait)) {
+                    if (!warp_look_wait(t_empty + 8 * done_slot, done_phase, abort_flag, p.status_word, kErrProducerWait)) {
                         alive = false;
                         break;
                     }
@@ -320,7 +321,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
                 }
                 const bool fetch = blocks >= ahead;
                 for (uint32_t term = 0; term < p.terms; ++term) {
-                    if (!mbar_wait(t_empty + 8 * slot, t_phase, abort_flag, p.status_word, kErrProducerWait)) {
+                    if (!warp_look_wait(t_empty + 8 * slot, t_phase, abort_flag, p.status_word, kErrProducerWait)) {
                         alive = false;
                         break;
                     }
@@ -357,13 +358,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         for (uint32_t index = 0; alive && index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
             // the epilogues of both CTAs must have drained the previous tile's accumulator
-            if (!mbar_wait(bar_tmem_empty, tmem_phase ^ 1, abort_flag, p.status_word, kErrMmaWaitTmem)) break;
+            if (!warp_look_wait(bar_tmem_empty, tmem_phase ^ 1, abort_flag, p.status_word, kErrMmaWaitTmem)) break;
             tc_fence_after();
             const uint32_t idesc = item.tile / m_pairs == half_tile ? kHalfTile : kWideTile;
             uint32_t accumulate = 0;
             for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb) {
                 const uint32_t k_steps = (kb + 1 < k_blocks) ? 4u : last_k_steps;
-                if (!weights_seen && !mbar_wait(w_full + 8 * w_stage, w_phase, abort_flag, p.status_word, kErrMmaWaitWeights)) {
+                if (!weights_seen && !warp_look_wait(w_full + 8 * w_stage, w_phase, abort_flag, p.status_word, kErrMmaWaitWeights)) {
                     alive = false;
                     break;
                 }
@@ -372,7 +373,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
                 if (++w_stage == depth.weights) { w_stage = 0; w_phase ^= 1; }
                 for (uint32_t term = 0; term < p.terms; ++term) {
                     // codes in shared memory (TMA) and block scales on their way to tensor memory (copy warp)
-                    if (!tokens_seen && !mbar_wait(t_full + 8 * slot, t_phase, abort_flag, p.status_word, kErrMmaWaitTokens)) {
+                    if (!tokens_seen && !warp_look_wait(t_full + 8 * slot, t_phase, abort_flag, p.status_word, kErrMmaWaitTokens)) {
                         alive = false;
                         break;
                     }
@@ -431,7 +432,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
             for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb) {
                 const uint32_t k_steps = (kb + 1 < k_blocks) ? 4u : last_k_steps;
                 for (uint32_t term = 0; term < per_block; ++term) {
-                    if (!mbar_wait(landed + 8 * slot, phase, abort_flag, p.status_word, kErrCopyWait)) {
+                    if (!warp_look_wait(landed + 8 * slot, phase, abort_flag, p.status_word, kErrCopyWait)) {
                         alive = false;
                         break;
                     }
@@ -481,7 +482,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         for (uint32_t index = 0; index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
             const uint32_t m_pair = item.tile % m_pairs, n_tile = item.tile / m_pairs;
-            if (!mbar_wait_suspended(bar_tmem_full, tmem_phase, abort_flag, p.status_word, kErrEpilogueWait)) break;
+            if (!warp_wait_suspended(bar_tmem_full, tmem_phase, abort_flag, p.status_word, kErrEpilogueWait)) break;
             tc_fence_after();
             const uint32_t accumulator = tmem_base + kTmemAcc + ((quadrant * 32) << 16) + half * 128;
             auto release = [&]() {   // the accumulator is free for the next tile's MMAs from here on

@@ -44,7 +44,7 @@ constexpr uint32_t kNarrowThreads = 32 * (4 + kNarrowEpilogueWarps);   // 12 war
 // 64 K registers and a quantiser CTA (5 K) fits beside one of them only, so half the CTAs began to load weights after the quantiser
 // instead of under it (6144 x 5120, three terms, quantiser included: 256 tokens 31.8 -> 29.4 us, 128 tokens 24.2 -> 23.0).
 constexpr uint32_t kNarrowBound = 32 * 14;
-constexpr uint32_t kNarrowState = 1024;                               // barriers, tensor-memory base, abort flag
+constexpr uint32_t kNarrowState = 1024;                               // barriers, tensor-memory base, abort flag, a counter per warp
 constexpr uint32_t kNarrowTurnPitch = 36;                             // floats between columns of the transposition area: 16-byte reads hit all banks
 constexpr uint32_t kNarrowSumPitch = 129;                             // 16-byte rows between groups of four columns of the partial sums, likewise
 constexpr uint32_t kNarrowRowPitch = kTileM + 4;                      // floats between columns of finished sums on their way to SwiGLU, likewise
@@ -53,6 +53,7 @@ constexpr uint32_t kNarrowRowPitch = kTileM + 4;                      // floats 
 constexpr uint32_t kNarrowSmem = 112 * 1024;
 constexpr uint32_t kNarrowTmemColumns = 256;
 constexpr uint32_t kNarrowMaxParts = 8;                               // portable cluster size
+static_assert((6 * kNarrowMaxDepth + 1) * 8 + 8 + kNarrowThreads / 32 * 4 <= kNarrowState, "the small state fits");
 static_assert(kTileM / 4 * kNarrowSumPitch * 16 + kTileM / 2 * kNarrowRowPitch * 4 <= kNarrowSmem - 1024 - kNarrowState,
               "partial sums of all columns and finished ones of half of them in the space of the rings");
 
@@ -145,6 +146,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
     if (threadIdx.x == 0) {
         for (uint32_t b = 0; b < 6 * kNarrowMaxDepth + 1; ++b) mbar_init(bar0 + 8 * b, 1);
         *abort_flag = 0;
+        for (uint32_t w = 0; w < kNarrowThreads / 32; ++w) abort_flag[1 + w] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -171,7 +173,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         const uint8_t* scales = g.weight_sf + static_cast<uint64_t>(row_tile) * atoms * kSfAtomBytes;
         uint32_t load_kb = kb0, load_stage = 0, load_phase = 1, stage = 0, phase = 0;
         auto load = [&]() {
-            if (!mbar_wait(w_empty + 8 * load_stage, load_phase, abort_flag, g.status_word, kErrNarrowWeights)) return false;
+            if (!warp_look_wait(w_empty + 8 * load_stage, load_phase, abort_flag, g.status_word, kErrNarrowWeights)) return false;
             const uint32_t full = w_full + 8 * load_stage, to = smem_u32(smem + load_stage * kNarrowStage);
             const uint32_t sf_bytes = (load_kb + 1 < k_blocks ? 4u : last_k_steps) * kSfAtomBytes;
             if (elect_one()) {
@@ -187,7 +189,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         bool alive = true;
         while (alive && load_kb < kb1 && load_kb < kb0 + p.weight_depth) alive = load();
         for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
-            if (!mbar_wait(w_full + 8 * stage, phase, abort_flag, g.status_word, kErrNarrowCopy)) break;
+            if (!warp_look_wait(w_full + 8 * stage, phase, abort_flag, g.status_word, kErrNarrowCopy)) break;
             tc_fence_after();
             if (elect_one()) {
                 narrow_copy_scales(tmem_base + p.sf_weight + stage * 16, desc0 + stage * (kNarrowStage >> 4), kb + 1 < k_blocks ? 4u : last_k_steps);
@@ -213,7 +215,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
             const uint8_t* from = scales + static_cast<uint64_t>(kb) * kNarrowScales;
             uint32_t row = token_row;
             for (uint32_t term = 0; term < g.terms; ++term) {
-                if (!mbar_wait(t_empty + 8 * slot, phase, abort_flag, g.status_word, kErrNarrowTokens)) {
+                if (!warp_look_wait(t_empty + 8 * slot, phase, abort_flag, g.status_word, kErrNarrowTokens)) {
                     alive = false;
                     break;
                 }
@@ -241,13 +243,13 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         // MMAs of this one are issued, and waited for only if they were not there.
         bool w_seen = false, t_seen = false;
         for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
-            if (!w_seen && !mbar_wait(w_ready + 8 * stage, w_phase, abort_flag, g.status_word, kErrNarrowFull)) break;
+            if (!w_seen && !warp_look_wait(w_ready + 8 * stage, w_phase, abort_flag, g.status_word, kErrNarrowFull)) break;
             const uint32_t k_steps = kb + 1 < k_blocks ? 4u : last_k_steps;
             const uint64_t w_desc = w_desc0 + stage * (kNarrowStage >> 4);
             const uint32_t sf_w = tmem_base + p.sf_weight + stage * 16, w_done = w_empty + 8 * stage;
             if (++stage == p.weight_depth) { stage = 0; w_phase ^= 1; }
             for (uint32_t term = 0; term < g.terms; ++term) {
-                if (!t_seen && !mbar_wait(t_ready + 8 * slot, t_phase, abort_flag, g.status_word, kErrNarrowScales)) {
+                if (!t_seen && !warp_look_wait(t_ready + 8 * slot, t_phase, abort_flag, g.status_word, kErrNarrowScales)) {
                     alive = false;
                     break;
                 }
@@ -284,7 +286,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
             const uint32_t k_steps = kb + 1 < k_blocks ? 4u : last_k_steps;
             for (uint32_t term = 0; term < g.terms; ++term) {
-                if (!mbar_wait(t_full + 8 * slot, phase, abort_flag, g.status_word, kErrNarrowCopy)) {
+                if (!warp_look_wait(t_full + 8 * slot, phase, abort_flag, g.status_word, kErrNarrowCopy)) {
                     alive = false;
                     break;
                 }
@@ -308,7 +310,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
     if (epilogue) {
         if (!p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing is written while an earlier kernel may still read it
         // suspended: sixteen polling warps per SM took 2 to 3 % of the launch from those that issue
-        complete = mbar_wait_suspended(acc_full, 0, abort_flag, g.status_word, kErrNarrowAccFull);
+        complete = warp_wait_suspended(acc_full, 0, abort_flag, g.status_word, kErrNarrowAccFull);
         tc_fence_after();
     }
     __syncwarp();

@@ -932,7 +932,14 @@ __global__ void __launch_bounds__(kWarps * 32, 1) gemv_kernel(const __grid_const
         }
         uint32_t spin = 0;
         while (!mbar_try_wait(my_bars + 8 * slot, parity)) {
-            if (++spin > kWaitLimit) { ring_ok = false; break; }
+            if (++spin > kWaitLimit) {
+                // A block is multiplied and reduced by all lanes together, so no lane may leave the others. They have polled equally often; what one
+                // of them has still seen arrive, the others see a millisecond later.
+#pragma unroll 1
+                for (uint32_t i = 0; i < 1000; ++i) __nanosleep(1000);
+                ring_ok = mbar_try_wait(my_bars + 8 * slot, parity);
+                break;
+            }
         }
         if (!ring_ok) break;
         compute_block(acc, my_ring + slot * kStreamBlockBytes, act + kbi * 128,

@@ -30,7 +30,7 @@ constexpr uint32_t kStreamWeightStage = kStageCodeBytes + kStageSfBytes;   // 18
 constexpr uint32_t kStreamActStage = kChunkBytes + kStageSfBytes;          // 10 KB
 constexpr uint32_t kStreamWeightDepth = 4, kStreamActDepth = 3;
 constexpr uint32_t kStreamExchange = 8 * 1024;                         // the cluster's sums of the token rows and weight rows this CTA finishes
-constexpr uint32_t kStreamState = 512;
+constexpr uint32_t kStreamState = 512;                                 // barriers, tensor-memory base, abort flag, a counter per warp
 constexpr uint32_t kStreamRings = kStreamWeightDepth * kStreamWeightStage + kStreamActDepth * kStreamActStage;
 constexpr uint32_t kStreamSmem = kStreamRings + kStreamExchange + kStreamState + 1024 /*alignment*/;
 constexpr uint32_t kStreamThreads = 32 * 12;
@@ -146,6 +146,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
     const uint32_t w_full = bar0, w_empty = w_full + 8 * kStreamWeightDepth, w_ready = w_empty + 8 * kStreamWeightDepth;
     const uint32_t t_full = w_ready + 8 * kStreamWeightDepth, t_empty = t_full + 8 * kStreamActDepth, t_ready = t_empty + 8 * kStreamActDepth;
     const uint32_t acc_full = t_ready + 8 * kStreamActDepth;
+    static_assert(kBars * 8 + 8 + kStreamThreads / 32 * 4 <= kStreamState, "the small state fits");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kBars);
     volatile uint32_t* abort_flag = tmem_slot + 1;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -154,6 +155,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
     if (threadIdx.x == 0) {
         for (uint32_t b = 0; b < kBars; ++b) mbar_init(bar0 + 8 * b, 1);
         *abort_flag = 0;
+        for (uint32_t w = 0; w < kStreamThreads / 32; ++w) abort_flag[1 + w] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -180,7 +182,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
         const uint8_t* scales = p.weight_sf + static_cast<uint64_t>(tile) * atoms * kSfAtomBytes;
         uint32_t load_kb = kb0, load_stage = 0, load_phase = 1, stage = 0, phase = 0;
         auto load = [&]() {
-            if (!mbar_wait(w_empty + 8 * load_stage, load_phase, abort_flag, p.status_word, kErrStreamWeights)) return false;
+            if (!warp_wait(w_empty + 8 * load_stage, load_phase, abort_flag, p.status_word, kErrStreamWeights)) return false;
             const uint32_t full = w_full + 8 * load_stage, to = smem_u32(smem + load_stage * kStreamWeightStage);
             const uint32_t sf_bytes = (load_kb + 1 < k_blocks ? 4u : last_k_steps) * kSfAtomBytes;
             if (elect_one()) {
@@ -196,7 +198,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
         bool alive = true;
         while (alive && load_kb < kb1 && load_kb < kb0 + kStreamWeightDepth) alive = load();
         for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
-            if (!mbar_wait(w_full + 8 * stage, phase, abort_flag, p.status_word, kErrStreamCopy)) break;
+            if (!warp_wait(w_full + 8 * stage, phase, abort_flag, p.status_word, kErrStreamCopy)) break;
             tc_fence_after();
             if (elect_one()) {
                 copy_scales(tmem_base + kStreamSfWeight + stage * 16, desc0 + stage * (kStreamWeightStage >> 4), kb + 1 < k_blocks ? 4u : last_k_steps);
@@ -215,7 +217,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
         const uint8_t* image_sf = p.split + split_code_bytes(p.cols);
         uint32_t slot = 0, phase = 1;
         for (uint32_t kb = kb0; kb < kb1; ++kb) {
-            if (!mbar_wait(t_empty + 8 * slot, phase, abort_flag, p.status_word, kErrStreamTokens)) break;
+            if (!warp_wait(t_empty + 8 * slot, phase, abort_flag, p.status_word, kErrStreamTokens)) break;
             const uint32_t to = smem_u32(slots + slot * kStreamActStage), full = t_full + 8 * slot;
             if (elect_one()) {
                 mbar_expect_tx(full, kStreamActStage);
@@ -233,8 +235,8 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
         const uint32_t idesc = instr_desc(kCols);
         const uint64_t w_desc0 = operand_desc(smem_u32(smem)), t_desc0 = operand_desc(smem_u32(slots));
         for (uint32_t kb = kb0; kb < kb1; ++kb) {
-            if ((!w_seen && !mbar_wait(w_ready + 8 * stage, w_phase, abort_flag, p.status_word, kErrStreamFull)) ||
-                (!t_seen && !mbar_wait(t_ready + 8 * slot, t_phase, abort_flag, p.status_word, kErrStreamScales))) {
+            if ((!w_seen && !warp_wait(w_ready + 8 * stage, w_phase, abort_flag, p.status_word, kErrStreamFull)) ||
+                (!t_seen && !warp_wait(t_ready + 8 * slot, t_phase, abort_flag, p.status_word, kErrStreamScales))) {
                 alive = false;
                 break;
             }
@@ -268,7 +270,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
         uint32_t slot = 0, phase = 0;
         const uint64_t desc0 = sf_desc(smem_u32(slots) + kChunkBytes);
         for (uint32_t kb = kb0; kb < kb1; ++kb) {
-            if (!mbar_wait(t_full + 8 * slot, phase, abort_flag, p.status_word, kErrStreamCopy)) break;
+            if (!warp_wait(t_full + 8 * slot, phase, abort_flag, p.status_word, kErrStreamCopy)) break;
             tc_fence_after();
             if (elect_one()) {
                 copy_scales(tmem_base + kStreamSfAct + slot * 16, desc0 + slot * (kStreamActStage >> 4), kb + 1 < k_blocks ? 4u : last_k_steps);
@@ -284,6 +286,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
     const bool epilogue = warp >= 4;
     const uint32_t task = warp - 4, quadrant = task & 3, token0 = (task >> 2) * 4;   // quadrant == warp % 4: the tensor-memory lanes it may read
     float y[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    bool complete = false;
     float scale[2][4];   // term 0 of a row has the global scale 2^(A - 155), which need not be an F32 number: as the product of two that are
     if (epilogue) {
         asm volatile("griddepcontrol.wait;" ::: "memory");   // the anchors; and nothing is written while an earlier kernel may still read it
@@ -294,7 +297,8 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
             scale[0][j] = __uint_as_float(static_cast<uint32_t>(127 + half) << 23);
             scale[1][j] = __uint_as_float(a == kNonFinite ? 0x7fc00000u : static_cast<uint32_t>(127 + exponent - half) << 23);
         }
-        if (mbar_wait(acc_full, 0, abort_flag, p.status_word, kErrStreamAccFull)) {
+        complete = warp_wait(acc_full, 0, abort_flag, p.status_word, kErrStreamAccFull);
+        if (complete) {
             tc_fence_after();
             uint32_t v[kTerms][4];
 #pragma unroll
@@ -331,7 +335,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const Stream
             }
         }
     }
-    if (epilogue && (p.parts == 1 || task % p.parts == part) && *abort_flag == 0) store_rows(p, tile * kTileM + quadrant * 32, token0, lane, y);
+    if (complete && (p.parts == 1 || task % p.parts == part)) store_rows(p, tile * kTileM + quadrant * 32, token0, lane, y);
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {

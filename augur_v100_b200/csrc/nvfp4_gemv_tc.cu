@@ -61,6 +61,7 @@ constexpr uint32_t kStages = 4;                        // per CTA; two CTAs shar
 constexpr uint32_t kCtasPerSm = 2;                     // two rings consumed in order stall less on a late stage than one of twice the depth
 constexpr uint32_t kThreads = 416;                     // warp 0 TMA of weights, 1 MMA, 2..9 split and epilogue, 10 and 12 scale copies, 11 TMA of activations
 constexpr uint32_t kSmemBytes = kStages * kStageBytes + 512 /*small state*/;   // the stages start the (1024-byte aligned) window
+constexpr uint32_t kSmallStateWarps = 2;               // counters behind the abort flag: of warps 0 and 1, the last being the one whose lanes wait together
 constexpr uint32_t kTmemAcc = 0;                       // two accumulators of 64 columns
 constexpr uint32_t kTmemSfWeight = 128;                // 16 columns per ring stage
 constexpr uint32_t kTmemSfAct = kTmemSfWeight + kStages * 16;
@@ -173,7 +174,7 @@ __device__ __forceinline__ bool counter_wait(const TcParams& p, const uint32_t* 
 // used again before meeting m + 2; nobody gets to meeting m + 2 before the last arriver of m, its store behind it,
 // has arrived at m + 1. A CTA may raise a flag as it arrives (the arrivals count in the low 16 bits, the flags
 // above them): `*raised` says afterwards whether any CTA did.
-__device__ __forceinline__ bool grid_meet(const TcParams& p, bool leader, uint32_t& meeting, bool raise, volatile uint32_t* raised,
+__device__ __forceinline__ void grid_meet(const TcParams& p, bool leader, uint32_t& meeting, bool raise, volatile uint32_t* raised,
                                           volatile uint32_t* abort_flag) {
     workers_sync();
     if (leader) {
@@ -198,7 +199,6 @@ __device__ __forceinline__ bool grid_meet(const TcParams& p, bool leader, uint32
     }
     meeting = (meeting + 1) % 3;
     workers_sync();
-    return *abort_flag == 0;
 }
 
 // ---- activation split (the worker warps of every CTA; warp w of the grid's W worker warps takes the group pairs w, w + W, ... of a job) ----
@@ -424,6 +424,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
     uint64_t* bars = reinterpret_cast<uint64_t*>(gathered + 16);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 * kStages + 4);
     volatile uint32_t* abort_flag = tmem_slot + 1;
+    static_assert((2 * 8 * kMaxJobs + 8 + 4 + 16) * 4 + (4 * kStages + 4) * 8 + 8 + kSmallStateWarps * 4 <= 512, "the small state fits");
 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (smem_u32(smem) & 1023u) {
@@ -477,6 +478,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             mbar_init(bar_acc_empty + 8 * b, 8);   // one arrival per epilogue warp
         }
         *abort_flag = 0;
+        for (uint32_t w = 0; w < kSmallStateWarps; ++w) abort_flag[1 + w] = 0;
         *input_ready = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // The weight halves of the first ring fill go out at once, before anything else is set up: weights depend
@@ -572,15 +574,15 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             const uint32_t buffer = item_count & 1;
             if (c.kb == c.kb0) {
                 // the epilogue must have drained this buffer (two items ago)
-                if (!mbar_wait(bar_acc_empty + 8 * buffer, acc_phase[buffer] ^ 1, abort_flag, p.header, kErrTcAccEmpty)) break;
+                if (!warp_wait(bar_acc_empty + 8 * buffer, acc_phase[buffer] ^ 1, abort_flag, p.header, kErrTcAccEmpty)) break;
                 tc_fence_after();
             }
             const uint32_t acc = tmem_base + kTmemAcc + buffer * 64;
             const uint32_t stage = step % kStages, parity = (step / kStages) & 1;
             // operands in shared memory (TMA) and their block scales on the way to tensor memory (copy thread):
             // a copy and a later MMA execute in issue order, so the copies only have to be issued
-            if (!mbar_wait(bar_full + 8 * stage, parity, abort_flag, p.header, kErrTcFull) ||
-                !mbar_wait(bar_scales_ready + 8 * stage, parity, abort_flag, p.header, kErrTcScalesReady)) {
+            if (!warp_wait(bar_full + 8 * stage, parity, abort_flag, p.header, kErrTcFull) ||
+                !warp_wait(bar_scales_ready + 8 * stage, parity, abort_flag, p.header, kErrTcScalesReady)) {
                 break;
             }
             tc_fence_after();
@@ -661,7 +663,8 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
                 for (uint32_t i = 8; i < 8 * p.jobs; ++i) p.header[kHeaderRowMax + i] = 0;
             }
         }
-        bool alive = true;
+        // A worker's wait that fails does not end its loop, since the others meet it at every workers_sync: they all go on to the end with
+        // whatever they find (the other waits see the abort flag), and the status word says that the launch has no results.
         {
             // ---- job 0: the input of the first step comes from outside ----
             // Its row maxima would take a meeting of their own. Instead every CTA looks at the same sample, the first
@@ -708,22 +711,20 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             }
             // every CTA's slice is in place before any CTA loads from the split (the thread that issues the loads puts
             // a proxy fence between the meeting and them)
-            alive = grid_meet(p, leader, meeting, *beyond != 0, raised, abort_flag);
-            if (alive && *raised) {
+            grid_meet(p, leader, meeting, *beyond != 0, raised, abort_flag);
+            if (*raised) {
                 job_scales(p, 0, worker, term_scale, anchor);
                 share_codes(p, 0, held, largest, nullptr, first_pair, pair_stride, lane);
                 share_scales(p, 0, anchor, held, largest, first_pair, pair_stride, lane);
-                alive = grid_meet(p, leader, meeting, false, raised, abort_flag);
+                grid_meet(p, leader, meeting, false, raised, abort_flag);
             }
-            if (alive) {
-                if (blockIdx.x == 0 && worker < 8) p.header[kHeaderRowMax + worker] = 0;   // clean for the next launch
-                if (leader) {
-                    __threadfence_block();
-                    *input_ready = 1;
-                }
+            if (blockIdx.x == 0 && worker < 8) p.header[kHeaderRowMax + worker] = 0;   // clean for the next launch
+            if (leader) {
+                __threadfence_block();
+                *input_ready = 1;
             }
         }
-        for (uint32_t s = 0; alive && s < p.steps; ++s) {
+        for (uint32_t s = 0; s < p.steps; ++s) {
             const TcStep& st = p.step[s];
             const TcPhase& ph = p.phase[st.phase];
             uint32_t* gather = st.feeds ? collected : nullptr;
@@ -734,10 +735,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             for (uint32_t item = blockIdx.x; item < items; item += gridDim.x, ++item_count) {
                 const uint32_t tile = item / st.parts, part = item - tile * st.parts;
                 const uint32_t buffer = item_count & 1;
-                if (!mbar_wait_suspended(bar_acc_full + 8 * buffer, acc_phase[buffer], abort_flag, p.header, kErrTcAccFull)) {
-                    alive = false;
-                    break;
-                }
+                mbar_wait_suspended(bar_acc_full + 8 * buffer, acc_phase[buffer], abort_flag, p.header, kErrTcAccFull);
                 acc_phase[buffer] ^= 1;
                 tc_fence_after();
                 // column = term * 8 + token: this warp's four token rows are four neighbouring columns of every term
@@ -764,7 +762,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
                 contribute_rows(ph, p.tokens, st.tile0 + tile, quadrant, token0, st.slot0 + part, lane, y, gather, st.keeps ? kept : nullptr);
                 kept_group = (st.tile0 + tile) * 4 + quadrant;
             }
-            if (!alive || !st.feeds) continue;
+            if (!st.feeds) continue;
             // ---- this step's outputs are the activations of job `feeds`: maxima, arrive, wait, split, arrive ----
             const uint32_t w = st.feeds - 1;
             const TcJob& job = p.job[st.feeds];
@@ -866,10 +864,6 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
                 if (leader) counter_wait(p, wave + 2 * w, kErrTcWave, abort_flag);
                 workers_sync();
             }
-            if (*abort_flag) {
-                alive = false;
-                break;
-            }
             if (!st.keeps) job_scales(p, st.feeds, worker, term_scale, anchor);
             if (st.keeps) {
                 if (kept_group != ~0u) {
@@ -898,7 +892,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             }
         }
         // the next launch goes on counting meetings where this one stopped, with the other half of the wave counters
-        if (alive && leader && blockIdx.x == 0) {
+        if (leader && blockIdx.x == 0 && *abort_flag == 0) {
             p.header[kHeaderEpoch] = meeting;
             p.header[kHeaderParity] = parity ^ 1;
         }
