@@ -9,7 +9,8 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <cstring>
+
+#include "nvfp4_rounding.h"
 
 namespace augur_sm100 {
 namespace tc {
@@ -159,7 +160,9 @@ __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint3
 // One pipeline step of a converged warp: the four MMAs of a 256-deep k block (64 k each: 32 bytes further in every operand row, four
 // scale columns further) and the commits that free what they read, `done` and, where `also` is not zero, `also_done`. The elected
 // lane is a predicate on the instructions, not a branch: the warp does not diverge, and the operands of all six are formed once
-// in uniform registers. Written as a branch around six separate instructions a step takes 400 cycles to issue, whatever its n.
+// in uniform registers. Written as a branch around six separate instructions a step takes 400 cycles to issue, whatever its n. Its MMAs
+// occupy the pipe for 156 cycles at n = 16, 176 at 48 and 256 at 128, twice that for the two CTAs of an SM: so issue was the bound of
+// small n, and what is gained at 128 is little.
 __device__ __forceinline__ void tc_step(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t accumulate,
                                         uint32_t done, uint32_t also, uint32_t also_done) {
     asm volatile(
@@ -259,15 +262,11 @@ __device__ __forceinline__ uint32_t e2m1_nearest(float v, float* level) {
 }
 
 // Eight quotients -> eight codes, element i in nibble i, by the hardware converter: round to nearest even,
-// magnitudes above 6 (infinities too) to 6. It differs from "nearest, ties toward zero, zero always code 0" in
-// three places, put right here. At 0.75, 1.75 and 3.5 "even" is the larger level; at the other ties it is the smaller one. The
-// three have a significand of 1.5 or 1.75, the others of 1 or 1.25, so every quotient goes in one ulp nearer to zero if its
-// significand m is above 1.37 and as it is otherwise: q - q * 1.457 * 2^-25 takes 0.364 m
-// of an ulp off, which rounds to the neighbour once it exceeds half of one. A tie of the three then lies below itself, the value one ulp above it on the tie,
-// which rounds up as it must, and no other boundary has values so close (all F32 values from 2^-6 to 16 were compared). A negative
-// quotient that rounds to zero comes out as code 8. And a NaN comes out as +6 (the caller keeps groups with a NaN off this path).
+// magnitudes above 6 (infinities too) to 6. It differs from "nearest, ties toward zero, zero always code 0" in three places, put
+// right here: three of the ties (kTieNudge), a negative quotient that rounds to zero, which comes out as code 8, and a NaN, which
+// comes out as +6 (the caller keeps groups with a NaN off this path).
 __device__ __forceinline__ uint32_t e2m1x8_nearest(const float2 (&quotient)[4]) {
-    const float2 nudge = make_float2(-0x1.75p-25f, -0x1.75p-25f);
+    const float2 nudge = make_float2(kTieNudge, kTieNudge);
     float2 q[4];
 #pragma unroll
     for (uint32_t i = 0; i < 4; ++i) q[i] = __ffma2_rn(quotient[i], nudge, quotient[i]);
@@ -297,7 +296,7 @@ __device__ __forceinline__ void e2m1x8_levels(uint32_t codes, float2 (&level)[4]
 }
 
 // The 16 quotients of a group share one divisor. With y = RN(1/d), two Newton steps on the quotient (each
-// an exact FMA residual) end on the correctly rounded x / d whenever d and x are well inside the normal
+// an exact FMA residual; as quotient_by_reciprocal) end on the correctly rounded x / d whenever d and x are well inside the normal
 // range and d is not of the all-ones mantissa form; the kernel checks that once per group and otherwise
 // divides. An x so small that a residual of the steps is subnormal (below 2^-103) has a quotient under
 // 2^-40 (d is at least 2^-63 here), and the error that the lost bits leave in it is under 2^-87: code 0
@@ -365,34 +364,16 @@ __device__ __forceinline__ float group_divisor(float maximum, float global_scale
     return __fmul_rn(scale, global_scale);
 }
 
-// What a quantiser knows about its global scale before it has seen an element: 6 g, and its rounded reciprocal where the Newton
-// steps below end on the correctly rounded quotient (0 where they need not, see quantise_group_fast).
-struct QuantScale {
-    float global, six, six_reciprocal;
-};
-inline QuantScale quant_scale(float global_scale) {
-    const float six = 6.0f * global_scale;
-    uint32_t bits;
-    memcpy(&bits, &six, 4);
-    const uint32_t field = bits >> 23;
-    return QuantScale{global_scale, six, field >= 64u && field <= 180u && (bits & 0x7fffffu) != 0x7fffffu ? 1.0f / six : 0.0f};
-}
-
 // An E4M3 code as a float (hardware E4M3 -> F16, widened).
 __device__ __forceinline__ float e4m3_value(uint32_t code) {
     uint32_t pair;
     asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(pair) : "h"(static_cast<uint16_t>(code)));
     return __half2float(__ushort_as_half(static_cast<uint16_t>(pair & 0xffffu)));
 }
-// group_divisor for a `maximum` from 2^-63 to 2^64 and a scale with a reciprocal, without a branch: the quotient, which is a normal
-// number then, by two Newton steps (compared with IEEE division on 2 * 10^8 random cases), its ceiling as the hardware's nearest
-// value, or the one above where that is smaller.
+// group_divisor for a `maximum` from 2^-63 to 2^64 and a scale with a reciprocal, without a branch: the quotient is a normal number
+// then, and its ceiling the hardware's nearest value, or the one above where that is smaller.
 __device__ __forceinline__ float group_divisor_fast(float maximum, const QuantScale& s, uint32_t* scale_code_out) {
-    float desired = __fmul_rn(maximum, s.six_reciprocal);
-    float rest = __fmaf_rn(desired, -s.six, maximum);
-    desired = __fmaf_rn(rest, s.six_reciprocal, desired);
-    rest = __fmaf_rn(desired, -s.six, maximum);
-    desired = __fmaf_rn(rest, s.six_reciprocal, desired);
+    const float desired = quotient_by_reciprocal(maximum, s.six_reciprocal, s.six);
     uint16_t nearest;
     asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(nearest) : "f"(0.0f), "f"(desired));
     uint32_t code = nearest & 0xffu;
