@@ -954,9 +954,12 @@ struct PairSplit {
     uint32_t ns;
 };
 
-// Measured on a B200: a pipeline step (k block x term) of a pair takes 0.36 us, a launch 8 us beyond its steps. Handing the
-// parts of leftover tiles over takes the time of 16 steps and two more per part when nothing else is left to do, and about
-// 8 when it happens under whole tiles.
+// Fitted on a B200 to the kernel with one ring: a pipeline step (k block x term) of a pair 0.36 us, a launch 8 us beyond its steps; handing
+// the parts of leftover tiles over the time of 16 steps and two more per part when nothing else is left to do, and about 8 when it
+// happens under whole tiles. With the two rings a step takes 0.33 us at three terms, 0.37 to 0.43 at two and 0.46 to 0.50 at one, where
+// the weights of a k block come with every step (one tile per pair, 18944 rows, 256 tokens, 10 to 40 k blocks), a launch 9 to 11 us beyond.
+// The choice that these constants make is 0.7 % off the best on average, and 27 % where the two kernels are estimated alike: 10240 x
+// 5120, two terms, 300 tokens 38 us, narrow 32.
 constexpr uint32_t kPairStepNs = 360, kPairLaunchNs = 8000;
 constexpr uint32_t kSplitSteps = 16, kSplitPartSteps = 2, kSplitCoveredSteps = 8;
 
@@ -987,9 +990,9 @@ PairSplit pair_split(uint32_t token_pairs, uint32_t rows, uint32_t cols, uint32_
 }
 
 // How many of the token rows the pair kernel takes (in 256-row pairs); the narrow kernel takes the rest. The choice is the
-// quickest by the estimates of the two: narrow up to 128 tokens nearly always (6144 x 5120, three terms, 48 tokens: 12 us
-// against 23), pairs from about 256 on (17408 x 5120, 256 tokens: 29 against 37) unless the weight is small (1024 x 5120: 22
-// against 14), and pairs with a narrow tail when the tokens just exceed whole pairs (17408 x 5120, 300 tokens: 49 against
+// quickest by the estimates of the two: narrow up to 128 tokens nearly always (6144 x 5120, three terms, 48 tokens: 15 us
+// against 24), pairs from about 256 on (17408 x 5120, 256 tokens: 31 against 40) unless the weight is small (1024 x 5120: 27
+// against 18.5), and pairs with a narrow tail when the tokens just exceed whole pairs (17408 x 5120, 300 tokens: 52 against
 // 54). The tail starts when the pairs are nearly done, so it has to be clearly quicker to be taken.
 uint32_t token_pairs_for(const augur_cuda_nvfp4_sm100_plan_v1* plan, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
     const uint32_t all_pairs = plan->pair_clusters, pairs = (tokens + 2 * kTileM - 1) / (2 * kTileM), rest = tokens % (2 * kTileM);

@@ -4,8 +4,9 @@
 // The pair kernel of nvfp4_gemm.cu puts 256 token rows on its tile, so 9 tokens cost what 256 do. Here the weights are the
 // 128-row operand and the tokens sit on the MMA n dimension, whose size follows their number in steps of 16 (at most
 // 128): the work is that of the tokens there are, and what is left is streaming the weights once. What bounds a launch is a
-// chain of latencies, a pipeline step (k block x term) of 0.33 to 0.44 us behind the other, not HBM or the tensor pipe: 6144 x 5120 at
-// 48 tokens and three terms has them 13 % and 9 % busy.
+// chain of latencies, a pipeline step (k block x term) behind the other, not HBM or the tensor pipe alone: with two CTAs on every SM and
+// three terms a step takes 0.32 us at 16 tokens, 0.50 at 48 and 0.55 at 128, where the MMAs of the two CTAs occupy the pipe for 0.19 to 0.31 us
+// (at 1.65 GHz) and HBM delivers the weights in 0.28; 6144 x 5120 at 48 tokens, five parts, has them 13 % and 9 % busy.
 //
 //   D[feature][token] = sum over k blocks of 256, terms, k steps of 64:  W[128 x 64] * A_term[tokens x 64]^T
 //
@@ -461,9 +462,11 @@ uint32_t two_cta_clusters(int32_t ordinal, uint32_t parts) {
 
 namespace {
 // How a launch cuts its work, and about how long it takes: the waves of clusters times the pipeline steps of a part, of the
-// numbers of CTAs per item the one with the least. Measured on a B200 with two CTAs on every SM: a step (k block x term) of a
-// CTA takes 0.33 us at 16 tokens and 0.44 at 128, a launch about 6 us beyond its steps, a wave after the first 3; exchanging
-// the parts' sums takes 4 us more at 128 tokens.
+// numbers of CTAs per item the one with the least. Fitted on a B200 with two CTAs on every SM, before a step's MMAs became one block of
+// instructions and a cluster's sums were read where they are: a step (k block x term) 0.33 us at 16 tokens and 0.44 at 128, a launch about 6 us
+// beyond its steps, a wave after the first 3, the parts' sums 4 us more at 128 tokens. Measured since, three terms, one part: 0.32 to 0.34 us
+// a step at 16 tokens, 0.50 at 48, 0.55 at 128, and 5 to 9 us beyond. The number of parts chosen is 1.7 % off the best on average, 25 % at worst
+// (1024 x 5120, 200 tokens).
 struct NarrowCut {
     uint32_t token_tiles, tile_tokens, columns, parts, ns;
 };
