@@ -189,10 +189,9 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_plan_crea
         return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE, cudaGetLastError());
     }
     if (major != 10) return make_result(AUGUR_CUDA_STATUS_UNSUPPORTED_DEVICE);
-    // Kernels are loaded in this order. Where a kernel's code comes to lie is worth a few percent to the one-launch MLP block,
-    // whose code is larger than an instruction cache, so it comes first, where what the other kernels grow by does not move it: two
-    // layers of linears and blocks 157.1 us in this order, 157.4 to 158.6 with it third, second or ahead of the split; the block
-    // alone 39.8 to 40.0 us in all of them (41.2 before its MMAs became one block of instructions, 39.9 to 40.9 by place).
+    // Kernels are loaded in this order: the one-launch MLP block, whose code is larger than an instruction cache, first, where what the other
+    // kernels grow by does not move it. With the waits' poll loops unrolled in line, three linears and a block took 81.0 to 82.2 us in nine
+    // orders, 81.0 in this one; how much code there is counts for more (78.9 with the loops rolled up, see nvfp4_tc.cuh).
     e = gemv_tc_configure_device();
     if (e == cudaSuccess) e = gemv_configure_device();
     if (e == cudaSuccess) e = gemm_configure_device();
