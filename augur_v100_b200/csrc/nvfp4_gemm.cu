@@ -18,6 +18,7 @@
 #include "nvfp4_gemm.cuh"
 #include "nvfp4_internal.h"
 #include "nvfp4_layout.cuh"
+#include "nvfp4_pair_work.h"
 #include "nvfp4_tc.cuh"
 
 namespace augur_sm100 {
@@ -67,17 +68,20 @@ constexpr uint32_t kPairWeightStage = kPairBytesB + kBytesSfB;       // 20480
 constexpr uint32_t kPairTokenSlot = kBytesA + kBytesSfA;             // 18432
 constexpr uint32_t kPairMaxDepth = 8;                                // slots of either ring
 // Ring depths by activation terms: about as many k blocks ahead on either ring as shared memory holds. A weight stage is
-// free when the last term's step of its k block is complete, which that step's token slot says (no barrier and no commit of its
-// own: a second commit per step, and scales that queue behind codes, took one term from 157 to 178 us). For the slot's
-// phase to be the one meant, the step must not have left the token ring yet.
+// free when the last term's step of its k block is complete, which the wait for a token slot of a later step says (no barrier and no
+// commit of its own: a second commit per step, and scales that queue behind codes, took one term from 157 to 178 us): the slot of
+// term `weight_term` of block b was last used by that step of block b - weights, or by a later one.
 struct PairDepths {
     uint32_t weights, tokens;
 };
-__host__ __device__ constexpr PairDepths pair_depths(uint32_t terms) { return terms == 1 ? PairDepths{5, 5} : PairDepths{3, 8}; }
-__host__ __device__ constexpr bool pair_depths_ok(uint32_t terms) {
-    return pair_depths(terms).tokens > (pair_depths(terms).weights - 1) * terms && pair_depths(terms).tokens >= terms;
+__host__ __device__ constexpr PairDepths pair_depths(uint32_t terms) {
+    return terms == 1 ? PairDepths{5, 5} : terms == 2 ? PairDepths{4, 6} : PairDepths{3, 8};
 }
-static_assert(pair_depths_ok(1) && pair_depths_ok(2) && pair_depths_ok(3), "a freed weight stage shows in the token ring");
+__host__ __device__ constexpr uint32_t pair_weight_term(uint32_t terms) {
+    const uint32_t before = (pair_depths(terms).weights - 1) * terms + 1;
+    return pair_depths(terms).tokens > before ? pair_depths(terms).tokens - before : 0;
+}
+static_assert(pair_weight_term(1) < 1 && pair_weight_term(2) < 2 && pair_weight_term(3) < 3, "a freed weight stage shows in the token ring");
 __host__ __device__ constexpr uint32_t pair_ring_bytes(uint32_t terms) {
     return pair_depths(terms).weights * kPairWeightStage + pair_depths(terms).tokens * kPairTokenSlot;
 }
@@ -100,7 +104,7 @@ constexpr uint32_t kPairSmemBytes = kPairRingBytes + kPairOutBytes + 1024 + 512;
 static_assert(kPairSmemBytes <= 227 * 1024, "shared memory of a CTA");
 constexpr uint32_t kPairCopyWarp = 2 + kPairEpilogueWarps;    // token-row scales; the warp after it copies the weight-row scales
 constexpr uint32_t kPairThreads = 32 * (kPairCopyWarp + 2);   // TMA warp, MMA warp, epilogue warps, two scale-copy warps
-static_assert(kPairBarriers * 8 + 8 + kPairThreads / 32 * 4 <= 512, "barriers, tensor-memory base, abort flag and the warps' counters fit behind the rings");
+static_assert(kPairBarriers * 8 + 8 + kPairThreads / 32 * 4 + sizeof(PairWork) <= 512, "barriers, tensor-memory base, abort flag, the warps' counters and the pair's work fit behind the rings");
 constexpr uint32_t kSplitWays = 8;              // a leftover tile is cut into this many parts at most
 constexpr uint32_t kSplitWaitLimit = 1u << 20;  // polls of a handed-over part's flag (each a round trip to L2) before giving up
 constexpr uint64_t kSplitSlotBytes = 2ull * kPairEpilogueWarps * 32 * 128 * 4;   // one pair's accumulator: 256 x 256 f32
@@ -114,11 +118,31 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// TMA tile load whose bytes are counted on the barrier at `bar`'s offset in the pair's leader CTA.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t bar) {
+// The TMA loads of a converged warp for one slot of the token ring, and for one stage of the weight ring: block scales first, on a
+// barrier of their own, then operand rows, all counted on barriers of the pair's leader CTA (cta_group::2), whose producer (`leader`)
+// announces the bytes of both CTAs. As predicated instructions in one block, for the reason given at tc_step.
+__device__ __forceinline__ void tma_token_step(bool leader, uint32_t landed, uint32_t scales, const CUtensorMap* map_scales, uint32_t scale_y,
+                                               uint32_t scale_z, uint32_t full, uint32_t bytes, uint32_t codes, const CUtensorMap* map_codes, uint32_t x, uint32_t y) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar & kLeaderMask)
+        "{\n.reg .pred e, l;\nelect.sync _|e, 0xffffffff;\nsetp.ne.and.b32 l, %0, 0, e;\n"
+        "@l mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %2;\n"
+        "@e cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%3], [%4, {%5, %6, %7}], [%8];\n"
+        "@l mbarrier.arrive.expect_tx.shared::cta.b64 _, [%9], %10;\n"
+        "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%11], [%12, {%13, %14}], [%15];\n}"
+        ::"r"(leader ? 1u : 0u), "r"(landed), "r"(2 * kBytesSfA), "r"(scales), "l"(map_scales), "r"(0u), "r"(scale_y), "r"(scale_z), "r"(landed & kLeaderMask),
+          "r"(full), "r"(bytes), "r"(codes), "l"(map_codes), "r"(x), "r"(y), "r"(full & kLeaderMask)
+        : "memory");
+}
+__device__ __forceinline__ void tma_weight_step(bool leader, uint32_t landed, uint32_t scales, const CUtensorMap* map_scales, uint32_t scale_y,
+                                                uint32_t scale_z, uint32_t full, uint32_t codes, const CUtensorMap* map_codes, uint32_t x, uint32_t y) {
+    asm volatile(
+        "{\n.reg .pred e, l;\nelect.sync _|e, 0xffffffff;\nsetp.ne.and.b32 l, %0, 0, e;\n"
+        "@l mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %2;\n"
+        "@e cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%3], [%4, {%5, %6, %7}], [%8];\n"
+        "@l mbarrier.arrive.expect_tx.shared::cta.b64 _, [%9], %10;\n"
+        "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%11], [%12, {%13, %14}], [%15];\n}"
+        ::"r"(leader ? 1u : 0u), "r"(landed), "r"(2 * kBytesSfB), "r"(scales), "l"(map_scales), "r"(0u), "r"(scale_y), "r"(scale_z), "r"(landed & kLeaderMask),
+          "r"(full), "r"(2 * kPairBytesB), "r"(codes), "l"(map_codes), "r"(x), "r"(y), "r"(full & kLeaderMask)
         : "memory");
 }
 // Arrives on the barrier at this offset in both CTAs of the pair once the MMAs issued so far are done.
@@ -127,87 +151,223 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
                  ::"r"(bar), "h"(static_cast<uint16_t>(3))
                  : "memory");
 }
-__device__ __forceinline__ void tc_copy_sf_pair(uint32_t tmem, uint64_t desc) {
-    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem), "l"(desc) : "memory");
-}
-__device__ __forceinline__ void tc_mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb,
-                                            uint32_t accumulate) {
+// A step of a converged warp, as tc_step: the one to four MMAs of a k block (64 k each: 32 bytes further in every operand row,
+// `step_a` and `step_b` scale columns further) and the commit that frees what they read. `a` and `b` are the low words of operand
+// descriptors, whose high words are all alike.
+__device__ __forceinline__ void tc_step_pair(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t step_a,
+                                             uint32_t step_b, uint32_t accumulate, uint32_t k_steps, uint32_t done) {
+    constexpr uint32_t kHigh = (1024 >> 4) | (1u << 14) | (2u << 29);
     asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
-        "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n}"
-        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
+        "{\n.reg .pred e, p, q, e1, e2, e3;\n.reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n.reg .b32 l1, l2, l3, m1, m2, m3, s1, s2, s3, t1, t2, t3;\n"
+        "tcgen05.fence::after_thread_sync;\nelect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, %8, 0;\nsetp.eq.u32 q, 0, 0;\n"
+        "setp.gt.and.u32 e1, %9, 1, e;\nsetp.gt.and.u32 e2, %9, 2, e;\nsetp.gt.and.u32 e3, %9, 3, e;\n"
+        "add.s32 l1, %1, 2;\nadd.s32 l2, %1, 4;\nadd.s32 l3, %1, 6;\nadd.s32 m1, %2, 2;\nadd.s32 m2, %2, 4;\nadd.s32 m3, %2, 6;\n"
+        "mov.b64 a0, {%1, %11};\nmov.b64 a1, {l1, %11};\nmov.b64 a2, {l2, %11};\nmov.b64 a3, {l3, %11};\n"
+        "mov.b64 b0, {%2, %11};\nmov.b64 b1, {m1, %11};\nmov.b64 b2, {m2, %11};\nmov.b64 b3, {m3, %11};\n"
+        "add.s32 s1, %4, %6;\nadd.s32 s2, s1, %6;\nadd.s32 s3, s2, %6;\nadd.s32 t1, %5, %7;\nadd.s32 t2, t1, %7;\nadd.s32 t3, t2, %7;\n"
+        "@e tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a0, b0, %3, [%4], [%5], p;\n"
+        "@e1 tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a1, b1, %3, [s1], [t1], q;\n"
+        "@e2 tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a2, b2, %3, [s2], [t2], q;\n"
+        "@e3 tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a3, b3, %3, [s3], [t3], q;\n"
+        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%10], %12;\n}"
+        ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(step_a), "r"(step_b), "r"(accumulate), "r"(k_steps), "r"(done), "r"(kHigh),
+          "h"(static_cast<uint16_t>(3))
         : "memory");
 }
+// The scale atoms of a slot, four k steps of one 128-row block or of two (2 KB apart), on their way to both CTAs' tensor memory, four columns an
+// atom, those of one k step side by side; and the arrival that says so.
+template <uint32_t kBlocks>
+__device__ __forceinline__ void tc_copy_step_pair(uint32_t columns, uint64_t desc, uint32_t ready) {
+    static_assert(kSfAtomBytes >> 4 == 32, "steps of the descriptors below");
+    if (kBlocks == 1) {
+        asm volatile(
+            "{\n.reg .pred e;\n.reg .b64 a1, a2, a3;\n.reg .b32 c1, c2, c3;\ntcgen05.fence::after_thread_sync;\nelect.sync _|e, 0xffffffff;\n"
+            "add.s64 a1, %1, 32;\nadd.s64 a2, %1, 64;\nadd.s64 a3, %1, 96;\nadd.s32 c1, %0, 4;\nadd.s32 c2, %0, 8;\nadd.s32 c3, %0, 12;\n"
+            "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;\n@e tcgen05.cp.cta_group::2.32x128b.warpx4 [c1], a1;\n"
+            "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [c2], a2;\n@e tcgen05.cp.cta_group::2.32x128b.warpx4 [c3], a3;\n"
+            "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%2];\n}"
+            ::"r"(columns), "l"(desc), "r"(ready)
+            : "memory");
+    } else {
+        asm volatile(
+            "{\n.reg .pred e;\n.reg .b64 a1, a2, a3, b0, b1, b2, b3;\n.reg .b32 c1, c2, c3, d0, d1, d2, d3;\n"
+            "tcgen05.fence::after_thread_sync;\nelect.sync _|e, 0xffffffff;\n"
+            "add.s64 a1, %1, 32;\nadd.s64 a2, %1, 64;\nadd.s64 a3, %1, 96;\nadd.s64 b0, %1, 128;\nadd.s64 b1, %1, 160;\nadd.s64 b2, %1, 192;\nadd.s64 b3, %1, 224;\n"
+            "add.s32 c1, %0, 8;\nadd.s32 c2, %0, 16;\nadd.s32 c3, %0, 24;\nadd.s32 d0, %0, 4;\nadd.s32 d1, %0, 12;\nadd.s32 d2, %0, 20;\nadd.s32 d3, %0, 28;\n"
+            "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;\n@e tcgen05.cp.cta_group::2.32x128b.warpx4 [d0], b0;\n"
+            "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [c1], a1;\n@e tcgen05.cp.cta_group::2.32x128b.warpx4 [d1], b1;\n"
+            "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [c2], a2;\n@e tcgen05.cp.cta_group::2.32x128b.warpx4 [d2], b2;\n"
+            "@e tcgen05.cp.cta_group::2.32x128b.warpx4 [c3], a3;\n@e tcgen05.cp.cta_group::2.32x128b.warpx4 [d3], b3;\n"
+            "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%2];\n}"
+            ::"r"(columns), "l"(desc), "r"(ready)
+            : "memory");
+    }
+}
+template <bool kTail>
+struct PairTail {
+    __device__ constexpr operator bool() const { return kTail; }
+};
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar & kLeaderMask) : "memory");
 }
 
-// The work of one CTA pair, in the order it is done: the head or middle part of a leftover tile (its partial
-// accumulator is handed to the pair that finishes the tile), the part that finishes a leftover tile, then the
-// pair's whole tiles. Tiles are numbered m-pair fastest; whole tiles of pair p are p, p + pairs, ...; with `split` the
-// tiles past the last full round are cut along k into equal contiguous ranges, one per pair, so that every pair
-// issues the same number of k blocks. A range is at most one tile long: it holds the tail of one tile, the head
-// of the next, or both. A part handed over is its pair's first item and nothing waits in front of it; a
-// finishing part follows, and only its epilogue warps wait (for first items of other pairs, about as long as
-// its own), with the accumulator already released; the reads of the handed-over sums then run under the
-// MMAs of the whole tiles that follow.
-struct PairItem {
-    uint32_t tile, kb0, kb1;
-    uint32_t kind;           // 0: whole tile, 1: part handed over, 2: part that finishes the tile
-    uint32_t first_giver;    // kind 2: the pairs first_giver .. this pair - 1 hand their parts over
+// A tile of the pair kernel: 256 token rows on the MMA's row dimension and 256 features on its n (128 in a half tile at the end), or,
+// for the token rows past the last whole 256, a tail tile: the operands change places, 256 features are the rows (128 on either
+// CTA) and the tokens, in steps of 32, n. So 9 token rows cost the weights' way into shared memory and 32 columns, not 256 rows of
+// padding; and in one launch with the others the tail shares their balance over the pairs.
+struct PairTile {
+    uint32_t n_tile, token0;   // 256-feature tile; first token row
+    bool tail;
 };
-struct PairWork {
-    uint32_t items, whole;
-    PairItem given, finishing;
-    bool gives, finishes;
-    __device__ PairItem item(uint32_t index, uint32_t pair, uint32_t pairs, uint32_t k_blocks) const {
-        const uint32_t parts = (gives ? 1u : 0u) + (finishes ? 1u : 0u);
-        if (gives && index == 0) return given;
-        if (finishes && index + 1 == parts) return finishing;
-        return PairItem{pair + (index - parts) * pairs, 0, k_blocks, 0, 0};
-    }
-};
-// `sharers` (0: whole tiles only): the first `sharers` pairs share the leftover tiles (at most kSplitWays per tile).
-__device__ __forceinline__ PairWork pair_work(uint32_t pair, uint32_t pairs, uint32_t tiles, uint32_t k_blocks, uint32_t sharers) {
-    PairWork w{};
-    if (!sharers) {
-        w.whole = tiles > pair ? (tiles - pair + pairs - 1) / pairs : 0;
-        w.items = w.whole;
-        return w;
-    }
-    w.whole = tiles / pairs;
-    w.items = w.whole;
-    if (pair >= sharers) return w;
-    const uint32_t first_left = w.whole * pairs;
-    const uint64_t units = static_cast<uint64_t>(tiles - first_left) * k_blocks;   // k blocks of the leftover tiles
-    const uint64_t x0 = pair * units / sharers, x1 = (pair + 1) * units / sharers;  // this pair's range (not empty: units >= sharers)
-    const uint32_t a = static_cast<uint32_t>(x0 / k_blocks), b = static_cast<uint32_t>((x1 - 1) / k_blocks);
-    const uint64_t a_begin = static_cast<uint64_t>(a) * k_blocks, a_end = a_begin + k_blocks;
-    if (x1 >= a_end) {
-        // the range holds the tail of tile a: every pair from the one that owns the tile's first k block hands over
-        w.finishes = true;
-        w.finishing = PairItem{first_left + a, static_cast<uint32_t>(x0 - a_begin), k_blocks, 2,
-                               static_cast<uint32_t>(((a_begin + 1) * sharers - 1) / units)};
-        if (w.finishing.first_giver == pair) w.finishing.kind = 0;   // the whole tile
-    } else {
-        w.gives = true;
-        w.given = PairItem{first_left + a, static_cast<uint32_t>(x0 - a_begin), static_cast<uint32_t>(x1 - a_begin), 1, 0};
-    }
-    if (b > a) {
-        // and the head of tile b (never all of it: the range is at most one tile long)
-        w.gives = true;
-        w.given = PairItem{first_left + b, 0, static_cast<uint32_t>(x1 - static_cast<uint64_t>(b) * k_blocks), 1, 0};
-    }
-    w.items = w.whole + (w.gives ? 1u : 0u) + (w.finishes ? 1u : 0u);
-    return w;
+__device__ __forceinline__ PairTile pair_tile(uint32_t tile, uint32_t main_tiles, uint32_t m_pairs) {
+    if (tile >= main_tiles) return PairTile{tile - main_tiles, m_pairs * 2 * kTileM, true};
+    return PairTile{tile / m_pairs, tile % m_pairs * 2 * kTileM, false};
 }
 
-// One instantiation per set of ring depths: as constants they are worth 1.5 %.
-template <bool kResidualTerms>
+// 16 BF16 values of one token, one quantisation group, as the next GEMM's activations.
+__device__ __forceinline__ void quantise_row(const GemmParams& p, uint32_t token, uint32_t group, const uint32_t (&packed)[8]) {
+    const uint32_t width = p.rows / 2;
+    const uint64_t code_bytes = tcgen05_codes_bytes(p.padded_tokens, width), scale_bytes = tcgen05_scale_bytes(p.padded_tokens, width);
+    float2 residual[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) residual[i] = make_float2(__uint_as_float(packed[i] << 16), __uint_as_float(packed[i] & 0xffff0000u));
+#pragma unroll 1
+    for (uint32_t term = 0; term < p.quant_terms; ++term) {
+        uint32_t codes[2], scale_code;
+        quantise_term(residual, p.quant_scale, term + 1 < p.quant_terms, codes, &scale_code);
+        *reinterpret_cast<uint2*>(p.quant_out + term * code_bytes + static_cast<uint64_t>(token) * (width / 2) + group * 8) = make_uint2(codes[0], codes[1]);
+        p.quant_out[p.quant_terms * code_bytes + term * scale_bytes + tcgen05_scale_offset(token, group, width)] = static_cast<uint8_t>(scale_code);
+    }
+}
+
+// The first look at a barrier is in line, the rest suspended: what does not poll leaves the board's power to the MMAs (17408 x 5120 x 4096 with its
+// quantiser, one term 195.8 -> 194.4 us, MLP block of 4096 tokens 1328 -> 1322).
+__device__ __forceinline__ bool pair_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t* status_word, uint32_t code) {
+    return mbar_test(bar, parity) || warp_wait_suspended(bar, parity, abort_flag, status_word, code);
+}
+// Where the sums that a pair hands over pass through: a slot per epilogue warp of either CTA (`place` 0 .. 15).
+__device__ __forceinline__ uint32_t pair_slot(uint32_t giver, uint32_t place) { return giver * 2 * kPairEpilogueWarps + place; }
+__device__ __forceinline__ float4* pair_slot_sums(const GemmParams& p, uint32_t slot, uint32_t lane) {
+    return reinterpret_cast<float4*>(p.split_slots) + static_cast<uint64_t>(slot) * (32 * 32) + lane;
+}
+// The part that finishes a leftover tile waits for the parts handed over, which are then added in pair order.
+static __device__ __noinline__ bool pair_parts_arrived(const GemmParams& p, const PairItem& item, uint32_t pair, uint32_t place, volatile uint32_t* abort_flag) {
+    bool arrived = true;
+    for (uint32_t giver = item.first_giver; giver < pair; ++giver) {
+        const uint32_t slot = pair_slot(giver, place);
+        if ((threadIdx.x & 31) == 0) {
+            uint32_t spin = 0;
+            while (atomicAdd(p.split_flags + slot, 0u) == 0u) {
+                if (++spin > kSplitWaitLimit || ((spin & 255u) == 255u && *abort_flag)) {
+                    arrived = false;
+                    *abort_flag = 1;
+                    atomicCAS(p.status_word, 0u, kErrSplitWait);
+                    break;
+                }
+            }
+            // The flags read zero again when the launch is over, also those of parts that were given up on: that launch has
+            // failed and says so, and a late giver cannot leave one set for the next launch on this plan.
+            p.split_flags[slot] = 0;
+        }
+    }
+    __threadfence();
+    return __all_sync(0xffffffffu, arrived) != 0;
+}
+// 32 weight rows (one per lane) of 32 tokens of a tail tile on their way out: turned through shared memory, so that a row of it
+// is one token's.
+__device__ __forceinline__ void pair_store_tail(const GemmParams& p, uint8_t* rows, uint32_t token0, uint32_t row0, uint32_t lane, const uint32_t (&sums)[32]) {
+    if (!p.swiglu) {
+#pragma unroll
+        for (uint32_t i = 0; i < 32; ++i) {
+            *reinterpret_cast<__nv_bfloat16*>(rows + i * kPairOutRowBytes + lane * 2) = __float2bfloat16_rn(__uint_as_float(sums[i]) * p.scale);
+        }
+    } else {
+        // Lanes 0..15 hold gate rows and lanes 16..31 the matching up rows: the former finish the even tokens, the latter the odd ones.
+        const bool upper = lane >= 16;
+#pragma unroll
+        for (uint32_t i = 0; i < 32; i += 2) {
+            const float other = __uint_as_float(__shfl_xor_sync(0xffffffffu, upper ? sums[i] : sums[i + 1], 16));
+            const float gate = (upper ? other : __uint_as_float(sums[i])) * p.scale, up = (upper ? __uint_as_float(sums[i + 1]) : other) * p.scale_b;
+            *reinterpret_cast<__nv_bfloat16*>(rows + (i + (lane >> 4)) * kPairOutRowBytes + (lane & 15) * 2) =
+                __float2bfloat16_rn(__fdividef(gate, 1.0f + __expf(-gate)) * up);   // as in convert_chunk
+        }
+    }
+    __syncwarp();
+    if (p.quant_out && token0 + lane < p.tokens) {
+        const uint4 low = *reinterpret_cast<const uint4*>(rows + lane * kPairOutRowBytes), high = *reinterpret_cast<const uint4*>(rows + lane * kPairOutRowBytes + 16);
+        const uint32_t packed[8] = {low.x, low.y, low.z, low.w, high.x, high.y, high.z, high.w};
+        quantise_row(p, token0 + lane, row0 / 32, packed);
+    }
+    if (p.out) {
+        const uint32_t lanes = p.swiglu ? 2 : 4, width = p.swiglu ? p.rows / 2 : p.rows;   // 16 bytes a lane
+        uint8_t* out_base = reinterpret_cast<uint8_t*>(p.out + static_cast<uint64_t>(token0) * width + (p.swiglu ? row0 / 2 : row0));
+        for (uint32_t r = lane / lanes; r < 32 && token0 + r < p.tokens; r += 32 / lanes) {
+            const uint32_t piece = lane % lanes;
+            *reinterpret_cast<uint4*>(out_base + static_cast<uint64_t>(r) * width * 2 + piece * 16) =
+                *reinterpret_cast<const uint4*>(rows + r * kPairOutRowBytes + piece * 16);
+        }
+    }
+    __syncwarp();   // the rows are rewritten for the next chunk
+}
+// The epilogue of a tail tile, a function of its own so that it costs the main tiles' no registers: lanes are weight rows and columns tokens, at
+// most 64 of them per warp. Releases the accumulator; false if a part that was to be handed over did not come.
+static __device__ __noinline__ bool pair_tail_epilogue(const GemmParams& p, const PairItem& item, uint32_t accumulator, uint8_t* rows, uint32_t first_token,
+                                                       uint32_t row0, uint32_t pair, uint32_t place, uint32_t tmem_empty, volatile uint32_t* abort_flag) {
+    const uint32_t lane = threadIdx.x & 31;
+    const bool second = first_token + 32 < p.tokens;
+    uint32_t v[2][32];
+    tc_load32(accumulator, v[0]);
+    tc_load32(accumulator + 32, v[1]);   // past the tile's columns: never used
+    tc_wait_ld();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive_leader(tmem_empty);
+    if (item.kind == 1) {
+        float4* own = pair_slot_sums(p, pair_slot(pair, place), lane);
+#pragma unroll
+        for (uint32_t c = 0; c < 2; ++c) {
+            if (c && !second) break;
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                own[(c * 8 + i) * 32] = make_float4(__uint_as_float(v[c][4 * i]), __uint_as_float(v[c][4 * i + 1]),
+                                                    __uint_as_float(v[c][4 * i + 2]), __uint_as_float(v[c][4 * i + 3]));
+            }
+        }
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) atomicExch(p.split_flags + pair_slot(pair, place), 1u);
+        return true;
+    }
+    if (item.kind == 2) {
+        if (!pair_parts_arrived(p, item, pair, place, abort_flag)) return false;
+        for (uint32_t giver = item.first_giver; giver < pair; ++giver) {
+            const float4* src = pair_slot_sums(p, pair_slot(giver, place), lane);
+#pragma unroll
+            for (uint32_t c = 0; c < 2; ++c) {
+                if (c && !second) break;
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) {
+                    const float4 part = __ldcg(src + (c * 8 + i) * 32);
+                    v[c][4 * i] = __float_as_uint(__uint_as_float(v[c][4 * i]) + part.x);
+                    v[c][4 * i + 1] = __float_as_uint(__uint_as_float(v[c][4 * i + 1]) + part.y);
+                    v[c][4 * i + 2] = __float_as_uint(__uint_as_float(v[c][4 * i + 2]) + part.z);
+                    v[c][4 * i + 3] = __float_as_uint(__uint_as_float(v[c][4 * i + 3]) + part.w);
+                }
+            }
+        }
+    }
+    pair_store_tail(p, rows, first_token, row0, lane, v[0]);
+    if (second) pair_store_tail(p, rows, first_token + 32, row0, lane, v[1]);
+    return true;
+}
+
+// One instantiation per number of activation terms (the ring depths as constants are worth 1.5 %), with and without the fused quantiser, whose
+// registers the other epilogues need not pay for.
+template <uint32_t kTerms, bool kQuantised>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant__ CUtensorMap map_weight,
                  const __grid_constant__ CUtensorMap map_act_sf, const __grid_constant__ CUtensorMap map_weight_sf,
-                 const GemmParams p) {
+                 const __grid_constant__ CUtensorMap map_tail, const __grid_constant__ GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* out_stage = smem + kPairRingBytes;
@@ -218,13 +378,29 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();            // 0 = leader
     const uint32_t pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    constexpr PairDepths depth = pair_depths(kResidualTerms ? 3 : 1);
+    constexpr PairDepths depth = pair_depths(kTerms);
     const uint32_t smem_base = smem_u32(smem), tokens_base = smem_base + depth.weights * kPairWeightStage;
     const uint32_t bar0 = smem_u32(bars);
     const uint32_t w_full = bar0, w_landed = bar0 + 8 * kPairMaxDepth;
     const uint32_t t_full = bar0 + 16 * kPairMaxDepth, t_landed = bar0 + 24 * kPairMaxDepth, t_empty = bar0 + 32 * kPairMaxDepth;
     const uint32_t bar_tmem_full = bar0 + 40 * kPairMaxDepth, bar_tmem_empty = bar_tmem_full + 8;
 
+    // An odd number of 128-row token tiles leaves the second CTA of the last pair without rows of its own: it
+    // loads whatever follows (the next term's rows, or the fill value past the tensor) and stores nothing.
+    const uint32_t m_pairs = p.token_pairs;
+    // With an odd number of 128-row blocks of weights the last tile is half as wide (MMA n = 128): each CTA brings 64 of
+    // its rows, and the epilogue warps of the second column half have nothing to do.
+    const uint32_t n_tiles = (p.rows + kTileN - 1) / kTileN;
+    const uint32_t half_tile = p.rows % kTileN ? n_tiles - 1 : n_tiles;
+    const uint32_t main_tiles = m_pairs * n_tiles;
+    // A last k block that is only partly inside the tensor is loaded like the others (the TMA fills what lies past
+    // the edge); the MMA issuer only consumes the k steps inside.
+    const uint32_t k_blocks = (p.cols + kBlockK - 1) / kBlockK;
+    // What this pair does is kept in shared memory: fourteen registers less in every role (the epilogue holds 128 sums a thread).
+    PairWork& work = *reinterpret_cast<PairWork*>(tmem_slot + 2 + kPairThreads / 32);
+    if (threadIdx.x == 32 * 2) {
+        work = pair_work(pair, pairs, PairShares{main_tiles, p.tail_columns ? n_tiles : 0, k_blocks, p.split_sharers, p.cost_main, p.cost_tail});
+    }
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kPairMaxDepth; ++s) {
             mbar_init(w_full + 8 * s, 2);
@@ -252,20 +428,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_weights = tmem_base + kTmemPairScales, tmem_tokens = tmem_weights + depth.weights * 32;
 
-    // An odd number of 128-row token tiles leaves the second CTA of the last pair without rows of its own: it
-    // loads whatever follows (the next term's rows, or the fill value past the tensor) and stores nothing.
-    const uint32_t m_pairs = p.token_pairs;
-    // With an odd number of 128-row blocks of weights the last tile is half as wide (MMA n = 128): each CTA brings 64 of
-    // its rows, and the epilogue warps of the second column half have nothing to do.
-    const uint32_t n_tiles = (p.rows + kTileN - 1) / kTileN;
-    const uint32_t half_tile = p.rows % kTileN ? n_tiles - 1 : n_tiles;
-    const uint32_t total_tiles = m_pairs * n_tiles;
-    // A last k block that is only partly inside the tensor is loaded like the others (the TMA fills what lies past
-    // the edge); the MMA issuer only consumes the k steps inside.
-    const uint32_t k_blocks = (p.cols + kBlockK - 1) / kBlockK;
-    const uint32_t atoms_per_row_block = p.cols / 64;
-    const uint32_t act_term_atoms = p.padded_tokens / 128 * atoms_per_row_block;   // scale atoms of one activation term
-    const PairWork work = pair_work(pair, pairs, total_tiles, k_blocks, p.split_sharers);
     // The weights are constant, so the first ring of them, `ahead` k blocks of the first item, is under way while the launch before
     // this one, whose results the token rows are, still drains. What a role waits for on a barrier must not include that launch,
     // whose time would count against the bound of the wait: a role that depends on it waits for its end first.
@@ -281,61 +443,41 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         // them in tensor memory by the time the operand tiles arrive.
         uint32_t w_stage = 0, slot = 0, t_phase = 1;
         bool alive = true;
-        auto weight_scales = [&](uint32_t n_tile, uint32_t kb, uint32_t stage) {
-            const uint32_t to = smem_base + stage * kPairWeightStage + kPairBytesB, landed = w_landed + 8 * stage;
-            if (rank == 0) mbar_expect_tx(landed, 2 * kBytesSfB);
-            tma_load_2d_pair(to, &map_weight_sf, 0, (n_tile * 2) * atoms_per_row_block + kb * 4, landed);
-            tma_load_2d_pair(to + kBytesSfB / 2, &map_weight_sf, 0, (n_tile * 2 + 1) * atoms_per_row_block + kb * 4, landed);
-        };
-        auto weight_codes = [&](uint32_t n_tile, uint32_t kb, uint32_t stage) {
-            const uint32_t full = w_full + 8 * stage;
-            if (rank == 0) mbar_expect_tx(full, 2 * kPairBytesB);
-            tma_load_2d_pair(smem_base + stage * kPairWeightStage, &map_weight, kb * 128, n_tile * kTileN + rank * (n_tile == half_tile ? 64 : 128), full);
+        // As n operand the scales of all 256 features go to both CTAs, as row operand those of a CTA's own 128 (and the block behind, unused).
+        auto load_weights = [&](const PairTile& t, uint32_t kb, uint32_t stage) {
+            const uint32_t codes = smem_base + stage * kPairWeightStage;
+            tma_weight_step(rank == 0, w_landed + 8 * stage, codes + kPairBytesB, &map_weight_sf, kb * 4, t.n_tile * 2 + (t.tail ? rank : 0),
+                            w_full + 8 * stage, codes, &map_weight, kb * 128, t.n_tile * kTileN + rank * (!t.tail && t.n_tile == half_tile ? 64 : 128));
         };
         if (work.items) {
             const PairItem first = work.item(0, pair, pairs, k_blocks);
+            const PairTile tile = pair_tile(first.tile, main_tiles, m_pairs);
             for (uint32_t stage = 0; stage < ahead; ++stage) {
-                if (elect_one()) {
-                    weight_scales(first.tile / m_pairs, first.kb0 + stage, stage);
-                    weight_codes(first.tile / m_pairs, first.kb0 + stage, stage);
-                }
-                __syncwarp();
+                load_weights(tile, first.kb0 + stage, stage);
             }
         }
-        // The dependents start only after the wait: a narrow launch behind this one (`after_main`) skips its own wait until its
-        // end and relies on the quantiser, which this launch has waited for.
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (lane == 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-        uint32_t done_slot = p.terms - 1, done_phase = 0, blocks = 0;
+        uint32_t blocks = 0;
         for (uint32_t index = 0; alive && index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
-            const uint32_t n_tile = item.tile / m_pairs, token_row = item.tile % m_pairs * 2 * kTileM + rank * kTileM;
+            const PairTile tile = pair_tile(item.tile, main_tiles, m_pairs);
+            // a tail tile's tokens are the n operand: half of them on either CTA, the scales of their one 128-row block on both
+            const CUtensorMap* map_tokens = tile.tail ? &map_tail : &map_act;
+            const uint32_t pair_bytes = tile.tail ? p.tail_columns * 128 : 2 * kBytesA;
+            const uint32_t token_row = tile.token0 + rank * (tile.tail ? p.tail_columns / 2 : kTileM);
+            const uint32_t scale_block = (tile.tail ? tile.token0 : token_row) / 128;
             for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb, ++blocks) {
-                if (blocks >= depth.weights) {
-                    if (!warp_look_wait(t_empty + 8 * done_slot, done_phase, abort_flag, p.status_word, kErrProducerWait)) {
+#pragma unroll
+                for (uint32_t term = 0; term < kTerms; ++term) {
+                    if (!pair_wait(t_empty + 8 * slot, t_phase, abort_flag, p.status_word, kErrProducerWait)) {
                         alive = false;
                         break;
                     }
-                    done_slot += p.terms;
-                    if (done_slot >= depth.tokens) { done_slot -= depth.tokens; done_phase ^= 1; }
-                }
-                const bool fetch = blocks >= ahead;
-                for (uint32_t term = 0; term < p.terms; ++term) {
-                    if (!warp_look_wait(t_empty + 8 * slot, t_phase, abort_flag, p.status_word, kErrProducerWait)) {
-                        alive = false;
-                        break;
-                    }
-                    if (elect_one()) {
-                        const uint32_t base = tokens_base + slot * kPairTokenSlot, landed = t_landed + 8 * slot, full = t_full + 8 * slot;
-                        if (rank == 0) mbar_expect_tx(landed, 2 * kBytesSfA);
-                        tma_load_2d_pair(base + kBytesA, &map_act_sf, 0,
-                                         term * act_term_atoms + (token_row / 128) * atoms_per_row_block + kb * 4, landed);
-                        if (fetch && term == 0) weight_scales(n_tile, kb, w_stage);
-                        if (rank == 0) mbar_expect_tx(full, 2 * kBytesA);
-                        tma_load_2d_pair(base, &map_act, kb * 128, term * p.padded_tokens + token_row, full);
-                        if (fetch && term == 0) weight_codes(n_tile, kb, w_stage);
-                    }
-                    __syncwarp();
+                    if (term == pair_weight_term(kTerms) && blocks >= ahead) load_weights(tile, kb, w_stage);
+                    const uint32_t base = tokens_base + slot * kPairTokenSlot;
+                    tma_token_step(rank == 0, t_landed + 8 * slot, base + kBytesA, &map_act_sf, kb * 4, term * (p.padded_tokens / 128) + scale_block,
+                                   t_full + 8 * slot, pair_bytes, base, map_tokens, kb * 128, term * p.padded_tokens + token_row);
                     if (++slot == depth.tokens) { slot = 0; t_phase ^= 1; }
                 }
                 if (++w_stage == depth.weights) w_stage = 0;
@@ -349,58 +491,43 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         // bits hold address >> 4). Looking at a barrier takes as long as issuing an MMA or two, so those of the next
         // step are looked at before the MMAs of this one are issued, and waited for only if they were not there.
         uint32_t w_stage = 0, w_phase = 0, slot = 0, t_phase = 0, tmem_phase = 0;
-        bool alive = true, tokens_seen = false, weights_seen = false;
+        bool alive = true;
         constexpr uint32_t kWideTile = (1u << 7) | (1u << 10) | ((kTileN >> 3) << 17) | (((2 * kTileM) >> 4) << 24);
         constexpr uint32_t kHalfTile = (1u << 7) | (1u << 10) | ((kTileN / 2 >> 3) << 17) | (((2 * kTileM) >> 4) << 24);
-        const uint64_t w_desc0 = operand_desc(smem_base), t_desc0 = operand_desc(tokens_base);
+        const uint32_t w_desc0 = static_cast<uint32_t>(operand_desc(smem_base)), t_desc0 = static_cast<uint32_t>(operand_desc(tokens_base));
         const uint32_t last_k_steps = (p.cols - (k_blocks - 1) * kBlockK) / 64;   // 1..4 k steps of 64 in the last k block
         asm volatile("griddepcontrol.wait;" ::: "memory");   // the token rows
         for (uint32_t index = 0; alive && index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
-            // the epilogues of both CTAs must have drained the previous tile's accumulator
+            // The epilogues of both CTAs must have drained the previous tile's accumulator: the one wait that polls, since the tensor pipe
+            // stands still meanwhile.
             if (!warp_look_wait(bar_tmem_empty, tmem_phase ^ 1, abort_flag, p.status_word, kErrMmaWaitTmem)) break;
-            tc_fence_after();
-            const uint32_t idesc = item.tile / m_pairs == half_tile ? kHalfTile : kWideTile;
+            const PairTile tile = pair_tile(item.tile, main_tiles, m_pairs);
             uint32_t accumulate = 0;
-            for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb) {
-                const uint32_t k_steps = (kb + 1 < k_blocks) ? 4u : last_k_steps;
-                if (!weights_seen && !warp_look_wait(w_full + 8 * w_stage, w_phase, abort_flag, p.status_word, kErrMmaWaitWeights)) {
-                    alive = false;
-                    break;
-                }
-                const uint64_t w_desc = w_desc0 + w_stage * (kPairWeightStage >> 4);
-                const uint32_t sf_w = tmem_weights + w_stage * 32;
-                if (++w_stage == depth.weights) { w_stage = 0; w_phase ^= 1; }
-                for (uint32_t term = 0; term < p.terms; ++term) {
-                    // codes in shared memory (TMA) and block scales on their way to tensor memory (copy warp)
-                    if (!tokens_seen && !warp_look_wait(t_full + 8 * slot, t_phase, abort_flag, p.status_word, kErrMmaWaitTokens)) {
-                        alive = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint64_t t_desc = t_desc0 + slot * (kPairTokenSlot >> 4);
-                    const uint32_t sf_t = tmem_tokens + slot * 16, t_done = t_empty + 8 * slot;
-                    if (++slot == depth.tokens) { slot = 0; t_phase ^= 1; }
-                    tokens_seen = mbar_test(t_full + 8 * slot, t_phase);
-                    if (term + 1 == p.terms) weights_seen = mbar_test(w_full + 8 * w_stage, w_phase);
-                    if (elect_one()) {
-                        // each MMA consumes 64 k = 32 bytes of every row: start address + 2; only k steps inside the tensor
-                        if (k_steps == 4) {
+            // `Tail`: the weights are the row operand
+            auto multiply = [&](auto tail, uint32_t idesc) {
+                for (uint32_t kb = item.kb0; kb < item.kb1; ++kb) {
+                    if (!pair_wait(w_full + 8 * w_stage, w_phase, abort_flag, p.status_word, kErrMmaWaitWeights)) return false;
+                    const uint32_t w_desc = w_desc0 + w_stage * (kPairWeightStage >> 4), sf_w = tmem_weights + w_stage * 32;
+                    const uint32_t k_steps = kb + 1 < k_blocks ? 4u : last_k_steps;
+                    if (++w_stage == depth.weights) { w_stage = 0; w_phase ^= 1; }
 #pragma unroll
-                            for (uint32_t k = 0; k < 4; ++k) {
-                                tc_mma_pair(tmem_base + kTmemAcc, t_desc + 2 * k, w_desc + 2 * k, idesc, sf_t + 4 * k, sf_w + 8 * k, accumulate | k);
-                            }
-                        } else {
-                            for (uint32_t k = 0; k < k_steps; ++k) {
-                                tc_mma_pair(tmem_base + kTmemAcc, t_desc + 2 * k, w_desc + 2 * k, idesc, sf_t + 4 * k, sf_w + 8 * k, accumulate | k);
-                            }
-                        }
-                        tc_commit_pair(t_done);   // frees the slot, and with it the slot's scale columns, in both CTAs
+                    for (uint32_t term = 0; term < kTerms; ++term) {
+                        // codes in shared memory (TMA) and block scales on their way to tensor memory (copy warp)
+                        if (!pair_wait(t_full + 8 * slot, t_phase, abort_flag, p.status_word, kErrMmaWaitTokens)) return false;
+                        const uint32_t t_desc = t_desc0 + slot * (kPairTokenSlot >> 4), sf_t = tmem_tokens + slot * 16, t_done = t_empty + 8 * slot;
+                        // Each MMA consumes 64 k = 32 bytes of every row: start address + 2; only k steps inside the tensor. The commit frees
+                        // the slot, and with it the slot's scale columns, in both CTAs.
+                        if (tail) tc_step_pair(tmem_base + kTmemAcc, w_desc, t_desc, idesc, sf_w, sf_t, 8, 4, accumulate, k_steps, t_done);
+                        else tc_step_pair(tmem_base + kTmemAcc, t_desc, w_desc, idesc, sf_t, sf_w, 4, 8, accumulate, k_steps, t_done);
+                        if (++slot == depth.tokens) { slot = 0; t_phase ^= 1; }
+                        accumulate = 1;
                     }
-                    __syncwarp();
-                    accumulate = 1;
                 }
-            }
+                return true;
+            };
+            alive = tile.tail ? multiply(PairTail<true>(), kHalfTile - (((kTileN / 2 - p.tail_columns) >> 3) << 17))
+                              : multiply(PairTail<false>(), tile.n_tile == half_tile ? kHalfTile : kWideTile);
             if (alive && elect_one()) tc_commit_pair(bar_tmem_full);     // both accumulator halves complete
             __syncwarp();
             tmem_phase ^= 1;
@@ -413,59 +540,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         // A slot's scale atoms have landed. The producer refilled the slot only after the MMAs that used it last were
         // complete, so the slot's scale columns are free. The copies only have to be issued before the MMAs that read them: a
         // copy and a later MMA execute in issue order, and the fences on either side of the arrival order the two warps' issues.
-        const bool weights = warp != kPairCopyWarp;
-        uint32_t slot = 0, phase = 0;
-        const uint32_t slots = weights ? depth.weights : depth.tokens, per_block = weights ? 1u : p.terms;
-        const uint32_t landed = weights ? w_landed : t_landed, full = weights ? w_full : t_full;
-        const uint64_t desc0 = sf_desc(weights ? smem_base + kPairBytesB : tokens_base + kBytesA);
-        const uint32_t slot_step = (weights ? kPairWeightStage : kPairTokenSlot) >> 4;
-        const uint32_t columns0 = weights ? tmem_weights : tmem_tokens, slot_columns = weights ? 32 : 16;
-        constexpr uint32_t kAtomStep = kSfAtomBytes >> 4, kRowBlockStep = kBytesSfB / 2 >> 4;
-        const uint32_t last_k_steps = (p.cols - (k_blocks - 1) * kBlockK) / 64;
-        // the token rows; and weights beyond the first ring, whose stages are free when the token rows have been multiplied with
-        uint32_t before_wait = weights ? ahead : 0;
-        if (!before_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
-        bool alive = true;
-        for (uint32_t index = 0; alive && index < work.items; ++index) {
-            const PairItem item = work.item(index, pair, pairs, k_blocks);
-            const bool wide = item.tile / m_pairs != half_tile;   // a half tile has one row block of weight scales
-            for (uint32_t kb = item.kb0; alive && kb < item.kb1; ++kb) {
-                const uint32_t k_steps = (kb + 1 < k_blocks) ? 4u : last_k_steps;
-                for (uint32_t term = 0; term < per_block; ++term) {
-                    if (!warp_look_wait(landed + 8 * slot, phase, abort_flag, p.status_word, kErrCopyWait)) {
-                        alive = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    if (elect_one()) {
-                        const uint64_t desc = desc0 + slot * slot_step;
-                        const uint32_t columns = columns0 + slot * slot_columns;
-                        if (!weights) {
-                            if (k_steps == 4) {
-#pragma unroll
-                                for (uint32_t k = 0; k < 4; ++k) tc_copy_sf_pair(columns + 4 * k, desc + k * kAtomStep);
-                            } else {
-                                for (uint32_t k = 0; k < k_steps; ++k) tc_copy_sf_pair(columns + 4 * k, desc + k * kAtomStep);
-                            }
-                        } else if (k_steps == 4 && wide) {
-#pragma unroll
-                            for (uint32_t k = 0; k < 4; ++k) {
-                                tc_copy_sf_pair(columns + 8 * k, desc + k * kAtomStep);
-                                tc_copy_sf_pair(columns + 8 * k + 4, desc + kRowBlockStep + k * kAtomStep);
-                            }
-                        } else {
-                            for (uint32_t k = 0; k < k_steps; ++k) {
-                                tc_copy_sf_pair(columns + 8 * k, desc + k * kAtomStep);
-                                if (wide) tc_copy_sf_pair(columns + 8 * k + 4, desc + kRowBlockStep + k * kAtomStep);
-                            }
-                        }
-                        tc_fence_before();
-                        mbar_arrive(full + 8 * slot);
-                    }
-                    __syncwarp();
-                    if (++slot == slots) { slot = 0; phase ^= 1; }
-                    if (before_wait && --before_wait == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
-                }
+        // Slots are taken as they come, whatever tile they belong to, and whole: what a last k block or a tile does not have is not read.
+        const uint32_t blocks = work.blocks(k_blocks);
+        if (warp == kPairCopyWarp) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");   // the token rows
+            const uint64_t desc0 = sf_desc(tokens_base + kBytesA);
+            uint32_t slot = 0, phase = 0;
+            for (uint32_t left = blocks * kTerms; left; --left) {
+                if (!pair_wait(t_landed + 8 * slot, phase, abort_flag, p.status_word, kErrCopyWait)) break;
+                tc_copy_step_pair<1>(tmem_tokens + slot * 16, desc0 + slot * (kPairTokenSlot >> 4), t_full + 8 * slot);
+                if (++slot == depth.tokens) { slot = 0; phase ^= 1; }
+            }
+        } else {
+            const uint64_t desc0 = sf_desc(smem_base + kPairBytesB);
+            uint32_t stage = 0, phase = 0;
+            for (uint32_t block = 0; block < blocks; ++block) {
+                // stages beyond the first ring are free when the token rows have been multiplied with
+                if (block == ahead) asm volatile("griddepcontrol.wait;" ::: "memory");
+                if (!pair_wait(w_landed + 8 * stage, phase, abort_flag, p.status_word, kErrCopyWait)) break;
+                tc_copy_step_pair<2>(tmem_weights + stage * 32, desc0 + stage * (kPairWeightStage >> 4), w_full + 8 * stage);
+                if (++stage == depth.weights) { stage = 0; phase ^= 1; }
             }
         }
     } else if (warp >= 2 && warp < 2 + kPairEpilogueWarps) {
@@ -481,10 +575,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         uint8_t* my_rows = out_stage + (warp - 2) * 32 * kPairOutRowBytes;
         for (uint32_t index = 0; index < work.items; ++index) {
             const PairItem item = work.item(index, pair, pairs, k_blocks);
-            const uint32_t m_pair = item.tile % m_pairs, n_tile = item.tile / m_pairs;
+            const PairTile tile = pair_tile(item.tile, main_tiles, m_pairs);
+            const uint32_t n_tile = tile.n_tile;
             if (!warp_wait_suspended(bar_tmem_full, tmem_phase, abort_flag, p.status_word, kErrEpilogueWait)) break;
             tc_fence_after();
-            const uint32_t accumulator = tmem_base + kTmemAcc + ((quadrant * 32) << 16) + half * 128;
+            const uint32_t accumulator = tmem_base + kTmemAcc + ((quadrant * 32) << 16) + half * (tile.tail ? 64 : 128);
             auto release = [&]() {   // the accumulator is free for the next tile's MMAs from here on
                 tc_fence_before();
                 __syncwarp();
@@ -494,47 +589,58 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
             // Rows past the tokens, and the columns a half tile does not have: nothing to store, hand over or add. (Padding rows
             // hold whatever the staging buffer held; converting them cost more than real ones, since zeros and non-finite
             // values leave the quantiser's fast path.)
-            const uint32_t first_token = m_pair * 2 * kTileM + rank * kTileM + quadrant * 32;
-            if (first_token >= p.tokens || (half && n_tile == half_tile)) {
+            const uint32_t first_token = tile.token0 + (tile.tail ? half * 64 : rank * kTileM + quadrant * 32);
+            const uint32_t tail_row = n_tile * kTileN + rank * kTileM + quadrant * 32;   // of a tail tile: this warp's weight rows
+            if (first_token >= p.tokens || (tile.tail ? tail_row >= p.rows : half && n_tile == half_tile)) {
                 release();
                 continue;
             }
 
-            // One 32-column chunk of sums on its way out.
-            const uint32_t out_width = p.swiglu ? p.rows / 2 : p.rows, token = first_token + lane;
+            const uint32_t out_width = kQuantised || p.swiglu ? p.rows / 2 : p.rows, token = first_token + lane;
             uint32_t scale_words[3] = {0, 0, 0};   // SwiGLU, quantised: the scale bytes of this row's 4 groups, per term: one word of an atom
+            uint32_t held[8];
+            // The BF16 values this lane holds, quantised for the next GEMM while the next tile's MMAs run: groups c (`held`) and c + 1. Eight warps
+            // do not hide the latencies of one group's chain of three terms: two side by side, and stores of 16 bytes.
+            auto quantise_two = [&](uint32_t c, const uint32_t (&second)[16]) {
+                if (token >= p.tokens) return;
+                const uint64_t code_bytes = tcgen05_codes_bytes(p.padded_tokens, out_width);
+                const uint32_t group = n_tile * (kTileN / 32) + half * 4 + c;
+                float2 residual[2][8];
+#pragma unroll
+                for (uint32_t i = 0; i < 8; ++i) {
+                    residual[0][i] = make_float2(__uint_as_float(held[i] << 16), __uint_as_float(held[i] & 0xffff0000u));
+                    residual[1][i] = make_float2(__uint_as_float(second[i] << 16), __uint_as_float(second[i] & 0xffff0000u));
+                }
+#pragma unroll
+                for (uint32_t term = 0; term < 3; ++term) {
+                    if (term >= p.quant_terms) break;
+                    uint32_t codes[2][2], scale_code[2];
+                    if (term + 1 < p.quant_terms) quantise_groups_as<true>(residual, p.quant_scale, codes, scale_code);
+                    else quantise_groups_as<false>(residual, p.quant_scale, codes, scale_code);
+                    scale_words[term] |= scale_code[0] << (8 * c) | scale_code[1] << (8 * c + 8);
+                    *reinterpret_cast<uint4*>(p.quant_out + term * code_bytes + static_cast<uint64_t>(token) * (out_width / 2) + group * 8) =
+                        make_uint4(codes[0][0], codes[0][1], codes[1][0], codes[1][1]);
+                }
+                if (c == 2) {
+                    const uint64_t scale_bytes = tcgen05_scale_bytes(p.padded_tokens, out_width);
+#pragma unroll
+                    for (uint32_t term = 0; term < 3; ++term) {
+                        if (term >= p.quant_terms) break;
+                        *reinterpret_cast<uint32_t*>(p.quant_out + p.quant_terms * code_bytes + term * scale_bytes +
+                                                     tcgen05_scale_offset(token, n_tile * (kTileN / 32) + half * 4, out_width)) = scale_words[term];
+                    }
+                }
+            };
+            // One 32-column chunk of sums on its way out.
             auto store_chunk = [&](uint32_t c, const uint32_t (&sums)[32]) {
                 uint32_t packed[16];
-                if (p.swiglu) {
+                if (kQuantised || p.swiglu) {
                     // 32 accumulator columns = gate and up sums of 16 intermediate columns = one quantisation group per row
                     convert_chunk(sums, p.scale, p.scale_b, true, packed);
-                    if (p.quant_out && token < p.tokens) {
-                        // The BF16 values this lane holds, quantised for the next GEMM while the next tile's MMAs run.
-                        const uint64_t code_bytes = tcgen05_codes_bytes(p.padded_tokens, out_width);
-                        const uint32_t group = n_tile * (kTileN / 32) + half * 4 + c;
-                        float2 residual[8];
+                    if (kQuantised) {
+                        if (c & 1) quantise_two(c - 1, packed);
 #pragma unroll
-                        for (uint32_t i = 0; i < 8; ++i) {
-                            residual[i] = make_float2(__uint_as_float(packed[i] << 16), __uint_as_float(packed[i] & 0xffff0000u));
-                        }
-#pragma unroll
-                        for (uint32_t term = 0; term < 3; ++term) {
-                            if (term >= p.quant_terms) break;
-                            uint32_t codes[2], scale_code;
-                            quantise_term(residual, p.quant_scale, term + 1 < p.quant_terms, codes, &scale_code);
-                            scale_words[term] |= scale_code << (8 * c);
-                            *reinterpret_cast<uint2*>(p.quant_out + term * code_bytes + static_cast<uint64_t>(token) * (out_width / 2) + group * 8) =
-                                make_uint2(codes[0], codes[1]);
-                        }
-                        if (c == 3) {
-                            const uint64_t scale_bytes = tcgen05_scale_bytes(p.padded_tokens, out_width);
-#pragma unroll
-                            for (uint32_t term = 0; term < 3; ++term) {
-                                if (term >= p.quant_terms) break;
-                                *reinterpret_cast<uint32_t*>(p.quant_out + p.quant_terms * code_bytes + term * scale_bytes +
-                                                             tcgen05_scale_offset(token, n_tile * (kTileN / 32) + half * 4, out_width)) = scale_words[term];
-                            }
-                        }
+                        for (uint32_t i = 0; i < 8; ++i) held[i] = packed[i];
                     }
                     if (p.out) {
                         // transpose through shared memory: 32 bytes of every row, written out as 2 lanes per row
@@ -574,32 +680,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
                 }
                 __syncwarp();   // the rows are rewritten for the next chunk
             };
-            auto slot_of = [&](uint32_t giver) { return (giver * 2 + rank) * kPairEpilogueWarps + (warp - 2); };
-            auto slot_sums = [&](uint32_t slot) { return reinterpret_cast<float4*>(p.split_slots) + static_cast<uint64_t>(slot) * (32 * 32) + lane; };
-
-            // The part that finishes a leftover tile waits for the parts handed over and adds them in pair order.
-            auto parts_arrived = [&]() {
-                bool arrived = true;
-                for (uint32_t giver = item.first_giver; giver < pair; ++giver) {
-                    const uint32_t slot = slot_of(giver);
-                    if (lane == 0) {
-                        uint32_t spin = 0;
-                        while (atomicAdd(p.split_flags + slot, 0u) == 0u) {
-                            if (++spin > kSplitWaitLimit || ((spin & 255u) == 255u && *abort_flag)) {
-                                arrived = false;
-                                *abort_flag = 1;
-                                atomicCAS(p.status_word, 0u, kErrSplitWait);
-                                break;
-                            }
-                        }
-                        // The flags read zero again when the launch is over, also those of parts that were given up on: that launch has
-                        // failed and says so, and a late giver cannot leave one set for the next launch on this plan.
-                        p.split_flags[slot] = 0;
-                    }
-                }
-                __threadfence();
-                return __all_sync(0xffffffffu, arrived) != 0;
-            };
+            auto slot_of = [&](uint32_t giver) { return pair_slot(giver, rank * kPairEpilogueWarps + warp - 2); };
+            auto slot_sums = [&](uint32_t slot) { return pair_slot_sums(p, slot, lane); };
+            auto parts_arrived = [&]() { return pair_parts_arrived(p, item, pair, rank * kPairEpilogueWarps + warp - 2, abort_flag); };
+            if (tile.tail) {
+                if (!pair_tail_epilogue(p, item, accumulator, my_rows, first_token, tail_row, pair, rank * kPairEpilogueWarps + warp - 2, bar_tmem_empty, abort_flag)) break;
+                tmem_phase ^= 1;
+                continue;
+            }
             if (item.kind == 2 && index + 1 == work.items) {
                 if (!parts_arrived()) break;
                 // Nothing follows that waits for the accumulator: a chunk at a time stays in registers, and the same chunk of several
@@ -692,6 +780,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
     }
 }
 
+using PairKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GemmParams);
+constexpr PairKernel kPairKernels[6] = {gemm_pair_kernel<1, false>, gemm_pair_kernel<2, false>, gemm_pair_kernel<3, false>,
+                                        gemm_pair_kernel<1, true>, gemm_pair_kernel<2, true>, gemm_pair_kernel<3, true>};
+
 // ---- activation quantiser kernel ---------------------------------------------------------------
 // One thread per (token, 16-element group). Destination: the code planes of all terms
 // stacked ([terms][tokens][cols/2], one TMA tensor of terms*tokens rows), then the scale
@@ -772,16 +864,16 @@ bool make_code_map(CUtensorMap* map, uint64_t address, uint64_t rows, uint32_t c
 }
 
 namespace {
-// Block-scale atoms as a 2-D tensor [atoms][256 x u16] (512 bytes each); a box is the 4 atoms of
-// one 128-row block and one 256-deep k block.
-bool make_scale_map(CUtensorMap* map, uint64_t address, uint64_t atoms) {
+// Block-scale atoms as a tensor [128-row blocks][atoms of a block along k][256 x u16] (512 bytes an atom); a box is the 4 atoms of
+// `box_blocks` row blocks and one 256-deep k block.
+bool make_scale_map(CUtensorMap* map, uint64_t address, uint64_t row_blocks, uint64_t atoms, uint32_t box_blocks) {
     const EncodeTiled encode = encode_entry();
     if (!encode) return false;
-    const cuuint64_t dims[2] = {256, atoms};
-    const cuuint64_t strides[1] = {kSfAtomBytes};
-    const cuuint32_t box[2] = {256, 4};
-    const cuuint32_t element_strides[2] = {1, 1};
-    return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, reinterpret_cast<void*>(address), dims, strides, box,
+    const cuuint64_t dims[3] = {256, atoms, row_blocks};
+    const cuuint64_t strides[2] = {kSfAtomBytes, atoms * kSfAtomBytes};
+    const cuuint32_t box[3] = {256, 4, box_blocks};
+    const cuuint32_t element_strides[3] = {1, 1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, reinterpret_cast<void*>(address), dims, strides, box,
                   element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -870,7 +962,7 @@ uint32_t gemm_pair_resident_clusters() {
     config.attrs = &attribute;
     config.numAttrs = 1;
     int fewest = INT_MAX;
-    for (auto* kernel : {gemm_pair_kernel<false>, gemm_pair_kernel<true>}) {
+    for (PairKernel kernel : kPairKernels) {
         int clusters = 0;
         if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess || clusters < 1) {
             cudaGetLastError();
@@ -882,8 +974,11 @@ uint32_t gemm_pair_resident_clusters() {
 }
 
 cudaError_t gemm_configure_device() {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
+    for (PairKernel kernel : kPairKernels) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace augur_sm100
@@ -960,52 +1055,63 @@ struct PairSplit {
 // the weights of a k block come with every step (one tile per pair, 18944 rows, 256 tokens, 10 to 40 k blocks), a launch 9 to 11 us beyond.
 // The choice that these constants make is 0.7 % off the best on average, and 27 % where the two kernels are estimated alike: 10240 x
 // 5120, two terms, 300 tokens 38 us, narrow 32.
-constexpr uint32_t kPairStepNs = 360, kPairLaunchNs = 8000;
+constexpr uint32_t kPairStepCost = 36, kPairLaunchNs = 8000;   // a step in units of 10 ns
 constexpr uint32_t kSplitSteps = 16, kSplitPartSteps = 2, kSplitCoveredSteps = 8;
+
+// What a k block of a tile costs: a main tile's (`tail_columns` 0) or a tail tile's.
+uint32_t pair_block_cost(uint32_t terms, uint32_t tail_columns) {
+    return tail_columns ? 34 + terms * 10 + terms * (tail_columns - 32) / 20 : 22 + terms * 28;
+}
 
 // Tiles past the last full round of the pairs (all tiles, when there are fewer tiles than pairs) may be cut along k, in `ways`
 // parts each at most and over all pairs at most, when the plan's scratch has room for the partial accumulators handed
 // over: one slot per pair behind the counter regions, whose first words serve as the flags. Of the numbers of parts up to
 // kSplitWays the one with the least steps is taken: cut in eight, the 4 tiles of 1024 rows and 256 tokens took 25 us, whole 15.
-PairSplit pair_split(uint32_t token_pairs, uint32_t rows, uint32_t cols, uint32_t terms, uint32_t all_pairs, uint64_t scratch_bytes) {
-    const uint32_t tiles = token_pairs * ((rows + kTileN - 1) / kTileN), k_blocks = (cols + kBlockK - 1) / kBlockK;
-    const uint32_t whole = tiles / all_pairs, left = tiles % all_pairs;
-    PairSplit best{tiles < all_pairs ? tiles : all_pairs, 0, 0};
-    uint64_t least = static_cast<uint64_t>(whole + (left ? 1 : 0)) * k_blocks * terms;
-    for (uint32_t ways = 2; left && ways <= kSplitWays; ++ways) {
-        uint32_t sharers = left * ways < all_pairs ? left * ways : all_pairs;
-        if (sharers > static_cast<uint64_t>(left) * k_blocks) sharers = left * k_blocks;      // every part holds a k block
-        if (sharers <= left || scratch_bytes < kCounterBytes + sharers * kSplitSlotBytes) break;
-        const uint32_t parts = (sharers + left - 1) / left;
-        const uint64_t steps = static_cast<uint64_t>(whole) * k_blocks * terms + static_cast<uint64_t>(left * k_blocks + sharers - 1) / sharers * terms +
-                               (whole ? kSplitCoveredSteps : kSplitSteps + kSplitPartSteps * parts);
-        if (steps < least) {
-            least = steps;
-            best.sharers = sharers;
+PairSplit pair_split(uint32_t token_pairs, uint32_t tail_columns, uint32_t rows, uint32_t cols, uint32_t terms, uint32_t all_pairs, uint64_t scratch_bytes) {
+    const uint32_t n_tiles = (rows + kTileN - 1) / kTileN, k_blocks = (cols + kBlockK - 1) / kBlockK;
+    const uint32_t main = token_pairs * n_tiles, tail = tail_columns ? n_tiles : 0;
+    const uint64_t cost_main = pair_block_cost(terms, 0), cost_tail = tail ? pair_block_cost(terms, tail_columns) : 0;
+    const uint32_t rounds = main / all_pairs, left = main % all_pairs;
+    PairSplit best{main + tail < all_pairs ? main + tail : all_pairs, 0, 0};
+    // not cut: the first pair has the most tiles of either kind
+    const uint64_t most_main = (main + all_pairs - 1) / all_pairs, most = (main + tail + all_pairs - 1) / all_pairs;
+    uint64_t least = k_blocks * (most_main * cost_main + (most - most_main) * cost_tail);
+    const uint64_t line = k_blocks * (left * cost_main + tail * cost_tail), largest = left ? cost_main : cost_tail;
+    for (uint32_t ways = 2; line && ways <= kSplitWays; ++ways) {
+        uint64_t sharers = line * ways / (k_blocks * largest);
+        if (sharers > all_pairs) sharers = all_pairs;
+        if (sharers > line / cost_main) sharers = line / cost_main;      // every range holds a k block
+        if (sharers < 2 || (!tail && sharers <= left) || scratch_bytes < kCounterBytes + sharers * kSplitSlotBytes) break;
+        const uint64_t parts = (sharers * k_blocks * largest + line - 1) / line;
+        const uint64_t cost = k_blocks * rounds * cost_main + (line + sharers - 1) / sharers +
+                              (rounds ? kSplitCoveredSteps : kSplitSteps + kSplitPartSteps * parts) * kPairStepCost;
+        if (cost < least) {
+            least = cost;
+            best.sharers = static_cast<uint32_t>(sharers);
         }
     }
     if (best.pairs < best.sharers) best.pairs = best.sharers;
-    best.ns = static_cast<uint32_t>(least * kPairStepNs > UINT32_MAX / 2 ? UINT32_MAX / 2 : least * kPairStepNs) + kPairLaunchNs;
+    best.ns = static_cast<uint32_t>(least * 10 > UINT32_MAX / 2 ? UINT32_MAX / 2 : least * 10) + kPairLaunchNs;
     return best;
 }
 
-// How many of the token rows the pair kernel takes (in 256-row pairs); the narrow kernel takes the rest. The choice is the
-// quickest by the estimates of the two: narrow up to 128 tokens nearly always (6144 x 5120, three terms, 48 tokens: 15 us
-// against 24), pairs from about 256 on (17408 x 5120, 256 tokens: 31 against 40) unless the weight is small (1024 x 5120: 27
-// against 18.5), and pairs with a narrow tail when the tokens just exceed whole pairs (17408 x 5120, 300 tokens: 52 against
-// 54). The tail starts when the pairs are nearly done, so it has to be clearly quicker to be taken.
-uint32_t token_pairs_for(const augur_cuda_nvfp4_sm100_plan_v1* plan, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
+// Which token rows the pair kernel takes, and how: all of them or none (the narrow kernel's then). The choice is the quickest by the
+// estimates.
+struct PairPlan {
+    uint32_t token_pairs, tail_columns;
+    PairSplit split;
+};
+PairPlan pair_plan(const augur_cuda_nvfp4_sm100_plan_v1* plan, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
     const uint32_t all_pairs = plan->pair_clusters, pairs = (tokens + 2 * kTileM - 1) / (2 * kTileM), rest = tokens % (2 * kTileM);
-    if (!all_pairs) return 0;
+    if (!all_pairs) return PairPlan{};
     const uint32_t narrow_ns = gemm_narrow_ns(plan->ordinal, rows, cols, tokens, terms);
-    const uint32_t pair_ns = pair_split(pairs, rows, cols, terms, all_pairs, plan->scratch_bytes).ns;
-    uint32_t best = pair_ns < narrow_ns ? pairs : 0;
+    PairPlan best{pairs, 0, pair_split(pairs, 0, rows, cols, terms, all_pairs, plan->scratch_bytes)};
     if (pairs > 1 && rest != 0 && rest <= kTileM) {
-        const uint64_t mixed = static_cast<uint64_t>(pair_split(pairs - 1, rows, cols, terms, all_pairs, plan->scratch_bytes).ns) +
-                               gemm_narrow_ns(plan->ordinal, rows, cols, rest, terms) - 3000;
-        if (mixed * 100 < static_cast<uint64_t>(best ? pair_ns : narrow_ns) * 93) best = pairs - 1;
+        const uint32_t columns = (rest + 31) / 32 * 32;
+        const PairPlan tail{pairs - 1, columns, pair_split(pairs - 1, columns, rows, cols, terms, all_pairs, plan->scratch_bytes)};
+        if (tail.split.ns < best.split.ns) best = tail;
     }
-    return best;
+    return best.split.ns < narrow_ns ? best : PairPlan{};
 }
 
 augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
@@ -1030,29 +1136,35 @@ augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_s
     p.quant_out = reinterpret_cast<uint8_t*>(quant.destination);
     p.quant_terms = quant.terms;
     p.quant_scale = quant_scale(quant.global_scale);
-    p.token_pairs = token_pairs_for(plan, a->rows, a->cols, a->tokens, a->activation_terms);
+    const PairPlan pairs = pair_plan(plan, a->rows, a->cols, a->tokens, a->activation_terms);
+    p.token_pairs = pairs.token_pairs;
     if (p.token_pairs) {
         // 256 x 256 tiles on pairs of CTAs (clusters of two); the grid is a whole number of pairs.
         CUtensorMap map_act, map_act_sf, map_weight_sf;
-        const uint64_t atoms_per_row_block = a->cols / 64;
+        const uint64_t atoms = a->cols / 64;
         if (!make_code_map(&map_act, a->activation, static_cast<uint64_t>(a->activation_terms) * padded, a->cols) ||
-            !make_scale_map(&map_weight_sf, reinterpret_cast<uint64_t>(p.weight_sf), (a->rows / 128) * atoms_per_row_block) ||
+            !make_scale_map(&map_weight_sf, reinterpret_cast<uint64_t>(p.weight_sf), a->rows / 128, atoms, 2) ||
             !make_scale_map(&map_act_sf, reinterpret_cast<uint64_t>(p.act_sf),
-                            static_cast<uint64_t>(a->activation_terms) * (padded / 128) * atoms_per_row_block)) {
+                            static_cast<uint64_t>(a->activation_terms) * (padded / 128), atoms, 1)) {
             return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
         }
-        const PairSplit split = pair_split(p.token_pairs, a->rows, a->cols, a->activation_terms, plan->pair_clusters, plan->scratch_bytes);
-        if (split.sharers) {
-            p.split_sharers = split.sharers;
+        p.tail_columns = pairs.tail_columns;
+        CUtensorMap map_tail = map_act;
+        if (p.tail_columns && !make_code_map(&map_tail, a->activation, static_cast<uint64_t>(a->activation_terms) * padded, a->cols, p.tail_columns / 2)) {
+            return make_result(AUGUR_CUDA_STATUS_RUNTIME_FAILURE);
+        }
+        p.cost_main = pair_block_cost(a->activation_terms, 0);
+        p.cost_tail = pair_block_cost(a->activation_terms, p.tail_columns);
+        if (pairs.split.sharers) {
+            p.split_sharers = pairs.split.sharers;
             p.split_flags = reinterpret_cast<uint32_t*>(plan->scratch);
             p.split_slots = reinterpret_cast<float*>(plan->scratch + kCounterBytes);
         }
-        launch_dependent(s->stream, a->activation_terms > 1 ? gemm_pair_kernel<true> : gemm_pair_kernel<false>, 2 * split.pairs, kPairThreads, kPairSmemBytes, map_act, map_weight, map_act_sf, map_weight_sf, p);
+        launch_dependent(s->stream, kPairKernels[a->activation_terms - 1 + (p.quant_out ? 3 : 0)], 2 * pairs.split.pairs, kPairThreads, kPairSmemBytes, map_act, map_weight, map_act_sf, map_weight_sf, map_tail, p);
         count_launch();
-        const augur_cuda_result_v1 result = submitted();
-        if (result.status != AUGUR_CUDA_STATUS_OK || p.token_pairs * 2 * kTileM >= a->tokens) return result;
+        return submitted();
     }
-    return launch_gemm_narrow(s, plan, map_weight, a->activation, p, p.token_pairs * 2 * kTileM, p.token_pairs != 0);
+    return launch_gemm_narrow(s, plan, map_weight, a->activation, p);
 }
 
 static_assert(sizeof(augur_cuda_nvfp4_sm100_gemm_swiglu_args_v1) == 88, "gemm_swiglu ABI");

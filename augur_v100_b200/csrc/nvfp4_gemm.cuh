@@ -19,6 +19,8 @@ struct GemmParams {
     uint32_t* status_word;
     uint32_t rows, cols, tokens, terms;
     uint32_t token_pairs;          // 256-token row pairs of the pair kernel's launch
+    uint32_t tail_columns;         // tokens past them, in steps of 32 (0: none), on tail tiles
+    uint32_t cost_main, cost_tail; // of a k block of a whole tile and of a tail tile, for the balance of the leftover tiles
     uint32_t padded_tokens;        // tokens rounded up to whole 128-row tiles: row stride of the staged activation planes
     float scale;                   // g_w * g_a
     float scale_b;                 // SwiGLU: g_w of the up rows * g_a
@@ -72,11 +74,9 @@ __device__ __forceinline__ void convert_chunk(const uint32_t (&v)[32], float sca
 // computation: no allocation and no device access.
 bool make_code_map(CUtensorMap* map, uint64_t address, uint64_t rows, uint32_t cols, uint32_t box_rows = 128);
 
-// The GEMM over the token rows from `token0` (a multiple of 128) on, for a range that is narrow next to the weights
-// (csrc/nvfp4_gemm_narrow.cu). `map_weight`: boxes of 128 rows. `p` describes the whole GEMM. With `after_main` the launch
-// before it on the stream is the pair kernel on the token rows before `token0`.
+// The GEMM for token counts that are narrow next to the weights (csrc/nvfp4_gemm_narrow.cu). `map_weight`: boxes of 128 rows.
 augur_cuda_result_v1 launch_gemm_narrow(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan, const CUtensorMap& map_weight,
-                                        uint64_t activation, const GemmParams& p, uint32_t token0, bool after_main);
+                                        uint64_t activation, const GemmParams& p);
 // About how long it takes.
 uint32_t gemm_narrow_ns(int32_t ordinal, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms);
 

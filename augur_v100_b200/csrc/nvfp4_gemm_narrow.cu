@@ -63,9 +63,8 @@ constexpr uint32_t kErrNarrowWeights = 0x111, kErrNarrowTokens = 0x112, kErrNarr
 
 struct NarrowParams {
     GemmParams g;
-    uint32_t token0, tile_tokens, token_tiles, columns;   // columns: MMA n, tile_tokens rounded up to 16
+    uint32_t tile_tokens, token_tiles, columns;   // columns: MMA n, tile_tokens rounded up to 16
     uint32_t parts;                                       // CTAs per item (the cluster size)
-    uint32_t after_main;
     uint32_t weight_depth, token_depth, slot_bytes;       // ring slots, size of an activation slot
     uint32_t sf_weight, sf_token;                         // first tensor-memory columns of either ring's scales
 };
@@ -142,8 +141,8 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
     volatile uint32_t* abort_flag = tmem_slot + 1;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    // Normally the next kernel of the stream may become resident from here on (it waits for this one's end before it reads).
-    if (!p.after_main) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // The next kernel of the stream may become resident from here on (it waits for this one's end before it reads).
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) {
         for (uint32_t b = 0; b < 6 * kNarrowMaxDepth + 1; ++b) mbar_init(bar0 + 8 * b, 1);
         *abort_flag = 0;
@@ -160,7 +159,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
     const uint32_t tmem_base = *tmem_slot;
 
     const uint32_t part = blockIdx.x % p.parts, item = blockIdx.x / p.parts;
-    const uint32_t row_tile = item / p.token_tiles, token_row = p.token0 + item % p.token_tiles * p.tile_tokens;
+    const uint32_t row_tile = item / p.token_tiles, token_row = item % p.token_tiles * p.tile_tokens;
     const uint32_t token_end = min(token_row + p.tile_tokens, g.tokens);
     const uint32_t k_blocks = (g.cols + kNarrowK - 1) / kNarrowK, atoms = g.cols / 64;      // scale atoms of a 128-row block along k
     const uint32_t kb0 = part * k_blocks / p.parts, kb1 = (part + 1) * k_blocks / p.parts;
@@ -200,14 +199,13 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
             __syncwarp();
             if (++stage == p.weight_depth) { stage = 0; phase ^= 1; }
             // the first wait for a stage to be free, which it is when the activations are there
-            if (kb == kb0 + 1 && !p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");
+            if (kb == kb0 + 1) asm volatile("griddepcontrol.wait;" ::: "memory");
             if (kb != kb0 && load_kb < kb1) alive = load();
         }
     } else if (warp == 2) {
         // ---------------- TMA of activations ----------------
-        // They come from the launch before this one; after the pair kernel on the other tokens, from the launch before that,
-        // which is complete since that kernel lets its successor start only once its own wait is over.
-        if (!p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");
+        // They come from the launch before this one.
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         uint32_t slot = 0, phase = 1;
         bool alive = true;
         const uint8_t* scales = g.act_sf + static_cast<uint64_t>(token_row / 128) * atoms * kSfAtomBytes;
@@ -234,7 +232,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (!p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         uint32_t stage = 0, w_phase = 0, slot = 0, t_phase = 0, accumulate = 0;
         bool alive = true;
         const uint32_t idesc = instr_desc(p.columns);
@@ -279,7 +277,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         // A slot lands after the MMAs that used it last are complete, so its scale columns are free. The copies only have to be
         // issued before the MMAs that read them: both execute in issue order, and the fences on either side of the arrival
         // order the two warps' issues. The codes landed on the same barrier, so the MMA warp waits for this arrival only.
-        if (!p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         uint32_t slot = 0, phase = 0;
         bool alive = true;
         const uint64_t desc0 = sf_desc(smem_u32(slots) + p.columns * 128);
@@ -309,7 +307,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
     const uint32_t row0 = row_tile * kTileM + quadrant * 32;
     bool complete = true;
     if (epilogue) {
-        if (!p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing is written while an earlier kernel may still read it
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing is written while an earlier kernel may still read it
         // suspended: sixteen polling warps per SM took 2 to 3 % of the launch from those that issue
         complete = warp_wait_suspended(acc_full, 0, abort_flag, g.status_word, kErrNarrowAccFull);
         tc_fence_after();
@@ -408,8 +406,6 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         }
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");     // and the others of this one
     }
-    // the successor's wait covers this launch only, so this launch ends after the one before it
-    if (p.after_main) asm volatile("griddepcontrol.wait;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -497,16 +493,14 @@ uint32_t gemm_narrow_ns(int32_t ordinal, uint32_t rows, uint32_t cols, uint32_t 
 }
 
 augur_cuda_result_v1 launch_gemm_narrow(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan, const CUtensorMap& map_weight,
-                                        uint64_t activation, const GemmParams& g, uint32_t token0, bool after_main) {
+                                        uint64_t activation, const GemmParams& g) {
     NarrowParams p{};
     p.g = g;
-    p.token0 = token0;
-    const NarrowCut cut = narrow_cut(plan->ordinal, g.rows, g.cols, g.tokens - token0, g.terms);
+    const NarrowCut cut = narrow_cut(plan->ordinal, g.rows, g.cols, g.tokens, g.terms);
     p.token_tiles = cut.token_tiles;
     p.tile_tokens = cut.tile_tokens;
     p.columns = cut.columns;
     p.parts = cut.parts;
-    p.after_main = after_main ? 1u : 0u;
     // Two k blocks of activations ahead, but not at the price of fewer than four weight stages; three slots at least.
     const uint32_t room = kNarrowSmem - 1024 /*alignment*/ - kNarrowState;
     p.slot_bytes = p.columns * 128 + kNarrowScales;

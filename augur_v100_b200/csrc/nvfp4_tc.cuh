@@ -382,21 +382,29 @@ __device__ __forceinline__ float group_divisor_fast(float maximum, const QuantSc
     return __fmul_rn(e4m3_value(code), s.global);
 }
 
+// The largest magnitude of a group, its divisor and scale code on the fast path, and whether it may take that path.
+__device__ __forceinline__ bool group_is_fast(const float2 (&residual)[8], const QuantScale& s, float* largest, float* divisor_out, uint32_t* scale_code_out) {
+    // This maximum carries a NaN along, which keeps the group off the fast path; the reference's maximum
+    // leaves NaNs out, and only the other path computes it.
+    float maximum = 0.0f;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) maximum = max_or_nan(maximum, fabsf(residual[i].x), fabsf(residual[i].y));
+    const float divisor = group_divisor_fast(maximum, s, scale_code_out);
+    const uint32_t divisor_field = (__float_as_uint(divisor) >> 23) & 0xffu, largest_field = (__float_as_uint(maximum) >> 23) & 0xffu;
+    *largest = maximum;
+    *divisor_out = divisor;
+    return divisor_field >= 64u && divisor_field <= 190u && (__float_as_uint(divisor) & 0x7fffffu) != 0x7fffffu &&
+           largest_field >= 64u && largest_field <= 190u && s.six_reciprocal != 0.0f;
+}
+
 // One residual term of one 16-element group: the block scale, the 16 codes (nearest level of x / (scale * g),
 // ties toward zero) and, if another term follows, the residual it quantises.
 // `kMoreTerms` is a compile-time choice: the last term of a group needs neither the levels nor the residual.
 template <bool kMoreTerms>
 __device__ __forceinline__ void quantise_term_as(float2 (&residual)[8], const QuantScale& s, uint32_t (&packed)[2],
                                                  uint32_t* scale_code_out) {
-    // This maximum carries a NaN along, which keeps the group off the fast path; the reference's maximum
-    // leaves NaNs out, and only the other path computes it.
-    float maximum = 0.0f;
-#pragma unroll
-    for (uint32_t i = 0; i < 8; ++i) maximum = max_or_nan(maximum, fabsf(residual[i].x), fabsf(residual[i].y));
-    float divisor = group_divisor_fast(maximum, s, scale_code_out);
-    const uint32_t divisor_field = (__float_as_uint(divisor) >> 23) & 0xffu, largest_field = (__float_as_uint(maximum) >> 23) & 0xffu;
-    const bool fast = divisor_field >= 64u && divisor_field <= 190u && (__float_as_uint(divisor) & 0x7fffffu) != 0x7fffffu &&
-                      largest_field >= 64u && largest_field <= 190u && s.six_reciprocal != 0.0f;
+    float maximum, divisor;
+    const bool fast = group_is_fast(residual, s, &maximum, &divisor, scale_code_out);
     packed[0] = packed[1] = 0;
     if (fast) {
         quantise_group_fast<kMoreTerms>(residual, divisor, __frcp_rn(divisor), packed);
@@ -406,6 +414,25 @@ __device__ __forceinline__ void quantise_term_as(float2 (&residual)[8], const Qu
         for (uint32_t i = 0; i < 8; ++i) maximum = fmaxf(maximum, fmaxf(fabsf(residual[i].x), fabsf(residual[i].y)));
         divisor = group_divisor(maximum, s.global, scale_code_out);
         quantise_group_any<kMoreTerms>(residual, divisor, packed);
+    }
+}
+// Several groups of one lane, in one run of instructions where all of them take the fast path.
+template <bool kMoreTerms, uint32_t kGroups>
+__device__ __forceinline__ void quantise_groups_as(float2 (&residual)[kGroups][8], const QuantScale& s, uint32_t (&packed)[kGroups][2],
+                                                   uint32_t (&scale_code)[kGroups]) {
+    float divisor[kGroups];
+    bool fast = true;
+#pragma unroll
+    for (uint32_t g = 0; g < kGroups; ++g) {
+        float maximum;
+        fast = group_is_fast(residual[g], s, &maximum, &divisor[g], &scale_code[g]) && fast;
+    }
+    if (fast) {
+#pragma unroll
+        for (uint32_t g = 0; g < kGroups; ++g) quantise_group_fast<kMoreTerms>(residual[g], divisor[g], __frcp_rn(divisor[g]), packed[g]);
+    } else {
+#pragma unroll
+        for (uint32_t g = 0; g < kGroups; ++g) quantise_term_as<kMoreTerms>(residual[g], s, packed[g], &scale_code[g]);
     }
 }
 __device__ __forceinline__ void quantise_term(float2 (&residual)[8], const QuantScale& s, bool more_terms, uint32_t (&packed)[2],
