@@ -23,8 +23,9 @@
 //
 // Roles: warp 0 TMA and scale copies of the weights, 1 MMA, 2 TMA of the activations, 3 their scale copies to tensor memory,
 // 4..11 epilogue. What a step costs beyond its bytes is the time its warps take to issue it: each waits on as few barriers
-// as possible, its MMAs are one block of predicated instructions (tc_step; 15.3 -> 14.7 us at 6144 x 5120, 48 tokens, three terms), its copies unrolled. (One thread copying all
-// scales in a loop took 980 cycles per step.)
+// as possible, and what it issues is one block of predicated instructions (tc_step, tc_copy_step, tma_step), one instantiation per number of
+// terms: 9 tokens, three terms, quantiser included, 34816 x 5120 27.3 -> 24.0 us, 17408 x 5120 18.5 -> 16.8, 5120 x 17408 20.3 -> 18.5; 6144 x 5120 at 48
+// 14.15 -> 13.7. From 96 tokens on nothing changed: there the bytes into shared memory are the bound, 24 KB a step and CTA, 80 a ns and SM.
 // Every wait is bounded; a wait that runs out records a code in the plan's status word, raises a CTA-wide abort flag, and
 // all roles fall through to the common exits. What a role waits for on a barrier never includes the launch before: a role that
 // depends on it waits for its end first, so that its time does not count against the bound.
@@ -102,16 +103,6 @@ __device__ __forceinline__ void narrow_store(const GemmParams& g, uint32_t token
     }
 }
 
-// The scale atoms of up to four k steps (four tensor-memory columns each).
-__device__ __forceinline__ void narrow_copy_scales(uint32_t columns, uint64_t desc, uint32_t k_steps) {
-    if (k_steps == 4) {
-#pragma unroll
-        for (uint32_t k = 0; k < 4; ++k) tc_copy_sf(columns + 4 * k, desc + k * (kSfAtomBytes >> 4));
-    } else {
-        for (uint32_t k = 0; k < k_steps; ++k) tc_copy_sf(columns + 4 * k, desc + k * (kSfAtomBytes >> 4));
-    }
-}
-
 // 16 bytes at this offset of another CTA's shared memory.
 __device__ __forceinline__ float4 narrow_read_cluster(uint32_t offset, uint32_t cta) {
     uint32_t at;
@@ -125,6 +116,7 @@ __device__ __forceinline__ void narrow_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+template <uint32_t kTerms>
 __global__ void __launch_bounds__(kNarrowBound, 2)
 gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_constant__ CUtensorMap map_act, const NarrowParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -174,14 +166,9 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         uint32_t load_kb = kb0, load_stage = 0, load_phase = 1, stage = 0, phase = 0;
         auto load = [&]() {
             if (!warp_look_wait(w_empty + 8 * load_stage, load_phase, abort_flag, g.status_word, kErrNarrowWeights)) return false;
-            const uint32_t full = w_full + 8 * load_stage, to = smem_u32(smem + load_stage * kNarrowStage);
-            const uint32_t sf_bytes = (load_kb + 1 < k_blocks ? 4u : last_k_steps) * kSfAtomBytes;
-            if (elect_one()) {
-                mbar_expect_tx(full, kNarrowCodes + sf_bytes);
-                tma_load_2d(to, &map_weight, load_kb * 128, row_tile * kTileM, full);
-                bulk_load(to + kNarrowCodes, scales + static_cast<uint64_t>(load_kb) * kNarrowScales, sf_bytes, full);
-            }
-            __syncwarp();
+            const uint32_t to = smem_u32(smem + load_stage * kNarrowStage), sf_bytes = (load_kb + 1 < k_blocks ? 4u : last_k_steps) * kSfAtomBytes;
+            tma_step(w_full + 8 * load_stage, kNarrowCodes + sf_bytes, to, &map_weight, load_kb * 128, row_tile * kTileM, to + kNarrowCodes,
+                     scales + static_cast<uint64_t>(load_kb) * kNarrowScales, sf_bytes);
             ++load_kb;
             if (++load_stage == p.weight_depth) { load_stage = 0; load_phase ^= 1; }
             return true;
@@ -190,13 +177,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         while (alive && load_kb < kb1 && load_kb < kb0 + p.weight_depth) alive = load();
         for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
             if (!warp_look_wait(w_full + 8 * stage, phase, abort_flag, g.status_word, kErrNarrowCopy)) break;
-            tc_fence_after();
-            if (elect_one()) {
-                narrow_copy_scales(tmem_base + p.sf_weight + stage * 16, desc0 + stage * (kNarrowStage >> 4), kb + 1 < k_blocks ? 4u : last_k_steps);
-                tc_fence_before();
-                mbar_arrive(w_ready + 8 * stage);
-            }
-            __syncwarp();
+            tc_copy_step(tmem_base + p.sf_weight + stage * 16, desc0 + stage * (kNarrowStage >> 4), w_ready + 8 * stage);
             if (++stage == p.weight_depth) { stage = 0; phase ^= 1; }
             // the first wait for a stage to be free, which it is when the activations are there
             if (kb == kb0 + 1) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -212,21 +193,15 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
             const uint32_t sf_bytes = (kb + 1 < k_blocks ? 4u : last_k_steps) * kSfAtomBytes;
             const uint8_t* from = scales + static_cast<uint64_t>(kb) * kNarrowScales;
-            uint32_t row = token_row;
-            for (uint32_t term = 0; term < g.terms; ++term) {
+#pragma unroll
+            for (uint32_t term = 0; term < kTerms; ++term) {
                 if (!warp_look_wait(t_empty + 8 * slot, phase, abort_flag, g.status_word, kErrNarrowTokens)) {
                     alive = false;
                     break;
                 }
-                const uint32_t to = smem_u32(slots + slot * p.slot_bytes), full = t_full + 8 * slot;
-                if (elect_one()) {
-                    mbar_expect_tx(full, p.columns * 128 + sf_bytes);
-                    tma_load_2d(to, &map_act, kb * 128, row, full);
-                    bulk_load(to + p.columns * 128, from, sf_bytes, full);
-                }
-                __syncwarp();
-                from += g.act_term_stride;
-                row += g.padded_tokens;
+                const uint32_t to = smem_u32(slots + slot * p.slot_bytes);
+                tma_step(t_full + 8 * slot, p.columns * 128 + sf_bytes, to, &map_act, kb * 128, token_row + term * g.padded_tokens, to + p.columns * 128,
+                         from + term * g.act_term_stride, sf_bytes);
                 if (++slot == p.token_depth) { slot = 0; phase ^= 1; }
             }
         }
@@ -236,37 +211,25 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         uint32_t stage = 0, w_phase = 0, slot = 0, t_phase = 0, accumulate = 0;
         bool alive = true;
         const uint32_t idesc = instr_desc(p.columns);
-        const uint64_t w_desc0 = operand_desc(smem_u32(smem)), t_desc0 = operand_desc(smem_u32(slots));
+        const uint32_t w_desc0 = static_cast<uint32_t>(operand_desc(smem_u32(smem))), t_desc0 = static_cast<uint32_t>(operand_desc(smem_u32(slots)));
         const uint32_t slot_step = p.slot_bytes >> 4;
-        // Looking at a barrier takes as long as issuing an MMA or two, so the barriers of the next step are looked at before the
-        // MMAs of this one are issued, and waited for only if they were not there.
-        bool w_seen = false, t_seen = false;
         for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
-            if (!w_seen && !warp_look_wait(w_ready + 8 * stage, w_phase, abort_flag, g.status_word, kErrNarrowFull)) break;
-            const uint32_t k_steps = kb + 1 < k_blocks ? 4u : last_k_steps;
-            const uint64_t w_desc = w_desc0 + stage * (kNarrowStage >> 4);
+            if (!warp_look_wait(w_ready + 8 * stage, w_phase, abort_flag, g.status_word, kErrNarrowFull)) {
+                alive = false;
+                break;
+            }
+            const uint32_t k_steps = kb + 1 < k_blocks ? 4u : last_k_steps, w_desc = w_desc0 + stage * (kNarrowStage >> 4);
             const uint32_t sf_w = tmem_base + p.sf_weight + stage * 16, w_done = w_empty + 8 * stage;
             if (++stage == p.weight_depth) { stage = 0; w_phase ^= 1; }
-            for (uint32_t term = 0; term < g.terms; ++term) {
-                if (!t_seen && !warp_look_wait(t_ready + 8 * slot, t_phase, abort_flag, g.status_word, kErrNarrowScales)) {
+#pragma unroll
+            for (uint32_t term = 0; term < kTerms; ++term) {
+                if (!warp_look_wait(t_ready + 8 * slot, t_phase, abort_flag, g.status_word, kErrNarrowScales)) {
                     alive = false;
                     break;
                 }
-                tc_fence_after();
-                const uint64_t t_desc = t_desc0 + slot * slot_step;
-                const uint32_t sf_t = tmem_base + p.sf_token + slot * 16, t_done = t_empty + 8 * slot;
+                tc_step(tmem_base, w_desc, t_desc0 + slot * slot_step, idesc, sf_w, tmem_base + p.sf_token + slot * 16, accumulate, k_steps, t_empty + 8 * slot,
+                        term + 1 == kTerms ? 1u : 0u, w_done);
                 if (++slot == p.token_depth) { slot = 0; t_phase ^= 1; }
-                t_seen = mbar_test(t_ready + 8 * slot, t_phase);
-                if (term + 1 == g.terms) w_seen = mbar_test(w_ready + 8 * stage, w_phase);
-                const uint32_t last_term = term + 1 == g.terms ? 1u : 0u;
-                if (k_steps == 4) {
-                    tc_step(tmem_base, w_desc, t_desc, idesc, sf_w, sf_t, accumulate, t_done, last_term, w_done);
-                } else if (elect_one()) {
-                    for (uint32_t k = 0; k < k_steps; ++k) tc_mma(tmem_base, w_desc + 2 * k, t_desc + 2 * k, idesc, sf_w + 4 * k, sf_t + 4 * k, accumulate | k);
-                    tc_commit(t_done);
-                    if (last_term) tc_commit(w_done);
-                }
-                __syncwarp();
                 accumulate = 1;
             }
         }
@@ -274,30 +237,16 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
         __syncwarp();
     } else if (warp == 3) {
         // ---------------- scale copies of the activations, shared memory -> tensor memory ----------------
-        // A slot lands after the MMAs that used it last are complete, so its scale columns are free. The copies only have to be
-        // issued before the MMAs that read them: both execute in issue order, and the fences on either side of the arrival
-        // order the two warps' issues. The codes landed on the same barrier, so the MMA warp waits for this arrival only.
+        // A slot lands after the MMAs that used it last are complete, so its scale columns are free. The codes landed on the same
+        // barrier, so the MMA warp waits for the copies only.
         asm volatile("griddepcontrol.wait;" ::: "memory");
         uint32_t slot = 0, phase = 0;
-        bool alive = true;
         const uint64_t desc0 = sf_desc(smem_u32(slots) + p.columns * 128);
         const uint32_t slot_step = p.slot_bytes >> 4;
-        for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
-            const uint32_t k_steps = kb + 1 < k_blocks ? 4u : last_k_steps;
-            for (uint32_t term = 0; term < g.terms; ++term) {
-                if (!warp_look_wait(t_full + 8 * slot, phase, abort_flag, g.status_word, kErrNarrowCopy)) {
-                    alive = false;
-                    break;
-                }
-                tc_fence_after();
-                if (elect_one()) {
-                    narrow_copy_scales(tmem_base + p.sf_token + slot * 16, desc0 + slot * slot_step, k_steps);
-                    tc_fence_before();
-                    mbar_arrive(t_ready + 8 * slot);
-                }
-                __syncwarp();
-                if (++slot == p.token_depth) { slot = 0; phase ^= 1; }
-            }
+        for (uint32_t left = (kb1 - kb0) * kTerms; left; --left) {
+            if (!warp_look_wait(t_full + 8 * slot, phase, abort_flag, g.status_word, kErrNarrowCopy)) break;
+            tc_copy_step(tmem_base + p.sf_token + slot * 16, desc0 + slot * slot_step, t_ready + 8 * slot);
+            if (++slot == p.token_depth) { slot = 0; phase ^= 1; }
         }
     }
 
@@ -415,6 +364,9 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid_
 }
 
 // ---- host side ----------------------------------------------------------------------------------
+using NarrowKernel = void (*)(CUtensorMap, CUtensorMap, NarrowParams);
+constexpr NarrowKernel kNarrowKernels[3] = {gemm_narrow_kernel<1>, gemm_narrow_kernel<2>, gemm_narrow_kernel<3>};
+
 // Clusters of `parts` CTAs that a launch may count on to run at once. The device holds 148 of 2, 93 of 3, 71 of 4, 56 of 5, 45 of
 // 6, 37 of 7 and 33 of 8 on a B200 (they do not fill its SMs evenly); of those larger than 2 a sixteenth is left out, because they
 // come to lie badly while the launch before still has CTAs of its own on the SMs, and a cluster that finds no place then waits for
@@ -530,13 +482,16 @@ augur_cuda_result_v1 launch_gemm_narrow(augur_cuda_stream_t s, const augur_cuda_
     config.gridDim = dim3(g.rows / kTileM * p.token_tiles * p.parts);
     config.blockDim = dim3(kNarrowThreads);
     config.dynamicSmemBytes = kNarrowSmem;
-    cudaLaunchKernelEx(&config, gemm_narrow_kernel, map_weight, map_act, p);
+    cudaLaunchKernelEx(&config, kNarrowKernels[g.terms - 1], map_weight, map_act, p);
     count_launch();
     return submitted();
 }
 
 cudaError_t gemm_narrow_configure_device() {
-    cudaError_t e = cudaFuncSetAttribute(gemm_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNarrowSmem);
+    cudaError_t e = cudaSuccess;
+    for (NarrowKernel kernel : kNarrowKernels) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNarrowSmem);
+    }
     if (e == cudaSuccess) e = cudaFuncSetAttribute(narrow_shape_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNarrowSmem);
     int ordinal = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&ordinal);

@@ -592,15 +592,8 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             const uint32_t k_steps = min(kStageK, p.phase[p.step[c.step].phase].cols - c.kb * kStageK) / 64;
             const uint32_t accumulate = c.kb != c.kb0 ? 1u : 0u, last = c.kb + 1 == c.kb1 ? 1u : 0u;
             // each MMA consumes 64 k = 32 bytes of every row; the commits free the stage and, behind an item's last k block, hand the accumulator over
-            if (k_steps == 4) {
-                tc_step(acc, weight_desc, act_desc, idesc, tmem_sf_weight, tmem_sf_act, accumulate, bar_empty + 8 * stage, last, bar_acc_full + 8 * buffer);
-            } else if (elect_one()) {
-                for (uint32_t k = 0; k < k_steps; ++k) {
-                    tc_mma(acc, weight_desc + 2 * k, act_desc + 2 * k, idesc, tmem_sf_weight + 4 * k, tmem_sf_act + 4 * k, accumulate | k);
-                }
-                tc_commit(bar_empty + 8 * stage);
-                if (last) tc_commit(bar_acc_full + 8 * buffer);
-            }
+            tc_step(acc, static_cast<uint32_t>(weight_desc), static_cast<uint32_t>(act_desc), idesc, tmem_sf_weight, tmem_sf_act, accumulate, k_steps,
+                    bar_empty + 8 * stage, last, bar_acc_full + 8 * buffer);
             __syncwarp();
             if (last) {
                 acc_phase[buffer] ^= 1;

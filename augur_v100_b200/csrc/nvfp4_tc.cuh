@@ -157,26 +157,54 @@ __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint3
         ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
         : "memory");
 }
-// One pipeline step of a converged warp: the four MMAs of a 256-deep k block (64 k each: 32 bytes further in every operand row, four
-// scale columns further) and the commits that free what they read, `done` and, where `also` is not zero, `also_done`. The elected
+// One pipeline step of a converged warp: the one to four MMAs of a k block (64 k each: 32 bytes further in every operand row, four
+// scale columns further) and the commits that free what they read, `done` and, where `also` is not zero, `also_done`. `a` and `b` are the low
+// words of operand descriptors, whose high words are all alike. The elected
 // lane is a predicate on the instructions, not a branch: the warp does not diverge, and the operands of all six are formed once
 // in uniform registers. Written as a branch around six separate instructions a step takes 400 cycles to issue, whatever its n. Its MMAs
 // occupy the pipe for 156 cycles at n = 16, 176 at 48 and 256 at 128, twice that for the two CTAs of an SM: so issue was the bound of
 // small n, and what is gained at 128 is little.
-__device__ __forceinline__ void tc_step(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t accumulate,
+__device__ __forceinline__ void tc_step(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb, uint32_t accumulate, uint32_t k_steps,
                                         uint32_t done, uint32_t also, uint32_t also_done) {
+    constexpr uint32_t kHigh = (1024 >> 4) | (1u << 14) | (2u << 29);
     asm volatile(
-        "{\n.reg .pred e, f, p, q;\n.reg .b64 a1, a2, a3, b1, b2, b3;\n.reg .b32 s1, s2, s3, t1, t2, t3;\n"
-        "elect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, %6, 0;\nsetp.eq.u32 q, 0, 0;\nsetp.ne.and.b32 f, %8, 0, e;\n"
-        "add.s64 a1, %1, 2;\nadd.s64 a2, %1, 4;\nadd.s64 a3, %1, 6;\nadd.s64 b1, %2, 2;\nadd.s64 b2, %2, 4;\nadd.s64 b3, %2, 6;\n"
+        "{\n.reg .pred e, f, p, q, e1, e2, e3;\n.reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n.reg .b32 l1, l2, l3, m1, m2, m3, s1, s2, s3, t1, t2, t3;\n"
+        "tcgen05.fence::after_thread_sync;\nelect.sync _|e, 0xffffffff;\nsetp.ne.b32 p, %6, 0;\nsetp.eq.u32 q, 0, 0;\nsetp.ne.and.b32 f, %9, 0, e;\n"
+        "setp.gt.and.u32 e1, %7, 1, e;\nsetp.gt.and.u32 e2, %7, 2, e;\nsetp.gt.and.u32 e3, %7, 3, e;\n"
+        "add.s32 l1, %1, 2;\nadd.s32 l2, %1, 4;\nadd.s32 l3, %1, 6;\nadd.s32 m1, %2, 2;\nadd.s32 m2, %2, 4;\nadd.s32 m3, %2, 6;\n"
+        "mov.b64 a0, {%1, %11};\nmov.b64 a1, {l1, %11};\nmov.b64 a2, {l2, %11};\nmov.b64 a3, {l3, %11};\n"
+        "mov.b64 b0, {%2, %11};\nmov.b64 b1, {m1, %11};\nmov.b64 b2, {m2, %11};\nmov.b64 b3, {m3, %11};\n"
         "add.s32 s1, %4, 4;\nadd.s32 s2, %4, 8;\nadd.s32 s3, %4, 12;\nadd.s32 t1, %5, 4;\nadd.s32 t2, %5, 8;\nadd.s32 t3, %5, 12;\n"
-        "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n"
-        "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a1, b1, %3, [s1], [t1], q;\n"
-        "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a2, b2, %3, [s2], [t2], q;\n"
-        "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a3, b3, %3, [s3], [t3], q;\n"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n"
-        "@f tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%9];\n}"
-        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "r"(done), "r"(also), "r"(also_done)
+        "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a0, b0, %3, [%4], [%5], p;\n"
+        "@e1 tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a1, b1, %3, [s1], [t1], q;\n"
+        "@e2 tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a2, b2, %3, [s2], [t2], q;\n"
+        "@e3 tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], a3, b3, %3, [s3], [t3], q;\n"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%8];\n"
+        "@f tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%10];\n}"
+        ::"r"(d), "r"(a), "r"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "r"(k_steps), "r"(done), "r"(also), "r"(also_done), "r"(kHigh)
+        : "memory");
+}
+// The scale atoms of a slot (four k steps, four tensor-memory columns each) on their way to tensor memory, in the same way, and the commit that
+// says when they are there. (A plain arrival behind the copies, on the strength of copies and later MMAs executing in the order of their issue,
+// let MMAs of another warp see the last copy's columns before it in some launches, once steps were short.)
+__device__ __forceinline__ void tc_copy_step(uint32_t columns, uint64_t desc, uint32_t ready) {
+    asm volatile(
+        "{\n.reg .pred e;\n.reg .b64 a1, a2, a3;\n.reg .b32 c1, c2, c3;\ntcgen05.fence::after_thread_sync;\nelect.sync _|e, 0xffffffff;\n"
+        "add.s64 a1, %1, 32;\nadd.s64 a2, %1, 64;\nadd.s64 a3, %1, 96;\nadd.s32 c1, %0, 4;\nadd.s32 c2, %0, 8;\nadd.s32 c3, %0, 12;\n"
+        "@e tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n@e tcgen05.cp.cta_group::1.32x128b.warpx4 [c1], a1;\n"
+        "@e tcgen05.cp.cta_group::1.32x128b.warpx4 [c2], a2;\n@e tcgen05.cp.cta_group::1.32x128b.warpx4 [c3], a3;\n"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%2];\n}"
+        ::"r"(columns), "l"(desc), "r"(ready)
+        : "memory");
+}
+// A slot's loads, likewise: operand rows by TMA and `scale_bytes` of block scales, `bytes` in all on the barrier `full`.
+__device__ __forceinline__ void tma_step(uint32_t full, uint32_t bytes, uint32_t codes, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t scales,
+                                         const void* scales_from, uint32_t scale_bytes) {
+    asm volatile(
+        "{\n.reg .pred e;\nelect.sync _|e, 0xffffffff;\n@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
+        "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%2], [%3, {%4, %5}], [%0];\n"
+        "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%6], [%7], %8, [%0];\n}"
+        ::"r"(full), "r"(bytes), "r"(codes), "l"(map), "r"(x), "r"(y), "r"(scales), "l"(scales_from), "r"(scale_bytes)
         : "memory");
 }
 __device__ __forceinline__ void tc_load32(uint32_t taddr, uint32_t (&v)[32]) {
