@@ -22,7 +22,7 @@
 // there are at least about as many as CTAs, else every tile cut along k into equal
 // parts whose partial sums meet in plan scratch (arrival counter per 32 rows; the last arriver adds the parts in
 // a fixed order and finishes the rows; bit-reproducible). (A single linear as a program of one step took 17.3 us for
-// 17408 x 5120 at 8 tokens and 12.7 for 5120 x 5120; its two launches, which have no meeting, take 14.8 and 9.6.) The block is
+// 17408 x 5120 at 8 tokens and 12.7 for 5120 x 5120; nvfp4_gemv_split.cu, which has no meeting of all CTAs, takes 14.2 and 8.9.) The block is
 // two steps when the gate|up tiles fit the CTAs: gate|up in whole tiles, then down in k parts. The second product needs every CTA's
 // outputs of the first and their largest magnitudes per token row before it can split them: the CTAs arrive at
 // a counter when their outputs are stored, wait for all, split, arrive at a second counter, and the activation

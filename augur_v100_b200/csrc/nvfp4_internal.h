@@ -159,7 +159,8 @@ uint32_t two_cta_clusters(int32_t ordinal, uint32_t parts);
 // CTAs per 128-row tile of a small-token linear on tensor memory (a cluster) where `clusters[parts]` clusters of `parts` run at once.
 constexpr uint32_t kSplitMaxParts = 8;
 uint32_t split_linear_parts(uint32_t tiles, uint32_t k_blocks, const uint32_t (&clusters)[kSplitMaxParts + 1]);
-// The linear as two launches (nvfp4_gemv_split.cu); `split`: split_bytes(cols) of plan scratch.
+// The linear of 1..8 token rows on tensor memory (nvfp4_gemv_split.cu); `split`: split_bytes(cols) of plan scratch, where digits that a launch of
+// their own forms pass through.
 augur_cuda_result_v1 launch_split_linear(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
                                          const augur_cuda_nvfp4_sm100_gemv_args_v1* a, uint32_t physical_rows, uint8_t* split);
 // Two-CTA clusters of the pair GEMM that the device can hold at once (0 if the query fails).
