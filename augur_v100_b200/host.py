@@ -715,8 +715,8 @@ class Nvfp4Sm100Linear:
     """One weight matrix, any number of token rows: the dispatch a model runtime does per call site.
 
     Keeps the weight in both hot layouts (the small-token stream layout and the tcgen05 layout) and
-    binds the kernel its shape class calls for: tokens <= 8 -> `Nvfp4Sm100Projection`, or for the larger
-    weights `Nvfp4Sm100TcProjection`, otherwise `Nvfp4Sm100PrefillLinear` (activation quantiser with `terms`
+    binds the kernel its shape class calls for: tokens <= 8 -> `Nvfp4Sm100Projection`, or where it is the
+    quicker `Nvfp4Sm100TcProjection`, otherwise `Nvfp4Sm100PrefillLinear` (activation quantiser with `terms`
     residual terms, then the block-scaled GEMM). Bindings are made per (input, output) pair, exactly like the
     classes it chooses between.
 
@@ -741,6 +741,18 @@ class Nvfp4Sm100Linear:
             return False
         return self.rows >= (2560 if tokens <= 4 else 4096) and plan.snapshot().scratch_len_bytes >= gemv_tc_linear_scratch_bytes(self.cols)
 
+    def _on_tensor_memory_below(self, plan: Plan, tokens: int) -> bool:
+        """Most of what lies below that line is quicker there too, since the kernel forms the digits of its input itself and takes one launch. A tile
+        of 128 rows has eight CTAs at most, which bounds k next to the rows, the more so the more token rows there are; and beyond 32768 rows the
+        tiles no longer fit at once. B200, us on tensor memory / mma.sync at 1, 4, 5 and 8 token rows: 1024 x 2048 4.4 / 4.6, 4.6 / 5.0, 4.6 / 5.2, 4.8 / 5.4;
+        1024 x 5120 4.9 / 5.7, 5.7 / 5.9, 5.8 / 6.1, 6.6 / 6.2; 1024 x 17408 7.8 / 8.0, 8.5 / 8.7, 9.4 / 8.8, 9.9 / 9.2; 1536 x 8192 5.6 / 7.0, 6.4 / 7.6,
+        6.9 / 7.7, 8.0 / 7.8; 2048 x 5120 5.3 / 6.8, 6.1 / 7.0, 6.5 / 7.2, 7.3 / 7.3; 4096 x 4096 5.5 / 6.8, 6.3 / 7.5, 6.8 / 7.7, 7.5 / 7.9; 128 x 17408 7.0 / 5.6,
+        7.5 / 6.0, 8.2 / 6.2, 8.6 / 6.3; 49920 x 256 7.3 / 6.7, 7.6 / 7.0, 7.6 / 7.2, 7.9 / 7.1."""
+        if self.rows % 128 != 0 or self.rows > 32768:
+            return False
+        most = 32 if tokens <= 4 else 8 if tokens == 5 or self.rows >= 2048 else 4
+        return self.cols <= most * self.rows and plan.snapshot().scratch_len_bytes >= gemv_tc_linear_scratch_bytes(self.cols)
+
     def __init__(self, stream: Stream, rows: int, cols: int, codes, scales, global_scale: float):
         self.rows, self.cols = rows, cols
         self.small = Nvfp4Sm100Weight.upload_checkpoint_nvfp4(stream, abi.LAYOUT_STREAM, rows, cols, codes, scales, global_scale)
@@ -749,7 +761,7 @@ class Nvfp4Sm100Linear:
     def bind(self, plan: Plan, x: torch.Tensor, out: torch.Tensor | None = None, terms: int = 3,
              activation_global_scale: float = 2.0 ** -8):
         if classify_tokens(x.shape[0]) == SHAPE_SMALL_BATCH:
-            if self._on_tensor_memory(plan, x.shape[0]):
+            if self._on_tensor_memory(plan, x.shape[0]) or self._on_tensor_memory_below(plan, x.shape[0]):
                 return Nvfp4Sm100TcProjection.bind(plan, self.wide, x, out)
             return Nvfp4Sm100Projection.bind(plan, self.small, x, out)
         return Nvfp4Sm100PrefillLinear.bind(plan, self.wide, x, out, terms=terms, activation_global_scale=activation_global_scale)
