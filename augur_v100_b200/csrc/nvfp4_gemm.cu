@@ -1049,18 +1049,14 @@ struct PairSplit {
     uint32_t ns;
 };
 
-// Fitted on a B200 to the kernel with one ring: a pipeline step (k block x term) of a pair 0.36 us, a launch 8 us beyond its steps; handing
-// the parts of leftover tiles over the time of 16 steps and two more per part when nothing else is left to do, and about 8 when it
-// happens under whole tiles. With the two rings a step takes 0.33 us at three terms, 0.37 to 0.43 at two and 0.46 to 0.50 at one, where
-// the weights of a k block come with every step (one tile per pair, 18944 rows, 256 tokens, 10 to 40 k blocks), a launch 9 to 11 us beyond.
-// The choice that these constants make is 0.7 % off the best on average, and 27 % where the two kernels are estimated alike: 10240 x
-// 5120, two terms, 300 tokens 38 us, narrow 32.
-constexpr uint32_t kPairStepCost = 36, kPairLaunchNs = 8000;   // a step in units of 10 ns
-constexpr uint32_t kSplitSteps = 16, kSplitPartSteps = 2, kSplitCoveredSteps = 8;
-
-// What a k block of a tile costs: a main tile's (`tail_columns` 0) or a tail tile's.
+// In units of 10 ns, fitted on a B200 to 429 GEMMs (eleven weights from 1024 x 5120 to 34816 x 5120, 13 token counts from 48 to 1100, one to three terms),
+// each with every choice forced in turn: what a k block of a whole tile costs and of a tail tile, handing the parts of leftover tiles over when nothing
+// else is left to do (and per part) and when it happens under whole tiles, a launch beyond that. With the narrow kernel's estimate (gemm_narrow_ns) the
+// choice is 0.1 % off the best on average, 14 % at worst (2432 x 2176, 160 to 256 tokens, one term, 9.0 against 10.2 us).
+constexpr uint32_t kPairBlockCost[3] = {52, 93, 118};
+constexpr uint32_t kSplitCost = 450, kSplitPartCost = 170, kSplitCoveredCost = 480, kPairLaunchNs = 5500;
 uint32_t pair_block_cost(uint32_t terms, uint32_t tail_columns) {
-    return tail_columns ? 34 + terms * 10 + terms * (tail_columns - 32) / 20 : 22 + terms * 28;
+    return tail_columns ? 30 + terms * 9 + terms * (tail_columns - 32) * 7 / 100 : kPairBlockCost[terms - 1];
 }
 
 // Tiles past the last full round of the pairs (all tiles, when there are fewer tiles than pairs) may be cut along k, in `ways`
@@ -1084,7 +1080,7 @@ PairSplit pair_split(uint32_t token_pairs, uint32_t tail_columns, uint32_t rows,
         if (sharers < 2 || (!tail && sharers <= left) || scratch_bytes < kCounterBytes + sharers * kSplitSlotBytes) break;
         const uint64_t parts = (sharers * k_blocks * largest + line - 1) / line;
         const uint64_t cost = k_blocks * rounds * cost_main + (line + sharers - 1) / sharers +
-                              (rounds ? kSplitCoveredSteps : kSplitSteps + kSplitPartSteps * parts) * kPairStepCost;
+                              (rounds ? kSplitCoveredCost : kSplitCost + kSplitPartCost * parts);
         if (cost < least) {
             least = cost;
             best.sharers = static_cast<uint32_t>(sharers);

@@ -435,7 +435,11 @@ NarrowCut narrow_cut(int32_t ordinal, uint32_t rows, uint32_t cols, uint32_t tok
             cut.parts = parts;
         }
     }
-    cut.ns = static_cast<uint32_t>(least < UINT32_MAX / 2 ? least : UINT32_MAX / 2);
+    // Against the pair kernel the estimate counts, not only the order: fitted as kPairBlockCost.
+    const uint32_t clusters = two_cta_clusters(ordinal, cut.parts);
+    const uint64_t ns = (items + clusters - 1) / clusters * ((k_blocks + cut.parts - 1) / cut.parts * (terms * (350 + cut.columns) + 110) + 2900) + 2100 +
+                        cut.columns * 4000 / kTileM;
+    cut.ns = static_cast<uint32_t>(ns < UINT32_MAX / 2 ? ns : UINT32_MAX / 2);
     return cut;
 }
 }  // namespace
