@@ -490,7 +490,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         // (below) into the slots' scale columns, this one issues only the MMAs. Descriptors advance by additions (their low
         // bits hold address >> 4). Looking at a barrier takes as long as issuing an MMA or two, so those of the next
         // step are looked at before the MMAs of this one are issued, and waited for only if they were not there.
-        uint32_t w_stage = 0, w_phase = 0, slot = 0, t_phase = 0, tmem_phase = 0;
+        uint32_t w_stage = 0, w_phase = 0, slot = 0, t_phase = 0, tmem_phase = 0, behind = 0, behind_phase = 0, ahead_steps = 0;
         bool alive = true;
         constexpr uint32_t kWideTile = (1u << 7) | (1u << 10) | ((kTileN >> 3) << 17) | (((2 * kTileM) >> 4) << 24);
         constexpr uint32_t kHalfTile = (1u << 7) | (1u << 10) | ((kTileN / 2 >> 3) << 17) | (((2 * kTileM) >> 4) << 24);
@@ -515,6 +515,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
                     for (uint32_t term = 0; term < kTerms; ++term) {
                         // codes in shared memory (TMA) and block scales on their way to tensor memory (copy warp)
                         if (!pair_wait(t_full + 8 * slot, t_phase, abort_flag, p.status_word, kErrMmaWaitTokens)) return false;
+                        // No more than two steps of a whole tile are issued ahead of the pipe: the scale copies of later slots queue behind the MMAs and are
+                        // announced when they are done, too late for the next steps otherwise (18944 x 5120, 512 tokens, three terms 53.3 -> 51.6 us). At
+                        // one term, and in tail tiles, whose steps are short, nothing is gained.
+                        if (kTerms > 1 && ahead_steps == 2) {
+                            if (!tail && !pair_wait(t_empty + 8 * behind, behind_phase, abort_flag, p.status_word, kErrMmaWaitTokens)) return false;
+                            if (++behind == depth.tokens) { behind = 0; behind_phase ^= 1; }
+                        } else {
+                            ++ahead_steps;
+                        }
                         const uint32_t t_desc = t_desc0 + slot * (kPairTokenSlot >> 4), sf_t = tmem_tokens + slot * 16, t_done = t_empty + 8 * slot;
                         // Each MMA consumes 64 k = 32 bytes of every row: start address + 2; only k steps inside the tensor. The commit frees
                         // the slot, and with it the slot's scale columns, in both CTAs.
@@ -1054,7 +1063,7 @@ struct PairSplit {
 // else is left to do (and per part) and when it happens under whole tiles, a launch beyond that. With the narrow kernel's estimate (gemm_narrow_ns) the
 // choice is 0.1 % off the best on average, 14 % at worst (2432 x 2176, 160 to 256 tokens, one term, 9.0 against 10.2 us).
 constexpr uint32_t kPairBlockCost[3] = {52, 93, 118};
-constexpr uint32_t kSplitCost = 450, kSplitPartCost = 170, kSplitCoveredCost = 480, kPairLaunchNs = 5500;
+constexpr uint32_t kSplitCost = 450, kSplitPartCost = 170, kSplitCoveredCost = 480, kSplitAddCost = 300, kPairLaunchNs = 5500;
 uint32_t pair_block_cost(uint32_t terms, uint32_t tail_columns) {
     return tail_columns ? 30 + terms * 9 + terms * (tail_columns - 32) * 7 / 100 : kPairBlockCost[terms - 1];
 }
@@ -1079,8 +1088,11 @@ PairSplit pair_split(uint32_t token_pairs, uint32_t tail_columns, uint32_t rows,
         if (sharers > line / cost_main) sharers = line / cost_main;      // every range holds a k block
         if (sharers < 2 || (!tail && sharers <= left) || scratch_bytes < kCounterBytes + sharers * kSplitSlotBytes) break;
         const uint64_t parts = (sharers * k_blocks * largest + line - 1) / line;
+        // Under whole tiles the finishing pair has one tile's time to add the parts, 3 us each; what that takes longer keeps its accumulator waiting (4096 x
+        // 2688, 3584 tokens, two tiles left over, in eight parts each 61 us, three terms).
+        const uint64_t adding = kSplitAddCost * (parts - 1), tile = k_blocks * cost_main;
         const uint64_t cost = k_blocks * rounds * cost_main + (line + sharers - 1) / sharers +
-                              (rounds ? kSplitCoveredCost : kSplitCost + kSplitPartCost * parts);
+                              (rounds ? kSplitCoveredCost + (adding > tile ? adding - tile : 0) : kSplitCost + kSplitPartCost * parts);
         if (cost < least) {
             least = cost;
             best.sharers = static_cast<uint32_t>(sharers);
