@@ -58,8 +58,8 @@ constexpr uint32_t kErrProducerWait = 0x101, kErrMmaWaitTokens = 0x102, kErrMmaW
 // Barriers per slot of a ring (same offsets in both CTAs):
 //   landed  leader's only: the slot's block-scale atoms of both CTAs have landed (loaded before the operand tiles);
 //   full    leader's only: two arrivals, the leader's producer (expecting the operand bytes of both CTAs; both producers' TMA
-//           loads complete on it: cta_group::2 loads, leader's address) and the ring's copy warp, which has issued the
-//           shared -> tensor memory copies of the slot's scales;
+//           loads complete on it: cta_group::2 loads, leader's address) and the commit behind the copy warp's shared -> tensor
+//           memory copies of the slot's scales, which says that they are done;
 //   empty   token slots only, one per CTA, arrived by the leader's tcgen05.commit multicast to both CTAs.
 // And: tmem_full one per CTA, same multicast;   tmem_empty leader's only, one arrival per epilogue warp of either CTA (the
 // peer's through a cluster-scope arrive).
@@ -547,8 +547,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         // activation terms of a k block. (One thread issuing all twelve copies of a one-term step needed longer
         // than the step's MMAs: 193 us for 4096 tokens on 17408 x 5120.)
         // A slot's scale atoms have landed. The producer refilled the slot only after the MMAs that used it last were
-        // complete, so the slot's scale columns are free. The copies only have to be issued before the MMAs that read them: a
-        // copy and a later MMA execute in issue order, and the fences on either side of the arrival order the two warps' issues.
+        // complete, so the slot's scale columns are free. The MMA warp waits for a commit behind the copies: with a plain arrival, on the strength of copies and
+        // later MMAs executing in the order of their issue, most launches of 17408 x 5120, 1024 tokens, three terms multiplied some k block's last 64 k
+        // before the scales of its second 128 features were there, once a step of the MMA warp was as short as it is.
         // Slots are taken as they come, whatever tile they belong to, and whole: what a last k block or a tile does not have is not read.
         const uint32_t blocks = work.blocks(k_blocks);
         if (warp == kPairCopyWarp) {
