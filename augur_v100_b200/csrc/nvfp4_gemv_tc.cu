@@ -579,8 +579,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             }
             const uint32_t acc = tmem_base + kTmemAcc + buffer * 64;
             const uint32_t stage = step % kStages, parity = (step / kStages) & 1;
-            // operands in shared memory (TMA) and their block scales on the way to tensor memory (copy thread):
-            // a copy and a later MMA execute in issue order, so the copies only have to be issued
+            // operands in shared memory (TMA) and their block scales in tensor memory (copy threads)
             if (!warp_wait(bar_full + 8 * stage, parity, abort_flag, p.header, kErrTcFull) ||
                 !warp_wait(bar_scales_ready + 8 * stage, parity, abort_flag, p.header, kErrTcScalesReady)) {
                 break;
@@ -626,8 +625,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             } else {
                 for (uint32_t k = 0; k < k_steps; ++k) tc_copy_sf(columns + 4 * k, desc + k * (kSfAtomBytes >> 4));
             }
-            tc_fence_before();
-            mbar_arrive(bar_scales_ready + 8 * stage);
+            tc_commit(bar_scales_ready + 8 * stage);   // when the copies are done: their order against another warp's MMAs is not relied on (0.07 us a block)
             ++step;
             more = cursor_next(p, c);
         }

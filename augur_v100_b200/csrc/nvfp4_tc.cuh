@@ -149,14 +149,6 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
 __device__ __forceinline__ void tc_copy_sf(uint32_t tmem, uint64_t desc) {
     asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem), "l"(desc) : "memory");
 }
-__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb,
-                                       uint32_t accumulate) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %6, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%4], [%5], p;\n}"
-        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
-        : "memory");
-}
 // One pipeline step of a converged warp: the one to four MMAs of a k block (64 k each: 32 bytes further in every operand row, four
 // scale columns further) and the commits that free what they read, `done` and, where `also` is not zero, `also_done`. `a` and `b` are the low
 // words of operand descriptors, whose high words are all alike. The elected
