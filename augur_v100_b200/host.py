@@ -715,12 +715,13 @@ class Nvfp4Sm100Linear:
     """One weight matrix, any number of token rows: the dispatch a model runtime does per call site.
 
     Keeps the weight in both hot layouts (the small-token stream layout and the tcgen05 layout) and
-    binds the kernel its shape class calls for: tokens <= 8 -> `Nvfp4Sm100Projection`, or where it is the
-    quicker `Nvfp4Sm100TcProjection`, otherwise `Nvfp4Sm100PrefillLinear` (activation quantiser with `terms`
+    binds the kernel its shape class calls for: tokens <= 8 -> `Nvfp4Sm100Projection`, or for the larger
+    weights `Nvfp4Sm100TcProjection`, otherwise `Nvfp4Sm100PrefillLinear` (activation quantiser with `terms`
     residual terms, then the block-scaled GEMM). Bindings are made per (input, output) pair, exactly like the
     classes it chooses between.
 
-    Both small-token kernels take every BF16 row. The tensor-memory kernel holds an element exactly down to
+    Both small-token kernels take every BF16 row. `Nvfp4Sm100Projection` multiplies every element as it is, and an
+    infinity or a NaN reaches each output by the rules of IEEE arithmetic. The tensor-memory kernel holds an element exactly down to
     2^-14 of the largest of its 16-element group and to 2^-22 of that below (groups under 2^-17 of their
     row's largest, to 2^-39 of the latter), and a row with an infinity or a NaN gives NaN in all its outputs.
     """
@@ -729,29 +730,17 @@ class Nvfp4Sm100Linear:
     TENSOR_MEMORY_MAX_ROWS = 1 << 18        # what the entry takes
 
     def _on_tensor_memory(self, plan: Plan, tokens: int) -> bool:
-        """From 2^25 weights on the tensor-memory kernel is the faster of the two, whatever the token rows: below, its second
-        launch costs more at eight of them than the integer work per weight that it saves (4096 x 5120 9.5 us against 9.2 on
-        mma.sync). It cuts a tile of 128 weight rows in eight parts at most, so that weights of few rows leave SMs idle, which
-        costs the more the more token rows there are. B200, us on tensor memory / mma.sync at 1, 4 and 8 token rows: 17408 x 5120
-        13.3 / 15.4, 13.9 / 16.3, 14.6 / 17.1; 4096 x 8192 9.2 / 10.2, 9.9 / 10.6, 10.8 / 10.9; 3072 x 12288 9.9 / 10.9, 10.8 / 11.5,
-        12.1 / 11.8; 2560 x 13184 10.1 / 11.8, 11.2 / 11.3, 12.6 / 11.6; 2048 x 16384 10.3 / 9.9, 11.6 / 10.6, 12.9 / 11.1. (The
-        worst found above the line: 10880 x 3200 at 8 rows, 11.2 / 10.7.) A plan that does not hold the kernel's scratch keeps
-        the other; any other fault of the binding is the caller's to see."""
+        """Weights from 2^25 on, less those of few rows, on the tensor-memory kernel. It is the quicker one for most others too, and they keep the other
+        kernel all the same, since that multiplies every activation as it is: the lines are where they were drawn when the tensor-memory kernel took a
+        launch more and was slower beyond them. B200, us on tensor memory / mma.sync at 1, 4, 5 and 8 token rows: 17408 x 5120 11.6 / 15.4, 12.4 / 16.4,
+        13.0 / 16.5, 14.1 / 17.2; 4096 x 8192 7.4 / 10.3, 8.2 / 10.7, 8.9 / 10.8, 9.8 / 11.0; 2560 x 13184 7.7 / 11.7, 8.7 / 11.2, and on the other side of the line
+        10.0 / 11.5, 11.1 / 11.6; there too 2048 x 16384 8.2 / 10.0, 9.5 / 10.7, 10.5 / 10.9, 11.5 / 11.2; 4096 x 4096 5.5 / 6.7, 6.2 / 7.4, 6.7 / 7.6, 7.3 / 7.9; 2048 x 5120
+        5.2 / 6.7, 6.0 / 6.9, 6.4 / 7.1, 7.2 / 7.2; 1024 x 5120 4.9 / 5.6, 5.7 / 5.9, 6.0 / 6.1, 6.6 / 6.1. (A tile of 128 weight rows is cut in eight parts at most, which is
+        why few rows count for less, the more so the more token rows there are.) A plan that does not hold the kernel's scratch keeps the
+        other kernel; any other fault of the binding is the caller's to see."""
         if self.rows % 128 != 0 or self.rows > self.TENSOR_MEMORY_MAX_ROWS or self.rows * self.cols < self.TENSOR_MEMORY_WEIGHTS:
             return False
         return self.rows >= (2560 if tokens <= 4 else 4096) and plan.snapshot().scratch_len_bytes >= gemv_tc_linear_scratch_bytes(self.cols)
-
-    def _on_tensor_memory_below(self, plan: Plan, tokens: int) -> bool:
-        """Most of what lies below that line is quicker there too, since the kernel forms the digits of its input itself and takes one launch. A tile
-        of 128 rows has eight CTAs at most, which bounds k next to the rows, the more so the more token rows there are; and beyond 32768 rows the
-        tiles no longer fit at once. B200, us on tensor memory / mma.sync at 1, 4, 5 and 8 token rows: 1024 x 2048 4.4 / 4.6, 4.6 / 5.0, 4.6 / 5.2, 4.8 / 5.4;
-        1024 x 5120 4.9 / 5.7, 5.7 / 5.9, 5.8 / 6.1, 6.6 / 6.2; 1024 x 17408 7.8 / 8.0, 8.5 / 8.7, 9.4 / 8.8, 9.9 / 9.2; 1536 x 8192 5.6 / 7.0, 6.4 / 7.6,
-        6.9 / 7.7, 8.0 / 7.8; 2048 x 5120 5.3 / 6.8, 6.1 / 7.0, 6.5 / 7.2, 7.3 / 7.3; 4096 x 4096 5.5 / 6.8, 6.3 / 7.5, 6.8 / 7.7, 7.5 / 7.9; 128 x 17408 7.0 / 5.6,
-        7.5 / 6.0, 8.2 / 6.2, 8.6 / 6.3; 49920 x 256 7.3 / 6.7, 7.6 / 7.0, 7.6 / 7.2, 7.9 / 7.1."""
-        if self.rows % 128 != 0 or self.rows > 32768:
-            return False
-        most = 32 if tokens <= 4 else 8 if tokens == 5 or self.rows >= 2048 else 4
-        return self.cols <= most * self.rows and plan.snapshot().scratch_len_bytes >= gemv_tc_linear_scratch_bytes(self.cols)
 
     def __init__(self, stream: Stream, rows: int, cols: int, codes, scales, global_scale: float):
         self.rows, self.cols = rows, cols
@@ -761,7 +750,7 @@ class Nvfp4Sm100Linear:
     def bind(self, plan: Plan, x: torch.Tensor, out: torch.Tensor | None = None, terms: int = 3,
              activation_global_scale: float = 2.0 ** -8):
         if classify_tokens(x.shape[0]) == SHAPE_SMALL_BATCH:
-            if self._on_tensor_memory(plan, x.shape[0]) or self._on_tensor_memory_below(plan, x.shape[0]):
+            if self._on_tensor_memory(plan, x.shape[0]):
                 return Nvfp4Sm100TcProjection.bind(plan, self.wide, x, out)
             return Nvfp4Sm100Projection.bind(plan, self.small, x, out)
         return Nvfp4Sm100PrefillLinear.bind(plan, self.wide, x, out, terms=terms, activation_global_scale=activation_global_scale)

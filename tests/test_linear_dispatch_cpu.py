@@ -17,3 +17,18 @@ def test_kernel_by_shape(rows, cols, tokens, expected):
     plan = lambda bytes_: SimpleNamespace(snapshot=lambda: SimpleNamespace(scratch_len_bytes=bytes_))
     assert linear._on_tensor_memory(plan(need), tokens) is expected
     assert linear._on_tensor_memory(plan(need - 256), tokens) is False
+
+
+# What `bind` makes of it, below the line of the large weights too: those keep the kernel that multiplies every activation as it is.
+@pytest.mark.parametrize("rows,cols,tokens,expected", [
+    (17408, 5120, 8, "tensor memory"), (2560, 13184, 4, "tensor memory"), (2560, 13184, 8, "exact"), (3072, 12288, 8, "exact"), (2048, 16384, 8, "exact"),
+    (3968, 8704, 5, "exact"), (4096, 8064, 1, "exact"), (4096, 4096, 4, "exact"), (2048, 5120, 8, "exact"), (1024, 5120, 1, "exact"), (1024, 4096, 8, "exact"),
+    (128, 64, 1, "exact"), (32768, 64, 8, "exact"), (17440, 5120, 8, "exact")])
+def test_bind_by_shape(monkeypatch, rows, cols, tokens, expected):
+    monkeypatch.setattr(host.Nvfp4Sm100TcProjection, "bind", classmethod(lambda cls, plan, weight, x, out=None: ("tensor memory", weight)))
+    monkeypatch.setattr(host.Nvfp4Sm100Projection, "bind", classmethod(lambda cls, plan, weight, x, out=None: ("exact", weight)))
+    linear = host.Nvfp4Sm100Linear.__new__(host.Nvfp4Sm100Linear)
+    linear.rows, linear.cols, linear.small, linear.wide = rows, cols, "small", "wide"
+    plan = SimpleNamespace(snapshot=lambda: SimpleNamespace(scratch_len_bytes=1 << 30))
+    bound = linear.bind(plan, SimpleNamespace(shape=(tokens, cols)))
+    assert bound == (expected, "wide" if expected == "tensor memory" else "small")
