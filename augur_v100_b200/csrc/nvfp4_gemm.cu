@@ -265,8 +265,8 @@ static __device__ __noinline__ bool pair_parts_arrived(const GemmParams& p, cons
                     break;
                 }
             }
-            // The flags read zero again when the launch is over, also those of parts that were given up on: that launch has
-            // failed and says so, and a late giver cannot leave one set for the next launch on this plan.
+            // The flags read zero again when the launch is over, unless a part was given up on and came late: that launch has failed and says so, and
+            // reading the plan's status clears what it left.
             p.split_flags[slot] = 0;
         }
     }

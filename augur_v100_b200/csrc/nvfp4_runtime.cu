@@ -267,8 +267,11 @@ extern "C" augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_plan_devi
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(plan->owner_stream);
     if (e == cudaSuccess && *out_status != 0) {
-        // a wait ran out: the launch left its meeting counters and row maxima (header words 16..63, trailer) half used
+        // a wait ran out: the launch left its meeting counters and row maxima (header words 16..63, trailer) half used, and arrival counters and
+        // flags of handed-over parts (the scratch's counter regions), which a CTA that came late may have set after the one that gave up on it
         e = cudaMemsetAsync(plan->status_word + 16, 0, (64 - 16) * sizeof(uint32_t), plan->owner_stream);
+        const uint64_t counters = plan->scratch_bytes < kCounterBytes ? plan->scratch_bytes : kCounterBytes;
+        if (e == cudaSuccess) e = cudaMemsetAsync(plan->scratch, 0, counters, plan->owner_stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(plan->scratch + plan->scratch_bytes, 0, kPlanTrailerBytes, plan->owner_stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(plan->owner_stream);
     }

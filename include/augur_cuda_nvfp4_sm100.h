@@ -672,7 +672,8 @@ void AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_allocation_snapshot_v1(
 uint64_t AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_launch_count_v1(void);
 /* Device-side status word of the plan (0 = clean). Bounded waits inside the
  * kernels record where they gave up here instead of spinning for ever; reading
- * it synchronises the plan's stream. */
+ * it synchronises the plan's stream and, if it is not 0, clears the counters and
+ * flags that the launch which gave up may have left in the plan. */
 augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_plan_device_status_v1(
     augur_cuda_nvfp4_sm100_plan_v1* plan, uint32_t* out_status);
 
