@@ -584,8 +584,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
                 !warp_wait(bar_scales_ready + 8 * stage, parity, abort_flag, p.header, kErrTcScalesReady)) {
                 break;
             }
-            tc_fence_after();
-            const uint32_t stage_smem = smem_u32(smem + stage * kStageBytes);
+            const uint32_t stage_smem = smem_u32(smem + stage * kStageBytes);   // (the fence behind the waits is tc_step's: once more here: 0.04 us a block)
             const uint64_t weight_desc = operand_desc(stage_smem), act_desc = operand_desc(stage_smem + kStageActCodes);
             const uint32_t tmem_sf_weight = tmem_base + kTmemSfWeight + stage * 16, tmem_sf_act = tmem_base + kTmemSfAct + stage * 16;
             const uint32_t k_steps = min(kStageK, p.phase[p.step[c.step].phase].cols - c.kb * kStageK) / 64;
