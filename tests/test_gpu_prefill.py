@@ -271,7 +271,7 @@ def test_linear_dispatch_by_token_count(ctx, tokens):
     linear = host.Nvfp4Sm100Linear(ctx["stream"], rows, cols, codes, scales, glob)
     x_bits = synth.make_activation(3, 71, "x", tokens, cols)
     binding = linear.bind(ctx["plan"], torch_bf16_from_bits(x_bits, ctx["device"]))
-    assert isinstance(binding, host.Nvfp4Sm100Projection if tokens <= 8 else host.Nvfp4Sm100PrefillLinear)
+    assert type(binding) is (host.Nvfp4Sm100Projection if tokens <= 8 else host.Nvfp4Sm100PrefillLinear)
     assert host.classify_tokens(tokens) == (host.SHAPE_SMALL_BATCH if tokens <= 8 else host.SHAPE_PREFILL)
     binding.submit_for_plan()
     ctx["stream"].synchronize()

@@ -32,34 +32,39 @@ def env():
     stream.close()
 
 
-def _repack_args(weight, planes):
+def _repack_args(weight, planes, rows=ROWS, cols=COLS):
     args = abi.header(abi.RepackArgs)
     for name, tensor in (("codes", planes[0]), ("scales", planes[1]), ("destination", weight.packed)):
         setattr(args, name, tensor.data_ptr())
         setattr(args, name + "_len_bytes", tensor.numel())
-    args.rows, args.cols, args.layout = ROWS, COLS, weight.layout
+    args.rows, args.cols, args.layout = rows, cols, weight.layout
     return args
 
 
-# one launch; two launches; quantiser and narrow GEMM, whose weights are fetched behind a launch that triggers early; pair GEMM
-@pytest.mark.parametrize("kind,tokens", [("stream", 3), ("split", 8), ("gemm", 16), ("gemm", 300)])
-def test_repack_then_linear(env, kind, tokens):
+# one launch on mma.sync; one on tensor memory; two, and quantiser and narrow GEMM, whose weights are fetched behind a launch that triggers early;
+# pair GEMM
+@pytest.mark.parametrize("kind,tokens,rows,cols,launches", [("stream", 3, ROWS, COLS, 1), ("split", 8, ROWS, COLS, 1), ("split", 8, 1024, 8 * COLS, 2),
+                                                            ("gemm", 16, ROWS, COLS, 2), ("gemm", 300, ROWS, COLS, 2)])
+def test_repack_then_linear(env, kind, tokens, rows, cols, launches):
     torch, side, stream, plan = env["torch"], env["side"], env["stream"], env["plan"]
+    planes = [(codes.view(rows, cols // 2), scales.view(rows, cols // 16)) for codes, scales in env["planes"]]
     layout = abi.LAYOUT_STREAM if kind == "stream" else abi.LAYOUT_TCGEN05
     with torch.cuda.stream(side):
         generator = torch.Generator(device="cuda")
         generator.manual_seed(tokens)
-        x = torch.randn((tokens, COLS), device="cuda", generator=generator).to(torch.bfloat16)
-        weight = host.Nvfp4Sm100Weight.repack_device_planes(stream, layout, ROWS, COLS, *env["planes"][0], synth.GLOBAL_SCALE)
+        x = torch.randn((tokens, cols), device="cuda", generator=generator).to(torch.bfloat16)
+        weight = host.Nvfp4Sm100Weight.repack_device_planes(stream, layout, rows, cols, *planes[0], synth.GLOBAL_SCALE)
         binding = {"stream": host.Nvfp4Sm100Projection, "split": host.Nvfp4Sm100TcProjection, "gemm": host.Nvfp4Sm100PrefillLinear}[kind]
         program = binding.bind(plan, weight, x)
         submit = abi.lib().augur_cuda_nvfp4_sm100_repack_prevalidated_submit_v1
-        args = [_repack_args(weight, planes) for planes in env["planes"]]
+        args = [_repack_args(weight, both, rows, cols) for both in planes]
         wanted = []
         for which in range(2):
             assert submit(stream.ordinal, stream.handle, byref(args[which])).status == abi.STATUS_OK
             stream.synchronize()
+            before = host.launch_count()
             program.submit_for_plan()
+            assert host.launch_count() - before == launches
             stream.synchronize()
             wanted.append(program.out.clone())
         got = []
@@ -73,8 +78,8 @@ def test_repack_then_linear(env, kind, tokens):
     assert [torch.equal(out, wanted[turn % 2]) for turn, out in enumerate(got)] == [True] * 40
 
 
-# The quantiser reads what the launch before it writes, while that launch still runs: narrow GEMM, pair GEMM with a narrow tail,
-# small-token linear.
+# The quantiser reads what the launch before it writes, while that launch still runs: narrow GEMM, pair GEMM, small-token
+# linear on tensor memory.
 @pytest.mark.parametrize("tokens,producer", [(48, "gemm"), (300, "gemm"), (8, "split")])
 def test_linear_then_quantiser(env, tokens, producer):
     torch, side, stream, plan = env["torch"], env["side"], env["stream"], env["plan"]
@@ -131,14 +136,17 @@ def _lagging_launch(env, plan):
     return program, buffers
 
 
-# The bounded waits of a launch do not run out while it waits for a launch ahead of it that takes long: small-token linear, narrow
-# GEMM, pair GEMM, one-launch MLP block.
-@pytest.mark.parametrize("kind,tokens", [("split", 8), ("gemm", 16), ("gemm", 300), ("block", 8)])
-def test_waits_do_not_count_the_launch_before(env, kind, tokens):
+# The bounded waits of a launch do not run out while it waits for a launch ahead of it that takes long: small-token linear of one launch and of
+# two, narrow GEMM, pair GEMM, one-launch MLP block.
+@pytest.mark.parametrize("kind,tokens,rows,cols", [("split", 8, ROWS, COLS), ("split", 8, 1024, 8 * COLS), ("gemm", 16, ROWS, COLS), ("gemm", 300, ROWS, COLS),
+                                                   ("block", 8, ROWS, COLS)])
+def test_waits_do_not_count_the_launch_before(env, kind, tokens, rows, cols):
     torch, side, stream, plan = env["torch"], env["side"], env["stream"], env["plan"]
     with torch.cuda.stream(side):
-        x = torch.randn((tokens, COLS), device="cuda").to(torch.bfloat16)
-        weight = host.Nvfp4Sm100Weight.repack_device_planes(stream, abi.LAYOUT_TCGEN05, ROWS, COLS, *env["planes"][0], synth.GLOBAL_SCALE)
+        x = torch.randn((tokens, cols), device="cuda").to(torch.bfloat16)
+        codes, scales = env["planes"][0]
+        weight = host.Nvfp4Sm100Weight.repack_device_planes(stream, abi.LAYOUT_TCGEN05, rows, cols, codes.view(rows, cols // 2), scales.view(rows, cols // 16),
+                                                            synth.GLOBAL_SCALE)
         if kind == "block":
             weight.global_scale_b = synth.GLOBAL_SCALE   # the rows as gate and up of an intermediate half as wide
             codes, scales = (plane[:COLS] for plane in env["planes"][1])
