@@ -16,6 +16,7 @@
 
 
 #include "nvfp4_gemm.cuh"
+#include "nvfp4_gemm_choice.h"
 #include "nvfp4_internal.h"
 #include "nvfp4_layout.cuh"
 #include "nvfp4_pair_work.h"
@@ -105,7 +106,6 @@ static_assert(kPairSmemBytes <= 227 * 1024, "shared memory of a CTA");
 constexpr uint32_t kPairCopyWarp = 2 + kPairEpilogueWarps;    // token-row scales; the warp after it copies the weight-row scales
 constexpr uint32_t kPairThreads = 32 * (kPairCopyWarp + 2);   // TMA warp, MMA warp, epilogue warps, two scale-copy warps
 static_assert(kPairBarriers * 8 + 8 + kPairThreads / 32 * 4 + sizeof(PairWork) <= 512, "barriers, tensor-memory base, abort flag, the warps' counters and the pair's work fit behind the rings");
-constexpr uint32_t kSplitWays = 8;              // a leftover tile is cut into this many parts at most
 constexpr uint32_t kSplitWaitLimit = 1u << 20;  // polls of a handed-over part's flag (each a round trip to L2) before giving up
 constexpr uint64_t kSplitSlotBytes = 2ull * kPairEpilogueWarps * 32 * 128 * 4;   // one pair's accumulator: 256 x 256 f32
 constexpr uint32_t kLeaderMask = 0xFEFFFFFFu;   // clears the CTA-rank bit of a shared::cluster address within a pair
@@ -1053,74 +1053,11 @@ struct QuantTarget {
     float global_scale = 0.0f;
 };
 
-// How a launch of the pair kernel over `token_pairs` x 256 token rows shares its tiles out, and about how long it takes.
-struct PairSplit {
-    uint32_t pairs, sharers;     // sharers: pairs that share the leftover tiles (0: every tile is one pair's)
-    uint32_t ns;
-};
-
-// In units of 10 ns, fitted on a B200 to 429 GEMMs (eleven weights from 1024 x 5120 to 34816 x 5120, 13 token counts from 48 to 1100, one to three terms),
-// each with every choice forced in turn: what a k block of a whole tile costs and of a tail tile, handing the parts of leftover tiles over when nothing
-// else is left to do (and per part) and when it happens under whole tiles, a launch beyond that. With the narrow kernel's estimate (gemm_narrow_ns) the
-// choice is 0.1 % off the best on average, 14 % at worst (2432 x 2176, 160 to 256 tokens, one term, 9.0 against 10.2 us).
-constexpr uint32_t kPairBlockCost[3] = {52, 93, 118};
-constexpr uint32_t kSplitCost = 450, kSplitPartCost = 170, kSplitCoveredCost = 480, kSplitAddCost = 300, kPairLaunchNs = 5500;
-uint32_t pair_block_cost(uint32_t terms, uint32_t tail_columns) {
-    return tail_columns ? 30 + terms * 9 + terms * (tail_columns - 32) * 7 / 100 : kPairBlockCost[terms - 1];
-}
-
-// Tiles past the last full round of the pairs (all tiles, when there are fewer tiles than pairs) may be cut along k, in `ways`
-// parts each at most and over all pairs at most, when the plan's scratch has room for the partial accumulators handed
-// over: one slot per pair behind the counter regions, whose first words serve as the flags. Of the numbers of parts up to
-// kSplitWays the one with the least steps is taken: cut in eight, the 4 tiles of 1024 rows and 256 tokens took 25 us, whole 15.
-PairSplit pair_split(uint32_t token_pairs, uint32_t tail_columns, uint32_t rows, uint32_t cols, uint32_t terms, uint32_t all_pairs, uint64_t scratch_bytes) {
-    const uint32_t n_tiles = (rows + kTileN - 1) / kTileN, k_blocks = (cols + kBlockK - 1) / kBlockK;
-    const uint32_t main = token_pairs * n_tiles, tail = tail_columns ? n_tiles : 0;
-    const uint64_t cost_main = pair_block_cost(terms, 0), cost_tail = tail ? pair_block_cost(terms, tail_columns) : 0;
-    const uint32_t rounds = main / all_pairs, left = main % all_pairs;
-    PairSplit best{main + tail < all_pairs ? main + tail : all_pairs, 0, 0};
-    // not cut: the first pair has the most tiles of either kind
-    const uint64_t most_main = (main + all_pairs - 1) / all_pairs, most = (main + tail + all_pairs - 1) / all_pairs;
-    uint64_t least = k_blocks * (most_main * cost_main + (most - most_main) * cost_tail);
-    const uint64_t line = k_blocks * (left * cost_main + tail * cost_tail), largest = left ? cost_main : cost_tail;
-    for (uint32_t ways = 2; line && ways <= kSplitWays; ++ways) {
-        uint64_t sharers = line * ways / (k_blocks * largest);
-        if (sharers > all_pairs) sharers = all_pairs;
-        if (sharers > line / cost_main) sharers = line / cost_main;      // every range holds a k block
-        if (sharers < 2 || (!tail && sharers <= left) || scratch_bytes < kCounterBytes + sharers * kSplitSlotBytes) break;
-        const uint64_t parts = (sharers * k_blocks * largest + line - 1) / line;
-        // Under whole tiles the finishing pair has one tile's time to add the parts, 3 us each; what that takes longer keeps its accumulator waiting (4096 x
-        // 2688, 3584 tokens, two tiles left over, in eight parts each 61 us, three terms).
-        const uint64_t adding = kSplitAddCost * (parts - 1), tile = k_blocks * cost_main;
-        const uint64_t cost = k_blocks * rounds * cost_main + (line + sharers - 1) / sharers +
-                              (rounds ? kSplitCoveredCost + (adding > tile ? adding - tile : 0) : kSplitCost + kSplitPartCost * parts);
-        if (cost < least) {
-            least = cost;
-            best.sharers = static_cast<uint32_t>(sharers);
-        }
-    }
-    if (best.pairs < best.sharers) best.pairs = best.sharers;
-    best.ns = static_cast<uint32_t>(least * 10 > UINT32_MAX / 2 ? UINT32_MAX / 2 : least * 10) + kPairLaunchNs;
-    return best;
-}
-
-// Which token rows the pair kernel takes, and how: all of them or none (the narrow kernel's then). The choice is the quickest by the
-// estimates.
-struct PairPlan {
-    uint32_t token_pairs, tail_columns;
-    PairSplit split;
-};
-PairPlan pair_plan(const augur_cuda_nvfp4_sm100_plan_v1* plan, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
-    const uint32_t all_pairs = plan->pair_clusters, pairs = (tokens + 2 * kTileM - 1) / (2 * kTileM), rest = tokens % (2 * kTileM);
-    if (!all_pairs) return PairPlan{};
-    const uint32_t narrow_ns = gemm_narrow_ns(plan->ordinal, rows, cols, tokens, terms);
-    PairPlan best{pairs, 0, pair_split(pairs, 0, rows, cols, terms, all_pairs, plan->scratch_bytes)};
-    if (pairs > 1 && rest != 0 && rest <= kTileM) {
-        const uint32_t columns = (rest + 31) / 32 * 32;
-        const PairPlan tail{pairs - 1, columns, pair_split(pairs - 1, columns, rows, cols, terms, all_pairs, plan->scratch_bytes)};
-        if (tail.split.ns < best.split.ns) best = tail;
-    }
-    return best.split.ns < narrow_ns ? best : PairPlan{};
+// The choice of nvfp4_gemm_choice.h for this plan: a pair that hands a part over needs a slot of its scratch behind the counter regions, whose first words
+// serve as the flags.
+PairPlan plan_pairs(const augur_cuda_nvfp4_sm100_plan_v1* plan, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
+    const uint64_t slots = plan->scratch_bytes > kCounterBytes ? (plan->scratch_bytes - kCounterBytes) / kSplitSlotBytes : 0;
+    return pair_plan(rows, cols, tokens, terms, plan->pair_clusters, slots, gemm_narrow_ns(plan->ordinal, rows, cols, tokens, terms));
 }
 
 augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
@@ -1145,7 +1082,7 @@ augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_s
     p.quant_out = reinterpret_cast<uint8_t*>(quant.destination);
     p.quant_terms = quant.terms;
     p.quant_scale = quant_scale(quant.global_scale);
-    const PairPlan pairs = pair_plan(plan, a->rows, a->cols, a->tokens, a->activation_terms);
+    const PairPlan pairs = plan_pairs(plan, a->rows, a->cols, a->tokens, a->activation_terms);
     p.token_pairs = pairs.token_pairs;
     if (p.token_pairs) {
         // 256 x 256 tiles on pairs of CTAs (clusters of two); the grid is a whole number of pairs.

@@ -30,6 +30,7 @@
 // all roles fall through to the common exits. What a role waits for on a barrier never includes the launch before: a role that
 // depends on it waits for its end first, so that its time does not count against the bound.
 #include "nvfp4_gemm.cuh"
+#include "nvfp4_gemm_choice.h"
 
 namespace augur_sm100 {
 namespace {
@@ -54,7 +55,6 @@ constexpr uint32_t kNarrowRowPitch = kTileM + 4;                      // floats 
 // CTA found room beside two of them: 17408 x 5120, three terms, 128 tokens 33.8 -> 30.8 us, 48 tokens 26.1 -> 24.4.
 constexpr uint32_t kNarrowSmem = 112 * 1024;
 constexpr uint32_t kNarrowTmemColumns = 256;
-constexpr uint32_t kNarrowMaxParts = 8;                               // portable cluster size
 static_assert((6 * kNarrowMaxDepth + 1) * 8 + 8 + kNarrowThreads / 32 * 4 <= kNarrowState, "the small state fits");
 static_assert(kTileM / 4 * kNarrowSumPitch * 16 + kTileM / 2 * kNarrowRowPitch * 4 <= kNarrowSmem - 1024 - kNarrowState,
               "partial sums of all columns and finished ones of half of them in the space of the rings");
@@ -409,50 +409,22 @@ uint32_t two_cta_clusters(int32_t ordinal, uint32_t parts) {
 }
 
 namespace {
-// How a launch cuts its work, and about how long it takes: the waves of clusters times the pipeline steps of a part, of the
-// numbers of CTAs per item the one with the least. Fitted on a B200 with two CTAs on every SM, before a step's MMAs became one block of
-// instructions and a cluster's sums were read where they are: a step (k block x term) 0.33 us at 16 tokens and 0.44 at 128, a launch about 6 us
-// beyond its steps, a wave after the first 3, the parts' sums 4 us more at 128 tokens. Measured since, three terms, one part: 0.32 to 0.34 us
-// a step at 16 tokens, 0.50 at 48, 0.55 at 128, and 5 to 9 us beyond. The number of parts chosen is 1.7 % off the best on average, 25 % at worst
-// (1024 x 5120, 200 tokens).
-struct NarrowCut {
-    uint32_t token_tiles, tile_tokens, columns, parts, ns;
-};
-NarrowCut narrow_cut(int32_t ordinal, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
-    NarrowCut cut{};
-    cut.token_tiles = (tokens + kTileM - 1) / kTileM;
-    cut.tile_tokens = tokens < kTileM ? tokens : kTileM;
-    cut.columns = (cut.tile_tokens + 15) / 16 * 16;
-    const uint64_t items = static_cast<uint64_t>(rows / kTileM) * cut.token_tiles;
-    const uint32_t k_blocks = (cols + kNarrowK - 1) / kNarrowK, step_ns = 320 + cut.columns * 120 / kTileM;
-    uint64_t least = ~uint64_t(0);
-    for (uint32_t parts = 1; parts <= kNarrowMaxParts && parts <= k_blocks; ++parts) {
-        const uint32_t clusters = two_cta_clusters(ordinal, parts);
-        const uint64_t waves = (items + clusters - 1) / clusters;
-        const uint64_t ns = waves * ((k_blocks + parts - 1) / parts * terms * step_ns + 3000) + 3000 + cut.columns * 4000 / kTileM;
-        if (ns < least) {
-            least = ns;
-            cut.parts = parts;
-        }
-    }
-    // Against the pair kernel the estimate counts, not only the order: fitted as kPairBlockCost.
-    const uint32_t clusters = two_cta_clusters(ordinal, cut.parts);
-    const uint64_t ns = (items + clusters - 1) / clusters * ((k_blocks + cut.parts - 1) / cut.parts * (terms * (350 + cut.columns) + 110) + 2900) + 2100 +
-                        cut.columns * 4000 / kTileM;
-    cut.ns = static_cast<uint32_t>(ns < UINT32_MAX / 2 ? ns : UINT32_MAX / 2);
-    return cut;
+NarrowCut device_cut(int32_t ordinal, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
+    uint32_t clusters[kNarrowMaxParts + 1] = {};
+    for (uint32_t parts = 1; parts <= kNarrowMaxParts; ++parts) clusters[parts] = two_cta_clusters(ordinal, parts);
+    return narrow_cut(clusters, rows, cols, tokens, terms);
 }
 }  // namespace
 
 uint32_t gemm_narrow_ns(int32_t ordinal, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
-    return narrow_cut(ordinal, rows, cols, tokens, terms).ns;
+    return device_cut(ordinal, rows, cols, tokens, terms).ns;
 }
 
 augur_cuda_result_v1 launch_gemm_narrow(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan, const CUtensorMap& map_weight,
                                         uint64_t activation, const GemmParams& g) {
     NarrowParams p{};
     p.g = g;
-    const NarrowCut cut = narrow_cut(plan->ordinal, g.rows, g.cols, g.tokens, g.terms);
+    const NarrowCut cut = device_cut(plan->ordinal, g.rows, g.cols, g.tokens, g.terms);
     p.token_tiles = cut.token_tiles;
     p.tile_tokens = cut.tile_tokens;
     p.columns = cut.columns;

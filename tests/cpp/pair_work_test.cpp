@@ -1,4 +1,5 @@
-// pair_work (csrc/nvfp4_pair_work.h) over the launches that the command line asks for: every (tile, k block) is done exactly once;
+// pair_work (csrc/nvfp4_pair_work.h) over random launches and over those that pair_plan (csrc/nvfp4_gemm_choice.h) makes of random GEMMs, both as the
+// library includes them: every (tile, k block) is done exactly once;
 // a part handed over is its pair's first item and the only one; the pairs that hand parts of a tile over are exactly those that the
 // finishing pair waits for; no two pairs of those that share differ by more than two k blocks' cost, leaving the rounds aside.
 #include <cstdio>
@@ -6,6 +7,7 @@
 #include <map>
 #include <vector>
 
+#include "nvfp4_gemm_choice.h"
 #include "nvfp4_pair_work.h"
 
 using namespace augur_sm100;
@@ -44,8 +46,19 @@ static bool check(uint32_t pairs, const PairShares& s) {
     return givers == waits && (!s.sharers || most - least <= 2 * larger);
 }
 
-int main() {
-    std::srand(5);
+// Clusters of 1 .. 8 CTAs that a B200 holds, two CTAs on every SM, as two_cta_clusters counts them.
+static const uint32_t kClusters[kNarrowMaxParts + 1] = {0, 296, 148, 88, 67, 53, 43, 35, 31};
+
+static PairPlan plan_for(uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms, uint32_t all, uint64_t slots, bool pairs_only) {
+    return pair_plan(rows, cols, tokens, terms, all, slots, pairs_only ? UINT32_MAX : narrow_cut(kClusters, rows, cols, tokens, terms).ns);
+}
+static PairShares shares_of(const PairPlan& plan, uint32_t rows, uint32_t cols, uint32_t terms) {
+    const uint32_t n_tiles = (rows + 255) / 256;
+    return PairShares{plan.token_pairs * n_tiles, plan.tail_columns ? n_tiles : 0, (cols + 255) / 256, plan.split.sharers,
+                      pair_block_cost(terms, 0), pair_block_cost(terms, plan.tail_columns)};
+}
+
+static bool random_launches() {
     uint32_t cut = 0;
     for (uint32_t round = 0; round < 20000; ++round) {
         const uint32_t all = 1 + std::rand() % (round % 2 ? 74 : 8), n_tiles = 1 + std::rand() % 140, token_pairs = 1 + std::rand() % 5;
@@ -59,9 +72,61 @@ int main() {
         cut += s.sharers != 0;
         if (!check(pairs, s)) {
             std::printf("pairs %u main %u tail %u k blocks %u sharers %u costs %u %u\n", pairs, s.main, s.tail, s.k_blocks, s.sharers, s.cost_main, s.cost_tail);
-            return 1;
+            return false;
         }
     }
-    std::puts(cut > 10000 ? "ok" : "too few launches share tiles");
+    if (cut <= 10000) std::puts("too few launches share tiles");
+    return cut > 10000;
+}
+
+static bool chosen_launches() {
+    uint32_t cut = 0, tails = 0, cut_tails = 0;
+    for (uint32_t round = 0; round < 20000; ++round) {
+        const uint32_t rows = 128 * (1 + std::rand() % 272), cols = 64 * (1 + std::rand() % (round % 3 ? 80 : 300)), terms = 1 + std::rand() % 3;
+        const uint32_t tokens = 9 + std::rand() % (round % 2 ? 1100 : 4088), all = round % 4 ? 74 : 1 + std::rand() % 74;
+        const uint64_t slots = round % 5 ? all : std::rand() % 80;
+        const PairPlan plan = plan_for(rows, cols, tokens, terms, all, slots, round % 8 == 0);
+        if (!plan.token_pairs) continue;   // the narrow kernel's
+        const uint32_t covered = plan.token_pairs * 256 + plan.tail_columns;
+        const bool sound = plan.split.pairs <= all && plan.split.sharers <= plan.split.pairs && plan.split.sharers <= slots && covered >= tokens &&
+                           (plan.tail_columns ? plan.tail_columns % 32 == 0 && plan.tail_columns <= 128 && tokens > plan.token_pairs * 256 : true);
+        if (!sound || !check(plan.split.pairs, shares_of(plan, rows, cols, terms))) {
+            std::printf("rows %u cols %u tokens %u terms %u pairs %u slots %llu: %u x 256 + %u on %u, shared by %u\n", rows, cols, tokens, terms, all,
+                        static_cast<unsigned long long>(slots), plan.token_pairs, plan.tail_columns, plan.split.pairs, plan.split.sharers);
+            return false;
+        }
+        cut += plan.split.sharers != 0;
+        tails += plan.tail_columns != 0;
+        cut_tails += plan.split.sharers && plan.tail_columns;
+    }
+    if (cut <= 2000 || tails <= 2000 || cut_tails <= 500) std::printf("cut %u, with tail tiles %u, both %u\n", cut, tails, cut_tails);
+    return cut > 2000 && tails > 2000 && cut_tails > 500;
+}
+
+// Without arguments: the checks. With rows, cols, tokens, terms and slots: what a B200's 74 pairs do of such a GEMM, as token pairs, tail columns and
+// pairs that share tiles; of those, pairs that hand a part of a tail tile over, and tail tiles that are put together.
+int main(int count, char** text) {
+    if (count == 6) {
+        uint32_t v[5];
+        for (int i = 0; i < 5; ++i) v[i] = static_cast<uint32_t>(std::strtoul(text[1 + i], nullptr, 10));
+        const PairPlan plan = plan_for(v[0], v[1], v[2], v[3], 74, v[4], false);
+        uint32_t given = 0, finished = 0;
+        if (plan.token_pairs) {
+            const PairShares s = shares_of(plan, v[0], v[1], v[3]);
+            for (uint32_t pair = 0; pair < plan.split.pairs; ++pair) {
+                const PairWork w = pair_work(pair, plan.split.pairs, s);
+                for (uint32_t i = 0; i < w.items; ++i) {
+                    const PairItem item = w.item(i, pair, plan.split.pairs, s.k_blocks);
+                    given += item.kind == 1 && item.tile >= s.main;
+                    finished += item.kind == 2 && item.tile >= s.main;
+                }
+            }
+        }
+        std::printf("%u %u %u %u %u\n", plan.token_pairs, plan.tail_columns, plan.split.sharers, given, finished);
+        return 0;
+    }
+    std::srand(5);
+    if (!random_launches() || !chosen_launches()) return 1;
+    std::puts("ok");
     return 0;
 }
