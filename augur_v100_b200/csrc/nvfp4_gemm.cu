@@ -487,9 +487,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_const
         // ---------------- MMA issuer (leader only) ----------------
         // Issuing a tcgen05 operation keeps a warp busy for tens of cycles, and one warp issuing the 12 scale copies and
         // the 4 MMAs of every step could not keep the tensor pipe fed; the copies are issued by two warps of their own
-        // (below) into the slots' scale columns, this one issues only the MMAs. Descriptors advance by additions (their low
-        // bits hold address >> 4). Looking at a barrier takes as long as issuing an MMA or two, so those of the next
-        // step are looked at before the MMAs of this one are issued, and waited for only if they were not there.
+        // (below) into the slots' scale columns, this one issues only the MMAs, a step's as one block of predicated instructions. Descriptors advance by
+        // additions (their low bits hold address >> 4).
         uint32_t w_stage = 0, w_phase = 0, slot = 0, t_phase = 0, tmem_phase = 0, behind = 0, behind_phase = 0, ahead_steps = 0;
         bool alive = true;
         constexpr uint32_t kWideTile = (1u << 7) | (1u << 10) | ((kTileN >> 3) << 17) | (((2 * kTileM) >> 4) << 24);

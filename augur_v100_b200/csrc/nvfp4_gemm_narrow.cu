@@ -1,5 +1,5 @@
-// Prefill NVFP4 GEMM for token ranges that are narrow next to the weights (sm_100a): short prompts, batched decode of
-// more users than the small-token kernels take, and the tail of a longer prompt.
+// Prefill NVFP4 GEMM for token counts that are narrow next to the weights (sm_100a): short prompts, and batched decode of
+// more users than the small-token kernels take.
 //
 // The pair kernel of nvfp4_gemm.cu puts 256 token rows on its tile, so 9 tokens cost what 256 do. Here the weights are the
 // 128-row operand and the tokens sit on the MMA n dimension, whose size follows their number in steps of 16 (at most

@@ -8,7 +8,7 @@
 // range. The first MMA comes about two microseconds after the input is there. A launch of its own that splits the rows once for all CTAs takes
 // four, half of them its end and hand-over; it stays where a CTA has many chunks of many token rows (split_linear_own_digits), because the
 // integer work, 270 instructions for eight elements in every lane, is done by every CTA again. us, launch ahead / own digits: 17408 x 5120 at 1 token row
-// 13.5 / 11.7, at 8 14.9 / 14.2; 5120 x 5120 8.2 / 6.4, 9.9 / 8.9; 1024 x 5120 6.9 / 4.9, 7.0 / 6.5; two layers of linears and MLP blocks 155.5 / 148.7.
+// 13.7 / 12.3, at 8 14.9 / 14.6; 5120 x 5120 8.3 / 6.6, 9.8 / 8.8; 1024 x 5120 7.0 / 5.1, 7.0 / 7.0; two layers of linears and MLP blocks 155.7 / 149.4.
 //
 // Roles: warp 0 weights (TMA, scale copies), 1 MMA, 2 scale copies of the activations, 3 TMA of digits that a launch ahead left, 4..11 own digits, then
 // epilogue. What a warp issues
@@ -438,9 +438,10 @@ uint32_t split_linear_parts(uint32_t tiles, uint32_t k_blocks, const uint32_t (&
 }
 
 // Whether the stream kernel forms the digits itself, `chunks` of them per CTA. From six token rows on two of a CTA's eight warps share every quarter of the
-// SM and a chunk's digits take 0.94 us, its weights 0.82: what the launch ahead costs is lost again over some ten chunks. us at 6, 7 and 8
-// token rows, own digits / launch ahead: 17408 x 5120 (10 chunks) 13.9 / 14.4, 14.0 / 14.6, 14.2 / 14.9; 10240 x 8192 (11) 15.1 / 14.8, 15.2 / 15.0, 15.3 / 15.3;
-// 10240 x 10240 (14) 17.9 / 16.9, 17.9 / 17.2, 18.0 / 17.3; 34816 x 5120 (20) 22.5 / 20.9, 22.7 / 20.9, 23.0 / 21.1; at five 20.2 / 21.0, 10240 x 17408 (23) 24.2 / 24.7.
+// SM and a chunk's digits take 0.94 us, its weights 0.82: what the launch ahead costs is lost again over some ten chunks. us at 6 and 8
+// token rows, own digits / launch ahead: 17408 x 5120 (10 chunks) 14.3 / 14.4, 14.6 / 14.9; 10240 x 8192 (11) 15.6 / 14.8, 15.8 / 15.5; 17408 x 6144 (12) 16.9 / 16.1,
+// 17.2 / 16.6; 10240 x 10240 (14) 18.3 / 17.0, 18.6 / 17.6; 34816 x 5120 (20) 23.0 / 21.1, 23.3 / 21.1; at five 20.7 / 21.1, 10240 x 17408 (23) 24.8 / 24.7. A long k next to
+// the rows gives the launch ahead more to do, which the rule leaves out: 5120 x 17408 (12) 16.5 / 16.8, 16.8 / 17.9, 4096 x 16384 13.8 / 14.9, 14.1 / 15.6.
 static bool split_linear_own_digits(uint32_t tokens, uint32_t chunks) { return tokens <= 5 || chunks <= 10; }
 
 augur_cuda_result_v1 launch_split_linear(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,

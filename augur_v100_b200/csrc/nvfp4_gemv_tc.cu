@@ -22,7 +22,7 @@
 // there are at least about as many as CTAs, else every tile cut along k into equal
 // parts whose partial sums meet in plan scratch (arrival counter per 32 rows; the last arriver adds the parts in
 // a fixed order and finishes the rows; bit-reproducible). (A single linear as a program of one step took 17.3 us for
-// 17408 x 5120 at 8 tokens and 12.7 for 5120 x 5120; nvfp4_gemv_split.cu, which has no meeting of all CTAs, takes 14.2 and 8.9.) The block is
+// 17408 x 5120 at 8 tokens and 12.7 for 5120 x 5120; nvfp4_gemv_split.cu, which has no meeting of all CTAs, takes 14.6 and 8.8.) The block is
 // two steps when the gate|up tiles fit the CTAs: gate|up in whole tiles, then down in k parts. The second product needs every CTA's
 // outputs of the first and their largest magnitudes per token row before it can split them: the CTAs arrive at
 // a counter when their outputs are stored, wait for all, split, arrive at a second counter, and the activation
@@ -624,7 +624,7 @@ tc_program_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constan
             } else {
                 for (uint32_t k = 0; k < k_steps; ++k) tc_copy_sf(columns + 4 * k, desc + k * (kSfAtomBytes >> 4));
             }
-            tc_commit(bar_scales_ready + 8 * stage);   // when the copies are done: their order against another warp's MMAs is not relied on (0.07 us a block)
+            tc_commit(bar_scales_ready + 8 * stage);   // when the copies are done: their order against another warp's MMAs is not relied on (0.03 us a block)
             ++step;
             more = cursor_next(p, c);
         }

@@ -279,10 +279,10 @@ augur_cuda_result_v1 AUGUR_CUDA_CALL augur_cuda_nvfp4_sm100_gemv_bf16_prevalidat
  * (for EPILOGUE_SWIGLU_BF16: one tensor of 2 * rows physical rows, 16 gate rows alternating with the
  * matching 16 up rows, as interleave_gate_up_host_v1 makes it), rows (physical) a multiple of 128, cols a
  * multiple of 64. The weights reach the tensor cores (tcgen05.mma kind::mxf4nvf4) as TMA delivers them;
- * the BF16 activations are split, by a launch of their own, into eight NVFP4 terms (radix-8 digits with
- * power-of-two scales), exact for every element within 2^-14 of its 16-element group's largest magnitude and
- * to 2^-22 of that magnitude below (in a group more than 2^17 below its row's largest magnitude, to 2^-39 of the
- * latter); a token row with a non-finite element gives NaN outputs. A wait that runs out sets the plan's
+ * the BF16 activations are split, in the launch itself or, where that is quicker, by one ahead of it, into eight NVFP4
+ * terms (radix-8 digits with power-of-two scales), exact for every element within 2^-14 of its 16-element group's largest
+ * magnitude and to 2^-22 of that magnitude below (in a group more than 2^17 below the largest magnitude of its row, or of the
+ * part of it that is split together, to 2^-39 of the latter); a token row with a non-finite element gives NaN outputs. A wait that runs out sets the plan's
  * status word to 0x311..0x316. Needs the counter regions and the split activations of the plan's scratch, 10 KB per
  * 256 columns; the extent below is larger and also covers a member of mlp_tc. Replaces the same reference entry
  * points as gemv_bf16_*_v1 (augur_qwen35_nvfp4_qpn_abi.h:134-156), with one weight layout for every token count. */
