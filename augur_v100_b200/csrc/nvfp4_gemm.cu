@@ -1054,9 +1054,9 @@ struct QuantTarget {
 
 // The choice of nvfp4_gemm_choice.h for this plan: a pair that hands a part over needs a slot of its scratch behind the counter regions, whose first words
 // serve as the flags.
-PairPlan plan_pairs(const augur_cuda_nvfp4_sm100_plan_v1* plan, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms) {
+PairPlan plan_pairs(const augur_cuda_nvfp4_sm100_plan_v1* plan, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms, bool swiglu) {
     const uint64_t slots = plan->scratch_bytes > kCounterBytes ? (plan->scratch_bytes - kCounterBytes) / kSplitSlotBytes : 0;
-    return pair_plan(rows, cols, tokens, terms, plan->pair_clusters, slots, gemm_narrow_ns(plan->ordinal, rows, cols, tokens, terms));
+    return pair_plan(rows, cols, tokens, terms, swiglu, plan->pair_clusters, slots, gemm_narrow_ns(plan->ordinal, rows, cols, tokens, terms));
 }
 
 augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
@@ -1081,7 +1081,7 @@ augur_cuda_result_v1 launch_gemm(augur_cuda_stream_t s, const augur_cuda_nvfp4_s
     p.quant_out = reinterpret_cast<uint8_t*>(quant.destination);
     p.quant_terms = quant.terms;
     p.quant_scale = quant_scale(quant.global_scale);
-    const PairPlan pairs = plan_pairs(plan, a->rows, a->cols, a->tokens, a->activation_terms);
+    const PairPlan pairs = plan_pairs(plan, a->rows, a->cols, a->tokens, a->activation_terms, swiglu);
     p.token_pairs = pairs.token_pairs;
     if (p.token_pairs) {
         // 256 x 256 tiles on pairs of CTAs (clusters of two); the grid is a whole number of pairs.

@@ -34,10 +34,10 @@ inline NarrowCut narrow_cut(const uint32_t (&clusters)[kNarrowMaxParts + 1], uin
             cut.parts = parts;
         }
     }
-    // Against the pair kernel the estimate counts, not only the order: fitted as kPairBlockCost.
-    const uint64_t ns = (items + clusters[cut.parts] - 1) / clusters[cut.parts] *
-                            ((k_blocks + cut.parts - 1) / cut.parts * (terms * (350 + cut.columns) + 110) + 2900) +
-                        2100 + cut.columns * 4000 / kTile;
+    // Against the pair kernel the estimate counts, not only the order: fitted with it (pair_split).
+    const uint64_t ns = ((items + clusters[cut.parts] - 1) / clusters[cut.parts] *
+                             ((k_blocks + cut.parts - 1) / cut.parts * (terms * (350 + cut.columns) + 110) + 2900) +
+                         2100 + cut.columns * 4000 / kTile) * 924 / 1000;
     cut.ns = static_cast<uint32_t>(ns < UINT32_MAX / 2 ? ns : UINT32_MAX / 2);
     return cut;
 }
@@ -51,49 +51,65 @@ struct PairSplit {
     uint32_t ns;
 };
 
-// In units of 10 ns, fitted on a B200 to 429 GEMMs (eleven weights from 1024 x 5120 to 34816 x 5120, 13 token counts from 48 to 1100, one to three terms),
-// each with every choice forced in turn: what a k block of a whole tile costs and of a tail tile, handing the parts of leftover tiles over when nothing
-// else is left to do (and per part) and when it happens under whole tiles, a launch beyond that. With the narrow kernel's estimate the
-// choice is 0.1 % off the best on average, 14 % at worst (2432 x 2176, 160 to 256 tokens, one term, 9.0 against 10.2 us).
+// What a k block of a whole tile and of a tail tile counts when leftover tiles are shared out: only the ratio matters.
 constexpr uint32_t kPairBlockCost[3] = {52, 93, 118};
-constexpr uint32_t kSplitCost = 450, kSplitPartCost = 170, kSplitCoveredCost = 480, kSplitAddCost = 300, kPairLaunchNs = 5500;
 inline uint32_t pair_block_cost(uint32_t terms, uint32_t tail_columns) {
     return tail_columns ? 30 + terms * 9 + terms * (tail_columns - 32) * 7 / 100 : kPairBlockCost[terms - 1];
 }
 
+// The estimate, in ns, fitted on a B200 to 2560 GEMMs over the sizes of real layers (1024 to 17408 rows and columns, gate|up of twice that with their
+// quantiser, 130 to 4096 tokens, one to three terms), each with every choice forced in turn. Tile after tile a pair takes the k blocks, or the epilogue
+// where that is longer, which the last tile's follows; a last round of few tiles takes less of its time, since the board's power then goes to fewer SMs.
+// A cut costs its pairs their share and a fixed time, more when a share is parts of two tiles, and some per part; the pair that puts a tile together keeps its
+// accumulator waiting meanwhile, which a whole tile behind it hides only up to its own time. On 500 GEMMs more the choice is 1.0 % off the best on average
+// and 5 % in one of twenty. (With constants fitted to up to 1100 tokens and a cut taken for hidden under whole tiles 4.0 % and 18 %, us now and then: 1536 x
+// 6016, 3776 tokens, one term 27.5 / 32.8, gate|up 5120 x 1408, 810 tokens, two terms 13.0 / 22.0, 5376 x 4864, 2773 tokens, three terms 113 / 120.)
+constexpr uint32_t kBlockNs[3] = {446, 793, 1134}, kStoreNs = 1180, kQuantiseNs[3] = {3790, 6360, 8360}, kTailStartNs = 980, kPairLaunchNs = 3800;
+constexpr uint32_t kLastRoundShare[3] = {706, 857, 872};   // of 1000
+constexpr uint32_t kCutNs = 4350, kCutPartNs = 1660, kCutCoveredNs = 800, kCutWaitNs = 9520, kCutWaitPartNs = 3190;
+constexpr uint32_t kCutRaggedNs = 3420, kCutQuantiseNs = 3350, kCutTailNs = 4220, kNarrowQuantiseNs = 1190;
+inline uint64_t pair_tail_block_ns(uint32_t terms, uint32_t tail_columns) { return 169 + 115 * terms + terms * (tail_columns - 32) * 141 / 100; }
+
 // Tiles past the last full round of the pairs (all tiles, when there are fewer tiles than pairs) may be cut along k, in `ways`
 // parts each at most and over all pairs at most, when the plan's scratch has a slot for the partial accumulator of each pair that
-// shares them (`slots`). Of the numbers of parts up to kSplitWays the one with the least steps is taken: cut in eight, the 4 tiles of 1024
-// rows and 256 tokens took 25 us, whole 15.
-inline PairSplit pair_split(uint32_t token_pairs, uint32_t tail_columns, uint32_t rows, uint32_t cols, uint32_t terms, uint32_t all_pairs, uint64_t slots) {
+// shares them (`slots`). `swiglu`: gate and up with the quantiser of as many terms behind them; a launch that stores its BF16 result instead is cut in the
+// same way, so that both come to the same bits.
+inline PairSplit pair_split(uint32_t token_pairs, uint32_t tail_columns, uint32_t rows, uint32_t cols, uint32_t terms, bool swiglu, uint32_t all_pairs,
+                            uint64_t slots) {
     constexpr uint32_t kTile = 256, kDepth = 256;
     const uint32_t n_tiles = (rows + kTile - 1) / kTile, k_blocks = (cols + kDepth - 1) / kDepth;
-    const uint32_t main = token_pairs * n_tiles, tail = tail_columns ? n_tiles : 0;
-    const uint64_t cost_main = pair_block_cost(terms, 0), cost_tail = tail ? pair_block_cost(terms, tail_columns) : 0;
-    const uint32_t rounds = main / all_pairs, left = main % all_pairs;
-    PairSplit best{main + tail < all_pairs ? main + tail : all_pairs, 0, 0};
+    const uint32_t main = token_pairs * n_tiles, tail = tail_columns ? n_tiles : 0, rounds = main / all_pairs, left = main % all_pairs;
+    const auto larger = [](uint64_t a, uint64_t b) { return a > b ? a : b; };
+    const uint64_t out = swiglu ? kQuantiseNs[terms - 1] : kStoreNs, block = kBlockNs[terms - 1], last = k_blocks * block, tile = larger(last, out);
+    const uint64_t tail_block = tail ? pair_tail_block_ns(terms, tail_columns) : 0, tail_tile = k_blocks * tail_block + kTailStartNs;
     // not cut: the first pair has the most tiles of either kind
-    const uint64_t most_main = (main + all_pairs - 1) / all_pairs, most = (main + tail + all_pairs - 1) / all_pairs;
-    uint64_t least = k_blocks * (most_main * cost_main + (most - most_main) * cost_tail);
+    const uint64_t most_main = (main + all_pairs - 1) / all_pairs, most = (main + tail + all_pairs - 1) / all_pairs, share = kLastRoundShare[terms - 1];
+    uint64_t least = most > most_main ? most_main * tile + (most - most_main) * tail_tile : (most - 1) * tile + last;
+    if (!tail && left) least = rounds * tile + last * (share * all_pairs + (1000 - share) * left) / (1000 * all_pairs);
+    PairSplit best{main + tail < all_pairs ? main + tail : all_pairs, 0, 0};
+    const uint64_t cost_main = pair_block_cost(terms, 0), cost_tail = tail ? pair_block_cost(terms, tail_columns) : 0;
     const uint64_t line = k_blocks * (left * cost_main + tail * cost_tail), largest = left ? cost_main : cost_tail;
+    uint64_t before = 0;
     for (uint32_t ways = 2; line && ways <= kSplitWays; ++ways) {
         uint64_t sharers = line * ways / (k_blocks * largest);
         if (sharers > all_pairs) sharers = all_pairs;
         if (sharers > line / cost_main) sharers = line / cost_main;      // every range holds a k block
-        if (sharers < 2 || (!tail && sharers <= left) || sharers > slots) break;
+        if (sharers < 2 || (!tail && sharers <= left) || sharers > slots || sharers == before) break;
+        before = sharers;
         const uint64_t parts = (sharers * k_blocks * largest + line - 1) / line;
-        // Under whole tiles the finishing pair has one tile's time to add the parts, 3 us each; what that takes longer keeps its accumulator waiting (4096 x
-        // 2688, 3584 tokens, two tiles left over, in eight parts each 61 us, three terms).
-        const uint64_t adding = kSplitAddCost * (parts - 1), tile = k_blocks * cost_main;
-        const uint64_t cost = k_blocks * rounds * cost_main + (line + sharers - 1) / sharers +
-                              (rounds ? kSplitCoveredCost + (adding > tile ? adding - tile : 0) : kSplitCost + kSplitPartCost * parts);
-        if (cost < least) {
-            least = cost;
+        uint64_t ns = tail ? k_blocks * (left * block + tail * tail_block) / sharers + kCutTailNs : (left * k_blocks + sharers - 1) / sharers * block;
+        if (rounds == 0) ns += kCutNs + (parts - 1) * kCutPartNs;
+        else ns += kCutCoveredNs + larger(rounds > 1 ? tile : last, kCutWaitNs + (parts - 1) * kCutWaitPartNs) + (rounds > 1 ? (rounds - 2) * tile + last : 0);
+        if (!tail && sharers % left) ns += kCutRaggedNs;
+        if (swiglu) ns += kCutQuantiseNs;
+        if (ns < least) {
+            least = ns;
             best.sharers = static_cast<uint32_t>(sharers);
         }
     }
     if (best.pairs < best.sharers) best.pairs = best.sharers;
-    best.ns = static_cast<uint32_t>(least * 10 > UINT32_MAX / 2 ? UINT32_MAX / 2 : least * 10) + kPairLaunchNs;
+    least += kPairLaunchNs + out;
+    best.ns = static_cast<uint32_t>(least > UINT32_MAX / 2 ? UINT32_MAX / 2 : least);
     return best;
 }
 
@@ -103,17 +119,18 @@ struct PairPlan {
     uint32_t token_pairs, tail_columns;
     PairSplit split;
 };
-inline PairPlan pair_plan(uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms, uint32_t all_pairs, uint64_t slots, uint32_t narrow_ns) {
+inline PairPlan pair_plan(uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms, bool swiglu, uint32_t all_pairs, uint64_t slots,
+                          uint32_t narrow_ns) {
     constexpr uint32_t kTile = 256;
     const uint32_t pairs = (tokens + kTile - 1) / kTile, rest = tokens % kTile;
     if (!all_pairs) return PairPlan{};
-    PairPlan best{pairs, 0, pair_split(pairs, 0, rows, cols, terms, all_pairs, slots)};
+    PairPlan best{pairs, 0, pair_split(pairs, 0, rows, cols, terms, swiglu, all_pairs, slots)};
     if (pairs > 1 && rest != 0 && rest <= kTile / 2) {
         const uint32_t columns = (rest + 31) / 32 * 32;
-        const PairPlan tail{pairs - 1, columns, pair_split(pairs - 1, columns, rows, cols, terms, all_pairs, slots)};
+        const PairPlan tail{pairs - 1, columns, pair_split(pairs - 1, columns, rows, cols, terms, swiglu, all_pairs, slots)};
         if (tail.split.ns < best.split.ns) best = tail;
     }
-    return best.split.ns < narrow_ns ? best : PairPlan{};
+    return best.split.ns < narrow_ns + (swiglu ? terms * kNarrowQuantiseNs : 0) ? best : PairPlan{};
 }
 
 }  // namespace augur_sm100

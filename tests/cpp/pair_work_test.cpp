@@ -49,8 +49,8 @@ static bool check(uint32_t pairs, const PairShares& s) {
 // Clusters of 1 .. 8 CTAs that a B200 holds, two CTAs on every SM, as two_cta_clusters counts them.
 static const uint32_t kClusters[kNarrowMaxParts + 1] = {0, 296, 148, 88, 67, 53, 43, 35, 31};
 
-static PairPlan plan_for(uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms, uint32_t all, uint64_t slots, bool pairs_only) {
-    return pair_plan(rows, cols, tokens, terms, all, slots, pairs_only ? UINT32_MAX : narrow_cut(kClusters, rows, cols, tokens, terms).ns);
+static PairPlan plan_for(uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t terms, bool swiglu, uint32_t all, uint64_t slots, bool pairs_only) {
+    return pair_plan(rows, cols, tokens, terms, swiglu, all, slots, pairs_only ? UINT32_MAX : narrow_cut(kClusters, rows, cols, tokens, terms).ns);
 }
 static PairShares shares_of(const PairPlan& plan, uint32_t rows, uint32_t cols, uint32_t terms) {
     const uint32_t n_tiles = (rows + 255) / 256;
@@ -85,7 +85,7 @@ static bool chosen_launches() {
         const uint32_t rows = 128 * (1 + std::rand() % 272), cols = 64 * (1 + std::rand() % (round % 3 ? 80 : 300)), terms = 1 + std::rand() % 3;
         const uint32_t tokens = 9 + std::rand() % (round % 2 ? 1100 : 4088), all = round % 4 ? 74 : 1 + std::rand() % 74;
         const uint64_t slots = round % 5 ? all : std::rand() % 80;
-        const PairPlan plan = plan_for(rows, cols, tokens, terms, all, slots, round % 8 == 0);
+        const PairPlan plan = plan_for(rows, cols, tokens, terms, round % 3 == 0, all, slots, round % 8 == 0);
         if (!plan.token_pairs) continue;   // the narrow kernel's
         const uint32_t covered = plan.token_pairs * 256 + plan.tail_columns;
         const bool sound = plan.split.pairs <= all && plan.split.sharers <= plan.split.pairs && plan.split.sharers <= slots && covered >= tokens &&
@@ -103,13 +103,13 @@ static bool chosen_launches() {
     return cut > 2000 && tails > 2000 && cut_tails > 500;
 }
 
-// Without arguments: the checks. With rows, cols, tokens, terms and slots: what a B200's 74 pairs do of such a GEMM, as token pairs, tail columns and
+// Without arguments: the checks. With rows, cols, tokens, terms, 0 or 1 for gate|up and slots: what a B200's 74 pairs do of such a GEMM, as token pairs, tail columns and
 // pairs that share tiles; of those, pairs that hand a part of a tail tile over, and tail tiles that are put together.
 int main(int count, char** text) {
-    if (count == 6) {
-        uint32_t v[5];
-        for (int i = 0; i < 5; ++i) v[i] = static_cast<uint32_t>(std::strtoul(text[1 + i], nullptr, 10));
-        const PairPlan plan = plan_for(v[0], v[1], v[2], v[3], 74, v[4], false);
+    if (count == 7) {
+        uint32_t v[6];
+        for (int i = 0; i < 6; ++i) v[i] = static_cast<uint32_t>(std::strtoul(text[1 + i], nullptr, 10));
+        const PairPlan plan = plan_for(v[0], v[1], v[2], v[3], v[4] != 0, 74, v[5], false);
         uint32_t given = 0, finished = 0;
         if (plan.token_pairs) {
             const PairShares s = shares_of(plan, v[0], v[1], v[3]);

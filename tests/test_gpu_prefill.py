@@ -201,11 +201,11 @@ def test_gemm_pair_tiles_terms_share_weight_scales_across_tiles(ctx):
     _check_gemm(ctx, rows=2560, cols=768, tokens=2048, terms=2, seed=14)
 
 
-@pytest.mark.parametrize("cols,terms", [(4864, 1), (2560, 2), (320, 1)])
+@pytest.mark.parametrize("cols,terms", [(4864, 1), (2560, 2), (320, 1), (4864, 3)])
 def test_gemm_pair_tiles_leftover_round_cut_along_k(ctx, cols, terms):
     # 80 pair tiles for at most 74 pairs: with a plan that has room for the handed-over accumulators the 6 tiles
-    # of the last round are cut along k between the pairs (19 k blocks, 8 parts per tile; 10 k blocks with two
-    # terms); with 2 k blocks the idle time saved is not worth a hand-over and the tiles stay whole
+    # of the last round may be cut along k between the pairs (19 k blocks at three terms: five parts per tile); where the idle
+    # time saved is not worth a hand-over they stay whole
     host = ctx["host"]
     big = host.Plan(ctx["stream"], host.gemm_plan_scratch_bytes())
     try:
@@ -217,7 +217,7 @@ def test_gemm_pair_tiles_leftover_round_cut_along_k(ctx, cols, terms):
 
 
 def test_gemm_fewer_pair_tiles_than_pairs_all_cut_along_k(ctx):
-    # 2 pair tiles of 20 k blocks: with room in the plan every tile is cut between the pairs of the whole device
+    # 2 pair tiles of 20 k blocks, and one of 68: the narrow kernel's, since the pairs would have to cut them for the whole device
     host = ctx["host"]
     big = host.Plan(ctx["stream"], host.gemm_plan_scratch_bytes())
     try:

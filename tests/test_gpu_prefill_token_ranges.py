@@ -1,5 +1,5 @@
 """GPU parity of the prefill GEMM's two kernels over token counts: the narrow kernel, token pairs alone, and
-pairs with tail tiles; half tiles of an odd number of 128-row weight blocks; leftover tiles cut along k. Bounds as elsewhere:
+pairs with tail tiles; half tiles of an odd number of 128-row weight blocks. Bounds as elsewhere:
 helpers.rel_error <= 2e-2 (BF16 output) against the fp64 oracle fed the same quantised activations."""
 import numpy as np
 import pytest
@@ -27,7 +27,7 @@ def test_narrow_token_ranges(ctx, rows, cols, tokens, terms):  # noqa: F811
     assert _check_gemm(ctx, rows, cols, tokens, terms, seed=rows + tokens) <= TOLERANCE
 
 
-# Token pairs with a half tile at the end (one round; several rounds), leftover tiles cut along k with a half tile among them,
+# Token pairs with a half tile at the end (one round; several rounds; fewer tiles than pairs),
 # pairs with tail tiles of 44 tokens.
 @pytest.mark.parametrize("rows,cols,tokens,terms", [(17280, 576, 530, 3), (19072, 832, 1500, 1), (4992, 4352, 400, 3), (17408, 5120, 300, 3)])
 def test_pair_tiles_and_tails(ctx, split_plan, rows, cols, tokens, terms):  # noqa: F811
