@@ -152,8 +152,11 @@ split_rows_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ split, u
     split_scales(to, row_anchor, where, bits, group_largest, lane);
 }
 
-// The first look at a barrier is in line, the rest suspended: the issue slots are for the digits.
+// The first look at a barrier is in line, the rest suspended where the issue slots are for digits; where a launch ahead has formed them, polling: 10112 x 8448 at
+// seven token rows 15.2 us suspended, 15.0 polling, 10240 x 8192 at six 14.7 and 14.6, 5120 x 17408 at seven 18.1 and 17.9.
+template <bool kOwnDigits>
 __device__ __forceinline__ bool stream_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t* status_word, uint32_t code) {
+    if (!kOwnDigits) return warp_wait(bar, parity, abort_flag, status_word, code);
     return mbar_test(bar, parity) || warp_wait_suspended(bar, parity, abort_flag, status_word, code);
 }
 
@@ -243,7 +246,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid
         const uint8_t* scales = p.weight_sf + static_cast<uint64_t>(tile) * atoms * kSfAtomBytes;
         uint32_t load_kb = kb0, load_stage = 0, load_phase = 1, stage = 0, phase = 0;
         auto load = [&]() {
-            if (!stream_wait(w_empty + 8 * load_stage, load_phase, abort_flag, p.status_word, kErrStreamWeights)) return false;
+            if (!stream_wait<kOwnDigits>(w_empty + 8 * load_stage, load_phase, abort_flag, p.status_word, kErrStreamWeights)) return false;
             const uint32_t to = smem_u32(smem + load_stage * kStreamWeightStage), sf_bytes = (load_kb + 1 < k_blocks ? 4u : last_k_steps) * kSfAtomBytes;
             tma_step(w_full + 8 * load_stage, kStageCodeBytes + sf_bytes, to, &map_weight, load_kb * 128, tile * kTileM, to + kStageCodeBytes,
                      scales + static_cast<uint64_t>(load_kb) * kStageSfBytes, sf_bytes);
@@ -253,7 +256,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid
         };
         while (alive && load_kb < kb1 && load_kb < kb0 + kStreamWeightDepth) alive = load();
         for (uint32_t kb = kb0; alive && kb < kb1; ++kb) {
-            if (!stream_wait(w_full + 8 * stage, phase, abort_flag, p.status_word, kErrStreamCopy)) break;
+            if (!stream_wait<kOwnDigits>(w_full + 8 * stage, phase, abort_flag, p.status_word, kErrStreamCopy)) break;
             tc_copy_step(tmem_base + kStreamSfWeight + stage * 16, desc0 + stage * (kStreamWeightStage >> 4), w_ready + 8 * stage);
             if (++stage == kStreamWeightDepth) { stage = 0; phase ^= 1; }
             // the first wait for a stage to be free, which it is when the activations are there
@@ -267,8 +270,8 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid
         const uint32_t idesc = instr_desc(kCols);
         const uint32_t w_desc0 = static_cast<uint32_t>(operand_desc(smem_u32(smem))), t_desc0 = static_cast<uint32_t>(operand_desc(smem_u32(slots)));
         for (uint32_t kb = kb0; kb < kb1; ++kb) {
-            if (!stream_wait(w_ready + 8 * stage, w_phase, abort_flag, p.status_word, kErrStreamFull) ||
-                !stream_wait(t_ready + 8 * slot, t_phase, abort_flag, p.status_word, kErrStreamScales)) {
+            if (!stream_wait<kOwnDigits>(w_ready + 8 * stage, w_phase, abort_flag, p.status_word, kErrStreamFull) ||
+                !stream_wait<kOwnDigits>(t_ready + 8 * slot, t_phase, abort_flag, p.status_word, kErrStreamScales)) {
                 alive = false;
                 break;
             }
@@ -285,7 +288,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid
         uint32_t slot = 0, phase = 0;
         const uint64_t desc0 = sf_desc(smem_u32(slots) + kChunkBytes);
         for (uint32_t kb = kb0; kb < kb1; ++kb) {
-            if (!stream_wait(t_full + 8 * slot, phase, abort_flag, p.status_word, kErrStreamCopy)) break;
+            if (!stream_wait<kOwnDigits>(t_full + 8 * slot, phase, abort_flag, p.status_word, kErrStreamCopy)) break;
             tc_copy_step(tmem_base + kStreamSfAct + slot * 16, desc0 + slot * (kStreamActStage >> 4), t_ready + 8 * slot);
             if (++slot == kStreamActDepth) { slot = 0; phase ^= 1; }
         }
@@ -295,7 +298,7 @@ split_stream_kernel(const __grid_constant__ CUtensorMap map_weight, const __grid
         const uint8_t* image_sf = p.split + split_code_bytes(p.cols);
         uint32_t slot = 0, phase = 1;
         for (uint32_t kb = kb0; kb < kb1; ++kb) {
-            if (!stream_wait(t_empty + 8 * slot, phase, abort_flag, p.status_word, kErrStreamTokens)) break;
+            if (!stream_wait<kOwnDigits>(t_empty + 8 * slot, phase, abort_flag, p.status_word, kErrStreamTokens)) break;
             const uint32_t to = smem_u32(slots + slot * kStreamActStage), full = t_full + 8 * slot;
             if (elect_one()) {
                 mbar_expect_tx(full, kStreamActStage);
@@ -439,9 +442,9 @@ uint32_t split_linear_parts(uint32_t tiles, uint32_t k_blocks, const uint32_t (&
 
 // Whether the stream kernel forms the digits itself, `chunks` of them per CTA. From six token rows on two of a CTA's eight warps share every quarter of the
 // SM and a chunk's digits take 0.94 us, its weights 0.82: what the launch ahead costs is lost again over some ten chunks. us at 6 and 8
-// token rows, own digits / launch ahead: 17408 x 5120 (10 chunks) 14.3 / 14.4, 14.6 / 14.9; 10240 x 8192 (11) 15.6 / 14.8, 15.8 / 15.5; 17408 x 6144 (12) 16.9 / 16.1,
-// 17.2 / 16.6; 10240 x 10240 (14) 18.3 / 17.0, 18.6 / 17.6; 34816 x 5120 (20) 23.0 / 21.1, 23.3 / 21.1; at five 20.7 / 21.1, 10240 x 17408 (23) 24.8 / 24.7. A long k next to
-// the rows gives the launch ahead more to do, which the rule leaves out: 5120 x 17408 (12) 16.5 / 16.8, 16.8 / 17.9, 4096 x 16384 13.8 / 14.9, 14.1 / 15.6.
+// token rows, own digits / launch ahead: 17408 x 5120 (10 chunks) 14.3 / 14.1, 14.6 / 14.8; 10240 x 8192 (11) 15.6 / 14.7, 15.8 / 15.4; 17408 x 6144 (12) 16.9 / 15.9,
+// 17.2 / 16.6; 10240 x 10240 (14) 18.3 / 17.0, 18.6 / 17.5; 34816 x 5120 (20) 23.0 / 20.9, 23.3 / 21.1; at five 20.7 / 21.1, 10240 x 17408 (23) 24.8 / 24.7. A long k next to
+// the rows gives the launch ahead more to do, which the rule leaves out: 5120 x 17408 (12) 16.5 / 16.7, 16.8 / 17.9.
 static bool split_linear_own_digits(uint32_t tokens, uint32_t chunks) { return tokens <= 5 || chunks <= 10; }
 
 augur_cuda_result_v1 launch_split_linear(augur_cuda_stream_t s, const augur_cuda_nvfp4_sm100_plan_v1* plan,
