@@ -34,10 +34,14 @@ inline NarrowCut narrow_cut(const uint32_t (&clusters)[kNarrowMaxParts + 1], uin
             cut.parts = parts;
         }
     }
-    // Against the pair kernel the estimate counts, not only the order: fitted with it (pair_split).
-    const uint64_t ns = ((items + clusters[cut.parts] - 1) / clusters[cut.parts] *
-                             ((k_blocks + cut.parts - 1) / cut.parts * (terms * (350 + cut.columns) + 110) + 2900) +
-                         2100 + cut.columns * 4000 / kTile) * 924 / 1000;
+    // Against the pair kernel the time counts, not only the order, and it is an estimate of its own: fitted to 1660 GEMMs of 9 to 4096 tokens and 64 to 34816
+    // rows and columns, each by both kernels, as the pair kernel's estimate (pair_split) and the difference of the two times. The meeting of a cluster is
+    // 1.26 us per doubling of its CTAs. On 650 GEMMs more the choice between the kernels is 0.4 % off the best on average and 14 % at worst from 1024 rows
+    // and columns on below 129 tokens, 22 % beyond; with constants fitted to 130 tokens and more and real layers alone 4.3 %, us now and then: 9600 x 64, 15 tokens, one term
+    // 4.3 / 6.5, gate|up 18944 x 1088, 160 tokens, three terms 18.3 / 24.1.
+    constexpr uint32_t kMeetNs[kNarrowMaxParts + 1] = {0, 0, 1264, 2003, 2528, 2935, 3267, 3549, 3792};
+    const uint64_t waves = (items + clusters[cut.parts] - 1) / clusters[cut.parts], steps = (k_blocks + cut.parts - 1) / cut.parts;
+    const uint64_t ns = waves * (2310 + cut.columns * 216 / 10 + kMeetNs[cut.parts] + steps * (112 + terms * (414 + cut.columns * 79 / 100)));
     cut.ns = static_cast<uint32_t>(ns < UINT32_MAX / 2 ? ns : UINT32_MAX / 2);
     return cut;
 }
@@ -67,7 +71,7 @@ inline uint32_t pair_block_cost(uint32_t terms, uint32_t tail_columns) {
 constexpr uint32_t kBlockNs[3] = {446, 793, 1134}, kStoreNs = 1180, kQuantiseNs[3] = {3790, 6360, 8360}, kTailStartNs = 980, kPairLaunchNs = 3800;
 constexpr uint32_t kLastRoundShare[3] = {706, 857, 872};   // of 1000
 constexpr uint32_t kCutNs = 4350, kCutPartNs = 1660, kCutCoveredNs = 800, kCutWaitNs = 9520, kCutWaitPartNs = 3190;
-constexpr uint32_t kCutRaggedNs = 3420, kCutQuantiseNs = 3350, kCutTailNs = 4220, kNarrowQuantiseNs = 1190;
+constexpr uint32_t kCutRaggedNs = 3420, kCutQuantiseNs = 3350, kCutTailNs = 4220, kNarrowQuantiseNs = 485;
 inline uint64_t pair_tail_block_ns(uint32_t terms, uint32_t tail_columns) { return 169 + 115 * terms + terms * (tail_columns - 32) * 141 / 100; }
 
 // Tiles past the last full round of the pairs (all tiles, when there are fewer tiles than pairs) may be cut along k, in `ways`

@@ -27,6 +27,16 @@ def test_narrow_token_ranges(ctx, rows, cols, tokens, terms):  # noqa: F811
     assert _check_gemm(ctx, rows, cols, tokens, terms, seed=rows + tokens) <= TOLERANCE
 
 
+# The same on weights that stay with the narrow kernel by a margin (tests/test_pair_work_cpu.py asks the library's rule for these and those above): more tiles than
+# places, 301 and 390 of them, MMA n of 16, 48, 112 and 128, two and five token tiles, clusters of up to eight.
+NARROW = [(38528, 832, 9, 1), (49920, 1088, 16, 1), (49920, 2112, 40, 2), (384, 4352, 112, 2), (1152, 5120, 128, 1), (640, 4352, 200, 1), (512, 4352, 577, 1)]
+
+
+@pytest.mark.parametrize("rows,cols,tokens,terms", NARROW)
+def test_narrow_tiles(ctx, rows, cols, tokens, terms):  # noqa: F811
+    assert _check_gemm(ctx, rows, cols, tokens, terms, seed=rows + tokens) <= TOLERANCE
+
+
 # Token pairs with a half tile at the end (one round; several rounds; fewer tiles than pairs),
 # pairs with tail tiles of 44 tokens.
 @pytest.mark.parametrize("rows,cols,tokens,terms", [(17280, 576, 530, 3), (19072, 832, 1500, 1), (4992, 4352, 400, 3), (17408, 5120, 300, 3)])
@@ -51,7 +61,7 @@ def test_pair_tiles_and_tails(ctx, split_plan, rows, cols, tokens, terms):  # no
 
 
 # The fused intermediate quantiser in both kernels' epilogues: the whole block equals the one that quantises in a launch of its own.
-@pytest.mark.parametrize("hidden,inter,tokens", [(256, 640, 20), (384, 1152, 200), (5120, 8704, 300)])
+@pytest.mark.parametrize("hidden,inter,tokens", [(256, 640, 20), (384, 1152, 200), (5120, 8704, 300), (1536, 1408, 825)])
 def test_fused_quantiser_in_every_kernel(ctx, split_plan, hidden, inter, tokens):  # noqa: F811
     torch = ctx["torch"]
     generator = torch.Generator(device=ctx["device"])

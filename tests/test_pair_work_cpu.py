@@ -7,6 +7,7 @@ import subprocess
 import pytest
 
 from test_gpu_prefill_tails import BLOCKS, CASES, LEFTOVER, LEFTOVER_BLOCKS
+from test_gpu_prefill_token_ranges import NARROW
 
 ROOT = pathlib.Path(__file__).resolve().parents[1]
 PAIRS = 74      # of CTAs on a B200: as many slots has a plan with room to cut tiles
@@ -25,9 +26,11 @@ def test_every_part_of_every_tile_once(binary):
     assert done.returncode == 0 and done.stdout.strip() == "ok", done.stdout
 
 
-def _chosen(binary, rows, cols, tokens, terms, gate_up, slots):
+def _chosen(binary, rows, cols, tokens, terms, gate_up, slots, pairs=False):
     done = subprocess.run([str(binary)] + [str(v) for v in (rows, cols, tokens, terms, gate_up, slots)], capture_output=True, text=True, timeout=60, check=True)
-    _, tail_columns, sharers, given, finished = map(int, done.stdout.split())
+    token_pairs, tail_columns, sharers, given, finished = map(int, done.stdout.split())
+    if pairs:
+        return token_pairs
     return tail_columns, given > 0 and finished > 0, sharers
 
 
@@ -50,6 +53,25 @@ def test_leftover_cases(binary, rows, cols, tokens, terms, sharers):
 @pytest.mark.parametrize("hidden,inter,tokens,terms,sharers", LEFTOVER_BLOCKS)
 def test_leftover_blocks(binary, hidden, inter, tokens, terms, sharers):
     assert _chosen(binary, 2 * inter, hidden, tokens, terms, 1, PAIRS) == (0, False, sharers)
+
+
+@pytest.mark.parametrize("rows,cols,tokens,terms", NARROW + [(128, 64, 9, 1), (384, 192, 16, 3), (128, 320, 17, 2), (2944, 2112, 127, 3), (640, 1088, 129, 3),
+                                                             (128, 17408, 33, 2)])
+def test_narrow_cases(binary, rows, cols, tokens, terms):
+    assert _chosen(binary, rows, cols, tokens, terms, 0, PAIRS, pairs=True) == 0
+    assert _chosen(binary, rows, cols, tokens, terms, 0, 0, pairs=True) == 0
+
+
+# The choice between the two kernels. us by the narrow one and by pairs: an estimate fitted to 130 tokens and more had taken the slower of them.
+@pytest.mark.parametrize("rows,cols,tokens,terms,gate_up,narrow", [
+    (9600, 64, 15, 1, 0, True),         # 4.3 / 6.5
+    (14464, 1792, 69, 2, 0, True),      # 10.3 / 11.3
+    (18944, 1088, 160, 3, 1, True),     # 18.3 / 24.1
+    (7424, 1024, 450, 2, 1, True),      # 13.7 / 18.1
+    (2048, 1792, 1669, 1, 1, True),     # 13.3 / 18.6
+    (33536, 1024, 1402, 2, 1, False)])  # 105 / 89
+def test_quicker_kernel(binary, rows, cols, tokens, terms, gate_up, narrow):
+    assert (_chosen(binary, rows, cols, tokens, terms, gate_up, PAIRS, pairs=True) == 0) is narrow
 
 
 # GEMMs that a cut cost more than it saved, or that went to tail tiles whose quantiser takes longer than their k blocks: us as chosen here and as by a rule that took
